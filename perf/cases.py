@@ -37,19 +37,19 @@ LINEAR_SHAPES = ((4096, 4096), (6144, 4096), (28672, 4096), (14336, 4096), (4096
 def listed():
     return [
         # a single chat: the linear layer of one token, latency and weight streaming
-        {"name": "linear, one token", "kind": "linear", "m": 1, "n": 4096, "k": 4096},
+        {"name": "linear one token", "kind": "linear", "m": 1, "n": 4096, "k": 4096},
         # the down projection of a well filled decode batch
-        {"name": "linear, decode batch", "kind": "linear", "m": 128, "n": 4096, "k": 14336},
+        {"name": "linear decode batch", "kind": "linear", "m": 128, "n": 4096, "k": 14336},
         # the up projection of a long prompt
-        {"name": "linear, prompt", "kind": "linear", "m": 4096, "n": 14336, "k": 4096},
+        {"name": "linear prompt", "kind": "linear", "m": 4096, "n": 14336, "k": 4096},
         # the smallest attention call: a few chats, half precision, heads of 64
-        {"name": "paged decode, few", "kind": "paged_decode", "batch": 4, "least": 200, "most": 1100, "dim": 64, "type": "f16"},
+        {"name": "paged decode few", "kind": "paged_decode", "batch": 4, "least": 200, "most": 1100, "dim": 64, "type": "f16"},
         # an ordinary decode batch with contexts of all lengths
-        {"name": "paged decode, batch", "kind": "paged_decode", "batch": 32, "least": 128, "most": 4096, "dim": 128, "type": "bf16"},
+        {"name": "paged decode batch", "kind": "paged_decode", "batch": 32, "least": 128, "most": 4096, "dim": 128, "type": "bf16"},
         # four prompts read at once
-        {"name": "prefill, four prompts", "kind": "prefill", "prompts": 4, "least": 1024, "most": 8192, "spread": "halves", "dim": 128},
+        {"name": "prefill four prompts", "kind": "prefill", "prompts": 4, "least": 1024, "most": 8192, "spread": "halves", "dim": 128},
         # one step of continuous batching
-        {"name": "paged attention, mixed step", "kind": "paged_attention", "chunks": 4, "chunk": 512, "decoding": 28, "most": 3000,
+        {"name": "paged attention mixed step", "kind": "paged_attention", "chunks": 4, "chunk": 512, "decoding": 28, "most": 3000,
          "window": 0, "type": "bf16"},
         # an f32 encoder-sized attention
         {"name": "sdpa f32", "kind": "sdpa", "batch": 1, "heads": 8, "kv_heads": 8, "length": 512, "dim": 64, "causal": True},
