@@ -4,6 +4,7 @@
 #include <cmath>
 #include <mutex>
 
+#include "attention_f32.cuh"
 #include "attention_general.cuh"
 #include <type_traits>
 
@@ -937,6 +938,12 @@ int dense_entry(cudaStream_t stream, T *out, float *lse, const T *query, const T
     policy.lse_batch = static_cast<long long>(heads) * query_len;
     policy.lse_head = static_cast<long long>(query_len);
     policy.lse_row = 1;
+    if constexpr (std::is_same<T, float>::value) {
+        const DenseF32 dense = {query, out, lse, key, value, sinks, policy.heads, policy.kv_heads, policy.query_len,
+                                policy.key_len, policy.head_dim, policy.causal, policy.window, policy.q_batch, policy.q_head,
+                                policy.q_row, policy.k_batch, policy.k_head, policy.k_row, scale, softcap};
+        if (dense_attention_f32_takes(dense, batch)) return dense_attention_f32(stream, dense, batch);
+    }
     return launch_attention_general<T>(stream, policy, batch * heads * query_len, head_dim, scale,
                                        lse == nullptr ? LseKind::None : LseKind::Natural, -INFINITY, nullptr, softcap);
 }

@@ -1,0 +1,349 @@
+// Dense f32 attention in tiles: what Tensor::attend and fmha_prefill_lse compute for f32
+// (singe/src/backend/cpu/normalization/attention.rs:191-276, singe-kernel/src/cuda/attention/fmha.rs:48-140), in true
+// 32-bit arithmetic on the FMA pipe.
+//
+// Bound: issue slots and shared-memory reads, behind the FMA pipe (128 a clock and SM); up to 33 TFLOP/s.  One warp per query
+// row, the general kernel's way (1.2 - 2.2 TFLOP/s), reads every key and value from L1 once per row and folds each score over
+// the warp; here a CTA takes BM rows of one head, stages 64 keys at a time in shared memory, and a thread owns R rows x 4 keys
+// of the scores and R rows x D/16 columns of the output in registers, so a value read from shared memory feeds R or 4 FMAs.
+// Scores are summed as packed pairs, even and odd dimensions apart.  (Packed value products as well, with every weight stored
+// twice, cost 3 - 9 % more: the wider reads.)  Thread (ty, tx) owns rows ty, ty + BM/R, ... and keys tx,
+// tx + 16, ...: a row's scores lie in 16 neighbouring lanes, and rows one apart keep the 16-byte reads of a warp on
+// different banks (rows are padded by 16 bytes).
+// Teams of threads walk alternate key tiles, each in buffers of its own, and are folded at the end through shared memory: the
+// chain of key tiles is what a call of few CTAs waits for.
+// 8 heads x 512 causal keys of 64: 377 us -> 22.9; 6 x 1500: 2430 -> 114; 24 x 1500 of 128: 12340 -> 838.
+// Keys a row does not see take no part at all, whatever their bits are: in tiles that hold hidden keys the value
+// products are predicated, not multiplied by zero.
+#include "common.cuh"
+#include "attention_f32.cuh"
+
+namespace singe {
+
+namespace {
+
+constexpr int kKeys = 64;   // keys of a tile
+
+__device__ __forceinline__ void copy_16(float *dst, const float *src, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
+template <int D, int R, int BM, int G>
+struct Layout {
+    static constexpr int kTeam = 16 * BM / R;          // threads that share a key tile
+    static constexpr int kThreads = kTeam * G;
+    static constexpr int kRows = BM / R;               // distance between a thread's rows
+    static constexpr int kPitch = D + 4;               // floats between rows of Q and K
+    static constexpr int kWeightPitch = kKeys + 4;
+    static constexpr int kTeamFloats = kKeys * kPitch + kKeys * D + BM * kWeightPitch;
+    static constexpr int kFloats = BM * kPitch + G * kTeamFloats;
+    static_assert(G == 1 || kTeam * (R * D / 16 + 2 * R) <= kTeamFloats, "the fold reuses a team's buffers");
+};
+
+template <int D, int R, int BM, int G>
+__global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(const DenseF32 p, const int row_tiles) {
+    using L = Layout<D, R, BM, G>;
+    constexpr int kColumns = D / 64;   // float4 groups of output columns a thread owns
+    grid_launch_dependents();
+    extern __shared__ __align__(16) float shared[];
+    const int team = threadIdx.x / L::kTeam;
+    const int t = threadIdx.x % L::kTeam;
+    const int tx = t & 15, ty = t >> 4;
+    float *q_tile = shared;
+    float *k_tile = shared + BM * L::kPitch + team * L::kTeamFloats;
+    float *v_tile = k_tile + kKeys * L::kPitch;
+    float *weights = v_tile + kKeys * D;
+    auto team_sync = [&]() {
+        if (G == 1) {
+            __syncthreads();
+        } else {
+            asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(L::kTeam) : "memory");
+        }
+    };
+
+    // the heaviest row tiles (the last ones, under a causal mask) are dispatched first
+    const int pairs = gridDim.x / row_tiles;
+    const int first_row = (row_tiles - 1 - static_cast<int>(blockIdx.x) / pairs) * BM;
+    const int pair = static_cast<int>(blockIdx.x) % pairs;
+    const int head = pair % p.heads;
+    const long long batch = pair / p.heads;
+    const int kv_head = head / (p.heads / p.kv_heads);
+    const float *query = p.query + batch * p.q_batch + head * p.q_head;
+    const float *keys = p.key + batch * p.k_batch + kv_head * p.k_head;
+    const float *values = p.value + batch * p.k_batch + kv_head * p.k_head;
+    auto begin_of = [&](int row) { return p.window > 0 && row + 1 > p.window ? static_cast<int>(row + 1 - p.window) : 0; };
+    auto end_of = [&](int row) { return p.causal && row + 1 < p.key_len ? row + 1 : p.key_len; };
+    const int last_row = min(first_row + BM, p.query_len) - 1;
+    const int first_key = begin_of(first_row) / kKeys * kKeys;
+    const int end_key = end_of(last_row);
+
+    auto load_keys = [&](float *tile, const float *from, int pitch, int key0) {
+        for (int i = t; i < kKeys * (D / 4); i += L::kTeam) {
+            const int key = i / (D / 4), at = i % (D / 4) * 4;
+            const bool real = key0 + key < p.key_len && at < p.head_dim;
+            copy_16(tile + key * pitch + at, real ? from + (key0 + key) * p.k_row + at : from, real);
+        }
+        copy_commit();
+    };
+
+    grid_dependency_wait();
+    int key0 = first_key + team * kKeys;
+    if (key0 < end_key) {
+        load_keys(k_tile, keys, L::kPitch, key0);
+        load_keys(v_tile, values, D, key0);
+    }
+    for (int i = threadIdx.x; i < BM * (D / 4); i += L::kThreads) {
+        const int row = i / (D / 4), at = i % (D / 4) * 4;
+        float4 word = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (first_row + row < p.query_len && at < p.head_dim) {
+            word = *reinterpret_cast<const float4 *>(query + (first_row + row) * p.q_row + at);
+        }
+        *reinterpret_cast<float4 *>(q_tile + row * L::kPitch + at) =
+            make_float4(word.x * p.scale, word.y * p.scale, word.z * p.scale, word.w * p.scale);
+    }
+    __syncthreads();
+
+    float top[R], sum[R];
+    float4 out[R][kColumns];
+    int begin[R], end[R];
+    // a sink is one key of weight exp(sink - sink) = 1 and value zero; one thread of a row counts it
+    const float sink = p.sinks != nullptr && team == 0 ? p.sinks[head] : -INFINITY;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int row = first_row + ty + i * L::kRows;
+        begin[i] = row < p.query_len ? begin_of(row) : 0;
+        end[i] = row < p.query_len ? end_of(row) : 0;
+        top[i] = sink;
+        sum[i] = sink != -INFINITY && tx == 0 ? 1.0f : 0.0f;
+#pragma unroll
+        for (int c = 0; c < kColumns; ++c) out[i][c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+
+    for (; key0 < end_key; key0 += G * kKeys) {
+        copy_wait<1>();   // the keys; the values may still be on their way
+        team_sync();
+        // even and odd dimensions are summed apart, as packed pairs
+        float2 pairs2[R][4];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) pairs2[i][j] = make_float2(0.0f, 0.0f);
+        }
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+            float4 a[R], b[4];
+#pragma unroll
+            for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4 *>(q_tile + (ty + i * L::kRows) * L::kPitch + d);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(k_tile + (tx + 16 * j) * L::kPitch + d);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pairs2[i][j] = __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), pairs2[i][j]);
+            }
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pairs2[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), pairs2[i][j]);
+            }
+        }
+        float s[R][4];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = pairs2[i][j].x + pairs2[i][j].y;
+        }
+        team_sync();   // every thread has read the keys
+        const bool more = key0 + G * kKeys < end_key;
+        if (more) {
+            load_keys(k_tile, keys, L::kPitch, key0 + G * kKeys);
+        } else {
+            copy_commit();
+        }
+        // whether every row of the tile sees every key of it
+        const bool whole = begin_of(last_row) <= key0 && end_of(first_row) >= key0 + kKeys;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            if (p.softcap > 0.0f) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = p.softcap * tanhf(s[i][j] / p.softcap);
+            }
+            if (!whole) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int key = key0 + tx + 16 * j;
+                    if (key < begin[i] || key >= end[i]) s[i][j] = -INFINITY;
+                }
+            }
+            float most = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+#pragma unroll
+            for (int offset = 8; offset > 0; offset >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, offset));
+            most = fmaxf(most, top[i]);
+            const float base = most == -INFINITY ? 0.0f : most;
+            const float factor = expf(top[i] - base);
+            top[i] = most;
+            sum[i] *= factor;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float weight = expf(s[i][j] - base);
+                sum[i] += weight;
+                weights[(ty + i * L::kRows) * L::kWeightPitch + tx + 16 * j] = weight;
+            }
+#pragma unroll
+            for (int c = 0; c < kColumns; ++c) {
+                out[i][c].x *= factor;
+                out[i][c].y *= factor;
+                out[i][c].z *= factor;
+                out[i][c].w *= factor;
+            }
+        }
+        copy_wait<1>();   // the values; the next keys may still be on their way
+        team_sync();
+        auto weigh = [&](auto whole_tile) {
+#pragma unroll 4
+            for (int k = 0; k < kKeys; k += 4) {
+                float4 w[R];
+#pragma unroll
+                for (int i = 0; i < R; ++i) w[i] = *reinterpret_cast<const float4 *>(weights + (ty + i * L::kRows) * L::kWeightPitch + k);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float4 v[kColumns];
+#pragma unroll
+                    for (int c = 0; c < kColumns; ++c) v[c] = *reinterpret_cast<const float4 *>(v_tile + (k + u) * D + c * 64 + tx * 4);
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        if (!decltype(whole_tile)::value && (key0 + k + u < begin[i] || key0 + k + u >= end[i])) continue;
+                        const float weight = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+#pragma unroll
+                        for (int c = 0; c < kColumns; ++c) {
+                            out[i][c].x = fmaf(weight, v[c].x, out[i][c].x);
+                            out[i][c].y = fmaf(weight, v[c].y, out[i][c].y);
+                            out[i][c].z = fmaf(weight, v[c].z, out[i][c].z);
+                            out[i][c].w = fmaf(weight, v[c].w, out[i][c].w);
+                        }
+                    }
+                }
+            }
+        };
+        if (whole) {
+            weigh(std::true_type{});
+        } else {
+            weigh(std::false_type{});
+        }
+        team_sync();   // every thread has read the values
+        if (more) {
+            load_keys(v_tile, values, D, key0 + G * kKeys);
+        } else {
+            copy_commit();
+        }
+    }
+    copy_wait<0>();
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+#pragma unroll
+        for (int offset = 8; offset > 0; offset >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], offset);
+    }
+    // teams fold pairwise: the upper half parks its rows in the lower half's buffers, which nobody reads any more
+#pragma unroll
+    for (int half = G / 2; half > 0; half /= 2) {
+        __syncthreads();
+        constexpr int kEach = 2 + 4 * kColumns;
+        float *parked = shared + BM * L::kPitch + (team % half) * L::kTeamFloats + t;   // one float of every thread, then the next
+        if (team >= half && team < 2 * half) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                float *at = parked + i * kEach * L::kTeam;
+                at[0] = top[i];
+                at[L::kTeam] = sum[i];
+#pragma unroll
+                for (int c = 0; c < kColumns; ++c) {
+                    at[(2 + 4 * c) * L::kTeam] = out[i][c].x;
+                    at[(3 + 4 * c) * L::kTeam] = out[i][c].y;
+                    at[(4 + 4 * c) * L::kTeam] = out[i][c].z;
+                    at[(5 + 4 * c) * L::kTeam] = out[i][c].w;
+                }
+            }
+        }
+        __syncthreads();
+        if (team < half) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const float *at = parked + i * kEach * L::kTeam;
+                const float other = at[0];
+                const float most = fmaxf(top[i], other);
+                const float base = most == -INFINITY ? 0.0f : most;
+                const float mine = expf(top[i] - base), theirs = expf(other - base);
+                top[i] = most;
+                sum[i] = sum[i] * mine + at[L::kTeam] * theirs;
+#pragma unroll
+                for (int c = 0; c < kColumns; ++c) {
+                    out[i][c].x = out[i][c].x * mine + at[(2 + 4 * c) * L::kTeam] * theirs;
+                    out[i][c].y = out[i][c].y * mine + at[(3 + 4 * c) * L::kTeam] * theirs;
+                    out[i][c].z = out[i][c].z * mine + at[(4 + 4 * c) * L::kTeam] * theirs;
+                    out[i][c].w = out[i][c].w * mine + at[(5 + 4 * c) * L::kTeam] * theirs;
+                }
+            }
+        }
+    }
+    if (team > 0) return;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int row = first_row + ty + i * L::kRows;
+        if (row >= p.query_len) continue;
+        const bool empty = end[i] <= begin[i] && p.sinks == nullptr;
+        const float inverse = empty ? 0.0f : 1.0f / sum[i];
+        float *to = p.out + batch * p.q_batch + head * p.q_head + row * p.q_row;
+#pragma unroll
+        for (int c = 0; c < kColumns; ++c) {
+            if (c * 64 + tx * 4 < p.head_dim) {
+                *reinterpret_cast<float4 *>(to + c * 64 + tx * 4) =
+                    make_float4(out[i][c].x * inverse, out[i][c].y * inverse, out[i][c].z * inverse, out[i][c].w * inverse);
+            }
+        }
+        if (p.lse != nullptr && tx == 0) {
+            p.lse[(batch * p.heads + head) * p.query_len + row] = empty ? -INFINITY : top[i] + logf(sum[i]);
+        }
+    }
+}
+
+template <int D, int R, int BM, int G>
+int launch(cudaStream_t stream, const DenseF32 &p, size_t pairs) {
+    using L = Layout<D, R, BM, G>;
+    static int raised[kMaxDevices] = {0};
+    constexpr int kBytes = L::kFloats * 4;
+    SINGE_CUDA_TRY(ensure_dynamic_shared(dense_attention_f32_kernel<D, R, BM, G>, kBytes, raised));
+    const int row_tiles = (p.query_len + BM - 1) / BM;
+    SINGE_CUDA_TRY(launch_dependent(dense_attention_f32_kernel<D, R, BM, G>, dim3(static_cast<unsigned>(pairs * row_tiles)),
+                                    dim3(L::kThreads), kBytes, stream, kLaunchGlue, 1, p, row_tiles));
+    return launch_status();
+}
+
+}  // namespace
+
+bool dense_attention_f32_takes(const DenseF32 &p, size_t batch) {
+    const uintptr_t all = reinterpret_cast<uintptr_t>(p.query) | reinterpret_cast<uintptr_t>(p.key) |
+                          reinterpret_cast<uintptr_t>(p.value) | reinterpret_cast<uintptr_t>(p.out);
+    const size_t blocks = batch * static_cast<size_t>(p.heads) * ((static_cast<size_t>(p.query_len) + 31) / 32);
+    return p.head_dim % 4 == 0 && p.head_dim <= 128 && p.query_len >= kDenseF32LeastRows && (all & 15u) == 0 &&
+           blocks <= 0x7fffffffull && p.key_len <= 0x7fffffff - 2 * kKeys;
+}
+
+int dense_attention_f32(cudaStream_t stream, const DenseF32 &p, size_t batch) {
+    const size_t pairs = batch * static_cast<size_t>(p.heads);
+    const size_t sms = static_cast<size_t>(device_sm_count());
+    const size_t blocks = pairs * ((static_cast<size_t>(p.query_len) + 31) / 32);
+    if (p.head_dim <= 64) {
+        // A grid that does not cover the SMs leaves each CTA alone on its SM: four teams then (8 heads x 512 causal keys:
+        // 22.9 us, with two 34.3), which with more CTAs only take one another's shared memory (24 x 400 causal: 62.7
+        // against 47.2).  64 rows and no teams never win by more than 3 % (24 x 1500: 430 against 442) and lose up to half.
+        return blocks <= sms ? launch<64, 4, 32, 4>(stream, p, pairs) : launch<64, 4, 32, 2>(stream, p, pairs);
+    }
+    // Two teams' tiles of 128 columns fill an SM's shared memory, 64 rows without teams read each key half as often: that
+    // gains once the grid is two waves (24 heads x 1500 keys: 838 us against 924) and loses below (12 x 700: 99 against 61).
+    return blocks < 4 * sms ? launch<128, 4, 32, 2>(stream, p, pairs) : launch<128, 4, 64, 1>(stream, p, pairs);
+}
+
+}  // namespace singe
