@@ -42,6 +42,13 @@ int prefill_tcgen05(cudaStream_t stream, bool is_f16, void *out, float *lse, con
                     size_t head_dim, int causal, float scale, const uint32_t *block_table, size_t table_stride,
                     size_t cache_pages, size_t uniform_q, size_t uniform_kv);
 // kv_cache_write.cu
+bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t sequences,
+                          size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
+                          const void *value_cache, const void *out);
+int tensor_prefill(cudaStream_t stream, void *out, float *lse, const void *query, const void *key_cache, const void *value_cache,
+                   const void *query_offsets, const void *page_offsets, const void *pages, const void *last_page_lengths,
+                   int index_width, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t cache_pages,
+                   size_t sequences, size_t table_len, float scale, int causal, size_t window, uint32_t *status, unsigned **redo);
 int kv_cache_write(cudaStream_t stream, void *key_cache, void *value_cache, const void *keys, const void *values,
                    const void *write_pages, const void *write_slots, int index_width, size_t tokens, size_t kv_heads,
                    size_t head_dim, size_t pages, size_t page_size, uint32_t *status, size_t element_bytes);
@@ -92,7 +99,7 @@ int validate_ragged_prefill(size_t batch, size_t total_q, size_t total_kv, size_
 
 // paged_kv_decode_attention (singe-kernel/src/cpu/attention.rs:1172-1246): one query per sequence.
 template <typename T>
-struct DecodePagedPolicy {
+struct DecodePagedPolicy : RowPolicy {
     const T *query;
     T *out;
     const T *key_cache;
@@ -128,7 +135,7 @@ struct DecodePagedPolicy {
 
 // Queries that see the chunk of positions they stand in, over the paged cache of the sequence each belongs to.
 template <typename T>
-struct ChunkedPolicy {
+struct ChunkedPolicy : RowPolicy {
     const T *query;
     T *out;
     const T *key_cache;
@@ -165,7 +172,7 @@ struct ChunkedPolicy {
 
 // paged / ragged packed prefill (singe-kernel/src/cpu/attention.rs:1248-1420).  table == nullptr selects ragged.
 template <typename T>
-struct PackedPrefillPolicy {
+struct PackedPrefillPolicy : RowPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -232,7 +239,7 @@ struct PackedPrefillPolicy {
 // Tensor::paged_attention (singe/src/backend/cpu/normalization/attention.rs:424-540) with the refusals of
 // check_paged_values (singe/src/backend/spec/neural/attention.rs:363-416) applied to the row's own sequence.
 template <typename T, typename Index>
-struct TensorPagedPolicy {
+struct TensorPagedPolicy : RowPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -245,9 +252,26 @@ struct TensorPagedPolicy {
     int sequences, heads, kv_heads, head_dim, page_size, causal;
     long long tokens, cache_pages, table_len, window;
     const int *skip_when_zero;  // the planning kernel's verdict: 0 = the tiled decode kernel serves this call
+    const unsigned *redo;       // nullptr, or: the tensor-core kernel serves this call, and while this word is zero it has
+                                // left nothing; else the rows it marked and those of sequences it did not take are done here
 
+    __device__ bool nothing_left() const {
+        return (skip_when_zero != nullptr && *skip_when_zero == 0) || (redo != nullptr && *redo == 0u);
+    }
+    // Whether the tensor-core kernel left the sequence with these pages out: one of them lies outside the cache, or the query
+    // offsets of the call are out of range or run backwards.  The whole warp asks for one sequence.
+    __device__ bool left_out(long long first, long long last) const {
+        bool bad = false;
+        for (int s = threadIdx.x & 31; s < sequences && !bad; s += 32) {
+            bad = query_offsets[s] < 0 || query_offsets[s] > query_offsets[s + 1] || query_offsets[s + 1] > tokens;
+        }
+        for (long long i = first + (threadIdx.x & 31); i < last && !bad; i += 32) {
+            const long long page = static_cast<long long>(pages[i]);
+            bad = page < 0 || page >= cache_pages;
+        }
+        return __any_sync(0xffffffffu, bad) != 0;
+    }
     __device__ int locate(size_t row, RowPlan<T> &plan) const {
-        if (skip_when_zero != nullptr && *skip_when_zero == 0) return 0;
         const long long token = static_cast<long long>(row / heads);
         const int head = static_cast<int>(row - static_cast<size_t>(token) * heads);
         int owner = -1;
@@ -274,6 +298,7 @@ struct TensorPagedPolicy {
             if (last_length < 0 || last_length > page_size) return -1;
             keys = (page_count - 1) * page_size + last_length;
         }
+        if (redo != nullptr && !isnan(lse[row]) && !left_out(first_page, last_page)) return 0;
         const long long queries = end_query - first_query;
         long long position = keys + (token - first_query) - queries;  // queries are the sequence's last tokens
         if (position < 0) position = 0;
@@ -432,7 +457,7 @@ __global__ void check_and_plan_kernel(const Index *query_offsets, const Index *p
 // (singe/src/backend/cpu/normalization/attention.rs:191-276) and fmha_prefill_lse [B,L,H,D] over [B,S,G,D]
 // (singe-kernel/src/cpu/attention.rs:1758-1833).
 template <typename T>
-struct DensePolicy {
+struct DensePolicy : RowPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -476,7 +501,7 @@ struct DensePolicy {
 // out [B, H, splits, D] and its natural-log LSE in lse [B, H, splits] (fmha_decode_splitk_f32,
 // singe-kernel/src/cuda/attention/fmha.rs:1073-1117); splitk_reduce_kernel folds them.
 template <typename T>
-struct DenseSplitPolicy {
+struct DenseSplitPolicy : RowPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -779,6 +804,7 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
     policy.table_len = static_cast<long long>(table_len);
     policy.window = static_cast<long long>(window);
     policy.skip_when_zero = nullptr;
+    policy.redo = nullptr;
     bool checked = status == nullptr;  // no status word, no whole-table check
     auto check_alone = [&]() -> int {
         const unsigned blocks = static_cast<unsigned>((sequences + 3) / 4);  // four warps, one sequence each
@@ -853,9 +879,22 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
         }
         // (workspace growth refused under stream capture: the general kernel serves the call)
     }
+    // Steps with prompts in them: the tensor-core kernel, which checks the paging tensors itself and follows the general
+    // kernel's meaning row by row (what it leaves, the general kernel does).
+    if (std::is_same<T, __nv_bfloat16>::value && tokens != sequences && softcap == 0.0f &&
+        tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, sequences, table_len, causal, window, query, key_cache,
+                             value_cache, out)) {
+        unsigned *redo = nullptr;
+        SINGE_TRY(tensor_prefill(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
+                                 last_page_lengths, static_cast<int>(sizeof(Index)), tokens, heads, kv_heads, head_dim, cache_pages,
+                                 sequences, table_len, scale, causal, window, status, &redo));
+        policy.redo = redo;
+        checked = true;
+    }
     if (!checked) SINGE_TRY(check_alone());
+    const size_t most_blocks = policy.redo != nullptr ? static_cast<size_t>(device_sm_count()) * 16 : 0x7fffffff;
     return launch_attention_general<T>(stream, policy, tokens * heads, head_dim, scale, LseKind::Base2, -INFINITY,
-                                       status, softcap);
+                                       status, softcap, most_blocks);
 }
 
 template <typename T>

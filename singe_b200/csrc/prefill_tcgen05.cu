@@ -37,6 +37,9 @@
 // WINDOW: a query sees itself and the window - 1 keys before it.  A tile starts at the key tile where its first row begins
 // to see; a row whose first visible key lies in a later tile takes its base from that tile.
 // Keys have offsets and a row stride of their own, and the epilogue may gate a head's rows by a sigmoid.
+// TENSOR: the Tensor surface's paged attention (see TensorPaging).  A row is a (token, head) pair of one key/value head's
+// group, so that a sequence's few new tokens share one pass over its keys, and the value product takes the
+// probabilities as two terms hi + lo: that surface computes them in 32 bits.
 // Every mbarrier wait is bounded; on a timeout the CTA records status 2, frees tensor memory and leaves.
 #include <type_traits>
 
@@ -95,6 +98,84 @@ struct PrefillParams {
     const __nv_bfloat16 *gate;  // nullptr, or row t of head h is multiplied by sigmoid(gate[t * gate_stride + h])
     long long gate_stride;
 };
+
+// The Tensor surface's paging tensors (Tensor::paged_attention, singe/src/tensor/neural.rs:405-457), read as the caller
+// gave them: query_offsets and page_offsets [sequences + 1], pages [table_len], last_page_lengths [sequences], 32- or
+// 64-bit.  Every CTA checks all of them at its start and lists the sequences in shared memory; a sequence with a value
+// out of range gets no work here and raises `redo`, after which the general kernel computes what it can of it.  The
+// same word has the general kernel redo rows that this one marks with a NaN as their LSE: rows that leave the
+// single-pass range, and rows whose output is not finite (a hidden key's value may be anything, and zero times
+// infinity is not zero).
+// Bound by the tensor core and the special-function unit alike: 8 + 16 MMAs of 128 x 128 x 16 and 16384 exponentials a
+// key tile.  One step of four 510-token chunks and 28 decoding sequences behind 0 - 3000 tokens of context, 32 query heads on 8:
+// 238 us, 40.2 ms by one warp per row and head.
+struct TensorPaging {
+    const void *query_offsets;
+    const void *page_offsets;
+    const void *pages;
+    const void *last_page_lengths;
+    int index_width;   // 4 or 8
+    int sequences;
+    int tokens;
+    int table_len;
+    int pack;          // log2 of the query heads whose rows stand together; p.heads counts such packs
+    uint32_t *status;
+    unsigned *redo;
+};
+struct NoPaging {};
+
+constexpr int kMaxTensorSequences = 1024;
+constexpr unsigned kRedoMarkedRows = 1u, kRedoBadPaging = 2u;
+__device__ unsigned g_tensor_redo = 0;
+
+__device__ __forceinline__ long long paging_value(const void *list, int width, int at) {
+    return width == 8 ? static_cast<const long long *>(list)[at] : static_cast<const int *>(list)[at];
+}
+
+// Per sequence: rows (tokens << pack), keys, first token, first place in the page list.
+struct SequenceTable {
+    int *rows, *keys, *first_token, *first_page;
+};
+
+// Fills the table; every thread of the CTA takes part.  Query offsets that run backwards would have two sequences own a
+// token: then the whole call is left to the general kernel, which gives it to the first.
+__device__ __forceinline__ void list_sequences(const TensorPaging &g, int cache_pages, const SequenceTable &table, int warp, int lane) {
+    bool backwards = false;
+    for (int s = warp; s < g.sequences; s += kPrefillThreads / 32) {
+        const long long qf = paging_value(g.query_offsets, g.index_width, s);
+        const long long ql = paging_value(g.query_offsets, g.index_width, s + 1);
+        const long long pf = paging_value(g.page_offsets, g.index_width, s);
+        const long long pl = paging_value(g.page_offsets, g.index_width, s + 1);
+        bool bad = !(0 <= qf && qf <= ql && ql <= g.tokens);
+        backwards |= bad;
+        bad |= !(0 <= pf && pf <= pl && pl <= g.table_len);
+        long long keys = 0;
+        if (!bad && pf != pl) {
+            const long long last = paging_value(g.last_page_lengths, g.index_width, s);
+            bad = last < 0 || last > kPageTokens;
+            keys = (pl - pf - 1) * kPageTokens + last;
+            for (long long i = pf + lane; i < pl && !bad; i += 32) {
+                const long long page = paging_value(g.pages, g.index_width, static_cast<int>(i));
+                bad = page < 0 || page >= cache_pages;
+            }
+        }
+        bad = __any_sync(0xffffffffu, bad) != 0;
+        if (lane == 0) {
+            table.rows[s] = bad ? 0 : static_cast<int>(ql - qf) << g.pack;
+            table.keys[s] = bad ? 0 : static_cast<int>(keys);
+            table.first_token[s] = bad ? 0 : static_cast<int>(qf);
+            table.first_page[s] = bad ? 0 : static_cast<int>(pf);
+            if (bad && blockIdx.x == 0) {
+                report_status(g.status, kStatusIndexOutOfBounds);
+                atomicOr(g.redo, kRedoBadPaging);
+            }
+        }
+    }
+    if (__syncthreads_or(backwards ? 1 : 0) != 0) {
+        for (int s = threadIdx.x; s < g.sequences; s += kPrefillThreads) table.rows[s] = 0;
+        __syncthreads();
+    }
+}
 
 // Lengths and first rows of sequence b.  DENSE is a template argument of the kernel: as run-time branches these four
 // cost the packed form 2.5 % (every warp of a CTA decodes every work item).
@@ -157,10 +238,11 @@ __device__ __forceinline__ void chunk_max(const uint32_t (&sc)[kChunk], int low,
 // columns at `tmem_p`), the unrounded values are added to two running f32x2 sums.  Scores are handled as f32x2
 // pairs.  (Evaluating part of the exponentials as a polynomial on the FMA pipe was measured slower at every ratio:
 // with one softmax warp per scheduler the extra instructions cost more than the special-function unit saves.)
-template <typename T, int MASK>
+// SPLIT: 16 columns of leading terms, then 16 of what rounding them left out, over the chunk's own 32 score columns.
+template <typename T, int MASK, bool SPLIT>
 __device__ __forceinline__ void chunk_exp_store(const uint32_t (&sc)[kChunk], uint32_t tmem_p, float2 scale2,
                                                 float2 bias2, int low, int limit, float2 (&sum)[2]) {
-    uint32_t packed[kChunk / 2];
+    uint32_t packed[SPLIT ? kChunk : kChunk / 2];
 #pragma unroll
     for (int i = 0; i < kChunk; i += 2) {
         const float2 x = __ffma2_rn(make_float2(__uint_as_float(sc[i]), __uint_as_float(sc[i + 1])), scale2, bias2);
@@ -173,13 +255,22 @@ __device__ __forceinline__ void chunk_exp_store(const uint32_t (&sc)[kChunk], ui
         }
         sum[(i >> 1) & 1] = __fadd2_rn(sum[(i >> 1) & 1], e);
         packed[i >> 1] = pack2<T>(e.x, e.y);
+        if constexpr (SPLIT) {
+            static_assert(std::is_same<T, __nv_bfloat16>::value, "a bf16 pair is two f32 upper halves");
+            const float2 lead = make_float2(__uint_as_float(packed[i >> 1] << 16), __uint_as_float(packed[i >> 1] & 0xffff0000u));
+            packed[(i >> 1) + kChunk / 2] = pack2<T>(e.x - lead.x, e.y - lead.y);
+        }
     }
-    tmem_st_x16(tmem_p, packed);
+    if constexpr (SPLIT) {
+        tmem_st_x32(tmem_p, packed);
+    } else {
+        tmem_st_x16(tmem_p, packed);
+    }
 }
 
 // One row of one key tile: S (128 f32 columns at `tmem_s`) -> P (64 packed columns over the same place), chunk by
 // chunk with the next chunk's load in flight.
-template <typename T, int MASK>
+template <typename T, int MASK, bool SPLIT>
 __device__ __forceinline__ void tile_exp(uint32_t tmem_s, float2 scale2, float2 bias2, int low, int limit, float2 (&sum)[2]) {
     uint32_t buf[2][kChunk];
     tmem_ld_x32(tmem_s, buf[0]);
@@ -187,8 +278,8 @@ __device__ __forceinline__ void tile_exp(uint32_t tmem_s, float2 scale2, float2 
     for (int c = 0; c < kTile / kChunk; ++c) {
         tmem_wait_ld_into(buf[c & 1]);
         if (c + 1 < kTile / kChunk) tmem_ld_x32(tmem_s + (c + 1) * kChunk, buf[(c + 1) & 1]);
-        chunk_exp_store<T, MASK>(buf[c & 1], tmem_s + c * (kChunk / 2), scale2, bias2, low - c * kChunk, limit - c * kChunk,
-                                 sum);
+        chunk_exp_store<T, MASK, SPLIT>(buf[c & 1], tmem_s + c * (SPLIT ? kChunk : kChunk / 2), scale2, bias2, low - c * kChunk,
+                                        limit - c * kChunk, sum);
     }
 }
 
@@ -237,6 +328,7 @@ struct Item {
     int first[2];   // first key tile tile A / tile B needs (0 unless a window hides the ones before); A's is the lower
     int tiles[2];   // one past the last key tile tile A / tile B needs (0: no real row, or no visible key)
     int key_tiles;  // max of the two
+    int first_page; // TENSOR: place of the sequence's first page in the page list
     bool valid;     // false: the sequence's offsets leave the packed tensors
 };
 
@@ -246,8 +338,10 @@ __device__ __forceinline__ int pairs_of(int len_q) { return (max(len_q, 0) + kPa
 // pair index down (under a causal mask a pair's work grows with its index), head = index % heads.  `counts[t]` is
 // the number of sequences that have a pair t, `tmax` the largest pair count.  Every lane of the calling warp
 // takes part and receives the same answer.
-template <bool DENSE, bool WINDOW>
-__device__ __forceinline__ Item decode_item(const PrefillParams &p, const int *counts, int tmax, int index, int lane) {
+// TENSOR: rows are (token, head) pairs, `table` lists the sequences and `pack` is the log2 of a token's rows.
+template <bool DENSE, bool WINDOW, bool TENSOR>
+__device__ __forceinline__ Item decode_item(const PrefillParams &p, const SequenceTable &table, int pack, const int *counts, int tmax,
+                                            int index, int lane) {
     constexpr unsigned kFull = 0xffffffffu;
     Item item;
     int rank = index / p.heads;
@@ -275,7 +369,7 @@ __device__ __forceinline__ Item decode_item(const PrefillParams &p, const int *c
     int seq = -1;
     for (int first = 0; first < p.batch && seq < 0 && pair >= 0; first += 32) {
         const int b = first + lane;
-        const bool has = b < p.batch && pairs_of(seq_len_q<DENSE>(p, b)) > pair;
+        const bool has = b < p.batch && pairs_of(TENSOR ? table.rows[b] : seq_len_q<DENSE>(p, b)) > pair;
         const unsigned mask = __ballot_sync(kFull, has);
         const int n = __popc(mask);
         if (rank < n) {
@@ -295,26 +389,42 @@ __device__ __forceinline__ Item decode_item(const PrefillParams &p, const int *c
     item.first[0] = item.first[1] = 0;
     item.tiles[0] = item.tiles[1] = 0;
     item.key_tiles = 0;
+    item.first_page = 0;
     if (seq < 0) return item;
-    item.len_q = max(seq_len_q<DENSE>(p, seq), 0);
-    item.len_kv = max(seq_len_kv<DENSE>(p, seq), 0);
-    item.offset = seq_offset_q<DENSE>(p, seq);
-    item.offset_kv = seq_offset_kv<DENSE, WINDOW>(p, seq);
-    item.valid = item.offset >= 0 && item.offset_kv >= 0 && item.offset + item.len_q <= p.total_q &&
-                 (p.block_table != nullptr ? item.len_kv <= p.table_stride * kPageTokens
-                                           : item.offset_kv + item.len_kv <= p.total_kv);
-    if (!item.valid) return item;
-    item.shift = p.causal == 2 ? item.len_kv - item.len_q : 0;
+    if (TENSOR) {
+        item.len_q = table.rows[seq];
+        item.len_kv = table.keys[seq];
+        item.offset = table.first_token[seq];
+        item.first_page = table.first_page[seq];
+        item.valid = true;
+        item.shift = item.len_kv - (item.len_q >> pack);
+    } else {
+        item.len_q = max(seq_len_q<DENSE>(p, seq), 0);
+        item.len_kv = max(seq_len_kv<DENSE>(p, seq), 0);
+        item.offset = seq_offset_q<DENSE>(p, seq);
+        item.offset_kv = seq_offset_kv<DENSE, WINDOW>(p, seq);
+        item.valid = item.offset >= 0 && item.offset_kv >= 0 && item.offset + item.len_q <= p.total_q &&
+                     (p.block_table != nullptr ? item.len_kv <= p.table_stride * kPageTokens
+                                               : item.offset_kv + item.len_kv <= p.total_kv);
+        if (!item.valid) return item;
+        item.shift = p.causal == 2 ? item.len_kv - item.len_q : 0;
+    }
     if (WINDOW) {
 #pragma unroll
-        for (int x = 0; x < 2; ++x) item.first[x] = max(item.q0 + x * kTile + item.shift - p.window + 1, 0) / kTile;
+        for (int x = 0; x < 2; ++x) {
+            const int row = item.q0 + x * kTile;
+            item.first[x] = max((TENSOR ? row >> pack : row) + item.shift - p.window + 1, 0) / kTile;
+        }
     }
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         const int first = item.q0 + x * kTile;
         const int real = min(max(item.len_q - first, 0), kTile);
         int visible = real > 0 ? item.len_kv : 0;
-        if (p.causal && real > 0) visible = min(visible, max(first + real - 1 + item.shift, 0) + 1);
+        if (p.causal && real > 0) {
+            const int last = first + real - 1;
+            visible = min(visible, max((TENSOR ? last >> pack : last) + item.shift, 0) + 1);
+        }
         item.tiles[x] = (visible + kTile - 1) / kTile;
     }
     item.key_tiles = max(item.tiles[0], item.tiles[1]);
@@ -331,10 +441,11 @@ __device__ __forceinline__ Item decode_item(const PrefillParams &p, const int *c
 // 128-key tile and 64-wide half; the boxes land back to back, which is the layout one 128-row box would have).
 // HD = 128 or 64: with 64 a tile is a single 128-byte-wide box (the second half of every 32 KB buffer stays unused).
 // DENSE: uniform lengths, sequences back to back, LSE laid out [batch, heads, queries] (fmha_prefill_lse).
-template <typename T, int HD, bool SAFE, bool PAGED, bool DENSE, bool WINDOW>
+template <typename T, int HD, bool SAFE, bool PAGED, bool DENSE, bool WINDOW, bool TENSOR>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
     prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
-                           const __grid_constant__ CUtensorMap v_map, const PrefillParams p) {
+                           const __grid_constant__ CUtensorMap v_map, const PrefillParams p,
+                           const std::conditional_t<TENSOR, TensorPaging, NoPaging> paging) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -365,6 +476,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
+    SequenceTable table = {};
+    int pack = 0;
+    if constexpr (TENSOR) {
+        // (the redo list's place and what follows it)
+        table.rows = counts + kMaxRankTiles;
+        table.keys = table.rows + kMaxTensorSequences;
+        table.first_token = table.keys + kMaxTensorSequences;
+        table.first_page = table.first_token + kMaxTensorSequences;
+        pack = paging.pack;
+        list_sequences(paging, p.cache_pages, table, warp, lane);
+    }
     if (SAFE && !p.exact && *reinterpret_cast<volatile unsigned *>(&g_out_of_range_seen) == 0u) {
         return;  // no first launch on this device has ever marked a row
     }
@@ -372,11 +494,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     // ---- the table behind the heaviest-first item order ----
     {
         int tmax = 0;
-        for (int b = 0; b < p.batch; ++b) tmax = max(tmax, pairs_of(seq_len_q<DENSE>(p, b)));
+        for (int b = 0; b < p.batch; ++b) tmax = max(tmax, pairs_of(TENSOR ? table.rows[b] : seq_len_q<DENSE>(p, b)));
         tmax = min(tmax, kMaxRankTiles);
         for (int t = tid; t < tmax; t += kPrefillThreads) {
             int count = 0;
-            for (int b = 0; b < p.batch; ++b) count += pairs_of(seq_len_q<DENSE>(p, b)) > t ? 1 : 0;
+            for (int b = 0; b < p.batch; ++b) count += pairs_of(TENSOR ? table.rows[b] : seq_len_q<DENSE>(p, b)) > t ? 1 : 0;
             counts[t] = count;
         }
         __syncthreads();
@@ -389,6 +511,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         __syncthreads();
     }
     const int tmax = *shared_tmax;
+    auto decode = [&](int index) { return decode_item<DENSE, WINDOW, TENSOR>(p, table, pack, counts, tmax, index, lane); };
     const long long total_items = static_cast<long long>(*shared_ranks) * p.heads;
     // index of this CTA's share number `round`, or -1 past the end
     auto share_index = [&](int round) -> int {
@@ -401,6 +524,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         if (DENSE) {
             return p.lse + (static_cast<size_t>(item.seq) * p.heads + item.head) * p.lse_rows + row;
         }
+        if (TENSOR) {
+            return p.lse + (((static_cast<size_t>(item.offset) + (row >> pack)) * p.heads + item.head) << pack) + (row & ((1 << pack) - 1));
+        }
         return p.lse + (static_cast<size_t>(item.offset) + row) * p.heads + item.head;
     };
     int listed = -1;  // SAFE: number of marked items in redo_list, or -1 = walk the whole share
@@ -411,7 +537,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         for (int round = 0;; ++round) {
             const int index = share_index(round);
             if (index < 0) break;
-            const Item item = decode_item<DENSE, WINDOW>(p, counts, tmax, index, lane);
+            const Item item = decode(index);
             const int row = item.q0 + tid;
             const bool marked = item.valid && item.key_tiles > 0 && tid < kPair && row < item.len_q &&
                                 isnan(*lse_at(item, row));
@@ -469,7 +595,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         for (int round = 0; !failed; ++round) {
             const int index = item_index(round);
             if (index < 0) break;
-            const Item item = decode_item<DENSE, WINDOW>(p, counts, tmax, index, lane);
+            const Item item = decode(index);
             if (item.key_tiles == 0) continue;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
@@ -482,11 +608,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 ++q_loads[x];
                 if (lane == 0) {
                     mbar_expect_tx(bar_q_full + x * 8, kLoadBytes);
-                    const int row0 = item.offset + item.q0 + x * kTile;
-                    tma_load_3d(q_smem + x * kTileBytes, &q_map, bar_q_full + x * 8, 0, item.head, row0);
+                    // TENSOR: a box holds the heads of a pack for 128 >> pack tokens, token by token
+                    const int row0 = item.offset + ((item.q0 + x * kTile) >> pack);
+                    const int head0 = item.head << pack;
+                    tma_load_3d(q_smem + x * kTileBytes, &q_map, bar_q_full + x * 8, 0, head0, row0);
                     if (kHalves == 2) {
                         tma_load_3d(q_smem + x * kTileBytes + kHalfTileBytes, &q_map, bar_q_full + x * 8, 64,
-                                    item.head, row0);
+                                    head0, row0);
                     }
                 }
             }
@@ -504,13 +632,18 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 if (PAGED) {
                     const int pages_of_sequence = (item.len_kv + kPageTokens - 1) / kPageTokens;
                     const int wanted = j * (kTile / kPageTokens) + (lane & 7);
-                    const uint32_t *row = p.block_table + static_cast<size_t>(item.seq) * p.table_stride;
-                    uint32_t id = row[wanted < pages_of_sequence ? wanted : 0];
-                    if (id >= static_cast<uint32_t>(p.cache_pages)) {
-                        report_status(p.error, kStatusIndexOutOfBounds);
-                        id = 0u;
+                    const int place = wanted < pages_of_sequence ? wanted : 0;
+                    if constexpr (TENSOR) {
+                        page = static_cast<int32_t>(paging_value(paging.pages, paging.index_width, item.first_page + place));
+                    } else {
+                        const uint32_t *row = p.block_table + static_cast<size_t>(item.seq) * p.table_stride;
+                        uint32_t id = row[place];
+                        if (id >= static_cast<uint32_t>(p.cache_pages)) {
+                            report_status(p.error, kStatusIndexOutOfBounds);
+                            id = 0u;
+                        }
+                        page = static_cast<int32_t>(id);
                     }
-                    page = static_cast<int32_t>(id);
                 }
                 if (lane == 0) mbar_expect_tx(bar_k_full + stage * 8, kLoadBytes);
                 __syncwarp();
@@ -579,9 +712,14 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 const uint32_t v_tile = v_smem + stage * kTileBytes;
 #pragma unroll
                 for (int ks = 0; ks < kTile / 16; ++ks) {
-                    umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + ks * 8,
-                            make_smem_desc(v_tile + ks * 2048, kHalfTileBytes, 1024), kIdescPV,
+                    // TENSOR: a chunk of 32 keys holds 16 columns of leading terms and 16 of the rest
+                    const uint32_t at = TENSOR ? (ks >> 1) * kChunk + (ks & 1) * 8 : ks * 8;
+                    const uint64_t v_desc = make_smem_desc(v_tile + ks * 2048, kHalfTileBytes, 1024);
+                    umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at, v_desc, kIdescPV,
                             (accumulate || ks > 0) ? 1u : 0u);
+                    if (TENSOR) {
+                        umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at + kChunk / 2, v_desc, kIdescPV, 1u);
+                    }
                 }
                 if (last) tcgen05_commit(bar_o_full + x * 8);
             }
@@ -603,7 +741,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     return item;
                 }
                 ++round;
-                item = decode_item<DENSE, WINDOW>(p, counts, tmax, index, lane);
+                item = decode(index);
                 if (item.key_tiles > 0) return item;
             }
         };
@@ -707,15 +845,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         for (int round = 0; !failed; ++round) {
             const int index = item_index(round);
             if (index < 0) break;
-            const Item item = decode_item<DENSE, WINDOW>(p, counts, tmax, index, lane);
+            const Item item = decode(index);
             if (!item.valid) {
                 if (warp == 0 && lane == 0) report_status(p.error, kStatusIndexOutOfBounds);
                 continue;
             }
             const int row = item.q0 + x * kTile + local_row;    // sequence-local query index
             const bool real = row < item.len_q;
-            const size_t token = static_cast<size_t>(item.offset) + (real ? row : 0);
-            T *dst = static_cast<T *>(p.out) + (token * p.heads + item.head) * HD;
+            const int turn = row >> pack;                       // sequence-local token of the row
+            const size_t token = static_cast<size_t>(item.offset) + (real ? turn : 0);
+            T *dst = static_cast<T *>(p.out) + (((token * p.heads + item.head) << pack) + (real ? row & ((1 << pack) - 1) : 0)) * HD;
             float *lse_row = lse_at(item, real ? row : 0);
             const int my_tiles = x == 0 ? item.tiles[0] : item.tiles[1];
             const int my_first = x == 0 ? item.first[0] : item.first[1];
@@ -724,7 +863,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 if (real) {
 #pragma unroll
                     for (int i = 0; i < HD / 8; ++i) reinterpret_cast<uint4 *>(dst)[i] = make_uint4(0u, 0u, 0u, 0u);
-                    *lse_row = -1.0e20f;
+                    *lse_row = TENSOR ? -INFINITY : -1.0e20f;
                 }
                 continue;
             }
@@ -740,9 +879,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 tcgen05_fence_after();  // S(j) is ready, and with it every earlier MMA of this tile: O holds P V up to j-1
                 // number of keys of this key tile the row may see
                 int limit = item.len_kv - j * kTile;
-                if (p.causal) limit = min(limit, max(row + item.shift, 0) + 1 - j * kTile);
+                if (p.causal) limit = min(limit, max(turn + item.shift, 0) + 1 - j * kTile);
                 limit = real ? limit : 0;
-                const int low = WINDOW ? row + item.shift - p.window + 1 - j * kTile : 0;  // first column the row sees
+                const int low = WINDOW ? turn + item.shift - p.window + 1 - j * kTile : 0;  // first column the row sees
                 const bool partial = __any_sync(0xffffffffu, limit < kTile);
                 const bool lower = WINDOW && __any_sync(0xffffffffu, low > 0);
 
@@ -782,11 +921,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 const float2 bias2 = make_float2(bias, bias);
                 float2 sum[2] = {make_float2(row_sum, 0.0f), make_float2(0.0f, 0.0f)};
                 if (WINDOW && lower) {
-                    tile_exp<T, kMaskBoth>(tmem_s, scale2, bias2, low, limit, sum);
+                    tile_exp<T, kMaskBoth, TENSOR>(tmem_s, scale2, bias2, low, limit, sum);
                 } else if (partial) {
-                    tile_exp<T, kMaskEnd>(tmem_s, scale2, bias2, low, limit, sum);
+                    tile_exp<T, kMaskEnd, TENSOR>(tmem_s, scale2, bias2, low, limit, sum);
                 } else {
-                    tile_exp<T, kMaskNone>(tmem_s, scale2, bias2, low, limit, sum);
+                    tile_exp<T, kMaskNone, TENSOR>(tmem_s, scale2, bias2, low, limit, sum);
                 }
                 row_sum = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
                 tmem_wait_st();
@@ -810,11 +949,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             if (WINDOW && p.gate != nullptr) {
                 inverse /= 1.0f + __expf(-__bfloat162float(p.gate[token * p.gate_stride + item.head]));
             }
+            float probe = 0.0f;   // TENSOR: a NaN once an output is not finite
 #pragma unroll 1
             for (int c = 0; c < HD; c += 32) {
                 uint32_t r[32];
                 tmem_ld_x32(tmem_o + c, r);
                 tmem_wait_ld_into(r);
+                if (TENSOR) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) probe = fmaf(__uint_as_float(r[i]) * inverse, 0.0f, probe);
+                }
                 if (c + 32 == HD) {
                     // O is out of tensor memory: the next item's first P V may overwrite it
                     tcgen05_fence_before();
@@ -836,7 +980,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             }
             if (real) {
                 float value = empty ? -1.0e20f : (base_log2 + log2f(row_sum)) * 0.6931471805599453f;
-                if (!SAFE && !in_range) {
+                if constexpr (TENSOR) {
+                    value = base_log2 + log2f(row_sum);
+                    if (!in_range || empty || isnan(probe)) {
+                        value = __int_as_float(0x7fc00000);  // has the general kernel redo the row
+                        atomicOr(paging.redo, kRedoMarkedRows);
+                    }
+                } else if (!SAFE && !in_range) {
                     value = __int_as_float(0x7fc00000);  // has the second launch redo the item
                     atomicExch(&g_out_of_range_seen, 1u);
                 }
@@ -874,20 +1024,40 @@ namespace {
 template <typename T, int HD, bool PAGED, bool DENSE = false, bool WINDOW = false>
 int launch_prefill(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
                    const PrefillParams &params, unsigned persistent) {
-    SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW>,
+    SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem));
     if (std::is_same<T, __nv_bfloat16>::value) {
-        SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW>,
+        SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem));
-        prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW>
-            <<<persistent, kPrefillThreads, kPrefillSmem, stream>>>(q_map, k_map, v_map, params);
+        prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false>
+            <<<persistent, kPrefillThreads, kPrefillSmem, stream>>>(q_map, k_map, v_map, params, NoPaging{});
         SINGE_TRY(launch_status());
     }
     // bf16: the redo pass over the same shares, a no-op while the device's out-of-range flag has never been raised.
     // f16 (params.exact): the only pass.  P must stay below 65504 there, so every tile takes its exact row maximum.
-    prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW><<<persistent, kPrefillThreads, kPrefillSmem, stream>>>(q_map, k_map, v_map,
-                                                                                                  params);
+    prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false>
+        <<<persistent, kPrefillThreads, kPrefillSmem, stream>>>(q_map, k_map, v_map, params, NoPaging{});
     return launch_status();
+}
+
+template <int HD, bool WINDOW>
+int launch_tensor(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
+                  const PrefillParams &params, const TensorPaging &paging, unsigned persistent) {
+    static int raised[kMaxDevices] = {0};
+    constexpr int kBytes = kPrefillSmem + (4 * kMaxTensorSequences - kRedoCapacity) * 4;
+    const auto kernel = prefill_tcgen05_kernel<__nv_bfloat16, HD, false, true, false, WINDOW, true>;
+    SINGE_CUDA_TRY(ensure_dynamic_shared(kernel, kBytes, raised));
+    kernel<<<persistent, kPrefillThreads, kBytes, stream>>>(q_map, k_map, v_map, params, paging);
+    return launch_status();
+}
+
+// log2 of the query heads of a key/value head whose rows stand together: all of a group that divides a tile, else one.
+int pack_of(size_t heads, size_t kv_heads) {
+    const size_t group = heads / kv_heads;
+    for (int pack = 0; pack <= 4; ++pack) {
+        if (group == (size_t{1} << pack)) return pack;
+    }
+    return 0;
 }
 
 }  // namespace
@@ -1031,6 +1201,73 @@ int prefill_tcgen05_windowed(cudaStream_t stream, void *out, float *lse, const v
         return launch_prefill<__nv_bfloat16, 64, false, false, true>(stream, q_map, k_map, v_map, params, persistent);
     }
     return launch_prefill<__nv_bfloat16, 128, false, false, true>(stream, q_map, k_map, v_map, params, persistent);
+}
+
+// Whether tensor_prefill serves a call of the Tensor surface's paged attention (bf16, no score cap).
+bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t sequences,
+                          size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
+                          const void *value_cache, const void *out) {
+    const size_t rows = tokens << pack_of(heads, kv_heads);
+    return page_size == kPageTokens && sequences <= kMaxTensorSequences && table_len <= 0x7fffffff / kPageTokens - kTile &&
+           (window == 0 || (causal && window <= 0x3fffffff)) && rows <= 0x7fffffff / 2 &&
+           prefill_fast_path(heads, kv_heads, head_dim, rows, query, key_cache, value_cache, out);
+}
+
+// Tensor::paged_attention over 16-token pages.  `redo` (see TensorPaging) tells the general kernel, which follows on the
+// stream, whether rows are left to it.
+int tensor_prefill(cudaStream_t stream, void *out, float *lse, const void *query, const void *key_cache, const void *value_cache,
+                   const void *query_offsets, const void *page_offsets, const void *pages, const void *last_page_lengths,
+                   int index_width, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t cache_pages,
+                   size_t sequences, size_t table_len, float scale, int causal, size_t window, uint32_t *status, unsigned **redo) {
+    static unsigned *words[kMaxDevices] = {nullptr};
+    const int slot = device_slot();
+    if (slot < 0) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
+    if (words[slot] == nullptr) {
+        void *address = nullptr;
+        SINGE_CUDA_TRY(cudaGetSymbolAddress(&address, g_tensor_redo));
+        words[slot] = static_cast<unsigned *>(address);
+    }
+    const int pack = pack_of(heads, kv_heads);
+    const uint64_t width = head_dim;
+    const CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    CUtensorMap q_map, k_map, v_map;
+    const uint64_t q_dims[3] = {width, heads, tokens};
+    const uint64_t q_strides[2] = {width * 2, width * 2 * heads};
+    const uint32_t q_box[3] = {64, 1u << pack, static_cast<uint32_t>(kTile >> pack)};
+    SINGE_TRY(encode_tensor_map(&q_map, type, 3, query, q_dims, q_strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B));
+    const uint64_t dims[4] = {width, kv_heads, kPageTokens, cache_pages};
+    const uint64_t strides[3] = {width * 2, width * 2 * kv_heads, width * 2 * kv_heads * kPageTokens};
+    const uint32_t box[4] = {64, 1, kPageTokens, 1};
+    SINGE_TRY(encode_tensor_map(&k_map, type, 4, key_cache, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B));
+    SINGE_TRY(encode_tensor_map(&v_map, type, 4, value_cache, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B));
+    PrefillParams params = {};
+    params.out = out;
+    params.lse = lse;
+    params.batch = static_cast<int>(sequences);
+    params.heads = static_cast<int>(heads >> pack);
+    params.kv_heads = static_cast<int>(kv_heads);
+    params.total_q = static_cast<int>(tokens);
+    params.cache_pages = static_cast<int>(cache_pages);
+    params.causal = causal ? 1 : 0;
+    params.scale_log2 = scale * 1.4426950408889634f;
+    params.error = device_error_word();
+    params.window = static_cast<int>(window);
+    TensorPaging paging = {query_offsets, page_offsets, pages, last_page_lengths, index_width, static_cast<int>(sequences),
+                           static_cast<int>(tokens), static_cast<int>(table_len), pack, status, words[slot]};
+    const size_t items = ((tokens << pack) / kPair + sequences) * (heads >> pack);
+    if (items > 0x7fffffffull) return SINGE_ERR_LENGTH_EXCEEDS_I32;
+    const size_t sms = static_cast<size_t>(device_sm_count());
+    const unsigned persistent = static_cast<unsigned>(items < sms ? items : sms);
+    *redo = words[slot];
+    if (head_dim == 64) {
+        return window > 0 ? launch_tensor<64, true>(stream, q_map, k_map, v_map, params, paging, persistent)
+                          : launch_tensor<64, false>(stream, q_map, k_map, v_map, params, paging, persistent);
+    }
+    return window > 0 ? launch_tensor<128, true>(stream, q_map, k_map, v_map, params, paging, persistent)
+                      : launch_tensor<128, false>(stream, q_map, k_map, v_map, params, paging, persistent);
 }
 
 int prefill_tcgen05_bf16(cudaStream_t stream, void *out, float *lse, const void *query, const void *key,

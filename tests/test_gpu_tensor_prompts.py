@@ -1,0 +1,127 @@
+"""The Tensor surface's paged attention of steps with prompts in them: on the tensor core, with split probabilities.  The oracle
+is the CPU restatement; what a call leaves to the general kernel is compared with the f32 call on the same values, which that
+kernel serves whole."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle
+from singe_b200 import ops, workloads
+from tests.gpu_util import dev, host
+
+pytestmark = pytest.mark.gpu
+
+PAGE = 16
+
+
+def step(rng, new, every, heads, kv_heads, dim, spare=3):
+    counts = [-(-n // PAGE) for n in every]
+    pool = sum(counts) + spare
+    paging = {"query_offsets": np.concatenate([[0], np.cumsum(new)]), "page_offsets": np.concatenate([[0], np.cumsum(counts)]),
+              "pages": rng.permutation(pool)[: sum(counts)],
+              "last_page_lengths": np.asarray([(n - 1) % PAGE + 1 if n else 0 for n in every])}
+    q = workloads.normal_bf16(rng, (sum(new), heads, dim))
+    return q, workloads.normal_bf16(rng, (pool, PAGE, kv_heads, dim)), workloads.normal_bf16(rng, (pool, PAGE, kv_heads, dim)), paging
+
+
+def run_step(q, kc, vc, paging, kind=torch.bfloat16, index=np.int64, **options):
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tensors = [t.to(kind) if isinstance(t, torch.Tensor) else dev(t, kind) for t in (q, kc, vc)]
+    out, lse = ops.paged_attention(*tensors, *(dev(paging[name].astype(index)) for name in
+                                               ("query_offsets", "page_offsets", "pages", "last_page_lengths")),
+                                   scale=tensors[0].shape[2] ** -0.5, status=status, **options)
+    torch.cuda.synchronize()
+    return host(out), host(lse), int(status.item())
+
+
+def assert_rounded(out, ref, what):
+    """``out`` is ``ref`` rounded to bf16 (half a unit: 2^-8), up to what probabilities of 2^-17 relative error and f32 sums of
+    values below 6 leave."""
+    assert (np.abs(out - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-4).all(), f"{what}: {np.abs(out - ref).max()}"
+
+
+NEW = [1, 300, 0, 70, 1, 33, 1, 256, 2]
+EVERY = [517, 300, 40, 900, 16, 20, 1, 640, 0]     # more keys than new tokens, as many, fewer, none
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 128), (4, 4, 128), (8, 1, 64), (6, 2, 64), (32, 2, 128), (4, 2, 128)])
+@pytest.mark.parametrize("causal,window,index", [(True, 0, np.int64), (False, 0, np.int32), (True, 100, np.int64), (True, 1, np.int32),
+                                                 (True, 5000, np.int64)])
+def test_steps_with_prompts(heads, kv_heads, dim, causal, window, index):
+    rng = np.random.default_rng(heads + dim + window)
+    q, kc, vc, paging = step(rng, NEW, EVERY, heads, kv_heads, dim)
+    out, lse, status = run_step(q, kc, vc, paging, index=index, causal=causal, window=window)
+    code, ref, ref_lse = oracle.attend_paged_f32(q, kc, vc, *paging.values(), scale=dim ** -0.5, causal=causal, window=window)
+    assert code == oracle.OK and status == 0 and ops.take_device_error() == 0
+    assert_rounded(out, ref, "out")
+    assert (np.isneginf(lse) == np.isneginf(ref_lse)).all()
+    seen = np.isfinite(ref_lse)
+    assert np.abs(lse[seen] - ref_lse[seen]).max() < 2e-4
+
+
+def test_rows_of_no_sequence_are_left_alone():
+    rng = np.random.default_rng(3)
+    q, kc, vc, paging = step(rng, [40, 3, 20], [40, 80, 33], 8, 2, 128)
+    paging["query_offsets"] = np.asarray([5, 45, 45, 60])
+    out, lse, status = run_step(q, kc, vc, paging)
+    ref, ref_lse, _ = run_step(q, kc, vc, paging, torch.float32)
+    assert status == 0 and not out[:5].any() and not out[60:].any() and np.isneginf(lse[:5]).all()
+    assert_rounded(out, ref, "out")
+    assert np.abs(lse[5:60] - ref_lse[5:60]).max() < 2e-4
+
+
+def same_as_general(q, kc, vc, paging):
+    """The bf16 call against the f32 call on the same values."""
+    out, lse, status = run_step(q, kc, vc, paging)
+    ref, ref_lse, ref_status = run_step(q, kc, vc, paging, torch.float32)
+    assert status == ref_status
+    for mine, other in ((out, ref), (lse, ref_lse)):
+        assert (np.isnan(mine) == np.isnan(other)).all() and (np.isinf(mine) == np.isinf(other)).all()
+    fine = np.isfinite(ref)
+    assert_rounded(out[fine], ref[fine], "out")
+    fine = np.isfinite(ref_lse)
+    assert (np.abs(lse[fine] - ref_lse[fine]) <= 2e-4 + 1e-6 * np.abs(ref_lse[fine])).all()
+    return status
+
+
+@pytest.mark.parametrize("fault", ["page", "last", "page_offsets", "query_offsets", "backwards"])
+def test_paging_out_of_range_leaves_the_other_sequences_whole(fault):
+    rng = np.random.default_rng(11)
+    q, kc, vc, paging = step(rng, NEW, EVERY, 8, 2, 128)
+    if fault == "page":
+        paging["pages"][paging["page_offsets"][3] + 20] = kc.shape[0]    # rows before that page's keys are still computed
+    elif fault == "last":
+        paging["last_page_lengths"][1] = PAGE + 1
+    elif fault == "page_offsets":
+        paging["page_offsets"][-1] += 1
+    elif fault == "query_offsets":
+        paging["query_offsets"][-1] += 1
+    else:
+        paging["query_offsets"][4] -= 100
+    assert same_as_general(q, kc, vc, paging) == 1
+    q, kc, vc, paging = step(rng, NEW, EVERY, 8, 2, 128)                 # and the next call is served as ever
+    assert same_as_general(q, kc, vc, paging) == 0
+
+
+@pytest.mark.parametrize("what", ["hidden values", "hidden keys", "seen value", "infinite value", "unused slots", "jump", "all hidden low"])
+def test_values_the_tensor_core_cannot_carry(what):
+    rng = np.random.default_rng(13)
+    q, kc, vc, paging = step(rng, [200, 1, 30], [260, 300, 30], 8, 2, 128)
+    at = lambda sequence, key: (paging["pages"][paging["page_offsets"][sequence] + key // PAGE], key % PAGE)
+    if what == "hidden values":
+        vc[at(0, 200)] = np.nan           # seen from row 140 on
+    elif what == "hidden keys":
+        kc[at(0, 200)] = np.inf
+    elif what == "seen value":
+        vc[at(1, 7)] = np.nan
+    elif what == "infinite value":
+        vc[at(1, 7)] = np.inf
+    elif what == "unused slots":
+        vc[at(2, 30)] = np.nan
+        vc[at(0, 260)] = np.inf
+    elif what == "jump":
+        kc[at(0, 150)] = 60.0 * np.sign(q[150, 0])   # scores that outgrow the first key tile's by far more than 2^64
+    else:
+        q[:, 0] = 2.0 ** 100
+        kc[at(0, 0)] = -2.0 ** 100        # a score of minus infinity
+    same_as_general(q, kc, vc, paging)
