@@ -23,6 +23,17 @@ class PageTableError(ValueError):
     pass
 
 
+def token_array(tokens) -> np.ndarray:
+    """Token ids as int64, whatever sequence of integers they come in."""
+    try:
+        array = np.array(tokens, dtype=np.int64)
+        if array.ndim == 1:
+            return array
+    except (TypeError, ValueError):
+        pass
+    return np.fromiter(map(int, tokens), dtype=np.int64, count=len(tokens))
+
+
 @dataclass
 class DecodeStep:
     """The paging tensors of one step (singe/src/nn/decode/step.rs:13-30), as int64 numpy arrays."""
@@ -137,6 +148,7 @@ class PageTable:
         sequences = len(self.pages)
         if len(tokens) != sequences or all(len(t) == 0 for t in tokens):
             raise PageTableError("decode step needs a slice for every sequence, and tokens in one")
+        flats = [token_array(t) for t in tokens]   # (before anything changes: a token that is no integer is refused here)
         padding = total - self.step_tokens(tokens)
         if padding < 0:
             raise PageTableError("a decode step is padded to fewer rows than it has")
@@ -159,39 +171,36 @@ class PageTable:
             for place in places:
                 self.pages[row][place] = self.pool
 
-        flat, positions, write_pages, write_slots = [], [], [], []
-        query_offsets, last_rows, real_tokens, sequence_ids, visible = [0], [], [], [], []
-        for row, t in enumerate(tokens):
+        # rows of the step: a sequence's new tokens, or one idle row; then the padding behind the last sequence with tokens
+        counts = np.asarray([len(t) for t in tokens], dtype=np.int64)
+        starts = np.asarray(self.lengths, dtype=np.int64)
+        rows = np.maximum(counts, 1)
+        rows[padded] += padding
+        query_offsets = np.concatenate([[0], np.cumsum(rows)])
+        first_rows = query_offsets[:-1]
+        sequence_ids = np.repeat(np.arange(sequences, dtype=np.int64), rows)
+        place = np.arange(total, dtype=np.int64) - first_rows[sequence_ids]
+        unbounded = starts[sequence_ids] + place
+        positions = np.minimum(unbounded, self.capacity - 1)
+        write_slots = np.where(counts[sequence_ids] > 0, unbounded % self.page_size, 0)
+        write_pages = np.full(total, self.pool, dtype=np.int64)
+        flat = np.zeros(total, dtype=np.int64)
+        for row, (start, count, at) in enumerate(zip(self.lengths, counts.tolist(), first_rows.tolist())):
+            if count == 0:
+                continue
             held = self.pages[row]
-            for token in t:
-                position = self.lengths[row]
-                page = position // self.page_size
-                if page == len(held):
-                    held.append(self.free.pop())
-                flat.append(int(token))
-                positions.append(position)
-                write_pages.append(held[page])
-                write_slots.append(position % self.page_size)
-                self.lengths[row] += 1
-            if len(t) == 0:
-                flat.append(0)
-                positions.append(min(self.lengths[row], self.capacity - 1))
-                write_pages.append(self.pool)
-                write_slots.append(0)
-            last = len(flat) - 1
-            keys = self.lengths[row]
-            if row == padded:
-                for position in range(self.lengths[row], self.lengths[row] + padding):
-                    flat.append(0)
-                    positions.append(min(position, self.capacity - 1))
-                    write_pages.append(self.pool)
-                    write_slots.append(position % self.page_size)
-                keys += padding
-            visible.append(keys)
-            sequence_ids.extend([row] * (len(flat) - len(sequence_ids)))
-            query_offsets.append(len(flat))
-            last_rows.append(last)
-            real_tokens.append(len(t))
+            page, last_page = start // self.page_size, (start + count - 1) // self.page_size
+            while last_page >= len(held):
+                held.append(self.free.pop())
+            flat[at: at + count] = flats[row]
+            if page == last_page:
+                write_pages[at: at + count] = held[page]
+            else:
+                own = np.asarray(held[page: last_page + 1], dtype=np.int64)
+                write_pages[at: at + count] = own[unbounded[at: at + count] // self.page_size - page]
+            self.lengths[row] += count
+        visible = list(self.lengths)
+        visible[padded] += padding
 
         pages, page_offsets, last_page_lengths = [], [0], []
         for held, seen in zip(self.pages, visible):
@@ -205,12 +214,11 @@ class PageTable:
                 pages.extend([self.pool] * (used - kept))
                 last_page_lengths.append((seen - 1) % self.page_size + 1)
             page_offsets.append(len(pages))
-        pages.extend([0] * (self.table_length() - len(pages)))
+        listed = np.zeros(self.table_length(), dtype=np.int64)
+        listed[: len(pages)] = pages
         as_array = lambda values: np.asarray(values, dtype=np.int64)
-        return DecodeStep(as_array(flat), as_array(positions), as_array(write_pages), as_array(write_slots),
-                          as_array(query_offsets), as_array(page_offsets), as_array(pages),
-                          as_array(last_page_lengths), as_array(last_rows), as_array(real_tokens),
-                          as_array(sequence_ids))
+        return DecodeStep(flat, positions, write_pages, write_slots, query_offsets, as_array(page_offsets), listed,
+                          as_array(last_page_lengths), first_rows + np.maximum(counts, 1) - 1, counts, sequence_ids)
 
     def place_prompts(self, lengths) -> None:
         """Advances every sequence by ``lengths[b]`` tokens without building step tensors (bulk prompt placement)."""
@@ -263,6 +271,18 @@ class PagedDecoder:
 
     def _stream(self) -> int:
         return int(self.torch.cuda.current_stream().cuda_stream)
+
+    def _send(self, arrays: dict, kind) -> dict:
+        """Arrays of one integer type on the device, by one copy that the host does not wait for."""
+        torch = self.torch
+        sizes = [len(array) for array in arrays.values()]
+        starts = np.cumsum([0] + [(size + 15) // 16 * 16 for size in sizes])
+        packed = torch.empty(int(starts[-1]), dtype=getattr(torch, np.dtype(kind).name), pin_memory=True)
+        host = packed.numpy()
+        for (start, size), array in zip(zip(starts, sizes), arrays.values()):
+            host[start: start + size] = array
+        sent = packed.to("cuda", non_blocking=True)
+        return {name: sent[start: start + size] for name, start, size in zip(arrays, starts, sizes)}
 
     def _refresh_block_table(self) -> None:
         for b, held in enumerate(self.table.pages):

@@ -29,7 +29,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import kernel_sys as ks
-from .decoder import PagedDecoder, PageTable
+from .decoder import PagedDecoder, PageTable, token_array
 from .layer_ops import FEW_TOKENS, BlockRows, ChunkRows, ExpandedRows, Ops, StepRows, plan_chunks, round_up
 from .parallel_mixer import ParallelConfig, ParallelMixer
 from .residual import LayerNormResidual, StreamResidual, Sublayer
@@ -434,7 +434,7 @@ class HybridDecoder(PagedDecoder):
         sequence) the logits of those tokens, [wanted, vocab], in that order.  A step that cannot get its pages raises
         before anything changed."""
         torch = self.torch
-        tokens = [[int(v) for v in t] for t in tokens]
+        tokens = [token_array(t) for t in tokens]
         if all(len(t) <= 1 for t in tokens):
             step = self._plan_lists(tokens)
             self.run()
@@ -446,7 +446,7 @@ class HybridDecoder(PagedDecoder):
         logits = torch.empty((len(picked), self.config.vocab), dtype=torch.float32, device="cuda")
         if len(picked) > 0:
             last = self.ops.rows(len(picked), self.config.width)
-            last.copy_(normed.index_select(0, torch.from_numpy(picked).cuda()))
+            last.copy_(normed.index_select(0, self._send({"picked": picked}, np.int64)["picked"]))
             self.ops.linear_f32_out(self._stream(), logits, last, self.head)
         return logits
 
@@ -516,7 +516,8 @@ class HybridDecoder(PagedDecoder):
         chunks = {}
         for size, plan in plans.items():
             part = lambda name: n[f"{name}{size}"]
-            chunks[size] = ChunkRows(part("packed"), torch.from_numpy(plan["cached"]).cuda(), plan["keys"], part("moved"),
+            cached = self._send({"cached": plan["cached"]}, np.uint8)["cached"]
+            chunks[size] = ChunkRows(part("packed"), cached, plan["keys"], part("moved"),
                                      part("moved_to"), part("lens_q"), part("lens_kv"), part("offsets_q"), part("offsets_kv"),
                                      len(plan["lens_q"]))
         whole = None
@@ -528,16 +529,6 @@ class HybridDecoder(PagedDecoder):
                         n["table"].view(block_table.shape), w["positions"], n["sequence_of"], n["row_lens"],
                         int(fresh.max()), None if everything else w["short_rows"], n["short_sequences"], n["short_lens"],
                         len(short), expanded, blocks, chunks, whole)
-
-    def _send(self, arrays: dict, kind) -> dict:
-        torch = self.torch
-        sizes = [len(array) for array in arrays.values()]
-        starts = np.cumsum([0] + [round_up(size, 4) for size in sizes])
-        packed = np.zeros(int(starts[-1]), dtype=kind)
-        for (start, size), array in zip(zip(starts, sizes), arrays.values()):
-            packed[start: start + size] = array
-        sent = torch.from_numpy(packed).cuda()
-        return {name: sent[start: start + size] for name, start, size in zip(arrays, starts, sizes)}
 
 
 def random_weights(config: HybridConfig, names: dict, seed: int = 4) -> dict:

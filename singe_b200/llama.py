@@ -23,7 +23,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import kernel_sys as ks
-from .decoder import CachedDecoder, DecodeStep, PagedDecoder, PageTable, PageTableError  # noqa: F401 (one import for users)
+from .decoder import CachedDecoder, DecodeStep, PagedDecoder, PageTable, PageTableError, token_array  # noqa: F401 (one import for users)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -397,25 +397,23 @@ class LlamaDecoder(PagedDecoder):
             self.step([t[0] for t in tokens])
             logits = self._full_logits(self.logits)
             return logits if want is None else logits[[row for row, places in enumerate(want) for _ in places]]
-        step = self.table.step([[int(v) for v in t] for t in tokens])
+        step = self.table.step([token_array(t) for t in tokens])
         stream = int(torch.cuda.current_stream().cuda_stream)
         dev, bf16 = "cuda", torch.bfloat16
         t, s, w, d = len(step.tokens), self.sequences, c.hidden, c.head_dim
-        to_device = lambda array, dtype: torch.from_numpy(np.ascontiguousarray(array)).to(dev).to(dtype)
-        d_tokens, d_positions = to_device(step.tokens, torch.int64), to_device(step.positions, torch.int64)
-        d_pages, d_slots = to_device(step.write_pages, torch.int64), to_device(step.write_slots, torch.int64)
-        lens_q = np.diff(step.query_offsets).astype(np.int32)
         page_counts = np.diff(step.page_offsets)
-        lens_kv = ((page_counts - 1) * c.page_size + step.last_page_lengths).astype(np.int32)
         stride = max(int(page_counts.max()), 1)
-        table = np.zeros((s, stride), dtype=np.uint32)
+        table = np.zeros((s, stride), dtype=np.int32)
         for b in range(s):
             table[b, : page_counts[b]] = step.pages[step.page_offsets[b]: step.page_offsets[b + 1]]
-        d_lens_q, d_lens_kv = to_device(lens_q, torch.int32), to_device(lens_kv, torch.int32)
-        d_offsets = to_device(step.query_offsets[:-1].astype(np.int32), torch.int32)
-        d_table = to_device(table.view(np.int32), torch.int32)
         rows = step.last_rows if want is None else step.wanted_rows(want)
-        d_last = to_device(rows, torch.int64)
+        wide = self._send({"tokens": step.tokens, "positions": step.positions, "pages": step.write_pages, "slots": step.write_slots,
+                           "last": rows}, np.int64)
+        narrow = self._send({"lens_q": np.diff(step.query_offsets),
+                             "lens_kv": (page_counts - 1) * c.page_size + step.last_page_lengths,
+                             "offsets": step.query_offsets[:-1], "table": table.reshape(-1)}, np.int32)
+        d_tokens, d_positions, d_pages, d_slots, d_last = (wide[name] for name in ("tokens", "positions", "pages", "slots", "last"))
+        d_lens_q, d_lens_kv, d_offsets, d_table = (narrow[name] for name in ("lens_q", "lens_kv", "offsets", "table"))
         status = self.status.data_ptr()
         hidden = torch.empty((t, w), dtype=bf16, device=dev)
         normed = torch.empty((t, w), dtype=bf16, device=dev)
