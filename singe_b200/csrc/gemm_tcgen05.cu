@@ -5,10 +5,11 @@
 // singe-kernel/src/cpu/matmul/blocked.rs:27-95).  Replaces singe_tcgen05_matmul
 // (singe/src/backend/cuda/kernel_plan/source/tcgen05.rs:137-266), which is single-stage and cp.async-fed.
 //
-// Structure: persistent CTAs (one per SM), warp-specialised.
-//   warp 0   TMA producer: A tile [a_rows x 64] and B tile [BN x 64] of bf16 per stage, SWIZZLE_128B, ring of
+// Structure: persistent CTAs (one per SM), warp-specialised.  More than 128 rows run on pairs of SMs (gemm_pair.cuh); the
+// kernels here serve one row tile, batches of heads and [K, M] left operands.
+//   warp 0   TMA producer, one thread: A tile [a_rows x 64] and B tile [BN x 64] of bf16 per stage, SWIZZLE_128B, ring of
 //            `stages` mbarrier pairs.
-//   warp 1   MMA issuer: owns tensor memory (2 accumulators of BN columns), issues four
+//   warp 1   MMA issuer, one thread; the warp owns tensor memory (2 accumulators of BN columns), issues four
 //            tcgen05.mma 128 x BN x 16 per stage, commits the stage back to the producer and, after the last
 //            k-block, the accumulator to the epilogue.
 //   warps 2-5 epilogue: tcgen05.ld 32 columns at a time, convert, store; then hand the accumulator back, so
@@ -129,16 +130,36 @@ __device__ __forceinline__ void tile_coordinates(int tile, int tiles_m, int tile
     tn = within / rows;
 }
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t value;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(value));
+    return value;
+}
+
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t value;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(value));
+    return value;
+}
+
+// Every thread of every CTA of the cluster takes part; shared-memory writes before it are visible cluster-wide after.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+}  // namespace
+}  // namespace singe
+#include "gemm_pair.cuh"
+namespace singe {
+namespace {
+
 // KPS = 64-wide K slices per pipeline stage.  Skinny problems stream the weight matrix from HBM; with one
 // slice per stage every request touches 128 contiguous bytes of a weight row, which opens a DRAM page for two
 // bursts.  Several adjacent slices issued together give the memory controller 512-1024 contiguous bytes per row.
 // AT: the left operand is stored [K, M]; its 128 x 64 tile is two boxes of 64 K-rows x 64 M-columns, 8 KB apart, read
 // MN-major like a [K, N] right operand.
-// MT = 2: a tile is 256 rows, two 128-row MMAs per k step that read the same B slice: 64 KB of operands per 1024 clk
-// of tensor-core work instead of 48 KB per 512, which is what one SM can pull out of L2 (the 128 x 256 tile runs at the
-// SM's L2 read bandwidth, about 106 GB/s, not at the tensor core's rate).  Both accumulators belong to the one tile
-// (columns [0, BN) and [BN, 2 BN)), so the epilogue of a tile no longer overlaps the next tile's MMAs.
-template <int BN, int KPS, bool KN, bool AT = false, int MT = 1>
+template <int BN, int KPS, bool KN, bool AT = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
                      const GemmParams p) {
@@ -189,31 +210,29 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool failed = false;
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        // ---------------- TMA producer (one thread, see below) ----------------
+        if (elect_one()) {
             prefetch_tensor_map(&a_map);
             prefetch_tensor_map(&b_map);
-        }
-        // A stable weight operand does not depend on the kernels before this one: the B halves of the first tile's
-        // first `stages` ring slots are requested now (and a few more k-blocks pulled into L2), so that they cross
-        // HBM while the preceding kernel is still running.  Each slot's barrier expects the bytes of both operands;
-        // the A halves follow after the wait.
-        int preloaded = 0;
-        if (p.stable_rhs && blockIdx.x < total_tiles) {
-            int tm, tn;
-            const int batch = blockIdx.x / batch_tiles;
-            tile_coordinates(blockIdx.x - batch * batch_tiles, p.tiles_m, p.tiles_n, tm, tn);
-            const int b_row = batch * p.rhs_batch_rows + tn * BN;
-            preloaded = min(p.stages, p.k_blocks);
-            if (lane == 0) {
+            // A stable weight operand does not depend on the kernels before this one: the B halves of the first tile's
+            // first `stages` ring slots are requested now (and a few more k-blocks pulled into L2), so that they cross
+            // HBM while the preceding kernel is still running.  Each slot's barrier expects the bytes of both operands;
+            // the A halves follow after the wait.
+            int preloaded = 0;
+            if (p.stable_rhs && blockIdx.x < total_tiles) {
+                int tm, tn;
+                const int batch = blockIdx.x / batch_tiles;
+                tile_coordinates(blockIdx.x - batch * batch_tiles, p.tiles_m, p.tiles_n, tm, tn);
+                const int b_row = batch * p.rhs_batch_rows + tn * BN;
+                preloaded = min(p.stages, p.k_blocks);
                 for (int kb = 0; kb < preloaded; ++kb) {
                     const uint32_t stage = base + kb * p.stage_bytes;
                     const uint32_t full = bar_full + kb * 8;
-                    mbar_expect_tx(full, KPS * (MT * a_bytes + kBBytes));
+                    mbar_expect_tx(full, KPS * (a_bytes + kBBytes));
 #pragma unroll
                     for (int sub = 0; sub < KPS; ++sub) {
-                        load_b_slice<BN, KN>(stage + KPS * MT * a_bytes + sub * kBBytes, &b_map, full, (kb * KPS + sub) * kBlockK,
-                                         b_row);
+                        load_b_slice<BN, KN>(stage + KPS * a_bytes + sub * kBBytes, &b_map, full, (kb * KPS + sub) * kBlockK,
+                                             b_row);
                     }
                 }
                 const int last = min(p.k_blocks, preloaded + p.prefetch_blocks);
@@ -222,105 +241,97 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     for (int sub = 0; sub < KPS; ++sub) prefetch_b_slice<BN, KN>(&b_map, (kb * KPS + sub) * kBlockK, b_row);
                 }
             }
-        }
-        grid_dependency_wait();  // the A operand comes from the kernel before
-        int it = 0;
-        for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-            int tm, tn;
-            const int batch = tile / batch_tiles;
-            tile_coordinates(tile - batch * batch_tiles, p.tiles_m, p.tiles_n, tm, tn);
-            const int a_column = batch * p.lhs_batch_columns;
-            const int b_row = batch * p.rhs_batch_rows + tn * BN;
-            for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-                const int s = it % p.stages;
-                const uint32_t phase = (it / p.stages) & 1;
-                const bool early = it < preloaded;  // slot armed and its B half requested before the wait
-                int ok = 1;
-                if (lane == 0 && !early) ok = mbar_wait(bar_empty + s * 8, phase ^ 1) ? 1 : 0;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
-                    failed = true;
-                    break;
-                }
-                if (lane == 0) {
+            grid_dependency_wait();  // the A operand comes from the kernel before
+            int s = 0;
+            uint32_t phase = 0;
+            for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+                int tm, tn;
+                const int batch = tile / batch_tiles;
+                tile_coordinates(tile - batch * batch_tiles, p.tiles_m, p.tiles_n, tm, tn);
+                const int a_column = batch * p.lhs_batch_columns;
+                const int b_row = batch * p.rhs_batch_rows + tn * BN;
+                for (int kb = 0; kb < p.k_blocks; ++kb) {
+                    const bool early = preloaded > 0;  // slot armed and its B half requested before the wait
+                    if (!early && !mbar_wait(bar_empty + s * 8, phase ^ 1)) {
+                        failed = true;
+                        break;
+                    }
                     const uint32_t stage = base + s * p.stage_bytes;
                     const uint32_t full = bar_full + s * 8;
-                    if (!early) mbar_expect_tx(full, KPS * (MT * a_bytes + kBBytes));
+                    if (!early) mbar_expect_tx(full, KPS * (a_bytes + kBBytes));
 #pragma unroll
                     for (int sub = 0; sub < KPS; ++sub) {
                         // slices past K are zero-filled by TMA and add nothing
-#pragma unroll
-                        for (int mt = 0; mt < MT; ++mt) {
-                            const uint32_t a_at = stage + (sub * MT + mt) * a_bytes;
-                            const int row0 = (tm * MT + mt) * kBlockM;
-                            if (AT) {
-                                tma_load_2d(a_at, &a_map, full, row0, (kb * KPS + sub) * kBlockK);
-                                tma_load_2d(a_at + 8192, &a_map, full, row0 + 64, (kb * KPS + sub) * kBlockK);
-                            } else {
-                                tma_load_2d(a_at, &a_map, full, a_column + (kb * KPS + sub) * kBlockK, row0);
-                            }
+                        const uint32_t a_at = stage + sub * a_bytes;
+                        if (AT) {
+                            tma_load_2d(a_at, &a_map, full, tm * kBlockM, (kb * KPS + sub) * kBlockK);
+                            tma_load_2d(a_at + 8192, &a_map, full, tm * kBlockM + 64, (kb * KPS + sub) * kBlockK);
+                        } else {
+                            tma_load_2d(a_at, &a_map, full, a_column + (kb * KPS + sub) * kBlockK, tm * kBlockM);
                         }
                     }
                     if (!early) {
 #pragma unroll
                         for (int sub = 0; sub < KPS; ++sub) {
-                            load_b_slice<BN, KN>(stage + KPS * MT * a_bytes + sub * kBBytes, &b_map, full,
-                                             (kb * KPS + sub) * kBlockK, b_row);
+                            load_b_slice<BN, KN>(stage + KPS * a_bytes + sub * kBBytes, &b_map, full,
+                                                 (kb * KPS + sub) * kBlockK, b_row);
                         }
+                    }
+                    if (early) --preloaded;
+                    if (++s == p.stages) {
+                        s = 0;
+                        phase ^= 1;
                     }
                 }
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        int it = 0;
-        int local = 0;
-        for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local) {
-            // MT == 1: two accumulators take turns; MT == 2: both belong to every tile
-            const int acc = MT == 2 ? 0 : (local & 1);
-            const uint32_t acc_phase = MT == 2 ? (local & 1) : ((local >> 1) & 1);
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_acc_empty + acc * 8, acc_phase ^ 1) ? 1 : 0)) {
-                failed = true;
-                break;
-            }
-            tcgen05_fence_after();
-            const uint32_t tmem_d = tmem_base + acc * BN;
-            for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-                const int s = it % p.stages;
-                const uint32_t phase = (it / p.stages) & 1;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar_full + s * 8, phase) ? 1 : 0)) {
+        // One thread runs the whole loop.  With the warp in step (a vote after every wait, the issue under `lane == 0`) a
+        // stage cost 430 clk of issue alone, more than its four MMAs of 128 x 256 x 16 would take the tensor core; in an
+        // elected thread it costs 70.
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            int local = 0;
+            for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local) {
+                const int acc = local & 1;  // two accumulators take turns
+                if (!mbar_wait(bar_acc_empty + acc * 8, ((local >> 1) & 1) ^ 1)) {
                     failed = true;
                     break;
                 }
                 tcgen05_fence_after();
-                if (lane == 0) {
+                const uint32_t tmem_d = tmem_base + acc * BN;
+                for (int kb = 0; kb < p.k_blocks; ++kb) {
+                    if (!mbar_wait(bar_full + s * 8, phase)) {
+                        failed = true;
+                        break;
+                    }
+                    tcgen05_fence_after();
                     const uint32_t stage = base + s * p.stage_bytes;
 #pragma unroll
                     for (int sub = 0; sub < KPS; ++sub) {
+                        const uint64_t a_desc = make_smem_desc(stage + sub * a_bytes, BWalk<AT>::kLeadingBytes, 1024);
                         const uint64_t b_desc =
-                            make_smem_desc(stage + KPS * MT * a_bytes + sub * kBBytes, BWalk<KN>::kLeadingBytes, 1024);
+                            make_smem_desc(stage + KPS * a_bytes + sub * kBBytes, BWalk<KN>::kLeadingBytes, 1024);
 #pragma unroll
-                        for (int mt = 0; mt < MT; ++mt) {
-                            const uint64_t a_desc =
-                                make_smem_desc(stage + (sub * MT + mt) * a_bytes, BWalk<AT>::kLeadingBytes, 1024);
-#pragma unroll
-                            for (int ks = 0; ks < kBlockK / 16; ++ks) {
-                                // 16 bf16 of K: 2 descriptor address units along a K-major row, 128 down an MN-major tile
-                                umma_ss(tmem_d + mt * BN, a_desc + BWalk<AT>::kStep * ks, b_desc + BWalk<KN>::kStep * ks,
-                                        kIdesc, (kb > 0 || sub > 0 || ks > 0) ? 1u : 0u);
-                            }
+                        for (int ks = 0; ks < kBlockK / 16; ++ks) {
+                            // 16 bf16 of K: 2 descriptor address units along a K-major row, 128 down an MN-major tile
+                            umma_ss(tmem_d, a_desc + BWalk<AT>::kStep * ks, b_desc + BWalk<KN>::kStep * ks, kIdesc,
+                                    (kb > 0 || sub > 0 || ks > 0) ? 1u : 0u);
                         }
                     }
                     tcgen05_commit(bar_empty + s * 8);
+                    if (kb == p.k_blocks - 1) tcgen05_commit(bar_acc_full + acc * 8);
+                    if (++s == p.stages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
                 }
-                __syncwarp();
             }
-            if (failed) break;
-            if (lane == 0) {
-                tcgen05_commit(bar_acc_full + acc * 8);
-            }
-            __syncwarp();
         }
+        __syncwarp();
     } else {
         // ---------------- epilogue ----------------
         if (warp == 2) warm_l2(p.warm, blockIdx.x, gridDim.x, lane);
@@ -332,17 +343,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             const int batch = tile / batch_tiles;
             tile_coordinates(tile - batch * batch_tiles, p.tiles_m, p.tiles_n, tm, tn);
             const long long out_column = batch * p.out_batch_columns;
-            const int acc = MT == 2 ? 0 : (local & 1);
-            const uint32_t acc_phase = MT == 2 ? (local & 1) : ((local >> 1) & 1);
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_acc_full + acc * 8, acc_phase) ? 1 : 0)) {
+            const int acc = local & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_acc_full + acc * 8, (local >> 1) & 1) ? 1 : 0)) {
                 failed = true;
                 break;
             }
             tcgen05_fence_after();
-#pragma unroll 1
-            for (int mt = 0; mt < MT; ++mt) {
-            const int row = (tm * MT + mt) * kBlockM + quarter * 32 + lane;
-            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (acc + mt) * BN;
+            const int row = tm * kBlockM + quarter * 32 + lane;
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
                 uint32_t r[32];
@@ -419,7 +427,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     }
                 }
             }
-            }  // mt
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -427,9 +434,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             }
         }
     }
-    if (failed && lane == 0) {
-        report_status(p.error, kStatusWaitTimeout);
-    }
+    if (failed) report_status(p.error, kStatusWaitTimeout);
     if (failed) linger_after_timeout();
     tcgen05_fence_before();
     __syncthreads();
@@ -447,24 +452,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // them.  No workspace in global memory, no atomics, nothing to reset between launches.  A timeline of the earlier
 // form (partials parked locally, owners pulling them with remote loads, a second barrier before leaving) showed
 // 2.2 - 2.6 us in the pull and 0.8 us in the closing barrier of a 10 us kernel.
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t value;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(value));
-    return value;
-}
-
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t value;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(value));
-    return value;
-}
-
-// Every thread of every CTA of the cluster takes part; shared-memory writes before it are visible cluster-wide after.
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 template <int BN, int KPS, bool KN>
 __global__ void __launch_bounds__(kSplitKThreads, 1)
     gemm_splitk_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
@@ -523,17 +510,15 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
 
     bool failed = false;
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        // ---------------- TMA producer (one thread, see gemm_bf16_kernel) ----------------
+        if (elect_one()) {
             prefetch_tensor_map(&a_map);
             prefetch_tensor_map(&b_map);
-        }
-        // Stable weights: the B halves of this CTA's first ring slots are requested before the wait (see
-        // gemm_bf16_kernel), a few more k-blocks are pulled into L2.
-        int preloaded = 0;
-        if (p.stable_rhs && has_work) {
-            preloaded = min(p.stages, kb_last - kb_first);
-            if (lane == 0) {
+            // Stable weights: the B halves of this CTA's first ring slots are requested before the wait (see
+            // gemm_bf16_kernel), a few more k-blocks are pulled into L2.
+            int preloaded = 0;
+            if (p.stable_rhs && has_work) {
+                preloaded = min(p.stages, kb_last - kb_first);
                 for (int i = 0; i < preloaded; ++i) {
                     const int kb = kb_first + i;
                     const uint32_t stage = base + i * p.stage_bytes;
@@ -551,21 +536,15 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                     for (int sub = 0; sub < KPS; ++sub) prefetch_b_slice<BN, KN>(&b_map, (kb * KPS + sub) * kBlockK, tn * BN);
                 }
             }
-        }
-        grid_dependency_wait();  // the A operand comes from the kernel before
-        int it = 0;
-        for (int kb = kb_first; kb < kb_last; ++kb, ++it) {
-            const int s = it % p.stages;
-            const uint32_t phase = (it / p.stages) & 1;
-            const bool early = it < preloaded;
-            int ok = 1;
-            if (lane == 0 && !early) ok = mbar_wait(bar_empty + s * 8, phase ^ 1) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {
-                failed = true;
-                break;
-            }
-            if (lane == 0) {
+            grid_dependency_wait();  // the A operand comes from the kernel before
+            int s = 0;
+            uint32_t phase = 0;
+            for (int kb = kb_first; kb < kb_last; ++kb) {
+                const bool early = preloaded > 0;
+                if (!early && !mbar_wait(bar_empty + s * 8, phase ^ 1)) {
+                    failed = true;
+                    break;
+                }
                 const uint32_t stage = base + s * p.stage_bytes;
                 const uint32_t full = bar_full + s * 8;
                 if (!early) mbar_expect_tx(full, KPS * (a_bytes + kBBytes));
@@ -580,20 +559,25 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                                          tn * BN);
                     }
                 }
+                if (early) --preloaded;
+                if (++s == p.stages) {
+                    s = 0;
+                    phase ^= 1;
+                }
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        int it = 0;
-        for (int kb = kb_first; kb < kb_last; ++kb, ++it) {
-            const int s = it % p.stages;
-            const uint32_t phase = (it / p.stages) & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_full + s * 8, phase) ? 1 : 0)) {
-                failed = true;
-                break;
-            }
-            tcgen05_fence_after();
-            if (lane == 0) {
+        // ---------------- MMA issuer (one thread) ----------------
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            for (int kb = kb_first; kb < kb_last; ++kb) {
+                if (!mbar_wait(bar_full + s * 8, phase)) {
+                    failed = true;
+                    break;
+                }
+                tcgen05_fence_after();
                 const uint32_t stage = base + s * p.stage_bytes;
 #pragma unroll
                 for (int sub = 0; sub < KPS; ++sub) {
@@ -607,13 +591,14 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                     }
                 }
                 tcgen05_commit(bar_empty + s * 8);
+                if (kb == kb_last - 1) tcgen05_commit(bar_acc_full);
+                if (++s == p.stages) {
+                    s = 0;
+                    phase ^= 1;
+                }
             }
-            __syncwarp();
         }
-        if (!failed && has_work) {
-            if (lane == 0) tcgen05_commit(bar_acc_full);
-            __syncwarp();
-        }
+        __syncwarp();
     } else if (warp < 6) {
         // ---------------- hand the partial tile to the CTAs that own its rows ----------------
         // Row i of the tile belongs to cluster CTA i % splits.  The four warps park the CTA's f32 partial tile in its
@@ -677,9 +662,7 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
     // Every warp helps with the reduction (the producer and MMA warps have nothing left to do): all of them wait for
     // the bytes addressed to this CTA.
     if (!__all_sync(0xffffffffu, mbar_wait(bar_recv, 0) ? 1 : 0)) failed = true;
-    if (failed && lane == 0) {
-        report_status(p.error, kStatusWaitTimeout);
-    }
+    if (failed) report_status(p.error, kStatusWaitTimeout);
     if (failed) linger_after_timeout();
     // Arrive: "everything addressed to this CTA has landed".  When all CTAs have said so, every bulk copy of the
     // cluster has finished reading its source, and a CTA may leave (the matching wait is at the end).
@@ -746,11 +729,12 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                 if (p.gated) {
                     __nv_bfloat16 *dst =
                         static_cast<__nv_bfloat16 *>(p.out) + static_cast<long long>(row) * p.ldo + col / 2;
-                    if (col + 4 <= p.n) {
+                    if (p.vector_store && col + 4 <= p.n) {
                         *reinterpret_cast<uint32_t *>(dst) =
                             pack2<__nv_bfloat16>(gated_value(sum.x, sum.y), gated_value(sum.z, sum.w));
-                    } else if (col + 2 <= p.n) {
-                        dst[0] = __float2bfloat16_rn(gated_value(sum.x, sum.y));
+                    } else {
+                        if (col + 2 <= p.n) dst[0] = __float2bfloat16_rn(gated_value(sum.x, sum.y));
+                        if (col + 4 <= p.n) dst[1] = __float2bfloat16_rn(gated_value(sum.z, sum.w));
                     }
                 } else if (p.out_f32) {
                     float *dst = static_cast<float *>(p.out) + static_cast<long long>(row) * p.ldo + col;
@@ -881,13 +865,12 @@ int launch_gemm_splitk(cudaStream_t stream, GemmParams params, const void *lhs, 
     return launch_status();
 }
 
-template <int BN, int KPS, bool AT = false, int MT = 1>
+template <int BN, int KPS, bool AT = false>
 int launch_gemm(cudaStream_t stream, GemmParams params, const void *lhs, const void *rhs, size_t lhs_row_stride,
                 size_t rhs_row_stride) {
     const int kSmemLimit = shared_limit(params);
     const int b_bytes = BN * 128;
-    if (MT == 2) params.tiles_m = (params.m + 2 * kBlockM - 1) / (2 * kBlockM);  // 256-row tiles
-    params.stage_bytes = KPS * (MT * params.a_rows * 128 + b_bytes);
+    params.stage_bytes = KPS * (params.a_rows * 128 + b_bytes);
     params.k_blocks = (params.k + kBlockK * KPS - 1) / (kBlockK * KPS);
     params.prefetch_blocks = prefetch_blocks_for(params, KPS * b_bytes);
     params.pad_bytes = over_read_pad(params.a_rows, KPS * b_bytes);
@@ -905,9 +888,9 @@ int launch_gemm(cudaStream_t stream, GemmParams params, const void *lhs, const v
     static int configured[kMaxDevices] = {0};
     static int configured_kn[kMaxDevices] = {0};
     if (params.rhs_kn) {
-        SINGE_CUDA_TRY(ensure_dynamic_shared(gemm_bf16_kernel<BN, KPS, kHasKN, AT, MT>, smem, configured_kn));
+        SINGE_CUDA_TRY(ensure_dynamic_shared(gemm_bf16_kernel<BN, KPS, kHasKN, AT>, smem, configured_kn));
     } else {
-        SINGE_CUDA_TRY(ensure_dynamic_shared(gemm_bf16_kernel<BN, KPS, false, AT, MT>, smem, configured));
+        SINGE_CUDA_TRY(ensure_dynamic_shared(gemm_bf16_kernel<BN, KPS, false, AT>, smem, configured));
     }
 
     CUtensorMap a_map, b_map;
@@ -944,11 +927,102 @@ int launch_gemm(cudaStream_t stream, GemmParams params, const void *lhs, const v
     const int total = params.tiles_m * params.tiles_n * params.batch;
     const int grid = total < device_sm_count() ? total : device_sm_count();
     if (params.rhs_kn) {
-        SINGE_CUDA_TRY(launch_dependent(gemm_bf16_kernel<BN, KPS, kHasKN, AT, MT>, dim3(grid), dim3(kGemmThreads), smem,
+        SINGE_CUDA_TRY(launch_dependent(gemm_bf16_kernel<BN, KPS, kHasKN, AT>, dim3(grid), dim3(kGemmThreads), smem,
                                         stream, kLaunchGemm, 1, a_map, b_map, params));
     } else {
-        SINGE_CUDA_TRY(launch_dependent(gemm_bf16_kernel<BN, KPS, false, AT, MT>, dim3(grid), dim3(kGemmThreads), smem,
+        SINGE_CUDA_TRY(launch_dependent(gemm_bf16_kernel<BN, KPS, false, AT>, dim3(grid), dim3(kGemmThreads), smem,
                                         stream, kLaunchGemm, 1, a_map, b_map, params));
+    }
+    return launch_status();
+}
+
+// Columns of a pair's tile: the width whose rounds over the machine cost least.  A round's cost is the SM clocks of one
+// 64-wide K slice, measured on B200 over M = 136 .. 14400, (N, K) = (2048, 2048) .. (28672, 4096): a slice of 256 columns
+// runs at the tensor core's rate (512 clk of MMA), narrower ones approach what an SM reads from L2 (128 columns: 24 KB in
+// 350 - 400 clk; 64 columns: 20 KB in 330), so narrow tiles pay where they fill a machine that wide ones leave idle.
+// 2048 x 4096 x 4096: 48 us in tiles of 256 columns (2 rounds), 53 of 192, 57 of 128; 1500 rows: 44 / 38 / 44;
+// 256 rows: 25 / 21 / 17.
+int pair_columns(const GemmParams &params, int sms, int forced) {
+    constexpr int kWidths[5] = {256, 224, 192, 128, 64};
+    constexpr int kClocks[5] = {560, 500, 455, 370, 330};
+    if (forced != 0) return params.rhs_kn && forced % 128 != 0 ? 0 : forced;
+    int best = 0;
+    long long least = 0;
+    for (int i = 0; i < 5; ++i) {
+        const int bn = kWidths[i];
+        if (params.rhs_kn && bn % 128 != 0) continue;
+        const long long tiles = static_cast<long long>((params.m + kPairRows - 1) / kPairRows) * ((params.n + bn - 1) / bn);
+        const long long cost = (tiles + sms / 2 - 1) / (sms / 2) * kClocks[i];
+        if (best == 0 || cost < least) {
+            best = bn;
+            least = cost;
+        }
+    }
+    return best;
+}
+
+template <int BN>
+int launch_gemm_pair(cudaStream_t stream, GemmParams params, const void *lhs, const void *rhs, size_t lhs_row_stride,
+                     size_t rhs_row_stride) {
+    constexpr int kStageBytes = kBlockM * 128 + BN / 2 * 128;
+    params.tiles_m = (params.m + kPairRows - 1) / kPairRows;
+    params.tiles_n = (params.n + BN - 1) / BN;
+    params.k_blocks = (params.k + kBlockK - 1) / kBlockK;
+    const int fixed = kPairStaging + 2 * kMaxStages * 8 + 64 + 1024;
+    int stages = (shared_limit(params) - fixed) / kStageBytes;
+    if (stages > kMaxStages) stages = kMaxStages;
+    if (stages < 2) stages = 2;  // the limit is a preference; two stages is the least the pipeline runs with
+    params.stages = stages;
+    const int smem = stages * kStageBytes + fixed;
+    constexpr bool kHasKN = BN % 128 == 0;  // [K, N] operands are staged in boxes of 64 columns, half of a tile's in each CTA
+    if (params.rhs_kn && !kHasKN) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
+    static int configured[kMaxDevices] = {0};
+    static int configured_kn[kMaxDevices] = {0};
+    if (params.rhs_kn) {
+        SINGE_CUDA_TRY(ensure_dynamic_shared(gemm_pair_kernel<BN, kHasKN>, smem, configured_kn));
+    } else {
+        SINGE_CUDA_TRY(ensure_dynamic_shared(gemm_pair_kernel<BN, false>, smem, configured));
+    }
+
+    CUtensorMap a_map, b_map, out_map;
+    {
+        const uint64_t dims[2] = {static_cast<uint64_t>(params.k), static_cast<uint64_t>(params.m)};
+        const uint64_t strides[1] = {static_cast<uint64_t>(lhs_row_stride) * 2};
+        const uint32_t box[2] = {kBlockK, kBlockM};
+        SINGE_TRY(encode_tensor_map(&a_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, lhs, dims, strides, box,
+                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B));
+    }
+    {
+        const uint64_t n = static_cast<uint64_t>(params.n), k = static_cast<uint64_t>(params.k);
+        const uint64_t dims[2] = {params.rhs_kn ? n : k, params.rhs_kn ? k : n};
+        const uint64_t strides[1] = {static_cast<uint64_t>(rhs_row_stride) * 2};
+        const uint32_t box[2] = {64, params.rhs_kn ? static_cast<uint32_t>(kBlockK) : static_cast<uint32_t>(BN / 2)};
+        SINGE_TRY(encode_tensor_map(&b_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rhs, dims, strides, box,
+                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B));
+    }
+    if (params.vector_store) {
+        // boxes of 32 rows x 32 accumulators (16 gated values), 128, 64 or 32 bytes a row
+        const uint64_t element = params.out_f32 ? 4 : 2;
+        const uint64_t dims[2] = {static_cast<uint64_t>(params.gated ? params.n / 2 : params.n), static_cast<uint64_t>(params.m)};
+        const uint64_t strides[1] = {static_cast<uint64_t>(params.ldo) * element};
+        const uint32_t box[2] = {params.gated ? 16u : 32u, 32u};
+        SINGE_TRY(encode_tensor_map(&out_map,
+                                    params.out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                                    params.out, dims, strides, box,
+                                    params.out_f32 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                                   : params.gated ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+                                    CU_TENSOR_MAP_L2_PROMOTION_NONE));
+    } else {
+        out_map = a_map;  // not used
+    }
+    const int total = params.tiles_m * params.tiles_n;
+    const int pairs = total < device_sm_count() / 2 ? total : device_sm_count() / 2;
+    if (params.rhs_kn) {
+        SINGE_CUDA_TRY(launch_dependent(gemm_pair_kernel<BN, kHasKN>, dim3(2 * pairs), dim3(kGemmThreads), smem, stream,
+                                        kLaunchGemm, 2, a_map, b_map, out_map, params));
+    } else {
+        SINGE_CUDA_TRY(launch_dependent(gemm_pair_kernel<BN, false>, dim3(2 * pairs), dim3(kGemmThreads), smem, stream,
+                                        kLaunchGemm, 2, a_map, b_map, out_map, params));
     }
     return launch_status();
 }
@@ -1050,34 +1124,55 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
             while (slices > 1 && slices * slice_bytes * 2 > 200 * 1024) slices >>= 1;
         }
     }
-    // One M tile and too few N tiles for the machine: split K over a cluster instead of narrowing the tile.  The
-    // tile stays 128 wide with 2 slices per stage (the best streaming shape measured).  Measured on B200 (M = 16..128,
-    // N = 768..6144, K = 512..14336): the best cluster is the largest of 2 / 4 whose CTAs still fit the machine in one
-    // wave; 8 pays only when even 4 leave two thirds of the SMs idle (then with 64-wide tiles), and a split needs at
-    // least three pipeline stages of K to amortise its fill and the reduction.
+    // One M tile and too few 128-wide N tiles for the machine: tiles of 64 or 128 columns, K split over clusters of up to
+    // four CTAs; whichever fills most of the machine in one wave.  Clusters of four are kept to 128 CTAs, what
+    // the GPCs hold at once (2304 x 2048: 36 clusters of four take 12.9 us, 36 of two 8.9); 8 splits pay only where four leave two thirds of
+    // the SMs idle; a split needs at least three stages of K to amortise its fill and the reduction.  Where narrow tiles
+    // and twice the splits tie, the narrow ones cost less to reduce and the wide ones stream a long K in longer runs:
+    // measured on B200, M = 128, (N, K) = (8192, 2048): 64 columns unsplit 10.3 us, 128 in two splits 12.7;
+    // (4096, 4096): 64 in two 12.0, 128 in four 13.2; (4096, 14336): 28.0 and 26.9.  M = 16: 9.3 / 10.2, 10.7 / 10.4,
+    // 23.3 / 23.3.  One stage of two slices or (M > 64, few stages) more stages of one: 4 x 128 at M = 128, K = 14336 31.7 and 26.9.
     int splits = 1;
     const int forced_splits = g_tuning_splits.load(std::memory_order_relaxed);
     const int forced_block_n = g_tuning_block_n.load(std::memory_order_relaxed);
     const int forced_slices = g_tuning_slices.load(std::memory_order_relaxed);
-    if (params.m <= kBlockM && tiles(128) < (sms * 2) / 3 && forced_splits != 1 && params.batch == 1) {
-        int wide = 128;
-        int wanted = 1;
-        while (wanted < 4 && tiles(wide) * wanted * 2 <= sms) wanted <<= 1;
-        if (wanted == 4 && tiles(wide) * 4 <= sms / 3) {
-            wanted = 8;
-            wide = 64;
+    const bool splittable = params.m <= kBlockM && params.batch == 1 && params.row_gate == nullptr && !params.lhs_km;
+    if (splittable && tiles(128) < (sms * 2) / 3) {
+        const int k_stages = (params.k + 2 * kBlockK - 1) / (2 * kBlockK);
+        const bool few_splits = params.k <= 2048 || (params.m >= 64 && params.k <= 8192);
+        int wide = 0;
+        int most = 0;
+        for (int i = 0; i < 6; ++i) {
+            // the preferred one of equals first
+            const int s = 1 << (i / 2);
+            const int candidate = i % 2 == 0 ? 64 : 128;
+            const int ctas = s * tiles(candidate);
+            if (ctas > (s == 4 ? 128 : sms) || (s > 1 && (k_stages / s < 3 || forced_splits == 1))) continue;
+            if (ctas > most || (ctas == most && s > splits && !few_splits)) {
+                most = ctas;
+                wide = candidate;
+                splits = s;
+            }
         }
-        const int stage_k = kBlockK * 2;
-        const int k_stages = (params.k + stage_k - 1) / stage_k;
-        while (wanted > 1 && k_stages / wanted < 3) wanted >>= 1;
-        if (wanted < 8) wide = 128;
-        if (wanted > 1) {
-            splits = wanted;
+        if (splits == 4 && wide == 64 && most <= sms / 3 && k_stages / 8 >= 3) splits = 8;
+        if (most > 0 && (splits > 1 || wide == 128 || most >= (sms * 2) / 3)) {
             bn = wide;
+            const int receive = splits > 1 ? splits * ((params.m + splits - 1) / splits) * bn * 4 : 0;
+            slices = bn == 64 ? 4 : 2;
+            while (slices > 1 && (shared_limit(params) - 2048 - receive) / (slices * (a_rows + bn) * 128) < (splits > 1 ? 5 : 4)) {
+                slices >>= 1;
+            }
+        }
+    } else if (splittable && tiles(128) >= (sms * 2) / 3 && a_rows == kBlockM) {
+        slices = 1;  // three stages of two slices against seven of one: (28672, 4096) 52.2 and 51.5 us, (14336, 4096) 26.6 and 25.8
+    }
+    if (forced_splits != 0 && params.batch == 1) {
+        splits = forced_splits;
+        if (splits > 1 && bn < 64) {
+            bn = 64;
             slices = 2;
         }
     }
-    if (forced_splits != 0 && params.batch == 1) splits = forced_splits;
     if (forced_block_n != 0) bn = forced_block_n;
     if (params.rhs_kn && bn < 64) {
         // [K, N] tiles are staged in boxes of 64 columns
@@ -1111,10 +1206,16 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
 #undef SINGE_SPLITK_CASE
         return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
     }
-    // Many 256 x 256 tiles: the form with two M sub-tiles per CTA, which halves the A-and-B bytes an SM pulls per flop.
-    if (bn == 256 && slices == 1 && params.m >= 2 * kBlockM && params.batch == 1 &&
-        ((params.m + 2 * kBlockM - 1) / (2 * kBlockM)) * ((params.n + 255) / 256) >= sms) {
-        return launch_gemm<256, 1, false, 2>(stream, params, lhs, rhs, lhs_row_stride, rhs_row_stride);
+    if (params.m > kBlockM && params.batch == 1 && params.row_gate == nullptr && (forced_slices == 0 || forced_slices == 1)) {
+        const int wide = pair_columns(params, sms, forced_block_n);
+#define SINGE_PAIR_CASE(BN_)                                                                              \
+    if (wide == BN_) return launch_gemm_pair<BN_>(stream, params, lhs, rhs, lhs_row_stride, rhs_row_stride);
+        SINGE_PAIR_CASE(256)
+        SINGE_PAIR_CASE(224)
+        SINGE_PAIR_CASE(192)
+        SINGE_PAIR_CASE(128)
+        SINGE_PAIR_CASE(64)
+#undef SINGE_PAIR_CASE
     }
 #define SINGE_GEMM_CASE(BN_, KPS_)                                                                    \
     if (bn == BN_ && slices == KPS_)                                                                  \
