@@ -1155,7 +1155,7 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
             }
         }
         if (splits == 4 && wide == 64 && most <= sms / 3 && k_stages / 8 >= 3) splits = 8;
-        if (most > 0 && (splits > 1 || wide == 128 || most >= (sms * 2) / 3)) {
+        if (most > 0 && (splits > 1 || wide == 128 || tiles(32) > sms)) {
             bn = wide;
             const int receive = splits > 1 ? splits * ((params.m + splits - 1) / splits) * bn * 4 : 0;
             slices = bn == 64 ? 4 : 2;

@@ -29,8 +29,10 @@
 //              (S = Q K^T: 8 x tcgen05.mma 128x128x16, both operands K-major in shared memory; O += P V: 8 x
 //              tcgen05.mma with P read from tensor memory and V MN-major), so softmax_A(j) overlaps PV_B(j-1) and
 //              QK_B(j), softmax_B(j) overlaps PV_A(j) and QK_A(j+1).
-//   warp 9     TMA producer: both Q tiles once, then K and V tiles (128 keys x 128 dims, two SWIZZLE_128B boxes
-//              each) into two stages each, released by tcgen05.commit when the MMAs that read them retire.
+//   warps 9,10 TMA producers: both Q tiles once and K tiles, V tiles (128 keys x 128 dims, two SWIZZLE_128B boxes
+//              each) into two stages each, released by tcgen05.commit when the MMAs that read them retire.  One warp for
+//              both let the next K tile wait for the last V tile's stage: a lone tile over paged keys took 1.7 us a key
+//              tile and takes 1.3.
 // Tensor memory (all 512 columns): S_A/P_A [0,128), S_B/P_B [128,256), O_A [256,384), O_B [384,512).
 // Shared memory: Q_A, Q_B, 2 x K, 2 x V tiles of 32 KB = 192 KB.
 // Under a causal mask tile A sees one key tile less than tile B; CTAs are dispatched heaviest-first.
@@ -50,7 +52,7 @@ namespace singe {
 
 namespace {
 
-constexpr int kPrefillThreads = 320;
+constexpr int kPrefillThreads = 352;
 constexpr int kTile = 128;           // rows of one query tile, and keys per key tile
 constexpr int kPair = 2 * kTile;     // query rows per CTA
 constexpr int kChunk = 32;           // score columns taken out of tensor memory at a time
@@ -108,7 +110,9 @@ struct PrefillParams {
 // infinity is not zero).
 // Bound by the tensor core and the special-function unit alike: 8 + 16 MMAs of 128 x 128 x 16 and 16384 exponentials a
 // key tile.  One step of four 510-token chunks and 28 decoding sequences behind 0 - 3000 tokens of context, 32 query heads on 8:
-// 238 us, 40.2 ms by one warp per row and head.
+// 172 us, 238 with items in order of their pair index and lone tiles a key tile at a time, 40.2 ms by one warp per row and head.
+// A pair's key tile takes 4800 - 5000 clk (3072 of MMA; softmax and Q K^T of a tile are a chain), a lone tile's 3000 in this
+// mix, whose cold cache all SMs read at once.
 struct TensorPaging {
     const void *query_offsets;
     const void *page_offsets;
@@ -125,6 +129,8 @@ struct TensorPaging {
 struct NoPaging {};
 
 constexpr int kMaxTensorSequences = 1024;
+constexpr int kTensorBarriers = 22;  // (one of them only keeps what follows aligned)
+constexpr int kMaxOrdered = 1024;   // (sequence, pair) entries that are put in order of their cost
 constexpr unsigned kRedoMarkedRows = 1u, kRedoBadPaging = 2u;
 __device__ unsigned g_tensor_redo = 0;
 
@@ -140,31 +146,50 @@ struct SequenceTable {
 // Fills the table; every thread of the CTA takes part.  Query offsets that run backwards would have two sequences own a
 // token: then the whole call is left to the general kernel, which gives it to the first.
 __device__ __forceinline__ void list_sequences(const TensorPaging &g, int cache_pages, const SequenceTable &table, int warp, int lane) {
+    // A lane reads the offsets of one sequence, then the warp goes through its sequences' pages with several loads in
+    // flight: one load after the other, the pages of 32 sequences took each CTA some 10 us.
+    constexpr int kWarps = kPrefillThreads / 32, kFlight = 4;
     bool backwards = false;
-    for (int s = warp; s < g.sequences; s += kPrefillThreads / 32) {
-        const long long qf = paging_value(g.query_offsets, g.index_width, s);
-        const long long ql = paging_value(g.query_offsets, g.index_width, s + 1);
-        const long long pf = paging_value(g.page_offsets, g.index_width, s);
-        const long long pl = paging_value(g.page_offsets, g.index_width, s + 1);
-        bool bad = !(0 <= qf && qf <= ql && ql <= g.tokens);
-        backwards |= bad;
-        bad |= !(0 <= pf && pf <= pl && pl <= g.table_len);
-        long long keys = 0;
-        if (!bad && pf != pl) {
-            const long long last = paging_value(g.last_page_lengths, g.index_width, s);
-            bad = last < 0 || last > kPageTokens;
-            keys = (pl - pf - 1) * kPageTokens + last;
-            for (long long i = pf + lane; i < pl && !bad; i += 32) {
-                const long long page = paging_value(g.pages, g.index_width, static_cast<int>(i));
-                bad = page < 0 || page >= cache_pages;
+    for (int base = warp; base < g.sequences; base += 32 * kWarps) {
+        const int own = base + lane * kWarps;
+        long long qf = 0, ql = 0, pf = 0, pl = 0, keys = 0;
+        bool bad = false;
+        if (own < g.sequences) {
+            qf = paging_value(g.query_offsets, g.index_width, own);
+            ql = paging_value(g.query_offsets, g.index_width, own + 1);
+            pf = paging_value(g.page_offsets, g.index_width, own);
+            pl = paging_value(g.page_offsets, g.index_width, own + 1);
+            const long long last = paging_value(g.last_page_lengths, g.index_width, own);
+            bad = !(0 <= qf && qf <= ql && ql <= g.tokens);
+            backwards |= bad;
+            bad |= !(0 <= pf && pf <= pl && pl <= g.table_len);
+            if (!bad && pf != pl) {
+                bad = last < 0 || last > kPageTokens;
+                keys = (pl - pf - 1) * kPageTokens + last;
             }
         }
-        bad = __any_sync(0xffffffffu, bad) != 0;
-        if (lane == 0) {
-            table.rows[s] = bad ? 0 : static_cast<int>(ql - qf) << g.pack;
-            table.keys[s] = bad ? 0 : static_cast<int>(keys);
-            table.first_token[s] = bad ? 0 : static_cast<int>(qf);
-            table.first_page[s] = bad ? 0 : static_cast<int>(pf);
+        for (int i = 0; i < 32 && base + i * kWarps < g.sequences; ++i) {
+            const long long first = __shfl_sync(0xffffffffu, pf, i), end = __shfl_sync(0xffffffffu, pl, i);
+            bool outside = false;
+            if (__shfl_sync(0xffffffffu, bad ? 1 : 0, i) == 0) {
+                for (long long at = first + lane; at < end; at += 32 * kFlight) {
+#pragma unroll
+                    for (int u = 0; u < kFlight; ++u) {
+                        if (at + 32 * u < end) {
+                            const long long page = paging_value(g.pages, g.index_width, static_cast<int>(at + 32 * u));
+                            outside |= page < 0 || page >= cache_pages;
+                        }
+                    }
+                }
+            }
+            outside = __any_sync(0xffffffffu, outside) != 0;
+            if (lane == i) bad |= outside;
+        }
+        if (own < g.sequences) {
+            table.rows[own] = bad ? 0 : static_cast<int>(ql - qf) << g.pack;
+            table.keys[own] = bad ? 0 : static_cast<int>(keys);
+            table.first_token[own] = bad ? 0 : static_cast<int>(qf);
+            table.first_page[own] = bad ? 0 : static_cast<int>(pf);
             if (bad && blockIdx.x == 0) {
                 report_status(g.status, kStatusIndexOutOfBounds);
                 atomicOr(g.redo, kRedoBadPaging);
@@ -329,6 +354,7 @@ struct Item {
     int tiles[2];   // one past the last key tile tile A / tile B needs (0: no real row, or no visible key)
     int key_tiles;  // max of the two
     int first_page; // TENSOR: place of the sequence's first page in the page list
+    bool alternate; // TENSOR: a single query tile, whose key tiles go to tile A's and tile B's places in turn
     bool valid;     // false: the sequence's offsets leave the packed tensors
 };
 
@@ -338,16 +364,24 @@ __device__ __forceinline__ int pairs_of(int len_q) { return (max(len_q, 0) + kPa
 // pair index down (under a causal mask a pair's work grows with its index), head = index % heads.  `counts[t]` is
 // the number of sequences that have a pair t, `tmax` the largest pair count.  Every lane of the calling warp
 // takes part and receives the same answer.
-// TENSOR: rows are (token, head) pairs, `table` lists the sequences and `pack` is the log2 of a token's rows.
+// TENSOR: rows are (token, head) pairs, `table` lists the sequences and `pack` is the log2 of a token's rows; `order`, unless
+// it is nullptr, lists sequence and pair of every rank (see order_items).
 template <bool DENSE, bool WINDOW, bool TENSOR>
 __device__ __forceinline__ Item decode_item(const PrefillParams &p, const SequenceTable &table, int pack, const int *counts, int tmax,
-                                            int index, int lane) {
+                                            const unsigned *order, int index, int lane) {
     constexpr unsigned kFull = 0xffffffffu;
     Item item;
     int rank = index / p.heads;
     item.head = index - rank * p.heads;
     item.kv_head = item.head / (p.heads / p.kv_heads);
     int pair = -1;
+    int seq = -1;
+    if (TENSOR && order != nullptr) {
+        const unsigned entry = order[rank];
+        seq = static_cast<int>(entry % kMaxTensorSequences);
+        pair = static_cast<int>(entry / kMaxTensorSequences);
+        tmax = 0;
+    }
     for (int first = 0; first < tmax && pair < 0; first += 32) {
         const int t = tmax - 1 - (first + lane);
         const int count = t >= 0 ? counts[t] : 0;
@@ -366,7 +400,6 @@ __device__ __forceinline__ Item decode_item(const PrefillParams &p, const Sequen
             rank -= __shfl_sync(kFull, prefix, 31);
         }
     }
-    int seq = -1;
     for (int first = 0; first < p.batch && seq < 0 && pair >= 0; first += 32) {
         const int b = first + lane;
         const bool has = b < p.batch && pairs_of(TENSOR ? table.rows[b] : seq_len_q<DENSE>(p, b)) > pair;
@@ -390,6 +423,7 @@ __device__ __forceinline__ Item decode_item(const PrefillParams &p, const Sequen
     item.tiles[0] = item.tiles[1] = 0;
     item.key_tiles = 0;
     item.first_page = 0;
+    item.alternate = false;
     if (seq < 0) return item;
     if (TENSOR) {
         item.len_q = table.rows[seq];
@@ -428,7 +462,59 @@ __device__ __forceinline__ Item decode_item(const PrefillParams &p, const Sequen
         item.tiles[x] = (visible + kTile - 1) / kTile;
     }
     item.key_tiles = max(item.tiles[0], item.tiles[1]);
+    item.alternate = TENSOR && item.tiles[1] == 0 && item.tiles[0] - item.first[0] > 1;
     return item;
+}
+
+// TENSOR: lists the (sequence, pair) entries of a call by the key tiles they take, the longest first.  A chunk's pairs and a
+// decoding sequence's only one differ by what context lies behind them; dealt out by pair index alone, a CTA's share of
+// four 512-token chunks and 28 decoding sequences behind 0 - 3000 tokens came to twice the mean.  Every CTA computes the
+// same list; all its threads take part.  Returns the number of entries, or -1 with no list when there are more than
+// kMaxOrdered.  `first`: kMaxTensorSequences ints, `costs` and `entries`: kMaxOrdered each.
+template <bool WINDOW>
+__device__ __forceinline__ int order_items(const PrefillParams &p, const SequenceTable &table, int pack, int *first, int *costs,
+                                           unsigned *entries, unsigned *order, volatile int *total, int warp, int lane) {
+    if (warp == 0) {
+        int sum = 0;
+        for (int b = 0; b < p.batch; b += 32) {
+            const int own = b + lane < p.batch ? pairs_of(table.rows[b + lane]) : 0;
+            int prefix = own;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int other = __shfl_up_sync(0xffffffffu, prefix, d);
+                if (lane >= d) prefix += other;
+            }
+            if (b + lane < p.batch) first[b + lane] = sum + prefix - own;
+            sum = min(sum + __shfl_sync(0xffffffffu, prefix, 31), 2 * kMaxOrdered);  // (pairs of one sequence fit 22 bits)
+        }
+        if (lane == 0) *total = sum;
+    }
+    __syncthreads();
+    const int count = *total;
+    if (count > kMaxOrdered) return -1;
+    for (int b = warp; b < p.batch; b += kPrefillThreads / 32) {
+        const int rows = table.rows[b], keys = table.keys[b];
+        const int shift = keys - (rows >> pack);
+        for (int t = lane; t < pairs_of(rows); t += 32) {
+            const int last = min(rows, (t + 1) * kPair) - 1;
+            int visible = keys;
+            if (p.causal) visible = min(visible, max((last >> pack) + shift, 0) + 1);
+            int tiles = (visible + kTile - 1) / kTile;
+            if (WINDOW) tiles -= max(((t * kPair) >> pack) + shift - p.window + 1, 0) / kTile;
+            const bool single = rows - t * kPair <= kTile;  // half as long: see `alternate`
+            costs[first[b] + t] = single ? (tiles + 1) / 2 : tiles;
+            entries[first[b] + t] = static_cast<unsigned>(b + t * kMaxTensorSequences);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < count; i += kPrefillThreads) {
+        const int own = costs[i];
+        int place = 0;
+        for (int j = 0; j < count; ++j) place += costs[j] > own || (costs[j] == own && j < i) ? 1 : 0;
+        order[place] = entries[i];
+    }
+    __syncthreads();
+    return count;
 }
 
 // SAFE = false: the first launch.  One persistent CTA per SM walks its share of the items (item round r of CTA c is
@@ -465,7 +551,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     const uint32_t bar_p_full = bars + 112;   // [2 tiles], one arrival per softmax warp of the tile
     const uint32_t bar_o_full = bars + 128;   // [2 tiles]
     const uint32_t bar_o_empty = bars + 144;  // [2 tiles], one arrival per softmax warp of the tile
-    constexpr int kBarriers = 20;
+    const uint32_t bar_share = bars + 160;    // TENSOR: tile B's half of an alternating item, one arrival per softmax warp
+    constexpr int kBarriers = TENSOR ? kTensorBarriers : 20;
     const uint32_t words = bars + 8 * kBarriers;
     volatile uint32_t *holder_ptr = reinterpret_cast<volatile uint32_t *>(smem_raw + (words - raw));
     volatile int *shared_tmax = reinterpret_cast<volatile int *>(smem_raw + (words + 4 - raw));
@@ -478,6 +565,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     const int lane = tid & 31;
     SequenceTable table = {};
     int pack = 0;
+    int ordered = -1;                  // TENSOR: entries in `order`, or -1: items go by `counts`
+    unsigned *order = nullptr;
+    volatile float2 *share = nullptr;  // TENSOR: base and sum of tile B's rows of an alternating item
     if constexpr (TENSOR) {
         // (the redo list's place and what follows it)
         table.rows = counts + kMaxRankTiles;
@@ -485,14 +575,22 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         table.first_token = table.keys + kMaxTensorSequences;
         table.first_page = table.first_token + kMaxTensorSequences;
         pack = paging.pack;
+        int *costs = table.first_page + kMaxTensorSequences;
+        unsigned *entries = reinterpret_cast<unsigned *>(costs + kMaxOrdered);
+        order = entries + kMaxOrdered;
+        share = reinterpret_cast<volatile float2 *>(order + kMaxOrdered);
         list_sequences(paging, p.cache_pages, table, warp, lane);
+        __syncthreads();
+        ordered = order_items<WINDOW>(p, table, pack, counts, costs, entries, order, shared_ranks, warp, lane);
+        if (ordered < 0) order = nullptr;
+        __syncthreads();  // `counts` may be used again below
     }
     if (SAFE && !p.exact && *reinterpret_cast<volatile unsigned *>(&g_out_of_range_seen) == 0u) {
         return;  // no first launch on this device has ever marked a row
     }
 
     // ---- the table behind the heaviest-first item order ----
-    {
+    if (!TENSOR || ordered < 0) {
         int tmax = 0;
         for (int b = 0; b < p.batch; ++b) tmax = max(tmax, pairs_of(TENSOR ? table.rows[b] : seq_len_q<DENSE>(p, b)));
         tmax = min(tmax, kMaxRankTiles);
@@ -510,9 +608,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         }
         __syncthreads();
     }
-    const int tmax = *shared_tmax;
-    auto decode = [&](int index) { return decode_item<DENSE, WINDOW, TENSOR>(p, table, pack, counts, tmax, index, lane); };
-    const long long total_items = static_cast<long long>(*shared_ranks) * p.heads;
+    const int tmax = TENSOR && ordered >= 0 ? 0 : *shared_tmax;
+    auto decode = [&](int index) { return decode_item<DENSE, WINDOW, TENSOR>(p, table, pack, counts, tmax, order, index, lane); };
+    const long long total_items = static_cast<long long>(TENSOR && ordered >= 0 ? ordered : *shared_ranks) * p.heads;
     // index of this CTA's share number `round`, or -1 past the end
     auto share_index = [&](int round) -> int {
         const long long first = static_cast<long long>(round) * gridDim.x;
@@ -562,7 +660,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
 
     if (tid == 0) {
         for (int i = 0; i < kBarriers; ++i) {
-            const bool by_warps = i == 14 || i == 15 || i == 18 || i == 19;  // p_full[2], o_empty[2]
+            const bool by_warps = i == 14 || i == 15 || i >= 18;  // p_full[2], o_empty[2], share
             mbar_init(bars + 8 * i, by_warps ? 4 : 1);
         }
         mbar_init_fence();
@@ -578,12 +676,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
 
     bool failed = false;
 
-    if (warp == 9) {
-        // ---------------- TMA producer ----------------
+    if (warp >= 9) {
+        // ---------------- TMA producers: warp 9 Q and K, warp 10 V ----------------
+        const bool values = warp == 10;
+        const CUtensorMap *map = values ? &v_map : &k_map;
+        const uint32_t tiles_smem = values ? v_smem : k_smem;
+        const uint32_t bar_full = values ? bar_v_full : bar_k_full;
+        const uint32_t bar_empty = values ? bar_v_empty : bar_k_empty;
         if (lane == 0) {
-            prefetch_tensor_map(&q_map);
-            prefetch_tensor_map(&k_map);
-            prefetch_tensor_map(&v_map);
+            if (!values) prefetch_tensor_map(&q_map);
+            prefetch_tensor_map(map);
         }
         int g = 0;                // key tiles loaded so far, over all items: stage g & 1, use (g >> 1)
         int q_loads[2] = {0, 0};  // Q tiles loaded so far
@@ -599,14 +701,14 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             if (item.key_tiles == 0) continue;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                if (item.tiles[x] == 0 || failed) continue;
+                if (item.tiles[x] == 0 || failed || values) continue;
                 // the tile's buffer is free when the previous item's last Q K^T of this tile has retired
                 if (q_loads[x] > 0 && !wait_lane0(bar_q_empty + x * 8, (q_loads[x] - 1) & 1)) {
                     failed = true;
                     continue;
                 }
                 ++q_loads[x];
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_expect_tx(bar_q_full + x * 8, kLoadBytes);
                     // TENSOR: a box holds the heads of a pack for 128 >> pack tokens, token by token
                     const int row0 = item.offset + ((item.q0 + x * kTile) >> pack);
@@ -617,67 +719,53 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                                     head0, row0);
                     }
                 }
+                __syncwarp();
             }
+            // paged form: the page ids of a key tile, one per lane (by its low three bits), read a tile ahead; lanes 0-15 each
+            // own one (page, half) box.  A page past the sequence's last one is replaced by the sequence's first page (finite
+            // data that the mask hides), a page id outside the cache likewise, with status 1.
+            auto page_of = [&](int j) -> int32_t {
+                const int pages_of_sequence = (item.len_kv + kPageTokens - 1) / kPageTokens;
+                const int wanted = j * (kTile / kPageTokens) + (lane & 7);
+                const int place = wanted < pages_of_sequence ? wanted : 0;
+                if constexpr (TENSOR) {
+                    return static_cast<int32_t>(paging_value(paging.pages, paging.index_width, item.first_page + place));
+                } else {
+                    const uint32_t *row = p.block_table + static_cast<size_t>(item.seq) * p.table_stride;
+                    uint32_t id = row[place];
+                    if (id >= static_cast<uint32_t>(p.cache_pages)) {
+                        report_status(p.error, kStatusIndexOutOfBounds);
+                        id = 0u;
+                    }
+                    return static_cast<int32_t>(id);
+                }
+            };
+            int32_t page = PAGED ? page_of(item.first[0]) : 0;
             for (int j = item.first[0]; j < item.key_tiles && !failed; ++j, ++g) {
                 const int stage = g & 1;
-                const int row0 = item.offset_kv + j * kTile;
-                if (g >= 2 && !wait_lane0(bar_k_empty + stage * 8, ((g >> 1) - 1) & 1)) {
+                const int32_t coming = PAGED && j + 1 < item.key_tiles ? page_of(j + 1) : 0;
+                if (g >= 2 && !wait_lane0(bar_empty + stage * 8, ((g >> 1) - 1) & 1)) {
                     failed = true;
                     break;
                 }
-                // paged form: lanes 0-15 each own one (page, half) box of the tile; a page past the sequence's last
-                // one is replaced by the sequence's first page (finite data that the mask hides), a page id outside
-                // the cache likewise, with status 1
-                int32_t page = 0;
+                const uint32_t tile = tiles_smem + stage * kTileBytes;
                 if (PAGED) {
-                    const int pages_of_sequence = (item.len_kv + kPageTokens - 1) / kPageTokens;
-                    const int wanted = j * (kTile / kPageTokens) + (lane & 7);
-                    const int place = wanted < pages_of_sequence ? wanted : 0;
-                    if constexpr (TENSOR) {
-                        page = static_cast<int32_t>(paging_value(paging.pages, paging.index_width, item.first_page + place));
-                    } else {
-                        const uint32_t *row = p.block_table + static_cast<size_t>(item.seq) * p.table_stride;
-                        uint32_t id = row[place];
-                        if (id >= static_cast<uint32_t>(p.cache_pages)) {
-                            report_status(p.error, kStatusIndexOutOfBounds);
-                            id = 0u;
-                        }
-                        page = static_cast<int32_t>(id);
-                    }
-                }
-                if (lane == 0) mbar_expect_tx(bar_k_full + stage * 8, kLoadBytes);
-                __syncwarp();
-                if (PAGED) {
+                    if (lane == 0) mbar_expect_tx(bar_full + stage * 8, kLoadBytes);
+                    __syncwarp();
                     if (lane < 8 * kHalves) {
                         const int half = lane >> 3;
-                        tma_load_4d(k_smem + stage * kTileBytes + half * kHalfTileBytes + (lane & 7) * kPageBytes, &k_map,
-                                    bar_k_full + stage * 8, half * 64, item.kv_head, 0, page);
+                        tma_load_4d(tile + half * kHalfTileBytes + (lane & 7) * kPageBytes, map, bar_full + stage * 8, half * 64,
+                                    item.kv_head, 0, page);
                     }
-                } else if (lane == 0) {
-                    tma_load_3d(k_smem + stage * kTileBytes, &k_map, bar_k_full + stage * 8, 0, item.kv_head, row0);
-                    if (kHalves == 2) {
-                        tma_load_3d(k_smem + stage * kTileBytes + kHalfTileBytes, &k_map, bar_k_full + stage * 8, 64,
-                                    item.kv_head, row0);
+                    page = coming;
+                } else {
+                    if (elect_one()) {
+                        const int row0 = item.offset_kv + j * kTile;
+                        mbar_expect_tx(bar_full + stage * 8, kLoadBytes);
+                        tma_load_3d(tile, map, bar_full + stage * 8, 0, item.kv_head, row0);
+                        if (kHalves == 2) tma_load_3d(tile + kHalfTileBytes, map, bar_full + stage * 8, 64, item.kv_head, row0);
                     }
-                }
-                if (g >= 2 && !wait_lane0(bar_v_empty + stage * 8, ((g >> 1) - 1) & 1)) {
-                    failed = true;
-                    break;
-                }
-                if (lane == 0) mbar_expect_tx(bar_v_full + stage * 8, kLoadBytes);
-                __syncwarp();
-                if (PAGED) {
-                    if (lane < 8 * kHalves) {
-                        const int half = lane >> 3;
-                        tma_load_4d(v_smem + stage * kTileBytes + half * kHalfTileBytes + (lane & 7) * kPageBytes, &v_map,
-                                    bar_v_full + stage * 8, half * 64, item.kv_head, 0, page);
-                    }
-                } else if (lane == 0) {
-                    tma_load_3d(v_smem + stage * kTileBytes, &v_map, bar_v_full + stage * 8, 0, item.kv_head, row0);
-                    if (kHalves == 2) {
-                        tma_load_3d(v_smem + stage * kTileBytes + kHalfTileBytes, &v_map, bar_v_full + stage * 8, 64,
-                                    item.kv_head, row0);
-                    }
+                    __syncwarp();
                 }
             }
         }
@@ -689,10 +777,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool {
             return __all_sync(0xffffffffu, mbar_wait(bar, parity) ? 1 : 0) != 0;
         };
-        // S_x = Q_x K(stage)^T; `last` releases the Q tile
-        auto issue_qk = [&](int x, int stage, bool last) {
+        // S_x = Q_query K(stage)^T; `last` releases the Q tile
+        auto issue_qk = [&](int x, int stage, bool last, int query) {
             if (elect_one()) {
-                const uint32_t q_tile = q_smem + x * kTileBytes;
+                const uint32_t q_tile = q_smem + query * kTileBytes;
                 const uint32_t k_tile = k_smem + stage * kTileBytes;
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {
@@ -701,7 +789,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                             make_smem_desc(k_tile + within, 16, 1024), kIdescQK, ks > 0 ? 1u : 0u);
                 }
                 tcgen05_commit(bar_s_full + x * 8);
-                if (last) tcgen05_commit(bar_q_empty + x * 8);
+                if (last) tcgen05_commit(bar_q_empty + query * 8);
             }
             __syncwarp();
         };
@@ -751,7 +839,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             if (!wait_all(bar_q_full + x * 8, q_uses[x] & 1)) return false;
             ++q_uses[x];
             tcgen05_fence_after();
-            issue_qk(x, stage, item.tiles[x] == item.first[x] + 1);
+            issue_qk(x, stage, item.tiles[x] == item.first[x] + 1, x);
             return true;
         };
         Item item = next_item();
@@ -765,6 +853,57 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         }
         while (item.key_tiles > 0 && !failed) {
             const Item following = next_item();
+            if constexpr (TENSOR) {
+                // A single query tile: key tile j's scores stand in tile A's or tile B's place by turns, so that Q K^T of the
+                // next one runs beside this one's softmax, and each place has its own O.
+                for (int j = item.first[0]; item.alternate && j < item.key_tiles && !failed; ++j, ++g) {
+                    const int stage = g & 1;
+                    const int next = (g + 1) & 1;
+                    const int x = (j - item.first[0]) & 1;
+                    const bool more = j + 1 < item.key_tiles;
+                    auto next_keys = [&]() -> bool {
+                        if (!wait_all(bar_k_full + next * 8, ((g + 1) >> 1) & 1)) return false;
+                        tcgen05_fence_after();
+                        return true;
+                    };
+                    auto release_keys = [&]() {
+                        if (elect_one()) tcgen05_commit(bar_k_empty + next * 8);
+                        __syncwarp();
+                    };
+                    if (more) {
+                        if (!next_keys()) {
+                            failed = true;
+                            break;
+                        }
+                        issue_qk(x ^ 1, next, j + 2 == item.key_tiles, 0);
+                        release_keys();
+                    }
+                    if (!wait_all(bar_v_full + stage * 8, (g >> 1) & 1) ||
+                        (j < item.first[0] + 2 && o_done[x] > 0 && !wait_all(bar_o_empty + x * 8, (o_done[x] - 1) & 1)) ||
+                        !wait_all(bar_p_full + x * 8, p_uses[x] & 1)) {
+                        failed = true;
+                        break;
+                    }
+                    ++p_uses[x];
+                    tcgen05_fence_after();
+                    const bool last = j + 2 >= item.key_tiles;
+                    issue_pv(x, stage, j >= item.first[0] + 2, last);
+                    if (last) ++o_done[x];
+                    if (elect_one()) tcgen05_commit(bar_v_empty + stage * 8);
+                    __syncwarp();
+                    if (!more && following.key_tiles > 0) {
+                        if (!next_keys() || !first_qk(following, 0, next) || !first_qk(following, 1, next)) {
+                            failed = true;
+                            break;
+                        }
+                        release_keys();
+                    }
+                }
+                if (item.alternate) {
+                    item = following;
+                    continue;
+                }
+            }
             for (int j = item.first[0]; j < item.key_tiles && !failed; ++j, ++g) {
                 const int stage = g & 1;
                 const int next = (g + 1) & 1;
@@ -815,7 +954,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                                 tcgen05_fence_after();
                             }
                             if (j + 1 < item.tiles[x] && (!WINDOW || j + 1 >= item.first[x])) {
-                                issue_qk(x, next, j + 2 == item.tiles[x]);
+                                issue_qk(x, next, j + 2 == item.tiles[x], x);
                             }
                         } else if (!first_qk(following, x, next)) {
                             failed = true;
@@ -842,6 +981,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         const float sign = p.scale_log2 < 0.0f ? -1.0f : 1.0f;
         int s_uses = 0;   // score tiles consumed so far, over all items
         int o_uses = 0;   // outputs taken so far
+        int shares = 0, others_done = 0;  // TENSOR, tile A: alternating items so far, outputs of tile B so far
         for (int round = 0; !failed; ++round) {
             const int index = item_index(round);
             if (index < 0) break;
@@ -850,14 +990,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 if (warp == 0 && lane == 0) report_status(p.error, kStatusIndexOutOfBounds);
                 continue;
             }
-            const int row = item.q0 + x * kTile + local_row;    // sequence-local query index
+            // sequence-local query index
+            const int row = item.q0 + (TENSOR && item.alternate ? 0 : x * kTile) + local_row;
             const bool real = row < item.len_q;
             const int turn = row >> pack;                       // sequence-local token of the row
             const size_t token = static_cast<size_t>(item.offset) + (real ? turn : 0);
             T *dst = static_cast<T *>(p.out) + (((token * p.heads + item.head) << pack) + (real ? row & ((1 << pack) - 1) : 0)) * HD;
             float *lse_row = lse_at(item, real ? row : 0);
-            const int my_tiles = x == 0 ? item.tiles[0] : item.tiles[1];
-            const int my_first = x == 0 ? item.first[0] : item.first[1];
+            const bool alternate = TENSOR && item.alternate;  // both places hold tile A's rows, of every other key tile
+            const int my_tiles = x == 0 || alternate ? item.tiles[0] : item.tiles[1];
+            const int my_first = alternate ? item.first[0] + x : x == 0 ? item.first[0] : item.first[1];
+            const int my_step = alternate ? 2 : 1;
             if (my_tiles == 0) {
                 // No key is visible to this tile's rows: zeros and LSE -1e20.
                 if (real) {
@@ -871,7 +1014,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             float row_sum = 0.0f;
             bool in_range = true;
             bool unseen = WINDOW && real;  // no key seen yet: O and the sum are zero, so the base is free
-            for (int j = my_first; j < my_tiles && !failed; ++j, ++s_uses) {
+            bool seen = false;             // TENSOR: some key was visible
+            for (int j = my_first; j < my_tiles && !failed; j += my_step, ++s_uses) {
                 if (!__all_sync(0xffffffffu, mbar_wait(bar_s_full + x * 8, s_uses & 1) ? 1 : 0)) {
                     failed = true;
                     break;
@@ -884,6 +1028,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 const int low = WINDOW ? turn + item.shift - p.window + 1 - j * kTile : 0;  // first column the row sees
                 const bool partial = __any_sync(0xffffffffu, limit < kTile);
                 const bool lower = WINDOW && __any_sync(0xffffffffu, low > 0);
+                if (TENSOR) seen = seen || max(low, 0) < min(limit, kTile);
 
                 if (SAFE || j == my_first || (WINDOW && __any_sync(0xffffffffu, unseen))) {
                     float wanted;
@@ -944,6 +1089,41 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             }
             ++o_uses;
             tcgen05_fence_after();
+            // TENSOR, an alternating item: tile B's warps hand base and sum of their rows to tile A's, which fold the two
+            // outputs (both lie in tensor-memory lanes they may read) and store.  A place whose keys were visible but left no
+            // weight, or that left the range, passes a NaN.
+            float mine = 1.0f, others = 0.0f;  // weights of the two outputs
+            if constexpr (TENSOR) {
+                if (alternate) {
+                    if (row_sum == 0.0f) base_log2 = -INFINITY;
+                    if (!in_range || (seen && row_sum == 0.0f)) row_sum = __int_as_float(0x7fc00000);
+                    if (x == 1) {
+                        share[local_row].x = base_log2;
+                        share[local_row].y = row_sum;
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_share);
+                        continue;
+                    }
+                    // tile B's output: complete before its warps arrived, the second wait orders this thread's reads
+                    const bool there = mbar_wait(bar_share, shares & 1) && mbar_wait(bar_o_full + 8, others_done & 1);
+                    if (!__all_sync(0xffffffffu, there ? 1 : 0)) {
+                        failed = true;
+                        break;
+                    }
+                    ++shares;
+                    ++others_done;
+                    tcgen05_fence_after();
+                    const float base_b = share[local_row].x, sum_b = share[local_row].y;
+                    const float base = fmaxf(base_log2, base_b);
+                    mine = base_log2 == -INFINITY ? 0.0f : exp2_approx(base_log2 - base);
+                    others = base_b == -INFINITY ? 0.0f : exp2_approx(base_b - base);
+                    row_sum = row_sum * mine + sum_b * others;   // (no weight: 0 * 0, or a NaN that stays one)
+                    in_range = in_range && row_sum < kOverflowLimit;
+                    base_log2 = base;
+                } else if (x == 0 && item.tiles[1] > 0) {
+                    ++others_done;
+                }
+            }
             const bool empty = row_sum == 0.0f;
             float inverse = empty ? 0.0f : 1.0f / row_sum;
             if (WINDOW && p.gate != nullptr) {
@@ -955,6 +1135,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 uint32_t r[32];
                 tmem_ld_x32(tmem_o + c, r);
                 tmem_wait_ld_into(r);
+                if constexpr (TENSOR) {
+                    if (alternate) {
+                        uint32_t b[32];
+                        tmem_ld_x32(tmem_o + HD + c, b);
+                        tmem_wait_ld_into(b);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            r[i] = __float_as_uint(__uint_as_float(r[i]) * mine + __uint_as_float(b[i]) * others);
+                        }
+                    }
+                }
                 if (TENSOR) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) probe = fmaf(__uint_as_float(r[i]) * inverse, 0.0f, probe);
@@ -964,6 +1155,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     tcgen05_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_o_empty + x * 8);
+                    if (lane == 0 && alternate) mbar_arrive(bar_o_empty + 8);
                 }
                 if (real) {
 #pragma unroll
@@ -1044,7 +1236,9 @@ template <int HD, bool WINDOW>
 int launch_tensor(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
                   const PrefillParams &params, const TensorPaging &paging, unsigned persistent) {
     static int raised[kMaxDevices] = {0};
-    constexpr int kBytes = kPrefillSmem + (4 * kMaxTensorSequences - kRedoCapacity) * 4;
+    constexpr int kBytes = kPrefillSmem + (4 * kMaxTensorSequences - kRedoCapacity + 3 * kMaxOrdered) * 4 +
+                           (kTensorBarriers - 20) * 8 + kTile * 8;
+    static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
     const auto kernel = prefill_tcgen05_kernel<__nv_bfloat16, HD, false, true, false, WINDOW, true>;
     SINGE_CUDA_TRY(ensure_dynamic_shared(kernel, kBytes, raised));
     kernel<<<persistent, kPrefillThreads, kBytes, stream>>>(q_map, k_map, v_map, params, paging);
