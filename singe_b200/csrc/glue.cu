@@ -165,6 +165,84 @@ __global__ void add_rms_norm_kernel(__nv_bfloat16 *hidden, const __nv_bfloat16 *
     }
 }
 
+// The same for prompts: a warp per row, so that nothing waits for a CTA and 16 KB of a row are in flight from the start.  Bound
+// by HBM.  The virtual threads of a row (see square_chain) are kept: virtual warp w is the warp's w-th 256 values.
+// 17280 rows of 4096: 156 - 223 us a CTA per row (barriers, and one 16-byte load per thread at a time),
+// now 89 (6.4 TB/s); 8192 rows of 2048: 36 and 21.  With fewer than about eight rows per SM the warps leave it idle and a CTA
+// per row is done sooner (750 rows of 4096: 7.4 us against 8.8; 1500: 15.4 against 11.3).
+constexpr int kRowWarps = 4;         // rows of a CTA
+constexpr size_t kRowsPerSm = 8;     // from here on a warp takes a row
+
+template <int WARPS>
+__global__ void __launch_bounds__(kRowWarps * 32)
+    add_rms_norm_rows_kernel(__nv_bfloat16 *hidden, const __nv_bfloat16 *delta, __nv_bfloat16 *normed,
+                             const __nv_bfloat16 *weight, int rows, int width, float eps, const WarmRange warm) {
+    grid_launch_dependents();
+    if (threadIdx.x < 32) warm_l2(warm, blockIdx.x, gridDim.x, threadIdx.x);
+    grid_dependency_wait();
+    const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const int lane8 = (threadIdx.x & 31) * 8;
+    const size_t base = static_cast<size_t>(row) * width;
+    uint4 held[WARPS];
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        const int c = w * 256 + lane8;
+        held[w] = c < width ? *reinterpret_cast<const uint4 *>(hidden + base + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (delta != nullptr) {
+        uint4 other[WARPS];
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            const int c = w * 256 + lane8;
+            other[w] = c < width ? *reinterpret_cast<const uint4 *>(delta + base + c) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            uint32_t *mine = &held[w].x;
+            const uint32_t *others = &other[w].x;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                mine[i] = pack2<__nv_bfloat16>(__uint_as_float(mine[i] << 16) + __uint_as_float(others[i] << 16),
+                                               __uint_as_float(mine[i] & 0xffff0000u) + __uint_as_float(others[i] & 0xffff0000u));
+            }
+            const int c = w * 256 + lane8;
+            if (c < width) *reinterpret_cast<uint4 *>(hidden + base + c) = held[w];
+        }
+    }
+    if (normed == nullptr) return;
+    float square[WARPS];
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        const uint32_t *mine = &held[w].x;
+        square[w] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            square[w] = square_chain(square[w], __uint_as_float(mine[i] << 16));
+            square[w] = square_chain(square[w], __uint_as_float(mine[i] & 0xffff0000u));
+        }
+    }
+    float total = 0.0f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) total += warp_sum(square[w]);
+    const float scale = 1.0f / sqrtf(total / static_cast<float>(width) + eps);
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        const int c = w * 256 + lane8;
+        if (c < width) {
+            const Vec8 gain = load8(weight + c);
+            const uint32_t *mine = &held[w].x;
+            Vec8 result;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                result.v[2 * i] = __uint_as_float(mine[i] << 16) * scale * gain.v[2 * i];
+                result.v[2 * i + 1] = __uint_as_float(mine[i] & 0xffff0000u) * scale * gain.v[2 * i + 1];
+            }
+            store8(normed + base + c, result);
+        }
+    }
+}
+
 // One CTA per token.  qkv row = [heads*D | kv_heads*D | kv_heads*D].  Rotates Q into q_out and K into the cache at
 // (write_pages[t], write_slots[t]); V is copied into the cache.  Rounding follows the tensor-op chain of
 // rotate_pairs: first' = bf16(bf16(first*cos) - bf16(second*sin)), second' = bf16(bf16(second*cos) + bf16(first*sin)).
@@ -303,6 +381,96 @@ __global__ void rotary_cache_write_kernel(__nv_bfloat16 *q_out, const __nv_bfloa
     }
 }
 
+// The same for prompts, without norms: a warp per token.  A head's pairs lie on head_dim / 16 adjacent lanes, a power of two,
+// so a lane meets the same angles in every head and reads them once; eight heads a lane are requested before the token's
+// position, page and slot are waited for.  Bound by HBM.  32 heads on 8 of 128: 17280 tokens 127 us a CTA per token, 77 now;
+// 2000 tokens 12.8 and 10.5, 1200 9.7 and 10.3: the line lies between.
+constexpr size_t kTokensPerSm = 12;
+
+template <typename Index>
+__global__ void __launch_bounds__(kRowWarps * 32)
+    rotary_rows_kernel(__nv_bfloat16 *q_out, const __nv_bfloat16 *qkv, long long qkv_stride, const __nv_bfloat16 *cos_table,
+                       const __nv_bfloat16 *sin_table, const Index *positions, __nv_bfloat16 *key_cache,
+                       __nv_bfloat16 *value_cache, const Index *write_pages, const Index *write_slots, int tokens, int heads,
+                       int kv_heads, int head_dim, long long pages, long long page_size, long long capacity, uint32_t *status,
+                       const WarmRange warm) {
+    constexpr int kBatch = 8;
+    grid_launch_dependents();
+    if (threadIdx.x < 32) warm_l2(warm, blockIdx.x, gridDim.x, threadIdx.x);
+    grid_dependency_wait();
+    const int token = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (token >= tokens) return;
+    const int lane = threadIdx.x & 31;
+    const int half = head_dim >> 1;
+    const int per_head = half / 8;
+    const int heads_at_once = 32 / per_head;
+    const int i = (lane % per_head) * 8;
+    const int rotated = heads + kv_heads;
+    const __nv_bfloat16 *row = qkv + static_cast<size_t>(token) * qkv_stride;
+    Vec8 c, s;
+    size_t cache_row = 0;
+    bool slot_ok = false;
+    for (int first = lane / per_head; first - lane / per_head < rotated; first += kBatch * heads_at_once) {
+        uint4 low[kBatch], high[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int head = first + u * heads_at_once;
+            if (head < rotated) {
+                low[u] = *reinterpret_cast<const uint4 *>(row + static_cast<size_t>(head) * head_dim + i);
+                high[u] = *reinterpret_cast<const uint4 *>(row + static_cast<size_t>(head) * head_dim + i + half);
+            }
+        }
+        if (first == lane / per_head) {
+            long long position = static_cast<long long>(positions[token]);
+            long long page = static_cast<long long>(write_pages[token]);
+            long long slot = static_cast<long long>(write_slots[token]);
+            if (position < 0) position += capacity;
+            if (page < 0) page += pages;
+            if (slot < 0) slot += page_size;
+            const bool position_ok = position >= 0 && position < capacity;
+            slot_ok = page >= 0 && page < pages && slot >= 0 && slot < page_size;
+            if ((!position_ok || !slot_ok) && lane == 0) report_status(status, kStatusIndexOutOfBounds);
+            if (!position_ok) return;
+            c = load8(cos_table + static_cast<size_t>(position) * half + i);
+            s = load8(sin_table + static_cast<size_t>(position) * half + i);
+            cache_row = (static_cast<size_t>(page) * page_size + slot) * kv_heads * head_dim;
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int head = first + u * heads_at_once;
+            if (head >= rotated || (head >= heads && !slot_ok)) continue;
+            __nv_bfloat16 *target = head < heads ? q_out + (static_cast<size_t>(token) * heads + head) * head_dim
+                                                 : key_cache + cache_row + static_cast<size_t>(head - heads) * head_dim;
+            const uint32_t *low_words = &low[u].x, *high_words = &high[u].x;
+            Vec8 out_first, out_second;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float a = __uint_as_float((e & 1) ? low_words[e / 2] & 0xffff0000u : low_words[e / 2] << 16);
+                const float b = __uint_as_float((e & 1) ? high_words[e / 2] & 0xffff0000u : high_words[e / 2] << 16);
+                out_first.v[e] = round_bf16(a * c.v[e]) - round_bf16(b * s.v[e]);
+                out_second.v[e] = round_bf16(b * c.v[e]) + round_bf16(a * s.v[e]);
+            }
+            store8(target + i, out_first);
+            store8(target + i + half, out_second);
+        }
+    }
+    if (!slot_ok) return;
+    const __nv_bfloat16 *values = row + static_cast<size_t>(rotated) * head_dim;
+    for (int first = lane * 8; first < kv_heads * head_dim; first += 4 * 256) {
+        uint4 held[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (first + u * 256 < kv_heads * head_dim) held[u] = *reinterpret_cast<const uint4 *>(values + first + u * 256);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (first + u * 256 < kv_heads * head_dim) {
+                *reinterpret_cast<uint4 *>(value_cache + cache_row + first + u * 256) = held[u];
+            }
+        }
+    }
+}
+
 // out = bf16(bf16(silu(gate)) * up), the two roundings of activation-then-mul in GatedMlp
 // (singe/src/nn/layers/feed_forward/mod.rs:58-66).  Elementwise: grid (column chunks, rows).
 template <int VEC>
@@ -421,7 +589,17 @@ int singe_add_rms_norm_bf16(singe_stream_t stream, void *hidden, const void *del
     }
     const bool wide = width % 8 == 0 && aligned16(hidden) && aligned16(delta) && aligned16(normed) && aligned16(weight);
     const WarmRange warm = take_pending_warm();
-    if (wide) {
+    // A warp per row from the row count at which the warps fill the machine; below, a CTA per row is done sooner.
+    if (wide && width <= 4096 && rows >= static_cast<size_t>(device_sm_count()) * kRowsPerSm) {
+        const dim3 grid(static_cast<unsigned>((rows + kRowWarps - 1) / kRowWarps));
+        auto kernel = width <= 1024   ? add_rms_norm_rows_kernel<4>
+                      : width <= 2048 ? add_rms_norm_rows_kernel<8>
+                                      : add_rms_norm_rows_kernel<16>;
+        launch_dependent(kernel, grid, dim3(kRowWarps * 32), 0, static_cast<cudaStream_t>(stream), kLaunchGlue, 1,
+                         static_cast<__nv_bfloat16 *>(hidden), static_cast<const __nv_bfloat16 *>(delta),
+                         static_cast<__nv_bfloat16 *>(normed), static_cast<const __nv_bfloat16 *>(weight),
+                         static_cast<int>(rows), static_cast<int>(width), eps, warm);
+    } else if (wide) {
         int threads = static_cast<int>((width / 8 + 31) / 32 * 32);
         if (threads > 512) threads = 512;
         launch_dependent(add_rms_norm_kernel<8>, dim3(static_cast<unsigned>(rows)), dim3(threads), 0,
@@ -478,6 +656,23 @@ static int rotary_cache_write(singe_stream_t stream, void *q_out, const void *qk
         static_cast<int>(kv_heads), static_cast<int>(head_dim), static_cast<long long>(pages),                       \
         static_cast<long long>(page_size), static_cast<long long>(capacity), status, warm, norms)
     const WarmRange warm = take_pending_warm();
+    const size_t lanes = head_dim / 16;
+    if (wide && norms.query == 0 && norms.key == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 &&
+        tokens >= kTokensPerSm * static_cast<size_t>(device_sm_count())) {
+        const dim3 grid(static_cast<unsigned>((tokens + kRowWarps - 1) / kRowWarps));
+#define SINGE_ROTARY_ROWS(Index)                                                                                     \
+    launch_dependent(rotary_rows_kernel<Index>, grid, dim3(kRowWarps * 32), 0, s, kLaunchGlue, 1,                    \
+        static_cast<__nv_bfloat16 *>(q_out), static_cast<const __nv_bfloat16 *>(qkv),                                \
+        static_cast<long long>(qkv_row_stride), static_cast<const __nv_bfloat16 *>(cos_table),                       \
+        static_cast<const __nv_bfloat16 *>(sin_table), static_cast<const Index *>(positions),                        \
+        static_cast<__nv_bfloat16 *>(key_cache), static_cast<__nv_bfloat16 *>(value_cache),                          \
+        static_cast<const Index *>(write_pages), static_cast<const Index *>(write_slots), static_cast<int>(tokens),  \
+        static_cast<int>(heads), static_cast<int>(kv_heads), static_cast<int>(head_dim),                             \
+        static_cast<long long>(pages), static_cast<long long>(page_size), static_cast<long long>(capacity), status, warm)
+        if (index_width == 8) SINGE_ROTARY_ROWS(long long); else SINGE_ROTARY_ROWS(int);
+#undef SINGE_ROTARY_ROWS
+        return launch_status();
+    }
     if (index_width == 8) {
         if (wide) SINGE_ROTARY(long long, 8); else SINGE_ROTARY(long long, 1);
     } else {

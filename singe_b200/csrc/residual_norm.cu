@@ -5,7 +5,9 @@
 // T is the activation and weight type (bf16, or f32 for a decoder run entirely in 32-bit); arithmetic is f32.
 //   layer_norm(x) = (x - mean) / sqrt(mean((x - mean)^2) + eps) * w        (deviations squared, not x^2 - mean^2)
 //   rms_norm(x)   = x / sqrt(mean(x^2) + eps) * w
-// One CTA per row; a row is read once and kept in registers between the passes.
+// One CTA per row, or for prompts one warp; a row is read once and kept in registers between the passes.
+#include <type_traits>
+
 #include "row_pack.cuh"
 
 namespace singe {
@@ -108,6 +110,107 @@ __global__ void __launch_bounds__(kNormThreads)
     for (int h = 0; h < kHeldPacks; ++h) {
         const int c = threadIdx.x * VEC + h * stride;
         if (c < width) store_pack<VEC>(target + c, x[h]);
+    }
+}
+
+// The same for prompts: a warp per row, whose lane stands for the threads lane, lane + 32, ... of the CTA that the kernel
+// above would give the row (WARPS warps, at most four packs a thread), with their sums in their order.  Bound by HBM.  bf16 delta and output, 8192 rows of 2048: 43.9 us a CTA per row, 34.9 now
+// (5.8 TB/s); 17280 of 768: 37.3 and 25.5.  Below about eight rows per SM there is nothing to gain: 1200 rows of 768 take
+// 5.7 and 5.9 us.
+constexpr int kRowsOfCta = 4;
+
+template <typename T, int WARPS>
+__global__ void __launch_bounds__(kRowsOfCta * 32, sizeof(T) == 2 ? 4 : 3)
+    add_layer_norm_rows_kernel(float *residual, const T *delta, long long delta_stride, T *normed, long long normed_stride,
+                               const T *weight, int rows, int width, float eps) {
+    constexpr int kPacks = 4, kStride = WARPS * 32 * 4;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int at = blockIdx.x * kRowsOfCta + (threadIdx.x >> 5);
+    if (at >= rows) return;
+    const int lane4 = (threadIdx.x & 31) * 4;
+    float *row = residual + static_cast<size_t>(at) * width;
+    Pack<4> x[WARPS][kPacks];
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+#pragma unroll
+        for (int h = 0; h < kPacks; ++h) {
+            const int c = w * 128 + lane4 + h * kStride;
+            x[w][h] = Pack<4>{};
+            if (c < width) x[w][h] = load_pack<4>(row + c);
+        }
+    }
+    if (delta != nullptr) {
+        const T *change = delta + at * delta_stride;
+        using Raw = std::conditional_t<sizeof(T) == 2, uint2, float4>;  // kept as it came: half the registers in bf16
+        Raw raw[WARPS][kPacks];
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+#pragma unroll
+            for (int h = 0; h < kPacks; ++h) {
+                const int c = w * 128 + lane4 + h * kStride;
+                if (c < width) raw[w][h] = *reinterpret_cast<const Raw *>(change + c);
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+#pragma unroll
+            for (int h = 0; h < kPacks; ++h) {
+                const int c = w * 128 + lane4 + h * kStride;
+                if (c < width) {
+                    const Pack<4> other = load_pack<4>(reinterpret_cast<const T *>(&raw[w][h]));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[w][h].v[i] += other.v[i];
+                    store_pack<4>(row + c, x[w][h]);
+                }
+            }
+        }
+    }
+    if (normed == nullptr) return;
+    float total = 0.0f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int h = 0; h < kPacks; ++h) {
+            if (w * 128 + lane4 + h * kStride < width) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum += x[w][h].v[i];
+            }
+        }
+        total += warp_sum(sum);
+    }
+    const float mean = total / static_cast<float>(width);
+    total = 0.0f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        float square = 0.0f;
+#pragma unroll
+        for (int h = 0; h < kPacks; ++h) {
+            if (w * 128 + lane4 + h * kStride < width) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    x[w][h].v[i] -= mean;
+                    square = square_chain(square, x[w][h].v[i]);
+                }
+            }
+        }
+        total += warp_sum(square);
+    }
+    const float scale = 1.0f / sqrtf(total / static_cast<float>(width) + eps);
+    T *target = normed + at * normed_stride;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+#pragma unroll
+        for (int h = 0; h < kPacks; ++h) {
+            const int c = w * 128 + lane4 + h * kStride;
+            if (c < width) {
+                const Pack<4> gain = load_pack<4>(weight + c);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[w][h].v[i] = x[w][h].v[i] * scale * gain.v[i];
+                store_pack<4>(target + c, x[w][h]);
+            }
+        }
     }
 }
 
@@ -287,6 +390,20 @@ int add_layer_norm(singe_stream_t stream, float *residual, const void *delta, si
                       aligned_to(delta, 4 * sizeof(T)) && aligned_to(normed, 4 * sizeof(T)) &&
                       aligned_to(weight, 4 * sizeof(T));
     if (!row_fits(width, wide ? 4 : 1)) return SINGE_ERR_UNSUPPORTED_WIDTH;
+    // a warp per row for prompts (the line: see add_layer_norm_rows_kernel)
+    const unsigned warps = norm_threads(width, 4) / 32;
+    if (wide && warps <= 4 && rows >= static_cast<size_t>(device_sm_count()) * 8) {
+        auto kernel = warps == 1   ? add_layer_norm_rows_kernel<T, 1>
+                      : warps == 2 ? add_layer_norm_rows_kernel<T, 2>
+                      : warps == 3 ? add_layer_norm_rows_kernel<T, 3>
+                                   : add_layer_norm_rows_kernel<T, 4>;
+        SINGE_CUDA_TRY(launch_dependent(kernel, dim3(static_cast<unsigned>((rows + kRowsOfCta - 1) / kRowsOfCta)),
+                                        dim3(kRowsOfCta * 32), 0, static_cast<cudaStream_t>(stream), kLaunchGlue, 1, residual,
+                                        static_cast<const T *>(delta), static_cast<long long>(delta_stride),
+                                        static_cast<T *>(normed), static_cast<long long>(normed_stride),
+                                        static_cast<const T *>(weight), static_cast<int>(rows), static_cast<int>(width), eps));
+        return launch_status();
+    }
     auto kernel = wide ? add_layer_norm_kernel<T, 4> : add_layer_norm_kernel<T, 1>;
     SINGE_CUDA_TRY(launch_dependent(kernel, dim3(static_cast<unsigned>(rows)), dim3(norm_threads(width, wide ? 4 : 1)), 0,
                                     static_cast<cudaStream_t>(stream), kLaunchGlue, 1, residual,
