@@ -29,10 +29,10 @@
 //              (S = Q K^T: 8 x tcgen05.mma 128x128x16, both operands K-major in shared memory; O += P V: 8 x
 //              tcgen05.mma with P read from tensor memory and V MN-major), so softmax_A(j) overlaps PV_B(j-1) and
 //              QK_B(j), softmax_B(j) overlaps PV_A(j) and QK_A(j+1).
-//   warps 9,10 TMA producers: both Q tiles once and K tiles, V tiles (128 keys x 128 dims, two SWIZZLE_128B boxes
+//   warps 9,10 TMA producers: both Q tiles once and K tiles, V tiles of paged keys (128 keys x 128 dims, two SWIZZLE_128B boxes
 //              each) into two stages each, released by tcgen05.commit when the MMAs that read them retire.  One warp for
 //              both let the next K tile wait for the last V tile's stage: a lone tile over paged keys took 1.7 us a key
-//              tile and takes 1.3.
+//              tile and takes 1.3.  Ragged keys, two boxes a tile, are 0.6 % faster with one warp.
 // Tensor memory (all 512 columns): S_A/P_A [0,128), S_B/P_B [128,256), O_A [256,384), O_B [384,512).
 // Shared memory: Q_A, Q_B, 2 x K, 2 x V tiles of 32 KB = 192 KB.
 // Under a causal mask tile A sees one key tile less than tile B; CTAs are dispatched heaviest-first.
@@ -677,8 +677,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     bool failed = false;
 
     if (warp >= 9) {
-        // ---------------- TMA producers: warp 9 Q and K, warp 10 V ----------------
-        const bool values = warp == 10;
+        // ---------------- TMA producers: warp 9 Q and K, warp 10 V (ragged keys come in whole boxes: warp 9 alone) ----------------
+        const bool values = PAGED && warp == 10;
         const CUtensorMap *map = values ? &v_map : &k_map;
         const uint32_t tiles_smem = values ? v_smem : k_smem;
         const uint32_t bar_full = values ? bar_v_full : bar_k_full;
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             if (lane == 0) ok = mbar_wait(bar, parity) ? 1 : 0;
             return __shfl_sync(0xffffffffu, ok, 0) != 0;
         };
-        for (int round = 0; !failed; ++round) {
+        for (int round = 0; (PAGED || warp == 9) && !failed; ++round) {
             const int index = item_index(round);
             if (index < 0) break;
             const Item item = decode(index);
@@ -759,13 +759,21 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     }
                     page = coming;
                 } else {
-                    if (elect_one()) {
-                        const int row0 = item.offset_kv + j * kTile;
-                        mbar_expect_tx(bar_full + stage * 8, kLoadBytes);
-                        tma_load_3d(tile, map, bar_full + stage * 8, 0, item.kv_head, row0);
-                        if (kHalves == 2) tma_load_3d(tile + kHalfTileBytes, map, bar_full + stage * 8, 64, item.kv_head, row0);
+                    const int row0 = item.offset_kv + j * kTile;
+                    auto load = [&](uint32_t target, const CUtensorMap *from, uint32_t bar) {
+                        if (elect_one()) {
+                            mbar_expect_tx(bar, kLoadBytes);
+                            tma_load_3d(target, from, bar, 0, item.kv_head, row0);
+                            if (kHalves == 2) tma_load_3d(target + kHalfTileBytes, from, bar, 64, item.kv_head, row0);
+                        }
+                        __syncwarp();
+                    };
+                    load(tile, &k_map, bar_k_full + stage * 8);
+                    if (g >= 2 && !wait_lane0(bar_v_empty + stage * 8, ((g >> 1) - 1) & 1)) {
+                        failed = true;
+                        break;
                     }
-                    __syncwarp();
+                    load(v_smem + stage * kTileBytes, &v_map, bar_v_full + stage * 8);
                 }
             }
         }
