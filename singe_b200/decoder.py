@@ -277,11 +277,18 @@ class PagedDecoder:
         torch = self.torch
         sizes = [len(array) for array in arrays.values()]
         starts = np.cumsum([0] + [(size + 15) // 16 * 16 for size in sizes])
-        packed = torch.empty(int(starts[-1]), dtype=getattr(torch, np.dtype(kind).name), pin_memory=True)
-        host = packed.numpy()
+        # Up to 64 KB the driver takes a copy of ordinary memory before the call returns; allocating pinned memory for each of a
+        # short step's copies would cost it some 20 us apiece.
+        small = int(starts[-1]) * np.dtype(kind).itemsize <= 65536
+        if small:
+            host = np.zeros(int(starts[-1]), dtype=kind)
+            held = torch.from_numpy(host)
+        else:
+            held = torch.empty(int(starts[-1]), dtype=getattr(torch, np.dtype(kind).name), pin_memory=True)
+            host = held.numpy()
         for (start, size), array in zip(zip(starts, sizes), arrays.values()):
             host[start: start + size] = array
-        sent = packed.to("cuda", non_blocking=True)
+        sent = held.to("cuda", non_blocking=True)
         return {name: sent[start: start + size] for name, start, size in zip(arrays, starts, sizes)}
 
     def _refresh_block_table(self) -> None:
