@@ -6,13 +6,15 @@
 // row, the general kernel's way (1.2 - 2.2 TFLOP/s), reads every key and value from L1 once per row and folds each score over
 // the warp; here a CTA takes BM rows of one head, stages 64 keys at a time in shared memory, and a thread owns R rows x 4 keys
 // of the scores and R rows x D/16 columns of the output in registers, so a value read from shared memory feeds R or 4 FMAs.
-// Scores are summed as packed pairs, even and odd dimensions apart.  (Packed value products as well, with every weight stored
+// Scores are summed as packed pairs in four chains, a quarter of the dimensions each, and scaled afterwards: in two chains over a
+// scaled query the error of short rows was up to 1.4 times the general kernel's (1.5e-7 against 1.1e-7; now 1.2e-7, and from 230 keys on
+// below it), at 2 % less time, 14 % for the one form that spills (512 keys of 64: 23.9 us, now 27.3).  (Packed value products as well, with every weight stored
 // twice, cost 3 - 9 % more: the wider reads.)  Thread (ty, tx) owns rows ty, ty + BM/R, ... and keys tx,
 // tx + 16, ...: a row's scores lie in 16 neighbouring lanes, and rows one apart keep the 16-byte reads of a warp on
 // different banks (rows are padded by 16 bytes).
 // Teams of threads walk alternate key tiles, each in buffers of its own, and are folded at the end through shared memory: the
 // chain of key tiles is what a call of few CTAs waits for.
-// 8 heads x 512 causal keys of 64: 377 us -> 22.9; 6 x 1500: 2430 -> 114; 24 x 1500 of 128: 12340 -> 838.
+// 8 heads x 512 causal keys of 64: 417 us -> 27.3; x 900: 1011 -> 46.5; x 1500 of 128: 3367 -> 177.
 // Keys a row does not see take no part at all, whatever their bits are: in tiles that hold hidden keys the value
 // products are predicated, not multiplied by zero.
 #include "common.cuh"
@@ -101,8 +103,7 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
         if (first_row + row < p.query_len && at < p.head_dim) {
             word = *reinterpret_cast<const float4 *>(query + (first_row + row) * p.q_row + at);
         }
-        *reinterpret_cast<float4 *>(q_tile + row * L::kPitch + at) =
-            make_float4(word.x * p.scale, word.y * p.scale, word.z * p.scale, word.w * p.scale);
+        *reinterpret_cast<float4 *>(q_tile + row * L::kPitch + at) = word;
     }
     __syncthreads();
 
@@ -125,12 +126,12 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     for (; key0 < end_key; key0 += G * kKeys) {
         copy_wait<1>();   // the keys; the values may still be on their way
         team_sync();
-        // even and odd dimensions are summed apart, as packed pairs
-        float2 pairs2[R][4];
+        // every fourth dimension is summed apart, as packed pairs
+        float2 pairs2[R][4], others2[R][4];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) pairs2[i][j] = make_float2(0.0f, 0.0f);
+            for (int j = 0; j < 4; ++j) pairs2[i][j] = others2[i][j] = make_float2(0.0f, 0.0f);
         }
 #pragma unroll 4
         for (int d = 0; d < D; d += 4) {
@@ -147,14 +148,14 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
 #pragma unroll
             for (int i = 0; i < R; ++i) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) pairs2[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), pairs2[i][j]);
+                for (int j = 0; j < 4; ++j) others2[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), others2[i][j]);
             }
         }
         float s[R][4];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = pairs2[i][j].x + pairs2[i][j].y;
+            for (int j = 0; j < 4; ++j) s[i][j] = ((pairs2[i][j].x + pairs2[i][j].y) + (others2[i][j].x + others2[i][j].y)) * p.scale;
         }
         team_sync();   // every thread has read the keys
         const bool more = key0 + G * kKeys < end_key;
