@@ -68,6 +68,9 @@ struct GemmParams {
     int rhs_kn;        // 1: rhs is stored [K, N] (transpose_rhs == 0): its tiles are staged N-contiguous and the MMA
                        //    reads them as an MN-major operand; 0: [N, K], K-major (a linear layer's weight)
     uint32_t *error;   // sticky device error word (2 = a bounded wait ran out)
+    int part_blocks;   // k-blocks of one partial sum of K
+    int parts;         // partial sums of K, counted without those that are left no K
+    int chains;        // partial sums that one CTA computes, one after the other, each in an accumulator of its own
     int lhs_km;        // 1: lhs is stored [K, M] (transpose_lhs != 0), staged M-contiguous and read as an MN-major A operand
     WarmRange warm;    // pulled into L2 by the epilogue warps while they have nothing else to do
 };
@@ -163,9 +166,9 @@ template <int BN, int KPS, bool KN, bool AT = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
                      const GemmParams p) {
-    constexpr uint32_t kTmemColumns = 2 * BN < 32 ? 32 : 2 * BN;
     constexpr uint32_t kIdesc = make_instr_desc(kBlockM, BN, true, AT ? 1 : 0, KN ? 1 : 0);  // KN / AT: MN-major reads
     constexpr int kBBytes = BN * 128;
+    const uint32_t tmem_columns = 2 * BN * p.chains;
 
     grid_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         mbar_init_fence();
     }
     if (warp == 1) {
-        tmem_alloc(tmem_holder, kTmemColumns);
+        tmem_alloc(tmem_holder, tmem_columns);
         tmem_relinquish();
     }
     tcgen05_fence_before();
@@ -302,8 +305,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     break;
                 }
                 tcgen05_fence_after();
-                const uint32_t tmem_d = tmem_base + acc * BN;
+                uint32_t tmem_d = tmem_base + acc * p.chains * BN;
+                int within = 0;  // k-block of its partial sum
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
+                    if (within == p.part_blocks) {
+                        within = 0;
+                        tmem_d += BN;
+                    }
                     if (!mbar_wait(bar_full + s * 8, phase)) {
                         failed = true;
                         break;
@@ -319,9 +327,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                         for (int ks = 0; ks < kBlockK / 16; ++ks) {
                             // 16 bf16 of K: 2 descriptor address units along a K-major row, 128 down an MN-major tile
                             umma_ss(tmem_d, a_desc + BWalk<AT>::kStep * ks, b_desc + BWalk<KN>::kStep * ks, kIdesc,
-                                    (kb > 0 || sub > 0 || ks > 0) ? 1u : 0u);
+                                    (within > 0 || sub > 0 || ks > 0) ? 1u : 0u);
                         }
                     }
+                    ++within;
                     tcgen05_commit(bar_empty + s * 8);
                     if (kb == p.k_blocks - 1) tcgen05_commit(bar_acc_full + acc * 8);
                     if (++s == p.stages) {
@@ -350,12 +359,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             }
             tcgen05_fence_after();
             const int row = tm * kBlockM + quarter * 32 + lane;
-            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * p.chains * BN;
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
                 uint32_t r[32];
                 tmem_ld_x32(taddr + c, r);
                 tmem_wait_ld();
+                for (int part = 1; part < p.parts; ++part) {
+                    uint32_t more[32];
+                    tmem_ld_x32(taddr + part * BN + c, more);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(more[j]));
+                }
                 const int col = tn * BN + c;
                 if (p.squared_relu) {
 #pragma unroll
@@ -440,26 +456,29 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     __syncthreads();
     if (warp == 1) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, kTmemColumns);
+        tmem_dealloc(tmem_base, tmem_columns);
     }
 }
 
 // ---- split-K for one-M-tile problems whose N gives too few tiles to fill the machine ----
-// A thread-block cluster of `splits` CTAs owns one N tile; CTA r of the cluster streams K slice r (its own TMA ring,
-// its own accumulator in tensor memory) and pushes each row of its f32 partial tile into the shared memory of the
+// A thread-block cluster of `splits` CTAs owns one N tile; CTA r of the cluster streams K slice r (its own TMA
+// ring, its own accumulators in tensor memory) and pushes each row of its f32 partial tiles into the shared memory of the
 // cluster CTA that owns the row (distributed shared memory stores); after one cluster barrier every CTA sums its
-// rows' partials out of its own shared memory, in split order (so the result does not depend on timing), and stores
-// them.  No workspace in global memory, no atomics, nothing to reset between launches.  A timeline of the earlier
-// form (partials parked locally, owners pulling them with remote loads, a second barrier before leaving) showed
-// 2.2 - 2.6 us in the pull and 0.8 us in the closing barrier of a 10 us kernel.
+// rows' partials out of its own shared memory, in the order of K (so the result does not depend on timing), and stores
+// them.  A CTA's slice is `chains` partial sums of part_blocks k-blocks, each in an accumulator of its own: how K is cut for
+// the sums (see k_parts) is one thing, how many CTAs share the work another.  No workspace in global memory, no atomics,
+// nothing to reset between launches.  A timeline of the earlier form (partials parked locally, owners pulling them with
+// remote loads, a second barrier before leaving) showed 2.2 - 2.6 us in the pull and 0.8 us in the closing barrier of a
+// 10 us kernel.
 template <int BN, int KPS, bool KN>
 __global__ void __launch_bounds__(kSplitKThreads, 1)
     gemm_splitk_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
                        const GemmParams p) {
-    constexpr uint32_t kTmemColumns = BN < 32 ? 32 : BN;
     constexpr uint32_t kIdesc = make_instr_desc(kBlockM, BN, true, 0, KN ? 1 : 0);  // KN: B read MN-major
     constexpr int kBBytes = BN * 128;
     constexpr int kQuads = BN / 4;  // float4 groups per row
+    static_assert(BN >= 32, "the least that tensor memory allocates");
+    const uint32_t tmem_columns = BN * p.chains;
 
     grid_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
@@ -468,11 +487,12 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
     const uint32_t rank = cluster_rank();
     const uint32_t splits = cluster_size();
     const int rows_per_cta = (p.m + static_cast<int>(splits) - 1) / static_cast<int>(splits);
-    // [ring: stages x stage_bytes, its start reused for the parked partial tile][over-read pad]
-    // [receive area: splits x rows_per_cta x BN floats][barriers]
-    const uint32_t slot_bytes = static_cast<uint32_t>(rows_per_cta) * BN * 4;  // one CTA's rows of one split's partial
-    const uint32_t recv = base + max(static_cast<uint32_t>(p.stages * p.stage_bytes), splits * slot_bytes) + p.pad_bytes;
-    const uint32_t bars = recv + splits * slot_bytes;
+    const uint32_t parts = splits * p.chains;
+    // [ring: stages x stage_bytes, its start reused for the parked partial tiles][over-read pad]
+    // [receive area: parts x rows_per_cta x BN floats][barriers]
+    const uint32_t slot_bytes = static_cast<uint32_t>(rows_per_cta) * BN * 4;  // one CTA's rows of one partial
+    const uint32_t recv = base + max(static_cast<uint32_t>(p.stages * p.stage_bytes), parts * slot_bytes) + p.pad_bytes;
+    const uint32_t bars = recv + parts * slot_bytes;
     const uint32_t bar_full = bars;
     const uint32_t bar_empty = bars + kMaxStages * 8;
     const uint32_t bar_acc_full = bars + 2 * kMaxStages * 8;
@@ -484,10 +504,12 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
     const int lane = threadIdx.x & 31;
     const int a_bytes = p.a_rows * 128;
     const int tn = blockIdx.x / splits;
-    const int per_split = (p.k_blocks + splits - 1) / splits;
+    const int per_split = p.chains * p.part_blocks;
     const int kb_first = rank * per_split;
-    const int kb_last = min(kb_first + per_split, p.k_blocks);  // may leave this CTA without work: its partial is zero
+    const int kb_last = min(kb_first + per_split, p.k_blocks);  // may leave this CTA without work, or some of its chains
     const bool has_work = kb_first < kb_last;
+    const int first_part = rank * p.chains;
+    const int own_parts = min(max(p.parts - first_part, 0), p.chains);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -499,7 +521,7 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
         mbar_init_fence();
     }
     if (warp == 1) {
-        tmem_alloc(tmem_holder, kTmemColumns);
+        tmem_alloc(tmem_holder, tmem_columns);
         tmem_relinquish();
     }
     tcgen05_fence_before();
@@ -572,7 +594,13 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
         if (elect_one()) {
             int s = 0;
             uint32_t phase = 0;
+            uint32_t tmem_d = tmem_base;
+            int within = 0;  // k-block of its partial sum
             for (int kb = kb_first; kb < kb_last; ++kb) {
+                if (within == p.part_blocks) {
+                    within = 0;
+                    tmem_d += BN;
+                }
                 if (!mbar_wait(bar_full + s * 8, phase)) {
                     failed = true;
                     break;
@@ -586,10 +614,11 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                         make_smem_desc(stage + KPS * a_bytes + sub * kBBytes, BWalk<KN>::kLeadingBytes, 1024);
 #pragma unroll
                     for (int ks = 0; ks < kBlockK / 16; ++ks) {
-                        umma_ss(tmem_base, a_desc + 2 * ks, b_desc + BWalk<KN>::kStep * ks, kIdesc,
-                                (kb > kb_first || sub > 0 || ks > 0) ? 1u : 0u);
+                        umma_ss(tmem_d, a_desc + 2 * ks, b_desc + BWalk<KN>::kStep * ks, kIdesc,
+                                (within > 0 || sub > 0 || ks > 0) ? 1u : 0u);
                     }
                 }
+                ++within;
                 tcgen05_commit(bar_empty + s * 8);
                 if (kb == kb_last - 1) tcgen05_commit(bar_acc_full);
                 if (++s == p.stages) {
@@ -601,18 +630,17 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
         __syncwarp();
     } else if (warp < 6) {
         // ---------------- hand the partial tile to the CTAs that own its rows ----------------
-        // Row i of the tile belongs to cluster CTA i % splits.  The four warps park the CTA's f32 partial tile in its
-        // own shared memory grouped by owner ([owner][row / splits][BN], 16-byte groups XOR-swizzled by the row so the
+        // Row i of the tile belongs to cluster CTA i % splits.  The four warps park the CTA's f32 partial tiles in its
+        // own shared memory grouped by owner ([owner][chain][row / splits][BN], 16-byte groups XOR-swizzled by the row so the
         // one-row-per-thread writes spread over the banks), then one thread sends each other owner its group with a
-        // single bulk copy into that CTA's receive area (slot = this CTA's rank), completing bytes on the owner's
-        // receive barrier.  An owner waits for the bytes of all live splits and sums its rows out of its own shared
+        // single bulk copy into that CTA's receive area (slot = number of the partial sum), completing bytes on the owner's
+        // receive barrier.  An owner waits for the bytes of all live partials and sums its rows out of its own shared
         // memory: no thread ever waits for a remote load.  (Stores of one row per thread straight into the owners'
         // shared memory took 1.6 us for 24 KB per CTA: 4096 separate 16-byte transfers.)
         if (warp == 2) warm_l2(p.warm, blockIdx.x, gridDim.x, lane);
         grid_dependency_wait();  // these warps store the output: not while an earlier kernel may still read it
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
-        const int live = min(static_cast<int>(splits), (p.k_blocks + per_split - 1) / per_split);
         if (has_work && !__all_sync(0xffffffffu, mbar_wait(bar_acc_full, 0) ? 1 : 0)) failed = true;
         tcgen05_fence_after();
         if (has_work && !failed) {
@@ -620,17 +648,18 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
             const int owner = row % static_cast<int>(splits);
             const int local_row = row / static_cast<int>(splits);
             float *mine = reinterpret_cast<float *>(smem_raw + (base - raw)) +
-                          (static_cast<size_t>(owner) * rows_per_cta + local_row) * BN;
+                          (static_cast<size_t>(owner) * p.chains * rows_per_cta + local_row) * BN;
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
+            for (int c = 0; c < own_parts * BN; c += 32) {
                 uint32_t r[32];
                 tmem_ld_x32(taddr + c, r);
                 tmem_wait_ld();
                 if (row < p.m) {
+                    float *chain = mine + static_cast<size_t>(c / BN) * rows_per_cta * BN;
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
-                        const int quad = ((c + j) >> 2) ^ (row & (kQuads - 1));
-                        *reinterpret_cast<float4 *>(mine + quad * 4) =
+                        const int quad = ((c % BN + j) >> 2) ^ (row & (kQuads - 1));
+                        *reinterpret_cast<float4 *>(chain + quad * 4) =
                             make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
                                         __uint_as_float(r[j + 3]));
                     }
@@ -638,22 +667,21 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
             }
             fence_proxy_async_shared();  // the bulk copies below read what these threads wrote
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps: the whole tile is parked
+        asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps: all is parked
         if (threadIdx.x == 64) {
-            // bytes this CTA will receive: one slot from every other live split
-            const int senders = live - (static_cast<int>(rank) < live ? 1 : 0);
-            mbar_expect_tx(bar_recv, static_cast<uint32_t>(senders) * slot_bytes);
+            // bytes this CTA will receive: one slot for every live partial of the others
+            mbar_expect_tx(bar_recv, static_cast<uint32_t>(p.parts - own_parts) * slot_bytes);
             if (has_work && !failed) {
                 for (uint32_t o = 0; o < splits; ++o) {
                     if (o == rank) continue;
                     uint32_t remote_slot, remote_bar;
                     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
                                  : "=r"(remote_slot)
-                                 : "r"(recv + rank * slot_bytes), "r"(o));
+                                 : "r"(recv + rank * p.chains * slot_bytes), "r"(o));
                     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_bar) : "r"(bar_recv), "r"(o));
                     asm volatile(
                         "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                        ::"r"(remote_slot), "r"(base + o * slot_bytes), "r"(slot_bytes), "r"(remote_bar)
+                        ::"r"(remote_slot), "r"(base + o * p.chains * slot_bytes), "r"(own_parts * slot_bytes), "r"(remote_bar)
                         : "memory");
                 }
             }
@@ -672,7 +700,6 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
         if (warp < 2 || warp >= 6) grid_dependency_wait();  // (warps 2-5 did before they parked the tile)
         const int t = threadIdx.x;
         const int my_rows = (p.m - static_cast<int>(rank) + static_cast<int>(splits) - 1) / static_cast<int>(splits);
-        const int live = min(static_cast<int>(splits), (p.k_blocks + per_split - 1) / per_split);
         const float *received = reinterpret_cast<const float *>(smem_raw + (recv - raw));
         const float *parked = reinterpret_cast<const float *>(smem_raw + (base - raw));
         const int slot_floats = rows_per_cta * BN;
@@ -691,10 +718,9 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                 const int at = local_row * BN + ((quad ^ (row & (kQuads - 1))) << 2);
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
-                    if (index < items && s < live) {
-                        // this CTA's own partial never left its parked tile (group `rank` there)
-                        const float *from = s == static_cast<int>(rank) ? parked + rank * slot_floats
-                                                                         : received + s * slot_floats;
+                    if (index < items && s < p.parts) {
+                        // this CTA's own partials never left its parked tiles (group `rank` there): number s lies at place s
+                        const float *from = (s >= first_part && s < first_part + p.chains ? parked : received) + s * slot_floats;
                         part[u][s] = *reinterpret_cast<const float4 *>(from + at);
                     }
                 }
@@ -708,11 +734,10 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
                 const int quad = index % kQuads;
                 const int col = tn * BN + quad * 4;
                 if (col >= p.n) continue;
-                float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (live > 0) sum = part[u][0];
+                float4 sum = part[u][0];
 #pragma unroll
-                for (int s = 1; s < 8; ++s) {  // split order: the result does not depend on timing
-                    if (s < live) {
+                for (int s = 1; s < 8; ++s) {  // the order of K: the result does not depend on timing
+                    if (s < p.parts) {
                         sum.x += part[u][s].x;
                         sum.y += part[u][s].y;
                         sum.z += part[u][s].z;
@@ -765,7 +790,7 @@ __global__ void __launch_bounds__(kSplitKThreads, 1)
     __syncthreads();
     if (warp == 1) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, kTmemColumns);
+        tmem_dealloc(tmem_base, tmem_columns);
     }
 }
 
@@ -800,26 +825,49 @@ int prefetch_blocks_for(const GemmParams &params, int block_b_bytes) {
     return kb * 1024 / block_b_bytes;
 }
 
+// How many partial sums the K of a one-M-tile problem is cut into.  It decides the accuracy of the result, and nothing of how the
+// work is shared out may change it: the tensor core's accumulators drop what does not fit as they go, so the error of a sum grows
+// with its length.  Against 64 bits, f32 results of (M, N, K) = (64, 6144, 4096): one sum 4.4e-6, two 2.1e-6; (64, 4096, 4096):
+// two 2.1e-6, four 1.0e-6; (64, 2304, 2048): one 2.1e-6, two 1.0e-6, four 4.7e-7.
+int k_parts(int k, int tiles_128, int sms) {
+    int parts = 1;
+    while (parts < 4 && tiles_128 * parts * 2 <= sms) parts <<= 1;
+    if (parts == 4 && tiles_128 * 4 <= sms / 3) parts = 8;
+    const int k_stages = (k + 2 * kBlockK - 1) / (2 * kBlockK);
+    while (parts > 1 && k_stages / parts < 3) parts >>= 1;
+    return parts;
+}
+
+// k-blocks of `slices` 64-wide slices in one of `parts` partial sums, which are pairs of slices whatever a block is.
+int part_blocks(int k, int parts, int slices) {
+    const int pairs = (k + 2 * kBlockK - 1) / (2 * kBlockK);
+    return ((pairs + parts - 1) / parts * 2 + slices - 1) / slices;
+}
+
 template <int BN, int KPS>
 int launch_gemm_splitk(cudaStream_t stream, GemmParams params, const void *lhs, const void *rhs,
-                       size_t lhs_row_stride, size_t rhs_row_stride, int splits) {
+                       size_t lhs_row_stride, size_t rhs_row_stride, int splits, int chains) {
     const int kSmemLimit = shared_limit(params);
     const int b_bytes = BN * 128;
     params.stage_bytes = KPS * (params.a_rows * 128 + b_bytes);
     params.k_blocks = (params.k + kBlockK * KPS - 1) / (kBlockK * KPS);
     params.prefetch_blocks = prefetch_blocks_for(params, KPS * b_bytes);
-    const int per_split = (params.k_blocks + splits - 1) / splits;
+    params.chains = chains;
+    params.part_blocks = part_blocks(params.k, splits * chains, KPS);
+    params.parts = (params.k_blocks + params.part_blocks - 1) / params.part_blocks;
+    const int per_split = chains * params.part_blocks;
     params.pad_bytes = over_read_pad(params.a_rows, KPS * b_bytes);
-    const int receive = splits * ((params.m + splits - 1) / splits) * BN * 4;  // every split's partial of the CTA's rows
-    const int fixed = params.pad_bytes + receive + 2 * kMaxStages * 8 + 64 + 1024;
-    // (the ring is at least as large as the parked tile, which reuses it: checked below)
+    // every partial of the rows a CTA owns, received; as much is parked
+    const int parked = splits * chains * ((params.m + splits - 1) / splits) * BN * 4;
+    const int fixed = params.pad_bytes + parked + 2 * kMaxStages * 8 + 64 + 1024;
+    // (the ring is at least as large as the parked tiles, which reuse it: checked below)
     int stages = (kSmemLimit - fixed) / params.stage_bytes;
     if (stages > kMaxStages) stages = kMaxStages;
     if (stages > per_split + 1 && per_split + 1 >= 2) stages = per_split + 1;
     if (stages < 2) stages = 2;  // the limit is a preference; two stages is the least the pipeline runs with
     params.stages = stages;
     params.tiles_n = (params.n + BN - 1) / BN;
-    const int ring = stages * params.stage_bytes > receive ? stages * params.stage_bytes : receive;
+    const int ring = stages * params.stage_bytes > parked ? stages * params.stage_bytes : parked;
     const int smem = ring + fixed;
     if (smem > 227 * 1024) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
     // [K, N] right operands are staged in boxes of 64 columns: those kernels exist from 64-wide tiles up
@@ -867,11 +915,14 @@ int launch_gemm_splitk(cudaStream_t stream, GemmParams params, const void *lhs, 
 
 template <int BN, int KPS, bool AT = false>
 int launch_gemm(cudaStream_t stream, GemmParams params, const void *lhs, const void *rhs, size_t lhs_row_stride,
-                size_t rhs_row_stride) {
+                size_t rhs_row_stride, int chains = 1) {
     const int kSmemLimit = shared_limit(params);
     const int b_bytes = BN * 128;
     params.stage_bytes = KPS * (params.a_rows * 128 + b_bytes);
     params.k_blocks = (params.k + kBlockK * KPS - 1) / (kBlockK * KPS);
+    params.chains = chains;
+    params.part_blocks = chains > 1 ? part_blocks(params.k, chains, KPS) : params.k_blocks;
+    params.parts = (params.k_blocks + params.part_blocks - 1) / params.part_blocks;
     params.prefetch_blocks = prefetch_blocks_for(params, KPS * b_bytes);
     params.pad_bytes = over_read_pad(params.a_rows, KPS * b_bytes);
     const int fixed = params.pad_bytes + 2 * kMaxStages * 8 + 64 + 1024;
@@ -1124,22 +1175,24 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
             while (slices > 1 && slices * slice_bytes * 2 > 200 * 1024) slices >>= 1;
         }
     }
-    // One M tile and too few 128-wide N tiles for the machine: tiles of 64 or 128 columns, K split over clusters of up to
-    // four CTAs; whichever fills most of the machine in one wave.  Clusters of four are kept to 128 CTAs, what
-    // the GPCs hold at once (2304 x 2048: 36 clusters of four take 12.9 us, 36 of two 8.9); 8 splits pay only where four leave two thirds of
-    // the SMs idle; a split needs at least three stages of K to amortise its fill and the reduction.  Where narrow tiles
-    // and twice the splits tie, the narrow ones cost less to reduce and the wide ones stream a long K in longer runs:
-    // measured on B200, M = 128, (N, K) = (8192, 2048): 64 columns unsplit 10.3 us, 128 in two splits 12.7;
-    // (4096, 4096): 64 in two 12.0, 128 in four 13.2; (4096, 14336): 28.0 and 26.9.  M = 16: 9.3 / 10.2, 10.7 / 10.4,
-    // 23.3 / 23.3.  One stage of two slices or (M > 64, few stages) more stages of one: 4 x 128 at M = 128, K = 14336 31.7 and 26.9.
+    // One M tile and too few 128-wide N tiles for the machine: tiles of 64 or 128 columns, the partial sums of K (see k_parts)
+    // shared out over clusters of up to four CTAs; whichever fills most of the machine in one wave.  Clusters of four are
+    // kept to 128 CTAs, what the GPCs hold at once (4608 x 2048, M = 16: 36 clusters of four, 128 wide, take 12.5 us, 72 of two,
+    // 64 wide, 8.7); 8 splits of narrow tiles pay only where four leave two thirds of the SMs idle.
+    // Two partial sums in one CTA without a cluster are added in registers: (8192, 2048), two splits of 128 columns and 64
+    // unsplit, M = 16: 10.0 and 9.2 us, M = 128: 12.6 and 9.8; (6144, 4096): 12.9 and 12.9, 16.4 and 16.1; where K is long and
+    // rows are few the wide ones stream it in longer runs.  In a cluster they are parked and sent one by one: a CTA for every
+    // sum, with tiles twice as wide, does as well and mostly better, (2304, 2048), M = 1: 5.8 us against 6.8, M = 64: 7.1 and 7.4,
+    // M = 128: 9.0 and 9.0; (4096, 4096), M = 128: 13.1 and 13.5.
     int splits = 1;
     const int forced_splits = g_tuning_splits.load(std::memory_order_relaxed);
     const int forced_block_n = g_tuning_block_n.load(std::memory_order_relaxed);
     const int forced_slices = g_tuning_slices.load(std::memory_order_relaxed);
     const bool splittable = params.m <= kBlockM && params.batch == 1 && params.row_gate == nullptr && !params.lhs_km;
+    int chains = 1;
     if (splittable && tiles(128) < (sms * 2) / 3) {
-        const int k_stages = (params.k + 2 * kBlockK - 1) / (2 * kBlockK);
         const bool few_splits = params.k <= 2048 || (params.m >= 64 && params.k <= 8192);
+        const int parts = forced_splits == 1 ? 1 : k_parts(params.k, tiles(128), sms);
         int wide = 0;
         int most = 0;
         for (int i = 0; i < 6; ++i) {
@@ -1147,24 +1200,35 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
             const int s = 1 << (i / 2);
             const int candidate = i % 2 == 0 ? 64 : 128;
             const int ctas = s * tiles(candidate);
-            if (ctas > (s == 4 ? 128 : sms) || (s > 1 && (k_stages / s < 3 || forced_splits == 1))) continue;
+            if (ctas > (s == 4 ? 128 : sms) || s > parts) continue;
             if (ctas > most || (ctas == most && s > splits && !few_splits)) {
                 most = ctas;
                 wide = candidate;
                 splits = s;
             }
         }
-        if (splits == 4 && wide == 64 && most <= sms / 3 && k_stages / 8 >= 3) splits = 8;
-        if (most > 0 && (splits > 1 || wide == 128 || tiles(32) > sms)) {
+        if (splits == 4 && wide == 64 && most <= sms / 3 && parts == 8) splits = 8;
+        if (splits > 1 && parts == 2 * splits && parts * tiles(128) >= most && parts * tiles(128) <= 128) {
+            wide = 128;
+            splits = parts;
+        }
+        chains = parts / splits;
+        if (most > 0 && (parts > 1 || wide == 128 || tiles(32) > sms)) {
             bn = wide;
-            const int receive = splits > 1 ? splits * ((params.m + splits - 1) / splits) * bn * 4 : 0;
+            const int receive = splits > 1 ? parts * ((params.m + splits - 1) / splits) * bn * 4 : 0;
             slices = bn == 64 ? 4 : 2;
-            while (slices > 1 && (shared_limit(params) - 2048 - receive) / (slices * (a_rows + bn) * 128) < (splits > 1 ? 5 : 4)) {
+            while (slices > 1 && (shared_limit(params) - 2048 - receive) / (slices * (a_rows + bn) * 128) < (parts > 1 ? 5 : 4)) {
                 slices >>= 1;
             }
+            if (slices == 4 && part_blocks(params.k, parts, 1) % 4 != 0) slices = 2;
         }
     } else if (splittable && tiles(128) >= (sms * 2) / 3 && a_rows == kBlockM) {
         slices = 1;  // three stages of two slices against seven of one: (28672, 4096) 52.2 and 51.5 us, (14336, 4096) 26.6 and 25.8
+    }
+    if (forced_block_n != 0 || forced_slices != 0 || forced_splits != 0) {
+        // explicit tuning: a CTA for every partial sum
+        splits *= chains;
+        chains = 1;
     }
     if (forced_splits != 0 && params.batch == 1) {
         splits = forced_splits;
@@ -1196,7 +1260,7 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
         if (params.m > kBlockM || (splits != 2 && splits != 4 && splits != 8)) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
 #define SINGE_SPLITK_CASE(BN_, KPS_)                                                                             \
     if (bn == BN_ && slices == KPS_)                                                                             \
-        return launch_gemm_splitk<BN_, KPS_>(stream, params, lhs, rhs, lhs_row_stride, rhs_row_stride, splits);
+        return launch_gemm_splitk<BN_, KPS_>(stream, params, lhs, rhs, lhs_row_stride, rhs_row_stride, splits, chains);
         SINGE_SPLITK_CASE(128, 2)
         SINGE_SPLITK_CASE(128, 1)
         SINGE_SPLITK_CASE(64, 1)
@@ -1219,7 +1283,7 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
     }
 #define SINGE_GEMM_CASE(BN_, KPS_)                                                                    \
     if (bn == BN_ && slices == KPS_)                                                                  \
-        return launch_gemm<BN_, KPS_>(stream, params, lhs, rhs, lhs_row_stride, rhs_row_stride);
+        return launch_gemm<BN_, KPS_>(stream, params, lhs, rhs, lhs_row_stride, rhs_row_stride, chains);
     SINGE_GEMM_CASE(256, 1)
     SINGE_GEMM_CASE(128, 1)
     SINGE_GEMM_CASE(128, 2)

@@ -96,3 +96,25 @@ def test_one_row_tile(m, n, k):
     assert ops.take_device_error() == 0
     _check(out, exact, bound, "bf16")
     assert torch.equal(gated_odd[:, : n // 2], gated) and bool(gated_odd[:, n // 2:].isnan().all())
+
+
+@pytest.mark.parametrize("m,n,k,parts", [(64, 6144, 4096, 2), (128, 6144, 4096, 2), (64, 4096, 4096, 4), (128, 4096, 4096, 4),
+                                         (1, 8192, 2048, 2), (128, 8192, 2048, 2), (1, 4608, 2048, 4), (100, 2304, 2048, 4),
+                                         (16, 768, 4096, 8), (96, 1400, 4096, 8), (64, 8200, 1000, 2), (33, 4100, 1544, 4),
+                                         (128, 9600, 4096, 1)])
+def test_partial_sums_of_one_row_tile(m, n, k, parts):
+    # K is cut for the sums by N and K alone, however the work is shared out: the bits are those of one CTA for every partial sum
+    x, w, exact, bound = _inputs(m, n, k)
+    got = []
+    for splits in (0, parts):
+        assert ks.lib().singe_matmul_set_splits(splits) == ks.OK
+        try:
+            out = torch.full((m, n), float("nan"), device="cuda")
+            ops.matmul_bf16(out, x, w, ops.MatmulConfig.row_major_transposed_rhs(m, n, k))
+            got.append(out)
+        finally:
+            assert ks.lib().singe_matmul_set_splits(0) == ks.OK
+    torch.cuda.synchronize()
+    assert ops.take_device_error() == 0
+    _check(got[0], exact, bound, "f32")
+    assert torch.equal(*got)
