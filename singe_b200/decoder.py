@@ -24,14 +24,16 @@ class PageTableError(ValueError):
 
 
 def token_array(tokens) -> np.ndarray:
-    """Token ids as int64, whatever sequence of integers they come in."""
+    """Token ids as int64, whatever integers they come as: what ``int()`` makes of each, and what it refuses is refused."""
+    if not hasattr(tokens, "__len__"):
+        tokens = list(tokens)
     try:
-        array = np.array(tokens, dtype=np.int64)
-        if array.ndim == 1:
-            return array
-    except (TypeError, ValueError):
+        array = np.asarray(tokens)
+        if array.ndim == 1 and array.dtype.kind in "iub" and np.can_cast(array.dtype, np.int64):
+            return array.astype(np.int64)
+    except (TypeError, ValueError, RuntimeError, OverflowError):
         pass
-    return np.fromiter(map(int, tokens), dtype=np.int64, count=len(tokens))
+    return np.asarray([int(token) for token in tokens], dtype=np.int64)
 
 
 @dataclass

@@ -1,8 +1,11 @@
 """The step's arrays against a restatement that places one token at a time."""
+import itertools
 import random
+import warnings
 
 import numpy as np
 import pytest
+import torch
 
 from singe_b200.decoder import PageTable, PageTableError, token_array
 
@@ -61,3 +64,23 @@ def test_token_ids_come_in_any_sequence_of_integers():
     assert token_array([]).tolist() == []
     with pytest.raises((TypeError, ValueError)):
         token_array([None])
+
+
+@pytest.mark.parametrize("tokens", [
+    (v for v in (3, 1)), iter([7]), map(int, "12"), range(4), (5, 6), {9}, [], "34", ["8"], [True, 2], [1.9, -2.9], [np.int32(3), 4],
+    np.asarray([1.5, 2.5]), np.asarray([7], dtype=np.uint64), np.asarray(["6"]), torch.tensor([1, 2]), torch.tensor([2.5]),
+    [torch.tensor(4), torch.tensor(5)], [2 ** 62]], ids=lambda tokens: type(tokens).__name__)
+def test_what_counts_as_tokens(tokens):
+    tokens = tokens if hasattr(tokens, "__len__") else iter(list(tokens))
+    first, second = (tokens, tokens) if hasattr(tokens, "__len__") else itertools.tee(tokens)
+    array = token_array(first)
+    assert array.dtype == np.int64 and array.tolist() == [int(v) for v in second]
+
+
+@pytest.mark.parametrize("tokens", [
+    [float("nan")], np.asarray([float("nan")]), np.asarray([float("inf")]), [float("inf")], np.asarray([2 ** 63], dtype=np.uint64), [2 ** 63],
+    [[1, 2]], [None], ["a"], torch.tensor([float("nan")]), np.zeros((2, 2))], ids=repr)
+def test_what_is_no_token_is_refused(tokens):
+    with pytest.raises((TypeError, ValueError, OverflowError)), warnings.catch_warnings():
+        warnings.simplefilter("error")
+        token_array(tokens)
