@@ -294,18 +294,19 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     for (int i = 0; i < R; ++i) {
         const int row = first_row + ty + i * L::kRows;
         if (row >= p.query_len) continue;
-        const bool empty = end[i] <= begin[i] && p.sinks == nullptr;
-        const float inverse = empty ? 0.0f : 1.0f / sum[i];
+        const bool unseen = end[i] <= begin[i];   // no key: nothing is weighed, and the log sum is that of the sink, whatever it is
+        const float inverse = 1.0f / sum[i];
         float *to = p.out + batch * p.q_batch + head * p.q_head + row * p.q_row;
 #pragma unroll
         for (int c = 0; c < kColumns; ++c) {
             if (c * 64 + tx * 4 < p.head_dim) {
                 *reinterpret_cast<float4 *>(to + c * 64 + tx * 4) =
-                    make_float4(out[i][c].x * inverse, out[i][c].y * inverse, out[i][c].z * inverse, out[i][c].w * inverse);
+                    unseen ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
+                           : make_float4(out[i][c].x * inverse, out[i][c].y * inverse, out[i][c].z * inverse, out[i][c].w * inverse);
             }
         }
         if (p.lse != nullptr && tx == 0) {
-            p.lse[(batch * p.heads + head) * p.query_len + row] = empty ? -INFINITY : top[i] + logf(sum[i]);
+            p.lse[(batch * p.heads + head) * p.query_len + row] = unseen ? sink : top[i] + logf(sum[i]);
         }
     }
 }

@@ -54,3 +54,16 @@ def test_dense_f32_lse_and_what_hidden_keys_hold():
     call(again, lse_again)
     assert torch.equal(again[:, :100], out[:, :100]) and torch.equal(lse_again[:, :, :100], lse[:, :, :100])
     assert again[:, 102:].isnan().any(-1).all()
+
+
+@pytest.mark.parametrize("l", [15, 16, 40, 300])       # one warp per row, and tiles
+@pytest.mark.parametrize("b,d", [(1, 64), (1, 128), (120, 64), (120, 128)])   # two and four teams of threads, two and one
+def test_dense_f32_sinks_that_are_not_finite(l, b, d):
+    rng = np.random.default_rng(l)
+    s, window, h = l - 12, 5, 4                        # the last seven rows see no key
+    q, k, v = (dev(rng.standard_normal((b, h, n, d), dtype=np.float32)) for n in (l, s, s))
+    sinks = torch.tensor([float("-inf"), 0.5, float("inf"), float("nan")], device="cuda")
+    out = attend(q, k, v, 0.125, False, window, 0.0, sinks)
+    assert not out[:, :, s + window - 1:].any()        # zero for every sink: nothing is weighed, whatever the sum is
+    assert torch.equal(out[:, 0], attend(q, k, v, 0.125, False, window)[:, 0])
+    assert out[:, :2].isfinite().all() and out[:, 2:, : s + window - 1].isnan().all()
