@@ -24,7 +24,11 @@ namespace singe {
 
 namespace {
 
-constexpr int kKeys = 64;   // keys of a tile
+constexpr int kKeys = 64;      // keys of a tile
+constexpr int kMostTeams = 4;
+// Positions are ints: a walk may compute places up to a step of every team and a tile past the last key, and start where the
+// window of the last row does.
+constexpr int kMostPositions = 0x7fffffff - (kMostTeams + 1) * kKeys;
 
 __device__ __forceinline__ void copy_16(float *dst, const float *src, bool real) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(real ? 16 : 0) : "memory");
@@ -42,6 +46,7 @@ struct Layout {
     static constexpr int kWeightPitch = kKeys + 4;
     static constexpr int kTeamFloats = kKeys * kPitch + kKeys * D + BM * kWeightPitch;
     static constexpr int kFloats = BM * kPitch + G * kTeamFloats;
+    static_assert(G <= kMostTeams && BM <= kKeys, "see kMostPositions");
     static_assert(G == 1 || kTeam * (R * D / 16 + 2 * R) <= kTeamFloats, "the fold reuses a team's buffers");
 };
 
@@ -330,7 +335,7 @@ bool dense_attention_f32_takes(const DenseF32 &p, size_t batch) {
                           reinterpret_cast<uintptr_t>(p.value) | reinterpret_cast<uintptr_t>(p.out);
     const size_t blocks = batch * static_cast<size_t>(p.heads) * ((static_cast<size_t>(p.query_len) + 31) / 32);
     return p.head_dim % 4 == 0 && p.head_dim <= 128 && p.query_len >= kDenseF32LeastRows && (all & 15u) == 0 &&
-           blocks <= 0x7fffffffull && p.key_len <= 0x7fffffff - 2 * kKeys;
+           blocks <= 0x7fffffffull && p.query_len <= kMostPositions && p.key_len <= kMostPositions;
 }
 
 int dense_attention_f32(cudaStream_t stream, const DenseF32 &p, size_t batch) {
