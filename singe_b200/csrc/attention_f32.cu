@@ -6,15 +6,18 @@
 // row, the general kernel's way (1.2 - 2.2 TFLOP/s), reads every key and value from L1 once per row and folds each score over
 // the warp; here a CTA takes BM rows of one head, stages 64 keys at a time in shared memory, and a thread owns R rows x 4 keys
 // of the scores and R rows x D/16 columns of the output in registers, so a value read from shared memory feeds R or 4 FMAs.
-// Scores are summed as packed pairs in four chains, a quarter of the dimensions each, and scaled afterwards: in two chains over a
-// scaled query the error of short rows was up to 1.4 times the general kernel's (1.5e-7 against 1.1e-7; now 1.2e-7, and from 230 keys on
-// below it), at 2 % less time, 14 % for the one form that spills (512 keys of 64: 23.9 us, now 27.3).  (Packed value products as well, with every weight stored
+// The error of a sum grows with the length of its chains, and one warp per row has short ones (D / 32 products a lane, then a
+// tree).  So eight dimensions are summed as packed pairs, four such blocks are added, and groups of 32 dimensions pairwise; the
+// scale is applied by the FMA that takes a score's distance from the row's base.  Against 64 bits, 128 heads of 128 columns
+// over 16, 40 and 100 causal keys, in units of the general kernel's error: 1.00, 0.99, 0.95 (64 columns 0.99, 0.98, 0.94); four
+// chains of a quarter of the dimensions each, scaled afterwards: 1.19, 1.17, 1.11.  They took 4 % less time, but 8 % more in the
+// form of four teams, where their registers spilled.  (Packed value products as well, with every weight stored
 // twice, cost 3 - 9 % more: the wider reads.)  Thread (ty, tx) owns rows ty, ty + BM/R, ... and keys tx,
 // tx + 16, ...: a row's scores lie in 16 neighbouring lanes, and rows one apart keep the 16-byte reads of a warp on
 // different banks (rows are padded by 16 bytes).
 // Teams of threads walk alternate key tiles, each in buffers of its own, and are folded at the end through shared memory: the
 // chain of key tiles is what a call of few CTAs waits for.
-// 8 heads x 512 causal keys of 64: 417 us -> 27.3; x 900: 1011 -> 46.5; x 1500 of 128: 3367 -> 177.
+// 8 heads x 512 causal keys of 64: 417 us -> 24.1; x 900: 1011 -> 41.7; x 1500 of 128: 3367 -> 182.
 // Keys a row does not see take no part at all, whatever their bits are: in tiles that hold hidden keys the value
 // products are predicated, not multiplied by zero.
 #include "common.cuh"
@@ -54,6 +57,7 @@ template <int D, int R, int BM, int G>
 __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(const DenseF32 p, const int row_tiles) {
     using L = Layout<D, R, BM, G>;
     constexpr int kColumns = D / 64;   // float4 groups of output columns a thread owns
+    constexpr int kBlock = 8, kGroup = 32;   // dimensions that are summed in a row, and apart from the others
     grid_launch_dependents();
     extern __shared__ __align__(16) float shared[];
     const int team = threadIdx.x / L::kTeam;
@@ -128,39 +132,80 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
         for (int c = 0; c < kColumns; ++c) out[i][c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 
+    // A score is s * unit, rounded only together with the base it is weighed against.
+    const float unit = p.softcap > 0.0f || p.scale == 0.0f ? 1.0f : p.scale;
+    const float hidden = unit < 0.0f ? INFINITY : -INFINITY;
     for (; key0 < end_key; key0 += G * kKeys) {
         copy_wait<1>();   // the keys; the values may still be on their way
         team_sync();
-        // every fourth dimension is summed apart, as packed pairs
-        float2 pairs2[R][4], others2[R][4];
+        // Even and odd dimensions are summed apart, as packed pairs, kBlock dimensions in a row; then the blocks of a group,
+        // then the groups, two and two.
+        float s[R][4], two[R][4];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) pairs2[i][j] = others2[i][j] = make_float2(0.0f, 0.0f);
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
         }
-#pragma unroll 4
-        for (int d = 0; d < D; d += 4) {
-            float4 a[R], b[4];
+#pragma unroll 1
+        for (int group = 0; group < D; group += kGroup) {
+            // (in narrow heads, where threads have 128 registers, a pair is folded at the end of its block)
+            std::conditional_t<D == 64, float, float2> total[R][4];
 #pragma unroll
-            for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4 *>(q_tile + (ty + i * L::kRows) * L::kPitch + d);
+            for (int first = 0; first < kGroup; first += kBlock) {
+                float2 part[R][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(k_tile + (tx + 16 * j) * L::kPitch + d);
+                for (int i = 0; i < R; ++i) {
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
+                    for (int j = 0; j < 4; ++j) part[i][j] = make_float2(0.0f, 0.0f);
+                }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) pairs2[i][j] = __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), pairs2[i][j]);
+                for (int d = 0; d < kBlock; d += 4) {
+                    const int at = group + first + d;
+                    float4 a[R], b[4];
+#pragma unroll
+                    for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4 *>(q_tile + (ty + i * L::kRows) * L::kPitch + at);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(k_tile + (tx + 16 * j) * L::kPitch + at);
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) part[i][j] = __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), part[i][j]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) part[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), part[i][j]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if constexpr (D == 64) {
+                            const float sum_of_block = part[i][j].x + part[i][j].y;
+                            total[i][j] = first == 0 ? sum_of_block : total[i][j] + sum_of_block;
+                        } else {
+                            total[i][j] = first == 0 ? part[i][j] : __fadd2_rn(total[i][j], part[i][j]);
+                        }
+                    }
+                }
             }
 #pragma unroll
             for (int i = 0; i < R; ++i) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) others2[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), others2[i][j]);
+                for (int j = 0; j < 4; ++j) {
+                    if constexpr (D == 64) {
+                        s[i][j] += total[i][j];
+                    } else {
+                        const float sum_of_group = total[i][j].x + total[i][j].y;
+                        if (group % (2 * kGroup) == 0) {
+                            two[i][j] = sum_of_group;
+                        } else {
+                            s[i][j] += two[i][j] + sum_of_group;
+                        }
+                    }
+                }
             }
-        }
-        float s[R][4];
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = ((pairs2[i][j].x + pairs2[i][j].y) + (others2[i][j].x + others2[i][j].y)) * p.scale;
         }
         team_sync();   // every thread has read the keys
         const bool more = key0 + G * kKeys < end_key;
@@ -175,16 +220,19 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
         for (int i = 0; i < R; ++i) {
             if (p.softcap > 0.0f) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = p.softcap * tanhf(s[i][j] / p.softcap);
+                for (int j = 0; j < 4; ++j) s[i][j] = p.softcap * tanhf(s[i][j] * p.scale / p.softcap);
+            } else if (p.scale == 0.0f) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] *= 0.0f;
             }
             if (!whole) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int key = key0 + tx + 16 * j;
-                    if (key < begin[i] || key >= end[i]) s[i][j] = -INFINITY;
+                    if (key < begin[i] || key >= end[i]) s[i][j] = hidden;
                 }
             }
-            float most = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+            float most = fmaxf(fmaxf(s[i][0] * unit, s[i][1] * unit), fmaxf(s[i][2] * unit, s[i][3] * unit));
 #pragma unroll
             for (int offset = 8; offset > 0; offset >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, offset));
             most = fmaxf(most, top[i]);
@@ -194,7 +242,7 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
             sum[i] *= factor;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float weight = expf(s[i][j] - base);
+                const float weight = expf(fmaf(s[i][j], unit, -base));
                 sum[i] += weight;
                 weights[(ty + i * L::kRows) * L::kWeightPitch + tx + 16 * j] = weight;
             }
@@ -343,13 +391,18 @@ int dense_attention_f32(cudaStream_t stream, const DenseF32 &p, size_t batch) {
     const size_t sms = static_cast<size_t>(device_sm_count());
     const size_t blocks = pairs * ((static_cast<size_t>(p.query_len) + 31) / 32);
     if (p.head_dim <= 64) {
-        // A grid that does not cover the SMs leaves each CTA alone on its SM: four teams then (8 heads x 512 causal keys:
-        // 22.9 us, with two 34.3), which with more CTAs only take one another's shared memory (24 x 400 causal: 62.7
-        // against 47.2).  64 rows and no teams never win by more than 3 % (24 x 1500: 430 against 442) and lose up to half.
-        return blocks <= sms ? launch<64, 4, 32, 4>(stream, p, pairs) : launch<64, 4, 32, 2>(stream, p, pairs);
+        // Four teams need more than two key tiles to share.  A grid that does not cover the SMs leaves each CTA alone on its SM,
+        // and the longest walk decides (us with four teams and with two: 8 heads x 130 causal keys 11.3 and 12.6, x 512 24.1 and
+        // 26.4; x 128 whole 9.7 and 9.1).  Else the mean walk does: from three tiles on (200 heads x 200 whole keys
+        // 135 and 141, 64 x 400 causal 82 and 84, 24 x 1500 causal 270 and 297; 64 x 256 causal 41.6 and 41.2, 200 x 130 causal
+        // 65 and 62).  64 rows and no teams never win by more than 3 % and lose up to half.
+        long long walk = p.key_len;
+        if (blocks > sms && p.causal) walk = (min(p.query_len, p.key_len) + 1) / 2;
+        if (p.window > 0 && walk > p.window) walk = p.window;
+        return walk > (blocks > sms ? 3 : 2) * kKeys ? launch<64, 4, 32, 4>(stream, p, pairs) : launch<64, 4, 32, 2>(stream, p, pairs);
     }
     // Two teams' tiles of 128 columns fill an SM's shared memory, 64 rows without teams read each key half as often: that
-    // gains once the grid is two waves (24 heads x 1500 keys: 838 us against 924) and loses below (12 x 700: 99 against 61).
+    // gains once the grid is two waves (24 heads x 1500 keys: 883 us against 978) and loses below (12 x 700: 104 against 65).
     return blocks < 4 * sms ? launch<128, 4, 32, 2>(stream, p, pairs) : launch<128, 4, 64, 1>(stream, p, pairs);
 }
 

@@ -23,7 +23,9 @@ struct DenseF32 {
 };
 
 // Fewer rows a head than this leave most of a tile empty: one warp per row is the better split then (512 heads of 64:
-// 8 rows 8.6 us against 15.8, 16 rows 23.3 against 16.1).
+// 8 rows 8.6 us against 15.8).  16 rows over 256 keys take a fifth of its time or less at 4 - 512 heads of 4 - 128 columns;
+// over 16 keys the two are near each other (us in tiles and by warps, 4 - 128 heads: of 4 columns 8.0 - 8.2 and 9.1 - 12.8, of 64
+// 8.0 - 8.2 and 13.3 - 15.1; 512 heads: of 4 26.3 and 23.6, of 64 26.1 and 29.0, of 96 40.1 and 32.9), over 24 no longer.
 constexpr int kDenseF32LeastRows = 16;
 
 bool dense_attention_f32_takes(const DenseF32 &p, size_t batch);

@@ -67,3 +67,20 @@ def test_dense_f32_sinks_that_are_not_finite(l, b, d):
     assert not out[:, :, s + window - 1:].any()        # zero for every sink: nothing is weighed, whatever the sum is
     assert torch.equal(out[:, 0], attend(q, k, v, 0.125, False, window)[:, 0])
     assert out[:, :2].isfinite().all() and out[:, 2:, : s + window - 1].isnan().all()
+
+
+@pytest.mark.parametrize("d", [16, 32, 48, 64, 72, 96, 128])
+@pytest.mark.parametrize("l", [16, 24, 40, 100])
+@pytest.mark.parametrize("causal", [True, False])
+def test_dense_f32_error_is_no_larger_than_one_warp_per_rows(d, l, causal):
+    # Inputs four bytes off go by one warp per row.  The same values, 128 heads: the two mean errors are known to about 1 %
+    # (1024 row means of errors of some 0.5 each, correlated along a row), so two of those are allowed.
+    gen = torch.Generator(device="cuda").manual_seed(d * 1000 + l)
+    q, k, v = (torch.randn((16, 8, l, d), generator=gen, device="cuda") for _ in range(3))
+    shifted = torch.empty(q.numel() + 1, device="cuda")[1:].view(q.shape).copy_(q)
+    scores = q.double() @ k.double().transpose(-1, -2) * d ** -0.5
+    if causal:
+        scores.masked_fill_(torch.ones(l, l, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    exact = torch.softmax(scores, -1) @ v.double()
+    tiles, warps = ((attend(x, k, v, d ** -0.5, causal).double() - exact).norm() for x in (q, shifted))
+    assert tiles <= 1.02 * warps
