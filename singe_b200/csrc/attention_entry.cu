@@ -41,14 +41,14 @@ int prefill_tcgen05(cudaStream_t stream, bool is_f16, void *out, float *lse, con
                     size_t batch, size_t total_query_tokens, size_t total_kv_tokens, size_t heads, size_t kv_heads,
                     size_t head_dim, int causal, float scale, const uint32_t *block_table, size_t table_stride,
                     size_t cache_pages, size_t uniform_q, size_t uniform_kv);
-// kv_cache_write.cu
 bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t sequences,
                           size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
                           const void *value_cache, const void *out);
 int tensor_prefill(cudaStream_t stream, void *out, float *lse, const void *query, const void *key_cache, const void *value_cache,
                    const void *query_offsets, const void *page_offsets, const void *pages, const void *last_page_lengths,
                    int index_width, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t cache_pages,
-                   size_t sequences, size_t table_len, float scale, int causal, size_t window, uint32_t *status, unsigned **redo);
+                   size_t sequences, size_t table_len, float scale, int causal, size_t window, uint32_t *status);
+// kv_cache_write.cu
 int kv_cache_write(cudaStream_t stream, void *key_cache, void *value_cache, const void *keys, const void *values,
                    const void *write_pages, const void *write_slots, int index_width, size_t tokens, size_t kv_heads,
                    size_t head_dim, size_t pages, size_t page_size, uint32_t *status, size_t element_bytes);
@@ -99,7 +99,7 @@ int validate_ragged_prefill(size_t batch, size_t total_q, size_t total_kv, size_
 
 // paged_kv_decode_attention (singe-kernel/src/cpu/attention.rs:1172-1246): one query per sequence.
 template <typename T>
-struct DecodePagedPolicy : RowPolicy {
+struct DecodePagedPolicy {
     const T *query;
     T *out;
     const T *key_cache;
@@ -135,7 +135,7 @@ struct DecodePagedPolicy : RowPolicy {
 
 // Queries that see the chunk of positions they stand in, over the paged cache of the sequence each belongs to.
 template <typename T>
-struct ChunkedPolicy : RowPolicy {
+struct ChunkedPolicy {
     const T *query;
     T *out;
     const T *key_cache;
@@ -172,7 +172,7 @@ struct ChunkedPolicy : RowPolicy {
 
 // paged / ragged packed prefill (singe-kernel/src/cpu/attention.rs:1248-1420).  table == nullptr selects ragged.
 template <typename T>
-struct PackedPrefillPolicy : RowPolicy {
+struct PackedPrefillPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -239,7 +239,7 @@ struct PackedPrefillPolicy : RowPolicy {
 // Tensor::paged_attention (singe/src/backend/cpu/normalization/attention.rs:424-540) with the refusals of
 // check_paged_values (singe/src/backend/spec/neural/attention.rs:363-416) applied to the row's own sequence.
 template <typename T, typename Index>
-struct TensorPagedPolicy : RowPolicy {
+struct TensorPagedPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -252,26 +252,9 @@ struct TensorPagedPolicy : RowPolicy {
     int sequences, heads, kv_heads, head_dim, page_size, causal;
     long long tokens, cache_pages, table_len, window;
     const int *skip_when_zero;  // the planning kernel's verdict: 0 = the tiled decode kernel serves this call
-    const unsigned *redo;       // nullptr, or: the tensor-core kernel serves this call, and while this word is zero it has
-                                // left nothing; else the rows it marked and those of sequences it did not take are done here
 
-    __device__ bool nothing_left() const {
-        return (skip_when_zero != nullptr && *skip_when_zero == 0) || (redo != nullptr && *redo == 0u);
-    }
-    // Whether the tensor-core kernel left the sequence with these pages out: one of them lies outside the cache, or the query
-    // offsets of the call are out of range or run backwards.  The whole warp asks for one sequence.
-    __device__ bool left_out(long long first, long long last) const {
-        bool bad = false;
-        for (int s = threadIdx.x & 31; s < sequences && !bad; s += 32) {
-            bad = query_offsets[s] < 0 || query_offsets[s] > query_offsets[s + 1] || query_offsets[s + 1] > tokens;
-        }
-        for (long long i = first + (threadIdx.x & 31); i < last && !bad; i += 32) {
-            const long long page = static_cast<long long>(pages[i]);
-            bad = page < 0 || page >= cache_pages;
-        }
-        return __any_sync(0xffffffffu, bad) != 0;
-    }
     __device__ int locate(size_t row, RowPlan<T> &plan) const {
+        if (skip_when_zero != nullptr && *skip_when_zero == 0) return 0;
         const long long token = static_cast<long long>(row / heads);
         const int head = static_cast<int>(row - static_cast<size_t>(token) * heads);
         int owner = -1;
@@ -298,7 +281,6 @@ struct TensorPagedPolicy : RowPolicy {
             if (last_length < 0 || last_length > page_size) return -1;
             keys = (page_count - 1) * page_size + last_length;
         }
-        if (redo != nullptr && !isnan(lse[row]) && !left_out(first_page, last_page)) return 0;
         const long long queries = end_query - first_query;
         long long position = keys + (token - first_query) - queries;  // queries are the sequence's last tokens
         if (position < 0) position = 0;
@@ -324,6 +306,80 @@ struct TensorPagedPolicy : RowPolicy {
     __device__ const T *key_base() const { return key_cache; }
     __device__ const T *value_base() const { return value_cache; }
 };
+
+// What the tensor-core kernel of a step leaves: rows that it marked with a NaN as their log sum, and those of sequences that it
+// did not take because a page of theirs lies outside the cache, or because the query offsets leave the tokens or run backwards
+// (then it takes none).  A CTA looks eight tokens up, a warp each, before the tensor-core kernel has ended (which reads the paging
+// tensors as well, and started when whoever wrote them had ended), then reads their log sums; what is left is shared out over
+// its warps.  The tokens of a CTA lie far apart: a sequence that is left out is left to many.  So a call leaves nothing behind
+// that a later one could meet.  The step of 2072 tokens on 32 heads of prefill_tcgen05.cu's notes takes 163.3 us, as with a word of
+// the device that said whether anything was left (163.5; once raised, it made every later call take 193.8); with one of its four
+// chunks left out 3.6 ms (1.4 with a warp per row, which had every row look its sequence up).
+constexpr int kLeftTokens = 8, kLeftWarps = 16;
+
+template <typename T, typename Index, int MAX>
+__global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const TensorPagedPolicy<T, Index> policy, int head_dim, float scale,
+                                                                    uint32_t *status) {
+    __shared__ unsigned shared_left[kLeftTokens];
+    grid_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long slots = (policy.tokens + kLeftTokens - 1) / kLeftTokens;
+    for (long long slot = blockIdx.x; slot < slots; slot += gridDim.x) {
+        const long long token = slot + warp * slots;
+        const bool mine = warp < kLeftTokens && token < policy.tokens;
+        bool all = false;  // whether every row of the token is left
+        if (mine) {
+            int owner = -1;
+            for (int base = 0; base < policy.sequences; base += 32) {
+                const int s = base + lane;
+                const long long first = s < policy.sequences ? policy.query_offsets[s] : 0;
+                const long long last = s < policy.sequences ? policy.query_offsets[s + 1] : 0;
+                all |= first < 0 || first > last || last > policy.tokens;
+                const unsigned owns = __ballot_sync(0xffffffffu, token >= first && token < last);
+                if (owns != 0 && owner < 0) owner = base + __ffs(owns) - 1;
+            }
+            if (owner >= 0) {
+                const long long first = policy.page_offsets[owner], last = policy.page_offsets[owner + 1];
+                if (0 <= first && last <= policy.table_len) {
+                    for (long long i = first + lane; i < last; i += 32) {
+                        const long long page = policy.pages[i];
+                        all |= page < 0 || page >= policy.cache_pages;
+                    }
+                }
+            }
+            all = __any_sync(0xffffffffu, all) != 0;
+        }
+        grid_dependency_wait();
+        for (int base = 0; base < policy.heads; base += 32) {
+            if (warp < kLeftTokens) {
+                const bool left = mine && base + lane < policy.heads && (all || isnan(policy.lse[token * policy.heads + base + lane]));
+                const unsigned rows = __ballot_sync(0xffffffffu, left);
+                if (lane == 0) shared_left[warp] = rows;
+            }
+            __syncthreads();
+            int number = 0;
+            for (int t = 0; t < kLeftTokens; ++t) {
+                for (unsigned rows = shared_left[t]; rows != 0; rows &= rows - 1) {
+                    if (number++ % kLeftWarps == warp) {
+                        const size_t row = static_cast<size_t>((slot + t * slots) * policy.heads + base + __ffs(rows) - 1);
+                        attention_general_row<T, TensorPagedPolicy<T, Index>, MAX>(policy, row, head_dim, scale, LseKind::Base2, -INFINITY,
+                                                                                   status, 0.0f);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+template <typename T, typename Index>
+int launch_left_rows(cudaStream_t stream, const TensorPagedPolicy<T, Index> &policy, size_t tokens, size_t head_dim, float scale,
+                     uint32_t *status) {
+    const size_t blocks = (tokens + kLeftTokens - 1) / kLeftTokens, most = static_cast<size_t>(device_sm_count()) * 2;
+    SINGE_CUDA_TRY(launch_dependent(left_rows_kernel<T, Index, kMaxPerLane>, dim3(static_cast<unsigned>(blocks < most ? blocks : most)),
+                                    dim3(32 * kLeftWarps), 0, stream, kLaunchGlue, 1, policy, static_cast<int>(head_dim), scale, status));
+    return launch_status();
+}
 
 // The whole-table refusal of check_paged_values: any sequence with bad offsets, pages or last length sets the status.
 // One warp per sequence; its lanes share the sequence's page list.
@@ -457,7 +513,7 @@ __global__ void check_and_plan_kernel(const Index *query_offsets, const Index *p
 // (singe/src/backend/cpu/normalization/attention.rs:191-276) and fmha_prefill_lse [B,L,H,D] over [B,S,G,D]
 // (singe-kernel/src/cpu/attention.rs:1758-1833).
 template <typename T>
-struct DensePolicy : RowPolicy {
+struct DensePolicy {
     const T *query;
     T *out;
     float *lse;
@@ -501,7 +557,7 @@ struct DensePolicy : RowPolicy {
 // out [B, H, splits, D] and its natural-log LSE in lse [B, H, splits] (fmha_decode_splitk_f32,
 // singe-kernel/src/cuda/attention/fmha.rs:1073-1117); splitk_reduce_kernel folds them.
 template <typename T>
-struct DenseSplitPolicy : RowPolicy {
+struct DenseSplitPolicy {
     const T *query;
     T *out;
     float *lse;
@@ -804,7 +860,6 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
     policy.table_len = static_cast<long long>(table_len);
     policy.window = static_cast<long long>(window);
     policy.skip_when_zero = nullptr;
-    policy.redo = nullptr;
     bool checked = status == nullptr;  // no status word, no whole-table check
     auto check_alone = [&]() -> int {
         const unsigned blocks = static_cast<unsigned>((sequences + 3) / 4);  // four warps, one sequence each
@@ -880,21 +935,20 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
         // (workspace growth refused under stream capture: the general kernel serves the call)
     }
     // Steps with prompts in them: the tensor-core kernel, which checks the paging tensors itself and follows the general
-    // kernel's meaning row by row (what it leaves, the general kernel does).
-    if (std::is_same<T, __nv_bfloat16>::value && tokens != sequences && softcap == 0.0f &&
-        tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, sequences, table_len, causal, window, query, key_cache,
-                             value_cache, out)) {
-        unsigned *redo = nullptr;
-        SINGE_TRY(tensor_prefill(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
-                                 last_page_lengths, static_cast<int>(sizeof(Index)), tokens, heads, kv_heads, head_dim, cache_pages,
-                                 sequences, table_len, scale, causal, window, status, &redo));
-        policy.redo = redo;
-        checked = true;
+    // kernel's meaning row by row (what it leaves is done behind it).
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        if (tokens != sequences && softcap == 0.0f &&
+            tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, sequences, table_len, causal, window, query, key_cache,
+                                 value_cache, out)) {
+            SINGE_TRY(tensor_prefill(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
+                                     last_page_lengths, static_cast<int>(sizeof(Index)), tokens, heads, kv_heads, head_dim,
+                                     cache_pages, sequences, table_len, scale, causal, window, status));
+            return launch_left_rows<T, Index>(stream, policy, tokens, head_dim, scale, status);
+        }
     }
     if (!checked) SINGE_TRY(check_alone());
-    const size_t most_blocks = policy.redo != nullptr ? static_cast<size_t>(device_sm_count()) * 16 : 0x7fffffff;
     return launch_attention_general<T>(stream, policy, tokens * heads, head_dim, scale, LseKind::Base2, -INFINITY,
-                                       status, softcap, most_blocks);
+                                       status, softcap);
 }
 
 template <typename T>

@@ -29,35 +29,23 @@ struct RowPlan {
                        // (sinks of Tensor::attend, singe/src/backend/cpu/normalization/attention.rs:253-263)
 };
 
-// What every policy has unless it says otherwise: the kernel has work.
-struct RowPolicy {
-    __device__ bool nothing_left() const { return false; }
-};
-
 constexpr int kMaxPerLane = 8;    // head_dim <= 256
 constexpr int kWidePerLane = 32;  // head_dim <= 1024: attention over latents, where a "head" is a whole cached row
 
+// One row, by one warp.
 template <typename T, typename Policy, int MAX>
-__global__ void __launch_bounds__(128) attention_general_kernel(Policy policy, size_t rows, int head_dim, float scale,
-                                                                LseKind lse_kind, float empty_lse,
-                                                                uint32_t *status, float softcap) {
-    // Launched as a programmatic dependent: its CTAs may become resident while the kernel before still runs, and
-    // read or write nothing before that kernel has finished.
-    grid_launch_dependents();
-    grid_dependency_wait();
-    if (policy.nothing_left()) return;
+__device__ __forceinline__ void attention_general_row(const Policy &policy, size_t row, int head_dim, float scale, LseKind lse_kind,
+                                                      float empty_lse, uint32_t *status, float softcap) {
     const int lane = threadIdx.x & 31;
-    const size_t warps = static_cast<size_t>(gridDim.x) * (blockDim.x >> 5);
-    for (size_t row = static_cast<size_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
     RowPlan<T> plan;
     plan.sink = -INFINITY;
     const int located = policy.locate(row, plan);
     if (located == 0) {
-        continue;  // the row belongs to no sequence: nothing is written
+        return;  // the row belongs to no sequence: nothing is written
     }
     if (located < 0) {
         if (lane == 0) report_status(status, kStatusIndexOutOfBounds);
-        continue;
+        return;
     }
     const int per_lane = (head_dim + 31) >> 5;
     float q[MAX];
@@ -138,7 +126,7 @@ __global__ void __launch_bounds__(128) attention_general_kernel(Policy policy, s
     }
     if (failed) {
         if (lane == 0) report_status(status, kStatusIndexOutOfBounds);
-        continue;
+        return;
     }
     const bool empty = plan.end <= plan.start && plan.sink == -INFINITY;
     const float inverse = empty ? 0.0f : 1.0f / running_sum;
@@ -156,24 +144,36 @@ __global__ void __launch_bounds__(128) attention_general_kernel(Policy policy, s
         }
         *plan.lse = value;
     }
-    }  // rows
+}
+
+template <typename T, typename Policy, int MAX>
+__global__ void __launch_bounds__(128) attention_general_kernel(Policy policy, size_t rows, int head_dim, float scale,
+                                                                LseKind lse_kind, float empty_lse,
+                                                                uint32_t *status, float softcap) {
+    // Launched as a programmatic dependent: its CTAs may become resident while the kernel before still runs, and
+    // read or write nothing before that kernel has finished.
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const size_t row = static_cast<size_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= rows) {
+        return;
+    }
+    attention_general_row<T, Policy, MAX>(policy, row, head_dim, scale, lse_kind, empty_lse, status, softcap);
 }
 
 template <typename T, typename Policy>
 int launch_attention_general(cudaStream_t stream, const Policy &policy, size_t rows, size_t head_dim, float scale,
-                             LseKind lse_kind, float empty_lse, uint32_t *status, float softcap = 0.0f,
-                             size_t most_blocks = 0x7fffffff) {
+                             LseKind lse_kind, float empty_lse, uint32_t *status, float softcap = 0.0f) {
     if (head_dim > 32 * kWidePerLane) {
         return SINGE_ERR_UNSUPPORTED_WIDTH;
     }
     if (rows == 0) {
         return SINGE_OK;
     }
-    size_t blocks = (rows + 3) / 4;
+    const size_t blocks = (rows + 3) / 4;
     if (blocks > 0x7fffffffull) {
         return SINGE_ERR_LENGTH_EXCEEDS_I32;
     }
-    if (blocks > most_blocks) blocks = most_blocks;  // a launch that most likely finds nothing to do
     if (head_dim <= 32 * kMaxPerLane) {
         SINGE_CUDA_TRY(launch_dependent(attention_general_kernel<T, Policy, kMaxPerLane>, dim3(static_cast<unsigned>(blocks)),
                                         dim3(128), 0, stream, kLaunchGlue, 1, policy, rows, static_cast<int>(head_dim),

@@ -104,10 +104,9 @@ struct PrefillParams {
 // The Tensor surface's paging tensors (Tensor::paged_attention, singe/src/tensor/neural.rs:405-457), read as the caller
 // gave them: query_offsets and page_offsets [sequences + 1], pages [table_len], last_page_lengths [sequences], 32- or
 // 64-bit.  Every CTA checks all of them at its start and lists the sequences in shared memory; a sequence with a value
-// out of range gets no work here and raises `redo`, after which the general kernel computes what it can of it.  The
-// same word has the general kernel redo rows that this one marks with a NaN as their LSE: rows that leave the
-// single-pass range, and rows whose output is not finite (a hidden key's value may be anything, and zero times
-// infinity is not zero).
+// out of range gets no work here, and the kernel that follows (left_rows_kernel) computes what can be computed of it.  It
+// also does rows over that this one marks with a NaN as their LSE: rows that leave the single-pass range, and rows whose
+// output is not finite (a hidden key's value may be anything, and zero times infinity is not zero).
 // Bound by the tensor core and the special-function unit alike: 8 + 16 MMAs of 128 x 128 x 16 and 16384 exponentials a
 // key tile.  One step of four 510-token chunks and 28 decoding sequences behind 0 - 3000 tokens of context, 32 query heads on 8:
 // 172 us, 238 with items in order of their pair index and lone tiles a key tile at a time, 40.2 ms by one warp per row and head.
@@ -124,15 +123,12 @@ struct TensorPaging {
     int table_len;
     int pack;          // log2 of the query heads whose rows stand together; p.heads counts such packs
     uint32_t *status;
-    unsigned *redo;
 };
 struct NoPaging {};
 
 constexpr int kMaxTensorSequences = 1024;
 constexpr int kTensorBarriers = 22;  // (one of them only keeps what follows aligned)
 constexpr int kMaxOrdered = 1024;   // (sequence, pair) entries that are put in order of their cost
-constexpr unsigned kRedoMarkedRows = 1u, kRedoBadPaging = 2u;
-__device__ unsigned g_tensor_redo = 0;
 
 __device__ __forceinline__ long long paging_value(const void *list, int width, int at) {
     return width == 8 ? static_cast<const long long *>(list)[at] : static_cast<const int *>(list)[at];
@@ -190,10 +186,7 @@ __device__ __forceinline__ void list_sequences(const TensorPaging &g, int cache_
             table.keys[own] = bad ? 0 : static_cast<int>(keys);
             table.first_token[own] = bad ? 0 : static_cast<int>(qf);
             table.first_page[own] = bad ? 0 : static_cast<int>(pf);
-            if (bad && blockIdx.x == 0) {
-                report_status(g.status, kStatusIndexOutOfBounds);
-                atomicOr(g.redo, kRedoBadPaging);
-            }
+            if (bad && blockIdx.x == 0) report_status(g.status, kStatusIndexOutOfBounds);
         }
     }
     if (__syncthreads_or(backwards ? 1 : 0) != 0) {
@@ -569,6 +562,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     unsigned *order = nullptr;
     volatile float2 *share = nullptr;  // TENSOR: base and sum of tile B's rows of an alternating item
     if constexpr (TENSOR) {
+        grid_launch_dependents();
         // (the redo list's place and what follows it)
         table.rows = counts + kMaxRankTiles;
         table.keys = table.rows + kMaxTensorSequences;
@@ -1182,10 +1176,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 float value = empty ? -1.0e20f : (base_log2 + log2f(row_sum)) * 0.6931471805599453f;
                 if constexpr (TENSOR) {
                     value = base_log2 + log2f(row_sum);
-                    if (!in_range || empty || isnan(probe)) {
-                        value = __int_as_float(0x7fc00000);  // has the general kernel redo the row
-                        atomicOr(paging.redo, kRedoMarkedRows);
-                    }
+                    if (!in_range || empty || isnan(probe)) value = __int_as_float(0x7fc00000);  // has the row done again: see left_rows_kernel
                 } else if (!SAFE && !in_range) {
                     value = __int_as_float(0x7fc00000);  // has the second launch redo the item
                     atomicExch(&g_out_of_range_seen, 1u);
@@ -1415,20 +1406,11 @@ bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t h
            prefill_fast_path(heads, kv_heads, head_dim, rows, query, key_cache, value_cache, out);
 }
 
-// Tensor::paged_attention over 16-token pages.  `redo` (see TensorPaging) tells the general kernel, which follows on the
-// stream, whether rows are left to it.
+// Tensor::paged_attention over 16-token pages; left_rows_kernel has to follow on the stream.
 int tensor_prefill(cudaStream_t stream, void *out, float *lse, const void *query, const void *key_cache, const void *value_cache,
                    const void *query_offsets, const void *page_offsets, const void *pages, const void *last_page_lengths,
                    int index_width, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t cache_pages,
-                   size_t sequences, size_t table_len, float scale, int causal, size_t window, uint32_t *status, unsigned **redo) {
-    static unsigned *words[kMaxDevices] = {nullptr};
-    const int slot = device_slot();
-    if (slot < 0) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
-    if (words[slot] == nullptr) {
-        void *address = nullptr;
-        SINGE_CUDA_TRY(cudaGetSymbolAddress(&address, g_tensor_redo));
-        words[slot] = static_cast<unsigned *>(address);
-    }
+                   size_t sequences, size_t table_len, float scale, int causal, size_t window, uint32_t *status) {
     const int pack = pack_of(heads, kv_heads);
     const uint64_t width = head_dim;
     const CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -1458,12 +1440,11 @@ int tensor_prefill(cudaStream_t stream, void *out, float *lse, const void *query
     params.error = device_error_word();
     params.window = static_cast<int>(window);
     TensorPaging paging = {query_offsets, page_offsets, pages, last_page_lengths, index_width, static_cast<int>(sequences),
-                           static_cast<int>(tokens), static_cast<int>(table_len), pack, status, words[slot]};
+                           static_cast<int>(tokens), static_cast<int>(table_len), pack, status};
     const size_t items = ((tokens << pack) / kPair + sequences) * (heads >> pack);
     if (items > 0x7fffffffull) return SINGE_ERR_LENGTH_EXCEEDS_I32;
     const size_t sms = static_cast<size_t>(device_sm_count());
     const unsigned persistent = static_cast<unsigned>(items < sms ? items : sms);
-    *redo = words[slot];
     if (head_dim == 64) {
         return window > 0 ? launch_tensor<64, true>(stream, q_map, k_map, v_map, params, paging, persistent)
                           : launch_tensor<64, false>(stream, q_map, k_map, v_map, params, paging, persistent);
