@@ -41,8 +41,8 @@ int prefill_tcgen05(cudaStream_t stream, bool is_f16, void *out, float *lse, con
                     size_t batch, size_t total_query_tokens, size_t total_kv_tokens, size_t heads, size_t kv_heads,
                     size_t head_dim, int causal, float scale, const uint32_t *block_table, size_t table_stride,
                     size_t cache_pages, size_t uniform_q, size_t uniform_kv);
-bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t sequences,
-                          size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
+bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t cache_pages,
+                          size_t sequences, size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
                           const void *value_cache, const void *out);
 int tensor_prefill(cudaStream_t stream, void *out, float *lse, const void *query, const void *key_cache, const void *value_cache,
                    const void *query_offsets, const void *page_offsets, const void *pages, const void *last_page_lengths,
@@ -938,8 +938,8 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
     // kernel's meaning row by row (what it leaves is done behind it).
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
         if (tokens != sequences && softcap == 0.0f &&
-            tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, sequences, table_len, causal, window, query, key_cache,
-                                 value_cache, out)) {
+            tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, cache_pages, sequences, table_len, causal, window,
+                                 query, key_cache, value_cache, out)) {
             SINGE_TRY(tensor_prefill(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
                                      last_page_lengths, static_cast<int>(sizeof(Index)), tokens, heads, kv_heads, head_dim,
                                      cache_pages, sequences, table_len, scale, causal, window, status));

@@ -1397,11 +1397,12 @@ int prefill_tcgen05_windowed(cudaStream_t stream, void *out, float *lse, const v
 }
 
 // Whether tensor_prefill serves a call of the Tensor surface's paged attention (bf16, no score cap).
-bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t sequences,
-                          size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
+bool tensor_prefill_takes(size_t tokens, size_t heads, size_t kv_heads, size_t head_dim, size_t page_size, size_t cache_pages,
+                          size_t sequences, size_t table_len, int causal, size_t window, const void *query, const void *key_cache,
                           const void *value_cache, const void *out) {
     const size_t rows = tokens << pack_of(heads, kv_heads);
-    return page_size == kPageTokens && sequences <= kMaxTensorSequences && table_len <= 0x7fffffff / kPageTokens - kTile &&
+    return page_size == kPageTokens && cache_pages > 0 && sequences <= kMaxTensorSequences &&
+           table_len <= 0x7fffffff / kPageTokens - kTile &&
            (window == 0 || (causal && window <= 0x3fffffff)) && rows <= 0x7fffffff / 2 &&
            prefill_fast_path(heads, kv_heads, head_dim, rows, query, key_cache, value_cache, out);
 }

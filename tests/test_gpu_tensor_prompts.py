@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import oracle
-from singe_b200 import ops, workloads
+from singe_b200 import kernel_sys as ks, ops, workloads
 from tests.gpu_util import dev, host
 
 pytestmark = pytest.mark.gpu
@@ -199,3 +199,15 @@ def test_captured_steps_and_streams_of_their_own():
     assert statuses[0].item() == 0 and statuses[1].item() == 1
     for own, wanted in zip(found, (expected[0], refused)):
         assert all(torch.equal(*pair) for result in own for pair in zip(result, wanted))
+
+
+def test_a_cache_without_pages():
+    tensors = [torch.zeros((5, 4, 128), dtype=torch.bfloat16, device="cuda")] * 3
+    out, lse = torch.full_like(tensors[0], 7.0), torch.full((5, 4), 7.0, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    paging = [torch.tensor(v, device="cuda") for v in ([0, 3, 3, 5], [0, 0, 0, 0], [0], [0, 0, 0])]
+    code = ks.lib().singe_paged_attention_bf16(int(torch.cuda.current_stream().cuda_stream), out.data_ptr(), lse.data_ptr(),
+                                               *(t.data_ptr() for t in tensors + paging), 8, 5, 4, 2, 128, PAGE, 0, 3, 0, 0.1, 1, 0,
+                                               status.data_ptr())
+    torch.cuda.synchronize()
+    assert code == ks.OK and status.item() == 0 and not out.any() and bool(lse.isneginf().all())
