@@ -7,25 +7,30 @@ from singe_b200 import kernel_sys as ks
 
 pytestmark = pytest.mark.gpu
 
-ROWS, FEW = 8 * 148 + 3, 500     # the last CTA is not full
+
+def _counts():
+    """Rows and tokens from which a warp takes one (8 and 12 per SM) with a last CTA that is not full, and too few for that."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return 8 * sms + 3, 12 * sms + 5, 3 * sms
 
 
 def _stream():
     return int(torch.cuda.current_stream().cuda_stream)
 
 
-def _slices(rows):
-    return [slice(first, min(first + FEW, rows)) for first in range(0, rows, FEW)]
+def _slices(rows, few):
+    return [slice(first, min(first + few, rows)) for first in range(0, rows, few)]
 
 
 @pytest.mark.parametrize("width", [8, 256, 264, 1024, 1032, 2048, 2056, 4096])
 @pytest.mark.parametrize("delta,norm", [(True, True), (False, True), (True, False)])
 def test_rms_norm_rows(width, delta, norm):
+    rows, _, few = _counts()
     gen = torch.Generator(device="cuda").manual_seed(width)
     normal = lambda *shape: torch.randn(shape, generator=gen, device="cuda").to(torch.bfloat16)
-    hidden, change, weight = normal(ROWS, width), normal(ROWS, width), normal(width)
+    hidden, change, weight = normal(rows, width), normal(rows, width), normal(width)
     results = []
-    for parts in ([slice(0, ROWS)], _slices(ROWS)):
+    for parts in ([slice(0, rows)], _slices(rows, few)):
         h, out = hidden.clone(), torch.zeros_like(hidden)
         for part in parts:
             assert ks.lib().singe_add_rms_norm_bf16(
@@ -40,13 +45,14 @@ def test_rms_norm_rows(width, delta, norm):
 @pytest.mark.parametrize("width,padding", [(4, 0), (512, 4), (516, 0), (1028, 0), (1536, 8), (2048, 0), (2052, 0)])
 @pytest.mark.parametrize("delta,norm", [(True, True), (False, True), (True, False)])
 def test_layer_norm_rows(kind, width, padding, delta, norm):
+    rows, _, few = _counts()
     gen = torch.Generator(device="cuda").manual_seed(width)
-    residual = torch.randn((ROWS, width), generator=gen, device="cuda") + 3.0
-    change, weight = (torch.randn(shape, generator=gen, device="cuda").to(kind) for shape in ((ROWS, width + padding), (width,)))
+    residual = torch.randn((rows, width), generator=gen, device="cuda") + 3.0
+    change, weight = (torch.randn(shape, generator=gen, device="cuda").to(kind) for shape in ((rows, width + padding), (width,)))
     call = ks.lib().singe_add_layer_norm_bf16 if kind == torch.bfloat16 else ks.lib().singe_add_layer_norm_f32
     results = []
-    for parts in ([slice(0, ROWS)], _slices(ROWS)):
-        r, out = residual.clone(), torch.zeros((ROWS, width + padding), dtype=kind, device="cuda")
+    for parts in ([slice(0, rows)], _slices(rows, few)):
+        r, out = residual.clone(), torch.zeros((rows, width + padding), dtype=kind, device="cuda")
         for part in parts:
             assert call(_stream(), r[part].data_ptr(), change[part].data_ptr() if delta else None, width + padding,
                         out[part].data_ptr() if norm else None, width + padding, weight.data_ptr(), r[part].shape[0], width,
@@ -61,7 +67,8 @@ def test_layer_norm_rows(kind, width, padding, delta, norm):
                                                         (4, 2, 96, 0)])
 def test_rotary_rows(index, heads, kv_heads, dim, padding):
     # (the last has a head of six lanes, which stays with the CTA per token)
-    tokens, capacity, page = 12 * 148 + 5, 300, 16
+    _, tokens, few = _counts()
+    capacity, page = 300, 16
     gen = torch.Generator(device="cuda").manual_seed(dim)
     normal = lambda *shape: torch.randn(shape, generator=gen, device="cuda").to(torch.bfloat16)
     qkv, cosine, sine = normal(tokens, (heads + 2 * kv_heads) * dim + padding), normal(capacity, dim // 2), normal(capacity, dim // 2)
@@ -74,7 +81,7 @@ def test_rotary_rows(index, heads, kv_heads, dim, padding):
     write_slot[9] = page            # its key and value are refused
     write_page[tokens - 1] = pages
     results = []
-    for parts in ([slice(0, tokens)], _slices(tokens)):
+    for parts in ([slice(0, tokens)], _slices(tokens, few)):
         q = torch.zeros((tokens, heads, dim), dtype=torch.bfloat16, device="cuda")
         keys, values = (torch.zeros((pages, page, kv_heads, dim), dtype=torch.bfloat16, device="cuda") for _ in range(2))
         status = torch.zeros(1, dtype=torch.int32, device="cuda")

@@ -40,6 +40,13 @@ def assert_rounded(out, ref, what):
     assert (np.abs(out - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-4).all(), f"{what}: {np.abs(out - ref).max()}"
 
 
+def assert_log_sums(lse, ref):
+    """Of the largest score's size, some 20 here, or of the log sum where that is larger: eight steps of the tensor core, which drops
+    what lies below its accumulator's last bit (2^-23 each), and a few roundings of either side's exponentials and sums."""
+    worst = np.abs(lse - ref) / np.maximum(20.0, np.abs(ref))
+    assert worst.size == 0 or worst.max() < 20 * 2.0 ** -24, worst.max()
+
+
 NEW = [1, 300, 0, 70, 1, 33, 1, 256, 2]
 EVERY = [517, 300, 40, 900, 16, 20, 1, 640, 0]     # more keys than new tokens, as many, fewer, none
 
@@ -56,7 +63,7 @@ def test_steps_with_prompts(heads, kv_heads, dim, causal, window, index):
     assert_rounded(out, ref, "out")
     assert (np.isneginf(lse) == np.isneginf(ref_lse)).all()
     seen = np.isfinite(ref_lse)
-    assert np.abs(lse[seen] - ref_lse[seen]).max() < 2e-4
+    assert_log_sums(lse[seen], ref_lse[seen])
 
 
 def test_rows_of_no_sequence_are_left_alone():
@@ -67,7 +74,7 @@ def test_rows_of_no_sequence_are_left_alone():
     ref, ref_lse, _ = run_step(q, kc, vc, paging, torch.float32)
     assert status == 0 and not out[:5].any() and not out[60:].any() and np.isneginf(lse[:5]).all()
     assert_rounded(out, ref, "out")
-    assert np.abs(lse[5:60] - ref_lse[5:60]).max() < 2e-4
+    assert_log_sums(lse[5:60], ref_lse[5:60])
 
 
 def same_as_general(q, kc, vc, paging):
@@ -80,7 +87,7 @@ def same_as_general(q, kc, vc, paging):
     fine = np.isfinite(ref)
     assert_rounded(out[fine], ref[fine], "out")
     fine = np.isfinite(ref_lse)
-    assert (np.abs(lse[fine] - ref_lse[fine]) <= 2e-4 + 1e-6 * np.abs(ref_lse[fine])).all()
+    assert_log_sums(lse[fine], ref_lse[fine])
     return status
 
 
