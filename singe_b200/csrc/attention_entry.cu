@@ -309,12 +309,12 @@ struct TensorPagedPolicy {
 
 // What the tensor-core kernel of a step leaves: rows that it marked with a NaN as their log sum, and those of sequences that it
 // did not take because a page of theirs lies outside the cache, or because the query offsets leave the tokens or run backwards
-// (then it takes none).  A CTA looks eight tokens up, a warp each, before the tensor-core kernel has ended (which reads the paging
-// tensors as well, and started when whoever wrote them had ended), then reads their log sums; what is left is shared out over
-// its warps.  The tokens of a CTA lie far apart: a sequence that is left out is left to many.  So a call leaves nothing behind
-// that a later one could meet.  The step of 2072 tokens on 32 heads of prefill_tcgen05.cu's notes takes 163.3 us, as with a word of
-// the device that said whether anything was left (163.5; once raised, it made every later call take 193.8); with one of its four
-// chunks left out 3.6 ms (1.4 with a warp per row, which had every row look its sequence up).
+// (then it takes none).  It has raised the caller's status word over those; only if that word is raised, or there is none, are
+// sequences looked up again.  A CTA has eight tokens, a warp each, and shares what is left of them out over its warps.  The
+// tokens of a CTA lie far apart: a sequence that is left out is left to many.  Nothing is kept that a later call could meet.
+// The step of 2072 tokens on 32 heads of prefill_tcgen05.cu's notes takes 172.7 us, 171.7 with a word of the device that said
+// whether anything was left (once raised, it made every later call a fifth longer); steps of 60 - 950 tokens 0 - 1.8 us more than
+// with that word.  One of the four chunks left out: 3.2 ms (1.4 with a warp per row, which had every row look its sequence up).
 constexpr int kLeftTokens = 8, kLeftWarps = 16;
 
 template <typename T, typename Index, int MAX>
@@ -322,13 +322,17 @@ __global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const Ten
                                                                     uint32_t *status) {
     __shared__ unsigned shared_left[kLeftTokens];
     grid_launch_dependents();
+    grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t raised = status != nullptr ? *status : 1u;
     const long long slots = (policy.tokens + kLeftTokens - 1) / kLeftTokens;
     for (long long slot = blockIdx.x; slot < slots; slot += gridDim.x) {
         const long long token = slot + warp * slots;
         const bool mine = warp < kLeftTokens && token < policy.tokens;
         bool all = false;  // whether every row of the token is left
-        if (mine) {
+        // (both loads are on their way before either is waited for)
+        const bool first_marked = mine && lane < policy.heads && isnan(policy.lse[token * policy.heads + lane]);
+        if (mine && __shfl_sync(0xffffffffu, raised, 0) != 0u) {  // (one answer for a warp)
             int owner = -1;
             for (int base = 0; base < policy.sequences; base += 32) {
                 const int s = base + lane;
@@ -349,10 +353,11 @@ __global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const Ten
             }
             all = __any_sync(0xffffffffu, all) != 0;
         }
-        grid_dependency_wait();
         for (int base = 0; base < policy.heads; base += 32) {
             if (warp < kLeftTokens) {
-                const bool left = mine && base + lane < policy.heads && (all || isnan(policy.lse[token * policy.heads + base + lane]));
+                const bool marked = base == 0 ? first_marked
+                                              : mine && base + lane < policy.heads && isnan(policy.lse[token * policy.heads + base + lane]);
+                const bool left = marked || (all && base + lane < policy.heads);
                 const unsigned rows = __ballot_sync(0xffffffffu, left);
                 if (lane == 0) shared_left[warp] = rows;
             }

@@ -567,7 +567,6 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     unsigned *order = nullptr;
     volatile float2 *share = nullptr;  // TENSOR: base and sum of tile B's rows of an alternating item
     if constexpr (TENSOR) {
-        grid_launch_dependents();
         // (the redo list's place and what follows it)
         table.rows = counts + kMaxRankTiles;
         table.keys = table.rows + kMaxTensorSequences;
