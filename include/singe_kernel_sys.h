@@ -190,6 +190,12 @@ size_t singe_paged_kv_decode_split_tokens(size_t key_len_bound, size_t max_split
  * count to run the same launch. */
 size_t singe_paged_kv_decode_default_splits(size_t batch, size_t kv_heads, size_t key_len_bound, size_t block_size);
 
+/* For callers of singe_decode_step_attention_bf16 and singe_chunked_attention_bf16 (whose partials are the library's own
+ * matter): the max_splits whose scratch has room for the form that shares the cached pages evenly among the SMs, or 0 where
+ * the split grid serves the shape.  With less room the split grid serves it too. */
+size_t singe_paged_kv_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound,
+                                         size_t block_size);
+
 /* Writes the partials only (all `max_splits` slots of every row are defined afterwards). */
 int singe_paged_kv_decode_splitk_bf16(singe_stream_t stream, float *attn_scratch, float *lse_scratch,
                                       const void *query, const void *key_cache, const void *value_cache,

@@ -16,13 +16,14 @@ namespace singe {
 bool paged_decode_fast_path(size_t heads, size_t kv_heads, size_t head_dim, size_t block_size, const void *key_cache,
                             const void *value_cache, const void *query);
 size_t paged_decode_split_tokens(size_t key_len_bound, size_t max_splits, size_t block_size);
+size_t paged_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound);
 int paged_decode_splitk(cudaStream_t stream, int element, void *out, float *attn_scratch, float *lse_scratch,
                         const void *query, const void *key_cache, const void *value_cache,
                         const int32_t *actual_seq_lens, const uint32_t *block_table, size_t batch, size_t heads,
                         size_t kv_heads, size_t head_dim, size_t physical_blocks, size_t block_table_batch_stride,
                         size_t max_splits, float scale, bool partials_only, uint32_t *status,
                         const RaggedDecode *ragged, unsigned hints, const QueryRotation *rotation, uint32_t *tickets,
-                        const FusedStep *fused);
+                        const FusedStep *fused, bool even);
 int paged_decode_chunked(cudaStream_t stream, void *out, float *attn_scratch, float *lse_scratch, const void *query,
                          const void *key_cache, const void *value_cache, const int32_t *lens, const uint32_t *block_table,
                          const ChunkedDecode &chunked, size_t queries, size_t heads, size_t kv_heads, size_t head_dim,
@@ -733,13 +734,14 @@ int decode_half(cudaStream_t stream, int element, void *out, const void *query, 
     }
     // The tiled kernel puts the batch in a grid dimension of at most 65535; larger batches keep the general kernel.
     if (batch <= 65535 && paged_decode_fast_path(heads, kv_heads, head_dim, block_size, key_cache, value_cache, query)) {
-        const size_t splits = wave_aware_splits(batch, kv_heads, stride * block_size, block_size);
+        const size_t even = paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size);
+        const size_t splits = even > 0 ? even : wave_aware_splits(batch, kv_heads, stride * block_size, block_size);
         float *scratch = nullptr;
         const size_t rows = batch * heads * splits;
         SINGE_TRY(workspace_for(stream, rows * (head_dim + 1), &scratch));
         return paged_decode_splitk(stream, element, out, scratch, scratch + rows * head_dim, query, key_cache,
                                    value_cache, lens, table, batch, heads, kv_heads, head_dim, physical_blocks, stride,
-                                   splits, scale, false, device_error_word(), nullptr, 0u, nullptr, nullptr, nullptr);
+                                   splits, scale, false, device_error_word(), nullptr, 0u, nullptr, nullptr, nullptr, true);
     }
     if (element == 0) {
         return decode_general<__nv_bfloat16>(stream, out, query, key_cache, value_cache, lens, table, batch, heads,
@@ -768,7 +770,7 @@ int decode_splitk_half(cudaStream_t stream, int element, void *out, float *attn_
     return paged_decode_splitk(stream, element, out, attn_scratch, lse_scratch, query, key_cache, value_cache, lens,
                                table, batch, heads, kv_heads, head_dim, physical_blocks, stride, max_splits, scale,
                                partials_only, status != nullptr ? status : device_error_word(), nullptr, hints, rotation,
-                               tickets, fused);
+                               tickets, fused, fused != nullptr);
 }
 
 template <typename T>
@@ -932,7 +934,7 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
                                           value_cache, lens, nullptr, sequences, heads, kv_heads, head_dim,
                                           cache_pages, 1, splits, scale, false,
                                           status != nullptr ? status : device_error_word(), &ragged, 0u, nullptr,
-                                          nullptr, nullptr));
+                                          nullptr, nullptr, false));
             policy.skip_when_zero = control;
         } else if (grown != SINGE_ERR_AUTOTUNE_DURING_CAPTURE) {
             return grown;
@@ -1161,6 +1163,15 @@ int singe_paged_kv_decode_attention_f32(singe_stream_t stream, float *out, const
 size_t singe_paged_kv_decode_default_splits(size_t batch, size_t kv_heads, size_t key_len_bound, size_t block_size) {
     if (batch == 0 || kv_heads == 0 || key_len_bound == 0 || block_size == 0) return 1;
     return wave_aware_splits(batch, kv_heads, key_len_bound, block_size);
+}
+
+size_t singe_paged_kv_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound,
+                                         size_t block_size) {
+    if (batch == 0 || kv_heads == 0 || heads % kv_heads != 0 || key_len_bound == 0 || block_size != 16 || heads / kv_heads > 8 ||
+        (head_dim != 64 && head_dim != 128)) {
+        return 0;
+    }
+    return paged_decode_even_splits(batch, heads, kv_heads, head_dim, key_len_bound);
 }
 
 size_t singe_paged_kv_decode_split_tokens(size_t key_len_bound, size_t max_splits, size_t block_size) {

@@ -220,6 +220,10 @@ class LlamaDecoder(PagedDecoder):
         self.fast_decode = fast
         # rotary embedding, cache write and attention of a decode step in one launch (singe_decode_step_attention_bf16)
         self.fuse_attention = fuse_attention and fast
+        if max_splits <= 0 and self.fuse_attention and not fold_in_kernel:
+            # scratch for the form that shares the cached pages evenly among the SMs, where it serves this shape
+            max_splits = int(ks.lib().singe_paged_kv_decode_even_splits(sequences, self.heads, self.kv_heads, config.head_dim,
+                                                                        self.stride * config.page_size, config.page_size))
         if max_splits <= 0:
             max_splits = choose_decode_splits(sequences * self.kv_heads, self.stride * config.page_size,
                                               2 * 2 * config.head_dim,

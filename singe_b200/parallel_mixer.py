@@ -142,7 +142,8 @@ class ChunkedAttention:
             return None
         torch, c = self.ops.torch, self.config
         bound = min(c.chunk + TILED_PAGE - 1, key_bound)
-        splits = int(ks.lib().singe_paged_kv_decode_default_splits(rows, c.kv_heads, bound, TILED_PAGE))
+        splits = int(ks.lib().singe_paged_kv_decode_even_splits(rows, c.heads, c.kv_heads, self.size, bound, TILED_PAGE) or
+                     ks.lib().singe_paged_kv_decode_default_splits(rows, c.kv_heads, bound, TILED_PAGE))
         attn = torch.empty((rows, c.heads, splits, self.size), dtype=torch.float32, device="cuda")
         lse = torch.empty((rows, c.heads, splits), dtype=torch.float32, device="cuda")
         return splits, attn, lse

@@ -1,0 +1,130 @@
+"""Paged decode whose CTAs share the cached pages evenly, at the places where runs, segments and folds can go wrong."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import llama_ref, oracle
+from singe_b200 import kernel_sys as ks
+from singe_b200 import ops, workloads
+from singe_b200.layer_ops import Ops
+from singe_b200.llama import rotary_tables
+from tests.gpu_util import assert_close_bf16, dev, dev_u32, host
+from tests.test_gpu_decode import _config, _inputs, _oracle
+
+pytestmark = pytest.mark.gpu
+
+LONG = 65536     # a bound on the lengths that has the even form serve short ones too
+
+# one sequence; runs that end inside, at and before a sequence's last page; empty sequences; more sequences than threads
+LENGTHS = [[1], [16 * 300], [16 * 148 * 2], [0, 33, 0, 512, 0], [1, 15, 16, 17, 2049, 31, 32, 33, 4097, 100],
+           [(37 * i) % 90 for i in range(300)], [5000] + [3] * 40]
+
+
+def even_splits(case):
+    return ks.lib().singe_paged_kv_decode_even_splits(case.batch, case.heads, case.kv_heads, case.head_dim,
+                                                      case.block_table_batch_stride * case.block_size, case.block_size)
+
+
+@pytest.mark.parametrize("lens", LENGTHS, ids=lambda lens: f"{len(lens)}x{max(lens)}")
+@pytest.mark.parametrize("heads,kv_heads,head_dim,dtype", [(32, 8, 128, torch.bfloat16), (16, 8, 64, torch.float16), (16, 4, 128, torch.bfloat16),
+                                                           (32, 4, 64, torch.bfloat16), (12, 4, 128, torch.float16)])
+def test_even_decode(lens, heads, kv_heads, head_dim, dtype):
+    case = workloads.paged_decode_case(seed=3, heads=heads, kv_heads=kv_heads, head_dim=head_dim, lens=lens, max_len=LONG)
+    assert even_splits(case) > 0
+    q, k, v = _inputs(case, seed=len(lens))
+    out = torch.full((case.batch, heads, head_dim), float("nan"), dtype=dtype, device="cuda")
+    operands = [dev(x, dtype) for x in (q, k, v)]
+    for _ in range(2):      # the workspace is not clean the second time
+        ops.paged_kv_decode_attention(out, *operands, dev(case.lens), dev_u32(case.block_table), _config(case))
+    torch.cuda.synchronize()
+    assert ops.take_device_error() == 0
+    assert_close_bf16(host(out), _oracle(case, q, k, v), f"{len(lens)} sequences")
+    assert not host(out)[np.asarray(lens) == 0].any()
+
+
+def test_even_decode_reports_page_ids_outside_the_cache():
+    case = workloads.paged_decode_case(seed=4, heads=8, kv_heads=4, head_dim=64, lens=[700, 40], max_len=LONG)
+    q, k, v = _inputs(case, seed=5)
+    table = case.block_table.copy()
+    table[0, 20] = case.physical_blocks
+    out = torch.empty((2, 8, 64), dtype=torch.bfloat16, device="cuda")
+    ops.paged_kv_decode_attention(out, *[dev(x, torch.bfloat16) for x in (q, k, v)], dev(case.lens), dev_u32(table), _config(case))
+    assert ops.take_device_error() == ks.STATUS_INDEX_OUT_OF_BOUNDS
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(32, 8, 128), (8, 4, 64)])
+@pytest.mark.parametrize("hinted", [False, True])
+def test_even_decode_step_adds_its_key(heads, kv_heads, head_dim, hinted):
+    lens = [1, 300, 16, 17, 2049, 0, 513, 33]     # keys including the new one; an idle row
+    case = workloads.paged_decode_case(seed=6, heads=heads, kv_heads=kv_heads, head_dim=head_dim, lens=lens, max_len=LONG)
+    _, k, v = _inputs(case, seed=7)
+    width = (heads + 2 * kv_heads) * head_dim
+    qkv = workloads.normal_bf16(np.random.default_rng(8), (case.batch, width))
+    positions = np.maximum(np.asarray(lens, dtype=np.int64) - 1, 0)
+    pages = np.asarray([case.block_table[b, p // 16] for b, p in enumerate(positions)], dtype=np.int64)
+    pages[5] = case.physical_blocks - 1           # a page that no sequence holds
+    slots = positions % 16
+    cos, sin = rotary_tables(head_dim, 500000.0, 4096)
+    splits = even_splits(case)
+    attn = torch.full((case.batch, heads, splits, head_dim), float("nan"), device="cuda")
+    lse = torch.full((case.batch, heads, splits), float("nan"), device="cuda")
+    keys, values = dev(k, torch.bfloat16), dev(v, torch.bfloat16)
+    out = torch.full((case.batch, heads, head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    device = [dev(qkv, torch.bfloat16), dev(case.lens), dev_u32(case.block_table), dev(cos, torch.bfloat16), dev(sin, torch.bfloat16),
+              dev(positions), dev(pages), dev(slots)]
+    p = [t.data_ptr() for t in device]
+    code = ks.lib().singe_decode_step_attention_bf16(
+        int(torch.cuda.current_stream().cuda_stream), out.data_ptr(), attn.data_ptr(), lse.data_ptr(), p[0], width, keys.data_ptr(),
+        values.data_ptr(), p[1], p[2], p[3], p[4], p[5], p[6], p[7], 8, case.batch, heads, kv_heads, head_dim, 16,
+        case.physical_blocks, case.block_table_batch_stride, splits, 4096, case.scale, ks.HINT_STABLE_PAGING if hinted else 0, None,
+        status.data_ptr())
+    torch.cuda.synchronize()
+    assert code == ks.OK and int(status.item()) == 0 and ops.take_device_error() == 0
+    c, s = llama_ref.bf16(cos)[positions], llama_ref.bf16(sin)[positions]
+    parts = np.split(qkv.reshape(case.batch, -1, head_dim), [heads, heads + kv_heads], axis=1)
+    queries, fresh = llama_ref.rotate(parts[0], c, s), llama_ref.rotate(parts[1], c, s)
+    for b, n in enumerate(lens):
+        if n > 0:
+            k[pages[b], slots[b]], v[pages[b], slots[b]] = fresh[b], parts[2][b]
+            assert (host(keys)[pages[b], slots[b]] == fresh[b]).all() and (host(values)[pages[b], slots[b]] == parts[2][b]).all()
+    assert_close_bf16(host(out), _oracle(case, queries, k, v), "decode step")
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,chunk", [(16, 4, 128, 512), (8, 8, 64, 520), (8, 8, 64, 100), (4, 4, 64, 4096)])
+def test_even_chunked_decode(heads, kv_heads, head_dim, chunk):
+    # queries in another order than their sequences, one sequence twice, a query without keys; chunks that begin inside a page
+    rng = np.random.default_rng(chunk)
+    sequence_of, lens = [2, 0, 1, 1, 3, 0] * 40, [700, 1, 512, 513, 0, 37] * 40
+    stride, pool = 64, 256
+    table = rng.permutation(pool).reshape(4, stride).astype(np.int32)
+    q, k, v = (workloads.normal_bf16(rng, shape) for shape in ((len(lens), heads, head_dim), (pool, 16, kv_heads, head_dim),
+                                                                (pool, 16, kv_heads, head_dim)))
+    bound = min(chunk + 15, stride * 16)
+    splits = ks.lib().singe_paged_kv_decode_even_splits(len(lens), heads, kv_heads, head_dim, bound, 16)
+    if splits == 0:          # (the rule leaves short chunks to the split grid: both forms are held to the same)
+        splits = 2
+    attn = torch.full((len(lens), heads, splits, head_dim), float("nan"), device="cuda")
+    lse = torch.full((len(lens), heads, splits), float("nan"), device="cuda")
+    out = torch.full((len(lens), heads, head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    i32 = lambda x: dev(np.asarray(x, dtype=np.int32))
+    Ops("bfloat16").call("singe_chunked_attention_bf16", int(torch.cuda.current_stream().cuda_stream), out, attn, lse,
+                         *[dev(x, torch.bfloat16) for x in (q, k, v)], i32(sequence_of), i32(lens), i32(table), len(lens), heads, kv_heads,
+                         head_dim, 16, pool, 4, stride, chunk, splits, head_dim ** -0.5, status)
+    assert int(status.item()) == 0
+    # the same keys, moved so that each query's chunk begins a page of its own
+    first = [(n - 1) // chunk * chunk if n else 0 for n in lens]
+    visible = np.asarray([n - f for n, f in zip(lens, first)], dtype=np.int32)
+    rows = lambda cache, b: cache[table[b]].reshape(-1, kv_heads, head_dim)
+    pages = -(-int(visible.max()) // 16)
+    moved = []
+    for cache in (k, v):
+        parts = np.zeros((len(lens), pages * 16, kv_heads, head_dim), dtype=np.float32)
+        for i, (b, f, n) in enumerate(zip(sequence_of, first, lens)):
+            parts[i, : n - f] = rows(cache, b)[f:n]
+        moved.append(parts.reshape(-1, 16, kv_heads, head_dim))
+    expect = oracle.paged_kv_decode_attention_f32(q, *moved, visible, np.arange(len(lens) * pages, dtype=np.uint32).reshape(len(lens), pages),
+                                                  batch=len(lens), heads=heads, kv_heads=kv_heads, head_dim=head_dim, block_size=16,
+                                                  block_table_batch_stride=pages, scale=head_dim ** -0.5)
+    assert_close_bf16(host(out), expect, f"chunks of {chunk}")
