@@ -33,14 +33,16 @@ def _check(code: int, where: str) -> None:
         raise SingeError(code, where)
 
 
+# A small call's time is its host side, so what every call does is kept to a few built-in operations: the raw handle of the
+# current stream (torch.cuda.current_stream() makes an object of it), dimensions checked by ``in`` and ``max``.
 def _stream(stream) -> int:
     if stream is None:
-        stream = torch.cuda.current_stream()
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return int(stream.cuda_stream)
 
 
 def _ptr(tensor) -> int | None:
-    return None if tensor is None else int(tensor.data_ptr())
+    return None if tensor is None else tensor.data_ptr()
 
 
 def _ensure(tensor: torch.Tensor, minimum: int, name: str) -> None:
@@ -50,10 +52,11 @@ def _ensure(tensor: torch.Tensor, minimum: int, name: str) -> None:
 
 
 _I32_MAX = 2**31 - 1
+_SUFFIXES = {torch.bfloat16: "bf16", torch.float16: "f16", torch.float32: "f32"}
 
 
 def _suffix(dtype: torch.dtype) -> str:
-    return {torch.bfloat16: "bf16", torch.float16: "f16", torch.float32: "f32"}[dtype]
+    return _SUFFIXES[dtype]
 
 
 # ------------------------------------------------------------------------------------------------
@@ -82,9 +85,9 @@ class PagedKvDecodeAttentionConfig:
         # validate_paged_kv_decode_attention_config (singe-kernel/src/cuda/attention/mod.rs:2963-2985)
         dims = (self.batch, self.heads, self.kv_heads, self.head_dim, self.block_size, self.physical_blocks,
                 self.block_table_batch_stride)
-        if any(d == 0 for d in dims) or self.heads % self.kv_heads != 0 or not math.isfinite(self.scale):
+        if 0 in dims or self.heads % self.kv_heads != 0 or not math.isfinite(self.scale):
             raise SingeError(ks.ERR_INVALID_LENGTH, "PagedKvDecodeAttentionConfig")
-        if any(d > _I32_MAX for d in dims):
+        if max(dims) > _I32_MAX:
             raise SingeError(ks.ERR_LENGTH_EXCEEDS_I32, "PagedKvDecodeAttentionConfig")
 
     def validate_lengths(self, out, query, key_cache, value_cache, actual_seq_lens, block_table) -> None:
@@ -115,9 +118,9 @@ class PagedKvPrefillAttentionConfig:
     def validate(self) -> None:
         dims = (self.batch, self.total_query_tokens, self.heads, self.kv_heads, self.head_dim, self.block_size,
                 self.physical_blocks, self.block_table_batch_stride)
-        if any(d == 0 for d in dims) or self.heads % self.kv_heads != 0 or not math.isfinite(self.scale):
+        if 0 in dims or self.heads % self.kv_heads != 0 or not math.isfinite(self.scale):
             raise SingeError(ks.ERR_INVALID_LENGTH, "PagedKvPrefillAttentionConfig")
-        if any(d > _I32_MAX for d in dims):
+        if max(dims) > _I32_MAX:
             raise SingeError(ks.ERR_LENGTH_EXCEEDS_I32, "PagedKvPrefillAttentionConfig")
 
 
@@ -134,9 +137,9 @@ class RaggedKvPrefillAttentionConfig:
 
     def validate(self) -> None:
         dims = (self.batch, self.total_query_tokens, self.total_kv_tokens, self.heads, self.kv_heads, self.head_dim)
-        if any(d == 0 for d in dims) or self.heads % self.kv_heads != 0 or not math.isfinite(self.scale):
+        if 0 in dims or self.heads % self.kv_heads != 0 or not math.isfinite(self.scale):
             raise SingeError(ks.ERR_INVALID_LENGTH, "RaggedKvPrefillAttentionConfig")
-        if any(d > _I32_MAX for d in dims):
+        if max(dims) > _I32_MAX:
             raise SingeError(ks.ERR_LENGTH_EXCEEDS_I32, "RaggedKvPrefillAttentionConfig")
 
 
@@ -351,8 +354,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None = Non
     n = weight.shape[0]
     if out is None:
         out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    matmul_bf16(out, x, weight, MatmulConfig(m, n, k, x.stride(0), weight.stride(0), out.stride(0), False, True),
-                stream)
+    name = "singe_matmul_bf16_f32" if out.dtype == torch.float32 else "singe_matmul_bf16_bf16"
+    _check(getattr(ks.lib(), name)(_stream(stream), out.data_ptr(), x.data_ptr(), weight.data_ptr(), m, n, k, x.stride(0),
+                                   weight.stride(0), out.stride(0), 0, 1), name)
     return out
 
 
