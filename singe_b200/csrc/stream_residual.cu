@@ -164,6 +164,109 @@ __global__ void __launch_bounds__(kNormThreads, 1) stream_step_kernel(const Stre
     }
 }
 
+// The sums of `count` values of every thread over the CTA, behind one barrier.  `scratch` is the call's own.
+template <int COUNT>
+__device__ __forceinline__ void cta_sums(float (&value)[COUNT], float (*scratch)[32]) {
+    const int warps = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int k = 0; k < COUNT; ++k) {
+        value[k] = warp_sum(value[k]);
+        if ((threadIdx.x & 31) == 0) scratch[k][threadIdx.x >> 5] = value[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < COUNT; ++k) {
+        value[k] = 0.0f;
+        for (int i = 0; i < warps; ++i) value[k] += scratch[k][i];
+    }
+}
+
+// The same for few rows of at most 4 * kNormThreads columns, as in a decode step, where nothing but the chain from the wait to
+// the last store counts: a thread owns four columns, keeps them in registers and has all it reads on its way at
+// once.  Four streams of 2048 columns, us by the kernel above and here, with one output and with two: 64 rows 5.5 and 3.1, 6.5 and
+// 4.1; 296 rows 6.5 and 5.5, 8.2 and 7.9; 450 rows 9.2 and 10.6, 11.3 and 16.7.  A Vatolorn decode step of 64 sequences 1008 and 953.
+template <typename T, int S>
+__global__ void __launch_bounds__(kNormThreads, 1) stream_step_row_kernel(const StreamStep p) {
+    grid_launch_dependents();
+    constexpr int VEC = 4;
+    __shared__ float scratch[3][32];
+    const int c = threadIdx.x * VEC;
+    const bool live = c < p.width;
+    const size_t row = blockIdx.x;
+    float mix[S][S], out[S], in[S];
+    Pack<VEC> gain = {}, gain0 = {}, gain1 = {};
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        out[s] = p.delta != nullptr ? p.out[s] : 0.0f;
+        in[s] = p.in != nullptr ? p.in[s] : 1.0f;
+#pragma unroll
+        for (int t = 0; t < S; ++t) mix[s][t] = p.delta != nullptr ? p.mix[s * S + t] : 0.0f;
+    }
+    grid_dependency_wait();
+    if (live && p.normed != nullptr) gain = load_pack<VEC>(static_cast<const T *>(p.weight) + c);
+    if (live && p.delta != nullptr && p.parts == 2) {
+        gain0 = load_pack<VEC>(static_cast<const T *>(p.part_weights[0]) + c);
+        gain1 = load_pack<VEC>(static_cast<const T *>(p.part_weights[1]) + c);
+    }
+    float *streams = p.streams + row * S * p.width;
+    Pack<VEC> x[S] = {}, y = {}, other = {};
+    if (p.table != nullptr) {
+        long long id = p.ids[row];
+        if (id < 0) id += p.vocab;
+        const bool valid = id >= 0 && id < p.vocab;
+        if (!valid && threadIdx.x == 0) report_status(p.status, kStatusIndexOutOfBounds);
+        if (live) x[0] = load_pack<VEC>(static_cast<const T *>(p.table) + static_cast<size_t>(valid ? id : 0) * p.width + c);
+#pragma unroll
+        for (int s = 1; s < S; ++s) x[s] = x[0];
+    } else if (live) {
+#pragma unroll
+        for (int s = 0; s < S; ++s) x[s] = load_pack<VEC>(streams + static_cast<size_t>(s) * p.width + c);
+    }
+    if (p.delta != nullptr) {
+        const T *delta = static_cast<const T *>(p.delta) + row * p.delta_stride;
+        if (live) y = load_pack<VEC>(delta + c);
+        if (p.parts == 2) {
+            if (live) other = load_pack<VEC>(delta + p.second_at + c);
+            float square[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                square[0] = square_chain(square[0], y.v[i]);
+                square[1] = square_chain(square[1], other.v[i]);
+            }
+            cta_sums<2>(square, scratch);
+            const float scale0 = p.part_scale / sqrtf(square[0] / static_cast<float>(p.width) + p.eps);
+            const float scale1 = p.part_scale / sqrtf(square[1] / static_cast<float>(p.width) + p.eps);
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) y.v[i] = fmaf(y.v[i] * scale0, gain0.v[i], other.v[i] * scale1 * gain1.v[i]);
+        }
+    }
+    Pack<VEC> u = {};
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+        Pack<VEC> next = x[t];
+        if (p.delta != nullptr) {
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                next.v[i] = out[t] * y.v[i];
+#pragma unroll
+                for (int s = 0; s < S; ++s) next.v[i] = fmaf(mix[s][t], x[s].v[i], next.v[i]);
+            }
+        }
+        if (p.store && live) store_pack<VEC>(streams + static_cast<size_t>(t) * p.width + c, next);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) u.v[i] = fmaf(in[t], next.v[i], u.v[i]);
+    }
+    if (p.normed == nullptr) return;
+    float square[1] = {0.0f};
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) square[0] = square_chain(square[0], u.v[i]);
+    cta_sums<1>(square, scratch + 2);
+    const float scale = 1.0f / sqrtf(square[0] / static_cast<float>(p.width) + p.eps);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) u.v[i] = u.v[i] * scale * gain.v[i] * p.normed_scale;
+    if (live) store_pack<VEC>(static_cast<T *>(p.normed) + row * p.normed_stride + c, u);
+}
+
 template <typename T>
 int stream_step(singe_stream_t stream, const StreamStep &p, size_t rows) {
     if (rows == 0 || p.width <= 0 || p.count <= 0 || (p.parts != 1 && p.parts != 2)) return SINGE_ERR_INVALID_LENGTH;
@@ -187,6 +290,16 @@ int stream_step(singe_stream_t stream, const StreamStep &p, size_t rows) {
                       aligned_to(p.table, bytes) && aligned_to(p.part_weights[0], bytes) && aligned_to(p.part_weights[1], bytes);
     const size_t shared = static_cast<size_t>(p.width) * sizeof(float);
     if (shared > 200 * 1024) return SINGE_ERR_UNSUPPORTED_WIDTH;
+    const unsigned row_threads = static_cast<unsigned>((p.width + 127) / 128 * 32);
+    if (wide && row_threads <= kNormThreads && rows <= 2 * static_cast<size_t>(device_sm_count())) {   // (figures above)
+        auto row_kernel = p.count == 1 ? stream_step_row_kernel<T, 1> : p.count == 2 ? stream_step_row_kernel<T, 2>
+                        : p.count == 3 ? stream_step_row_kernel<T, 3> : p.count == 4 ? stream_step_row_kernel<T, 4> : nullptr;
+        if (row_kernel != nullptr) {
+            SINGE_CUDA_TRY(launch_dependent(row_kernel, dim3(static_cast<unsigned>(rows)), dim3(row_threads), 0,
+                                            static_cast<cudaStream_t>(stream), kLaunchGlue, 1, p));
+            return launch_status();
+        }
+    }
     auto kernel = wide ? stream_step_kernel<T, 4, 0> : stream_step_kernel<T, 1, 0>;
     int which = wide ? 0 : 1;
 #define SINGE_STREAMS(S_)                       \
