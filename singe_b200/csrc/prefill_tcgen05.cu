@@ -780,44 +780,38 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         constexpr bool kIsBf16 = std::is_same<T, __nv_bfloat16>::value;
         constexpr uint32_t kIdescQK = make_instr_desc(kTile, kTile, kIsBf16, 0, 0);      // A, B K-major
         constexpr uint32_t kIdescPV = make_instr_desc(kTile, HD, kIsBf16, 0, 1);   // B (V) MN-major
-        auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool {
-            return __all_sync(0xffffffffu, mbar_wait(bar, parity) ? 1 : 0) != 0;
-        };
+        // The loops over key tiles run in one elected thread, as those of the linear layers do: with every lane waiting, a vote
+        // behind each wait and the issue under a lane test, the 24 MMAs of a tile with two-term weights came late: the step of four chunks
+        // and 28 decoding sequences above 157 -> 131 us (kernel), 60 - 480 token prompts of 64 sequences 15.2 -> 13.0.  Long prompts are where
+        // they were, 616 and 613: there softmax is the longer part of the chain.
+        const uint64_t q_desc = make_smem_desc(q_smem, 16, 1024), k_desc = make_smem_desc(k_smem, 16, 1024);
+        const uint64_t v_desc = make_smem_desc(v_smem, kHalfTileBytes, 1024);   // (a descriptor's address counts in 16 bytes)
         // S_x = Q_query K(stage)^T; `last` releases the Q tile
         auto issue_qk = [&](int x, int stage, bool last, int query) {
-            if (elect_one()) {
-                const uint32_t q_tile = q_smem + query * kTileBytes;
-                const uint32_t k_tile = k_smem + stage * kTileBytes;
+            const uint64_t a = q_desc + query * (kTileBytes >> 4), b = k_desc + stage * (kTileBytes >> 4);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks) {
-                    const uint32_t within = (ks >> 2) * kHalfTileBytes + (ks & 3) * 32;
-                    umma_ss(tmem_base + x * kTile, make_smem_desc(q_tile + within, 16, 1024),
-                            make_smem_desc(k_tile + within, 16, 1024), kIdescQK, ks > 0 ? 1u : 0u);
-                }
-                tcgen05_commit(bar_s_full + x * 8);
-                if (last) tcgen05_commit(bar_q_empty + query * 8);
+            for (int ks = 0; ks < HD / 16; ++ks) {
+                const uint32_t within = ((ks >> 2) * kHalfTileBytes + (ks & 3) * 32) >> 4;
+                umma_ss(tmem_base + x * kTile, a + within, b + within, kIdescQK, ks > 0 ? 1u : 0u);
             }
-            __syncwarp();
+            tcgen05_commit(bar_s_full + x * 8);
+            if (last) tcgen05_commit(bar_q_empty + query * 8);
         };
         // O_x (+)= P_x V(stage): 16 keys per step, P advances 8 packed columns, V two 8-row groups (2 x 1024 bytes);
         // the second 64 dims of V are the next box, 16 KB further (leading byte offset).
         auto issue_pv = [&](int x, int stage, bool accumulate, bool last) {
-            if (elect_one()) {
-                const uint32_t v_tile = v_smem + stage * kTileBytes;
+            const uint64_t v = v_desc + stage * (kTileBytes >> 4);
 #pragma unroll
-                for (int ks = 0; ks < kTile / 16; ++ks) {
-                    // TENSOR: a chunk of 32 keys holds 16 columns of leading terms and 16 of the rest
-                    const uint32_t at = TENSOR ? (ks >> 1) * kChunk + (ks & 1) * 8 : ks * 8;
-                    const uint64_t v_desc = make_smem_desc(v_tile + ks * 2048, kHalfTileBytes, 1024);
-                    umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at, v_desc, kIdescPV,
-                            (accumulate || ks > 0) ? 1u : 0u);
-                    if (TENSOR) {
-                        umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at + kChunk / 2, v_desc, kIdescPV, 1u);
-                    }
+            for (int ks = 0; ks < kTile / 16; ++ks) {
+                // TENSOR: a chunk of 32 keys holds 16 columns of leading terms and 16 of the rest
+                const uint32_t at = TENSOR ? (ks >> 1) * kChunk + (ks & 1) * 8 : ks * 8;
+                umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at, v + ks * (2048 >> 4), kIdescPV,
+                        (accumulate || ks > 0) ? 1u : 0u);
+                if (TENSOR) {
+                    umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at + kChunk / 2, v + ks * (2048 >> 4), kIdescPV, 1u);
                 }
-                if (last) tcgen05_commit(bar_o_full + x * 8);
             }
-            __syncwarp();
+            if (last) tcgen05_commit(bar_o_full + x * 8);
         };
         int g = 0;                 // key tiles consumed so far, over all items
         int q_uses[2] = {0, 0};    // Q tiles consumed so far
@@ -842,23 +836,20 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         // first Q K^T of both tiles of `item` on key stage `stage` (already waited for)
         auto first_qk = [&](const Item &item, int x, int stage) -> bool {
             if (item.tiles[x] == 0 || (WINDOW && item.first[x] != item.first[0])) return true;  // (tile B's may come later)
-            if (!wait_all(bar_q_full + x * 8, q_uses[x] & 1)) return false;
+            if (!mbar_wait(bar_q_full + x * 8, q_uses[x] & 1)) return false;
             ++q_uses[x];
             tcgen05_fence_after();
             issue_qk(x, stage, item.tiles[x] == item.first[x] + 1, x);
             return true;
         };
-        Item item = next_item();
-        if (item.key_tiles > 0) {
-            if (!wait_all(bar_k_full, 0)) failed = true;
-            if (!failed && (!first_qk(item, 0, 0) || !first_qk(item, 1, 0))) failed = true;
-            if (!failed) {
-                if (elect_one()) tcgen05_commit(bar_k_empty);
-                __syncwarp();
+        // Everything of one item, and the first Q K^T of the following one; one thread.
+        bool begun = false;
+        auto run_item = [&](const Item &item, const Item &following) {
+            if (!begun) {
+                if (!mbar_wait(bar_k_full, 0)) failed = true;
+                if (!failed && (!first_qk(item, 0, 0) || !first_qk(item, 1, 0))) failed = true;
+                if (!failed) tcgen05_commit(bar_k_empty);
             }
-        }
-        while (item.key_tiles > 0 && !failed) {
-            const Item following = next_item();
             if constexpr (TENSOR) {
                 // A single query tile: key tile j's scores stand in tile A's or tile B's place by turns, so that Q K^T of the
                 // next one runs beside this one's softmax, and each place has its own O.
@@ -868,13 +859,12 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     const int x = (j - item.first[0]) & 1;
                     const bool more = j + 1 < item.key_tiles;
                     auto next_keys = [&]() -> bool {
-                        if (!wait_all(bar_k_full + next * 8, ((g + 1) >> 1) & 1)) return false;
+                        if (!mbar_wait(bar_k_full + next * 8, ((g + 1) >> 1) & 1)) return false;
                         tcgen05_fence_after();
                         return true;
                     };
                     auto release_keys = [&]() {
-                        if (elect_one()) tcgen05_commit(bar_k_empty + next * 8);
-                        __syncwarp();
+                        tcgen05_commit(bar_k_empty + next * 8);
                     };
                     if (more) {
                         if (!next_keys()) {
@@ -884,9 +874,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                         issue_qk(x ^ 1, next, j + 2 == item.key_tiles, 0);
                         release_keys();
                     }
-                    if (!wait_all(bar_v_full + stage * 8, (g >> 1) & 1) ||
-                        (j < item.first[0] + 2 && o_done[x] > 0 && !wait_all(bar_o_empty + x * 8, (o_done[x] - 1) & 1)) ||
-                        !wait_all(bar_p_full + x * 8, p_uses[x] & 1)) {
+                    if (!mbar_wait(bar_v_full + stage * 8, (g >> 1) & 1) ||
+                        (j < item.first[0] + 2 && o_done[x] > 0 && !mbar_wait(bar_o_empty + x * 8, (o_done[x] - 1) & 1)) ||
+                        !mbar_wait(bar_p_full + x * 8, p_uses[x] & 1)) {
                         failed = true;
                         break;
                     }
@@ -895,8 +885,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     const bool last = j + 2 >= item.key_tiles;
                     issue_pv(x, stage, j >= item.first[0] + 2, last);
                     if (last) ++o_done[x];
-                    if (elect_one()) tcgen05_commit(bar_v_empty + stage * 8);
-                    __syncwarp();
+                    tcgen05_commit(bar_v_empty + stage * 8);
                     if (!more && following.key_tiles > 0) {
                         if (!next_keys() || !first_qk(following, 0, next) || !first_qk(following, 1, next)) {
                             failed = true;
@@ -905,17 +894,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                         release_keys();
                     }
                 }
-                if (item.alternate) {
-                    item = following;
-                    continue;
-                }
             }
-            for (int j = item.first[0]; j < item.key_tiles && !failed; ++j, ++g) {
+            for (int j = item.first[0]; !item.alternate && j < item.key_tiles && !failed; ++j, ++g) {
                 const int stage = g & 1;
                 const int next = (g + 1) & 1;
                 const bool more = j + 1 < item.key_tiles;          // this item has another key tile
                 const bool onward = more || following.key_tiles > 0;  // some Q K^T follows on key tile g + 1
-                if (!wait_all(bar_v_full + stage * 8, (g >> 1) & 1)) {
+                if (!mbar_wait(bar_v_full + stage * 8, (g >> 1) & 1)) {
                     failed = true;
                     break;
                 }
@@ -924,11 +909,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     if (failed) continue;
                     if (j < item.tiles[x] && (!WINDOW || j >= item.first[x])) {
                         // the previous item's epilogue must have taken O out of tensor memory
-                        if (j == item.first[x] && o_done[x] > 0 && !wait_all(bar_o_empty + x * 8, (o_done[x] - 1) & 1)) {
+                        if (j == item.first[x] && o_done[x] > 0 && !mbar_wait(bar_o_empty + x * 8, (o_done[x] - 1) & 1)) {
                             failed = true;
                             continue;
                         }
-                        if (!wait_all(bar_p_full + x * 8, p_uses[x] & 1)) {
+                        if (!mbar_wait(bar_p_full + x * 8, p_uses[x] & 1)) {
                             failed = true;
                             continue;
                         }
@@ -939,12 +924,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                         if (last) ++o_done[x];
                     }
                     if (x == 1) {
-                        if (elect_one()) tcgen05_commit(bar_v_empty + stage * 8);
-                        __syncwarp();
+                        tcgen05_commit(bar_v_empty + stage * 8);
                     }
                     if (onward) {
                         if (x == 0) {
-                            if (!wait_all(bar_k_full + next * 8, ((g + 1) >> 1) & 1)) {
+                            if (!mbar_wait(bar_k_full + next * 8, ((g + 1) >> 1) & 1)) {
                                 failed = true;
                                 continue;
                             }
@@ -952,7 +936,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                         }
                         if (more) {
                             if (WINDOW && item.tiles[x] > 0 && item.first[x] != item.first[0] && j + 1 == item.first[x]) {
-                                if (!wait_all(bar_q_full + x * 8, q_uses[x] & 1)) {
+                                if (!mbar_wait(bar_q_full + x * 8, q_uses[x] & 1)) {
                                     failed = true;
                                     continue;
                                 }
@@ -967,12 +951,30 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                             continue;
                         }
                         if (x == 1) {
-                            if (elect_one()) tcgen05_commit(bar_k_empty + next * 8);
-                            __syncwarp();
+                            tcgen05_commit(bar_k_empty + next * 8);
                         }
                     }
                 }
             }
+        };
+        Item item = next_item();
+        while (item.key_tiles > 0 && !failed) {
+            const Item following = next_item();   // (the whole warp takes part)
+            const bool issues = elect_one();
+            if (issues) run_item(item, following);
+            __syncwarp();
+            // the elected lane's counts and verdict
+            begun = true;
+            const int leader = __ffs(__ballot_sync(0xffffffffu, issues)) - 1;
+            auto share = [&](int value) { return __shfl_sync(0xffffffffu, value, leader); };
+            g = share(g);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                q_uses[x] = share(q_uses[x]);
+                p_uses[x] = share(p_uses[x]);
+                o_done[x] = share(o_done[x]);
+            }
+            failed = share(failed ? 1 : 0) != 0;
             item = following;
         }
     } else {
