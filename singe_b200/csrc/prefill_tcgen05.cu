@@ -26,6 +26,8 @@
 //              recomputes exactly those.
 //   warp 8     MMA issuer and tensor-memory owner.  Issue order per key tile j:
 //                 PV_A(j), QK_A(j+1), PV_B(j), QK_B(j+1)
+//              (P V in two halves of the keys, each as soon as its weights are there: a tile's softmax, P V and Q K^T are a chain, and
+//              the first half's products come off it.  8192 + 4096 + 2048 + 1024 tokens 745 -> 721 us at the power limit, 613 -> 605 at full clocks)
 //              (S = Q K^T: 8 x tcgen05.mma 128x128x16, both operands K-major in shared memory; O += P V: 8 x
 //              tcgen05.mma with P read from tensor memory and V MN-major), so softmax_A(j) overlaps PV_B(j-1) and
 //              QK_B(j), softmax_B(j) overlaps PV_A(j) and QK_A(j+1).
@@ -109,12 +111,13 @@ struct PrefillParams {
 // output is not finite (a hidden key's value may be anything, and zero times infinity is not zero).
 // Bound by the tensor core and the special-function unit alike: 8 + 16 MMAs of 128 x 128 x 16 and 16384 exponentials a
 // key tile.  One step of four 510-token chunks and 28 decoding sequences behind 0 - 3000 tokens of context, 32 query heads on 8:
-// 172 us, 238 with items in order of their pair index and lone tiles a key tile at a time, 40.2 ms by one warp per row and head.
+// 158 us with the rows behind; 175 before one thread issued the MMAs and the weights came in halves, 238 with items in order of their pair
+// index and lone tiles a key tile at a time, 40.2 ms by one warp per row and head.
 // Against 64 bits, this step and twelve of other sizes: outputs 1.6585e-3 off by either kernel, which is their rounding to bf16
 // (the squares of the two errors differ by 4e-6 squared: two terms, and long sums in the tensor core); log sums 5.6e-8, by the
 // general kernel 6.3e-8.
-// A pair's key tile takes 4800 - 5000 clk (3072 of MMA; softmax and Q K^T of a tile are a chain), a lone tile's 3000 in this
-// mix, whose cold cache all SMs read at once.
+// A pair's key tile has 3072 clk of MMA, and a tile's softmax and Q K^T are a chain; a lone tile's step took 3000 in this mix, whose cold
+// cache all SMs read at once.
 struct TensorPaging {
     const void *query_offsets;
     const void *page_offsets;
@@ -130,7 +133,7 @@ struct TensorPaging {
 struct NoPaging {};
 
 constexpr int kMaxTensorSequences = 1024;
-constexpr int kTensorBarriers = 22;  // (one of them only keeps what follows aligned)
+constexpr int kTensorBarriers = 24;  // (one of them only keeps what follows aligned)
 constexpr int kMaxOrdered = 1024;   // (sequence, pair) entries that are put in order of their cost
 
 __device__ __forceinline__ long long paging_value(const void *list, int width, int at) {
@@ -289,10 +292,19 @@ __device__ __forceinline__ void chunk_exp_store(const uint32_t (&sc)[kChunk], ui
     }
 }
 
+// This warp's share of half a tile's weights is in tensor memory.
+__device__ __forceinline__ void hand_over(uint32_t bar, int lane) {
+    tmem_wait_st();
+    tcgen05_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
 // One row of one key tile: S (128 f32 columns at `tmem_s`) -> P (64 packed columns over the same place), chunk by
 // chunk with the next chunk's load in flight.
 template <typename T, int MASK, bool SPLIT>
-__device__ __forceinline__ void tile_exp(uint32_t tmem_s, float2 scale2, float2 bias2, int low, int limit, float2 (&sum)[2]) {
+__device__ __forceinline__ void tile_exp(uint32_t tmem_s, float2 scale2, float2 bias2, int low, int limit, float2 (&sum)[2],
+                                         uint32_t bar_half, int lane) {
     uint32_t buf[2][kChunk];
     tmem_ld_x32(tmem_s, buf[0]);
 #pragma unroll
@@ -301,6 +313,7 @@ __device__ __forceinline__ void tile_exp(uint32_t tmem_s, float2 scale2, float2 
         if (c + 1 < kTile / kChunk) tmem_ld_x32(tmem_s + (c + 1) * kChunk, buf[(c + 1) & 1]);
         chunk_exp_store<T, MASK, SPLIT>(buf[c & 1], tmem_s + c * (SPLIT ? kChunk : kChunk / 2), scale2, bias2, low - c * kChunk,
                                         limit - c * kChunk, sum);
+        if (c & 1) hand_over(bar_half + (c >> 1) * 8, lane);
     }
 }
 
@@ -546,11 +559,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     const uint32_t bar_v_full = bars + 64;    // [2]
     const uint32_t bar_v_empty = bars + 80;   // [2]
     const uint32_t bar_s_full = bars + 96;    // [2 tiles]
-    const uint32_t bar_p_full = bars + 112;   // [2 tiles], one arrival per softmax warp of the tile
-    const uint32_t bar_o_full = bars + 128;   // [2 tiles]
-    const uint32_t bar_o_empty = bars + 144;  // [2 tiles], one arrival per softmax warp of the tile
-    const uint32_t bar_share = bars + 160;    // TENSOR: tile B's half of an alternating item, one arrival per softmax warp
-    constexpr int kBarriers = TENSOR ? kTensorBarriers : 20;
+    const uint32_t bar_o_full = bars + 112;   // [2 tiles]
+    const uint32_t bar_p_full = bars + 128;   // [2 tiles][2 halves of the keys], one arrival per softmax warp of the tile
+    const uint32_t bar_o_empty = bars + 160;  // [2 tiles], one arrival per softmax warp of the tile
+    const uint32_t bar_share = bars + 176;    // TENSOR: tile B's half of an alternating item, one arrival per softmax warp
+    constexpr int kBarriers = TENSOR ? kTensorBarriers : 22;
     const uint32_t words = bars + 8 * kBarriers;
     volatile uint32_t *holder_ptr = reinterpret_cast<volatile uint32_t *>(smem_raw + (words - raw));
     volatile int *shared_tmax = reinterpret_cast<volatile int *>(smem_raw + (words + 4 - raw));
@@ -658,7 +671,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
 
     if (tid == 0) {
         for (int i = 0; i < kBarriers; ++i) {
-            const bool by_warps = i == 14 || i == 15 || i >= 18;  // p_full[2], o_empty[2], share
+            const bool by_warps = i >= 16;  // p_full, o_empty, share
             mbar_init(bars + 8 * i, by_warps ? 4 : 1);
         }
         mbar_init_fence();
@@ -786,6 +799,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         // they were, 616 and 613: there softmax is the longer part of the chain.
         const uint64_t q_desc = make_smem_desc(q_smem, 16, 1024), k_desc = make_smem_desc(k_smem, 16, 1024);
         const uint64_t v_desc = make_smem_desc(v_smem, kHalfTileBytes, 1024);   // (a descriptor's address counts in 16 bytes)
+        int p_uses[2] = {0, 0};    // P tiles consumed so far
         // S_x = Q_query K(stage)^T; `last` releases the Q tile
         auto issue_qk = [&](int x, int stage, bool last, int query) {
             const uint64_t a = q_desc + query * (kTileBytes >> 4), b = k_desc + stage * (kTileBytes >> 4);
@@ -799,10 +813,19 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         };
         // O_x (+)= P_x V(stage): 16 keys per step, P advances 8 packed columns, V two 8-row groups (2 x 1024 bytes);
         // the second 64 dims of V are the next box, 16 KB further (leading byte offset).
-        auto issue_pv = [&](int x, int stage, bool accumulate, bool last) {
+        // The weights come in halves, so that the first half's products run beside the softmax of the second.
+        auto issue_pv = [&](int x, int stage, bool accumulate, bool last) -> bool {
             const uint64_t v = v_desc + stage * (kTileBytes >> 4);
+            const uint32_t parity = p_uses[x] & 1;
+            ++p_uses[x];
+            if (!mbar_wait(bar_p_full + x * 16, parity)) return false;
+            tcgen05_fence_after();
 #pragma unroll
             for (int ks = 0; ks < kTile / 16; ++ks) {
+                if (ks == kTile / 32) {
+                    if (!mbar_wait(bar_p_full + x * 16 + 8, parity)) return false;
+                    tcgen05_fence_after();
+                }
                 // TENSOR: a chunk of 32 keys holds 16 columns of leading terms and 16 of the rest
                 const uint32_t at = TENSOR ? (ks >> 1) * kChunk + (ks & 1) * 8 : ks * 8;
                 umma_ts(tmem_base + 2 * kTile + x * HD, tmem_base + x * kTile + at, v + ks * (2048 >> 4), kIdescPV,
@@ -812,10 +835,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 }
             }
             if (last) tcgen05_commit(bar_o_full + x * 8);
+            return true;
         };
         int g = 0;                 // key tiles consumed so far, over all items
         int q_uses[2] = {0, 0};    // Q tiles consumed so far
-        int p_uses[2] = {0, 0};    // P tiles consumed so far
         int o_done[2] = {0, 0};    // outputs handed to the epilogue so far
         int round = 0;
         // the next item with work, or key_tiles == 0 when there is none
@@ -875,15 +898,15 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                         release_keys();
                     }
                     if (!mbar_wait(bar_v_full + stage * 8, (g >> 1) & 1) ||
-                        (j < item.first[0] + 2 && o_done[x] > 0 && !mbar_wait(bar_o_empty + x * 8, (o_done[x] - 1) & 1)) ||
-                        !mbar_wait(bar_p_full + x * 8, p_uses[x] & 1)) {
+                        (j < item.first[0] + 2 && o_done[x] > 0 && !mbar_wait(bar_o_empty + x * 8, (o_done[x] - 1) & 1))) {
                         failed = true;
                         break;
                     }
-                    ++p_uses[x];
-                    tcgen05_fence_after();
                     const bool last = j + 2 >= item.key_tiles;
-                    issue_pv(x, stage, j >= item.first[0] + 2, last);
+                    if (!issue_pv(x, stage, j >= item.first[0] + 2, last)) {
+                        failed = true;
+                        break;
+                    }
                     if (last) ++o_done[x];
                     tcgen05_commit(bar_v_empty + stage * 8);
                     if (!more && following.key_tiles > 0) {
@@ -913,14 +936,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                             failed = true;
                             continue;
                         }
-                        if (!mbar_wait(bar_p_full + x * 8, p_uses[x] & 1)) {
+                        const bool last = j == item.tiles[x] - 1;
+                        if (!issue_pv(x, stage, j > item.first[x], last)) {
                             failed = true;
                             continue;
                         }
-                        ++p_uses[x];
-                        tcgen05_fence_after();
-                        const bool last = j == item.tiles[x] - 1;
-                        issue_pv(x, stage, j > item.first[x], last);
                         if (last) ++o_done[x];
                     }
                     if (x == 1) {
@@ -1074,19 +1094,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 const float2 bias2 = make_float2(bias, bias);
                 float2 sum[2] = {make_float2(row_sum, 0.0f), make_float2(0.0f, 0.0f)};
                 if (WINDOW && lower) {
-                    tile_exp<T, kMaskBoth, TENSOR>(tmem_s, scale2, bias2, low, limit, sum);
+                    tile_exp<T, kMaskBoth, TENSOR>(tmem_s, scale2, bias2, low, limit, sum, bar_p_full + x * 16, lane);
                 } else if (partial) {
-                    tile_exp<T, kMaskEnd, TENSOR>(tmem_s, scale2, bias2, low, limit, sum);
+                    tile_exp<T, kMaskEnd, TENSOR>(tmem_s, scale2, bias2, low, limit, sum, bar_p_full + x * 16, lane);
                 } else {
-                    tile_exp<T, kMaskNone, TENSOR>(tmem_s, scale2, bias2, low, limit, sum);
+                    tile_exp<T, kMaskNone, TENSOR>(tmem_s, scale2, bias2, low, limit, sum, bar_p_full + x * 16, lane);
                 }
                 row_sum = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
-                tmem_wait_st();
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(bar_p_full + x * 8);
-                }
                 in_range = in_range && row_sum < kOverflowLimit;  // false for inf and NaN too
             }
             if (failed) break;
@@ -1203,7 +1217,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     }
 }
 
-constexpr int kPrefillSmem = 6 * kTileBytes + 8 * 20 + 32 + kMaxRankTiles * 4 + kRedoCapacity * 4 + 1024;
+constexpr int kPrefillSmem = 6 * kTileBytes + 8 * 22 + 32 + kMaxRankTiles * 4 + kRedoCapacity * 4 + 1024;
 
 }  // namespace
 
@@ -1242,7 +1256,7 @@ int launch_tensor(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorM
                   const PrefillParams &params, const TensorPaging &paging, unsigned persistent) {
     static int raised[kMaxDevices] = {0};
     constexpr int kBytes = kPrefillSmem + (4 * kMaxTensorSequences - kRedoCapacity + 3 * kMaxOrdered) * 4 +
-                           (kTensorBarriers - 20) * 8 + kTile * 8;
+                           (kTensorBarriers - 22) * 8 + kTile * 8;
     static_assert(kBytes <= 227 * 1024, "shared memory of one CTA");
     const auto kernel = prefill_tcgen05_kernel<__nv_bfloat16, HD, false, true, false, WINDOW, true>;
     SINGE_CUDA_TRY(ensure_dynamic_shared(kernel, kBytes, raised));
