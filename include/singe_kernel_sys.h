@@ -332,6 +332,21 @@ int singe_paged_attention_f32(singe_stream_t stream, float *out, float *lse, con
                               size_t page_size, size_t cache_pages, size_t sequences, size_t table_len, float scale,
                               int causal, size_t window, uint32_t *status);
 
+/* The same into uninitialised out and lse: rows that nothing is computed for (tokens of no sequence, rows of refused
+ * sequences) become zeros and -inf, where the two above leave them as they are. */
+int singe_paged_attention_whole_bf16(singe_stream_t stream, void *out, float *lse, const void *query,
+                               const void *key_cache, const void *value_cache, const void *query_offsets,
+                               const void *page_offsets, const void *pages, const void *last_page_lengths,
+                               int index_width, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim,
+                               size_t page_size, size_t cache_pages, size_t sequences, size_t table_len, float scale,
+                               int causal, size_t window, uint32_t *status);
+int singe_paged_attention_whole_f32(singe_stream_t stream, float *out, float *lse, const float *query,
+                              const float *key_cache, const float *value_cache, const void *query_offsets,
+                              const void *page_offsets, const void *pages, const void *last_page_lengths,
+                              int index_width, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim,
+                              size_t page_size, size_t cache_pages, size_t sequences, size_t table_len, float scale,
+                              int causal, size_t window, uint32_t *status);
+
 /* The same with the remaining AttentionOptions field of the path, the cap on the scaled scores
  * (singe/src/tensor/neural.rs:26-32; CPU: score = cap * tanh(score / cap) before the softmax,
  * singe/src/backend/cpu/normalization/attention.rs:445,500; CUDA: paged_attention.rs:112,662-672).  softcap == 0: none.

@@ -315,22 +315,31 @@ struct TensorPagedPolicy {
 // tokens of a CTA lie far apart: a sequence that is left out is left to many.  Nothing is kept that a later call could meet.
 // The step of 2072 tokens on 32 heads of prefill_tcgen05.cu's notes takes 172.7 us, 171.7 with a word of the device that said
 // whether anything was left (once raised, it made every later call a fifth longer); steps of 60 - 950 tokens 0 - 1.8 us more than
-// with that word.  One of the four chunks left out: 3.2 ms (1.4 with a warp per row, which had every row look its sequence up).
+// with that word.  WHOLE: `out` and `lse` come uninitialised, and the rows that nothing is computed for (tokens of no sequence,
+// rows of refused ones) become zeros and -inf here; two fills of the whole outputs in front took 10 us of the step above.  One of the four chunks left out: 3.2 ms (1.4 with a warp per row, which had every row look its sequence up).
 constexpr int kLeftTokens = 8, kLeftWarps = 16;
 
-template <typename T, typename Index, int MAX>
+template <typename T, typename Index, int MAX, bool WHOLE>
 __global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const TensorPagedPolicy<T, Index> policy, int head_dim, float scale,
                                                                     uint32_t *status) {
     __shared__ unsigned shared_left[kLeftTokens];
     grid_launch_dependents();
     grid_dependency_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t raised = status != nullptr ? *status : 1u;
+    uint32_t raised = status != nullptr ? *status : 1u;
+    // sequences that are all well-formed cover the tokens from the first offset to the last
+    if (WHOLE && (policy.query_offsets[0] != 0 || policy.query_offsets[policy.sequences] != policy.tokens)) raised = 1u;
+    auto clear_row = [&](size_t row) {
+        for (int d = lane; d < head_dim; d += 32) policy.out[row * head_dim + d] = from_float<T>(0.0f);
+        if (lane == 0) policy.lse[row] = -INFINITY;
+        __syncwarp();
+    };
     const long long slots = (policy.tokens + kLeftTokens - 1) / kLeftTokens;
     for (long long slot = blockIdx.x; slot < slots; slot += gridDim.x) {
         const long long token = slot + warp * slots;
         const bool mine = warp < kLeftTokens && token < policy.tokens;
         bool all = false;  // whether every row of the token is left
+        bool none = false; // WHOLE: no sequence owns the token, or one that is refused
         // (both loads are on their way before either is waited for)
         const bool first_marked = mine && lane < policy.heads && isnan(policy.lse[token * policy.heads + lane]);
         if (mine && __shfl_sync(0xffffffffu, raised, 0) != 0u) {  // (one answer for a warp)
@@ -353,12 +362,21 @@ __global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const Ten
                 }
             }
             all = __any_sync(0xffffffffu, all) != 0;
+            if (WHOLE) {
+                none = owner < 0;
+                if (!none) {   // a sequence whose paging is refused
+                    const long long first = policy.page_offsets[owner], last = policy.page_offsets[owner + 1];
+                    const long long length = policy.last_page_lengths[owner];
+                    none = !(0 <= first && first <= last && last <= policy.table_len) ||
+                           (first != last && (length < 0 || length > policy.page_size));
+                }
+            }
         }
         for (int base = 0; base < policy.heads; base += 32) {
             if (warp < kLeftTokens) {
                 const bool marked = base == 0 ? first_marked
                                               : mine && base + lane < policy.heads && isnan(policy.lse[token * policy.heads + base + lane]);
-                const bool left = marked || (all && base + lane < policy.heads);
+                const bool left = marked || ((all || none) && base + lane < policy.heads);
                 const unsigned rows = __ballot_sync(0xffffffffu, left);
                 if (lane == 0) shared_left[warp] = rows;
             }
@@ -368,6 +386,7 @@ __global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const Ten
                 for (unsigned rows = shared_left[t]; rows != 0; rows &= rows - 1) {
                     if (number++ % kLeftWarps == warp) {
                         const size_t row = static_cast<size_t>((slot + t * slots) * policy.heads + base + __ffs(rows) - 1);
+                        if (WHOLE) clear_row(row);
                         attention_general_row<T, TensorPagedPolicy<T, Index>, MAX>(policy, row, head_dim, scale, LseKind::Base2, -INFINITY,
                                                                                    status, 0.0f);
                     }
@@ -380,10 +399,29 @@ __global__ void __launch_bounds__(32 * kLeftWarps, 2) left_rows_kernel(const Ten
 
 template <typename T, typename Index>
 int launch_left_rows(cudaStream_t stream, const TensorPagedPolicy<T, Index> &policy, size_t tokens, size_t head_dim, float scale,
-                     uint32_t *status) {
+                     uint32_t *status, bool whole) {
     const size_t blocks = (tokens + kLeftTokens - 1) / kLeftTokens, most = static_cast<size_t>(device_sm_count()) * 2;
-    SINGE_CUDA_TRY(launch_dependent(left_rows_kernel<T, Index, kMaxPerLane>, dim3(static_cast<unsigned>(blocks < most ? blocks : most)),
+    const auto kernel = whole ? left_rows_kernel<T, Index, kMaxPerLane, true> : left_rows_kernel<T, Index, kMaxPerLane, false>;
+    SINGE_CUDA_TRY(launch_dependent(kernel, dim3(static_cast<unsigned>(blocks < most ? blocks : most)),
                                     dim3(32 * kLeftWarps), 0, stream, kLaunchGlue, 1, policy, static_cast<int>(head_dim), scale, status));
+    return launch_status();
+}
+
+// out = 0, lse = -inf: what rows hold that nothing is computed for.
+template <typename T>
+__global__ void clear_rows_kernel(T *out, float *lse, long long values, long long rows) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const long long threads = static_cast<long long>(gridDim.x) * blockDim.x, first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (long long i = first; i < values; i += threads) out[i] = from_float<T>(0.0f);
+    for (long long i = first; i < rows; i += threads) lse[i] = -INFINITY;
+}
+
+template <typename T>
+int clear_rows(cudaStream_t stream, void *out, float *lse, size_t rows, size_t head_dim) {
+    SINGE_CUDA_TRY(launch_dependent(clear_rows_kernel<T>, dim3(static_cast<unsigned>(device_sm_count()) * 4), dim3(512), 0, stream,
+                                    kLaunchGlue, 1, static_cast<T *>(out), lse, static_cast<long long>(rows * head_dim),
+                                    static_cast<long long>(rows)));
     return launch_status();
 }
 
@@ -845,7 +883,7 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
                  const void *value_cache, const void *query_offsets, const void *page_offsets, const void *pages,
                  const void *last_page_lengths, size_t tokens, size_t heads, size_t kv_heads, size_t head_dim,
                  size_t page_size, size_t cache_pages, size_t sequences, size_t table_len, float scale, int causal,
-                 size_t window, uint32_t *status, float softcap) {
+                 size_t window, uint32_t *status, float softcap, bool whole) {
     TensorPagedPolicy<T, Index> policy;
     policy.query = static_cast<const T *>(query);
     policy.out = static_cast<T *>(out);
@@ -867,6 +905,19 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
     policy.table_len = static_cast<long long>(table_len);
     policy.window = static_cast<long long>(window);
     policy.skip_when_zero = nullptr;
+    // Steps with prompts in them: the tensor-core kernel, which checks the paging tensors itself and follows the general
+    // kernel's meaning row by row (what it leaves is done behind it).
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        if (tokens != sequences && softcap == 0.0f &&
+            tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, cache_pages, sequences, table_len, causal, window,
+                                 query, key_cache, value_cache, out)) {
+            SINGE_TRY(tensor_prefill(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
+                                     last_page_lengths, static_cast<int>(sizeof(Index)), tokens, heads, kv_heads, head_dim,
+                                     cache_pages, sequences, table_len, scale, causal, window, status));
+            return launch_left_rows<T, Index>(stream, policy, tokens, head_dim, scale, status, whole);
+        }
+    }
+    if (whole) SINGE_TRY(clear_rows<T>(stream, out, lse, tokens * heads, head_dim));
     bool checked = status == nullptr;  // no status word, no whole-table check
     auto check_alone = [&]() -> int {
         const unsigned blocks = static_cast<unsigned>((sequences + 3) / 4);  // four warps, one sequence each
@@ -941,18 +992,6 @@ int tensor_paged(cudaStream_t stream, void *out, float *lse, const void *query, 
         }
         // (workspace growth refused under stream capture: the general kernel serves the call)
     }
-    // Steps with prompts in them: the tensor-core kernel, which checks the paging tensors itself and follows the general
-    // kernel's meaning row by row (what it leaves is done behind it).
-    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        if (tokens != sequences && softcap == 0.0f &&
-            tensor_prefill_takes(tokens, heads, kv_heads, head_dim, page_size, cache_pages, sequences, table_len, causal, window,
-                                 query, key_cache, value_cache, out)) {
-            SINGE_TRY(tensor_prefill(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
-                                     last_page_lengths, static_cast<int>(sizeof(Index)), tokens, heads, kv_heads, head_dim,
-                                     cache_pages, sequences, table_len, scale, causal, window, status));
-            return launch_left_rows<T, Index>(stream, policy, tokens, head_dim, scale, status);
-        }
-    }
     if (!checked) SINGE_TRY(check_alone());
     return launch_attention_general<T>(stream, policy, tokens * heads, head_dim, scale, LseKind::Base2, -INFINITY,
                                        status, softcap);
@@ -964,7 +1003,7 @@ int tensor_paged_entry(singe_stream_t stream, void *out, float *lse, const void 
                        const void *pages, const void *last_page_lengths, int index_width, size_t tokens, size_t heads,
                        size_t kv_heads, size_t head_dim, size_t page_size, size_t cache_pages, size_t sequences,
                        size_t table_len, float scale, int causal, size_t window, uint32_t *status,
-                       float softcap = 0.0f) {
+                       float softcap = 0.0f, bool whole = false) {
     if (!(softcap >= 0.0f) || !finite(softcap)) return SINGE_ERR_INVALID_ARGUMENT;
     // paged_attention_problem (singe/src/backend/spec/neural/attention.rs:337-361)
     if (heads == 0 || kv_heads == 0 || head_dim == 0 || page_size == 0 || heads % kv_heads != 0 || !finite(scale)) {
@@ -974,6 +1013,10 @@ int tensor_paged_entry(singe_stream_t stream, void *out, float *lse, const void 
     if (!fits_i32(tokens) || !fits_i32(heads) || !fits_i32(head_dim) || !fits_i32(page_size) ||
         !fits_i32(cache_pages) || !fits_i32(sequences) || !fits_i32(table_len)) {
         return SINGE_ERR_LENGTH_EXCEEDS_I32;
+    }
+    if (whole && tokens != 0 && sequences == 0) {
+        if (out == nullptr || lse == nullptr) return SINGE_ERR_NULL_POINTER;
+        return clear_rows<T>(static_cast<cudaStream_t>(stream), out, lse, tokens * heads, head_dim);
     }
     if (tokens == 0 || sequences == 0) return SINGE_OK;
     if (out == nullptr || lse == nullptr || query == nullptr || key_cache == nullptr || value_cache == nullptr ||
@@ -985,11 +1028,11 @@ int tensor_paged_entry(singe_stream_t stream, void *out, float *lse, const void 
     if (index_width == 8) {
         return tensor_paged<T, long long>(s, out, lse, query, key_cache, value_cache, query_offsets, page_offsets,
                                           pages, last_page_lengths, tokens, heads, kv_heads, head_dim, page_size,
-                                          cache_pages, sequences, table_len, scale, causal, window, status, softcap);
+                                          cache_pages, sequences, table_len, scale, causal, window, status, softcap, whole);
     }
     return tensor_paged<T, int>(s, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
                                 last_page_lengths, tokens, heads, kv_heads, head_dim, page_size, cache_pages, sequences,
-                                table_len, scale, causal, window, status, softcap);
+                                table_len, scale, causal, window, status, softcap, whole);
 }
 
 template <typename T>
@@ -1407,6 +1450,27 @@ int singe_paged_attention_f32(singe_stream_t stream, float *out, float *lse, con
     return tensor_paged_entry<float>(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets,
                                      pages, last_page_lengths, index_width, tokens, heads, kv_heads, head_dim,
                                      page_size, cache_pages, sequences, table_len, scale, causal, window, status);
+}
+
+// As singe_paged_attention_*, into uninitialised `out` and `lse`.
+int singe_paged_attention_whole_bf16(singe_stream_t stream, void *out, float *lse, const void *query, const void *key_cache,
+                                     const void *value_cache, const void *query_offsets, const void *page_offsets,
+                                     const void *pages, const void *last_page_lengths, int index_width, size_t tokens, size_t heads,
+                                     size_t kv_heads, size_t head_dim, size_t page_size, size_t cache_pages, size_t sequences,
+                                     size_t table_len, float scale, int causal, size_t window, uint32_t *status) {
+    return tensor_paged_entry<__nv_bfloat16>(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
+                                             last_page_lengths, index_width, tokens, heads, kv_heads, head_dim, page_size, cache_pages,
+                                             sequences, table_len, scale, causal, window, status, 0.0f, true);
+}
+
+int singe_paged_attention_whole_f32(singe_stream_t stream, float *out, float *lse, const float *query, const float *key_cache,
+                                    const float *value_cache, const void *query_offsets, const void *page_offsets, const void *pages,
+                                    const void *last_page_lengths, int index_width, size_t tokens, size_t heads, size_t kv_heads,
+                                    size_t head_dim, size_t page_size, size_t cache_pages, size_t sequences, size_t table_len,
+                                    float scale, int causal, size_t window, uint32_t *status) {
+    return tensor_paged_entry<float>(stream, out, lse, query, key_cache, value_cache, query_offsets, page_offsets, pages,
+                                     last_page_lengths, index_width, tokens, heads, kv_heads, head_dim, page_size, cache_pages,
+                                     sequences, table_len, scale, causal, window, status, 0.0f, true);
 }
 
 // Tensor::paged_attention with every AttentionOptions field the path has: window and softcap.

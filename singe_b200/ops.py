@@ -255,10 +255,10 @@ def paged_attention(query, key_cache, value_cache, query_offsets, page_offsets, 
     cache_pages, page_size, kv_heads, _ = key_cache.shape
     if scale is None:
         scale = 1.0 / math.sqrt(head_dim)
-    out = torch.zeros_like(query)
-    lse = torch.full((tokens, heads), float("-inf"), dtype=torch.float32, device=query.device)
+    out = torch.empty_like(query)
+    lse = torch.empty((tokens, heads), dtype=torch.float32, device=query.device)
     width = query_offsets.element_size()
-    fn = getattr(ks.lib(), f"singe_paged_attention_{_suffix(query.dtype)}")
+    fn = getattr(ks.lib(), f"singe_paged_attention_whole_{_suffix(query.dtype)}")
     _check(fn(_stream(stream), _ptr(out), _ptr(lse), _ptr(query), _ptr(key_cache), _ptr(value_cache),
               _ptr(query_offsets), _ptr(page_offsets), _ptr(pages), _ptr(last_page_lengths), width, tokens, heads,
               kv_heads, head_dim, page_size, cache_pages, last_page_lengths.numel(), pages.numel(), scale,
