@@ -1172,7 +1172,7 @@ int gemm_bf16(cudaStream_t stream, void *out, bool out_f32, const void *lhs, con
             bn = tiles(64) >= enough ? 64 : 32;
             const int slice_bytes = (params.a_rows + bn) * 128;
             slices = 8;
-            while (slices > 1 && slices * slice_bytes * 2 > 200 * 1024) slices >>= 1;
+            while (slices > 1 && (slices * slice_bytes * 2 > 200 * 1024 || slices / 2 * kBlockK >= params.k)) slices >>= 1;
         }
     }
     // One M tile and too few 128-wide N tiles for the machine: tiles of 64 or 128 columns, the partial sums of K (see k_parts)

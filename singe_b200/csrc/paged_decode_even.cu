@@ -56,9 +56,10 @@ constexpr int even_merge_bytes() {
     return KVH == kEvenWarps ? 0 : KVH * 8 * (HD + 2) * 4;
 }
 
+// (what a call of few sequences leaves of an SM's shared memory is for the CTAs of kernels beside it)
 template <int HD, int KVH>
-constexpr int even_smem_bytes() {
-    return kEvenRing + even_merge_bytes<HD, KVH>() + 16 * even_slots<HD>() + 16 * KVH + (2 * kEvenMaxBatch + 1) * 4 + 64 + 1024;
+constexpr int even_smem_bytes(int batch) {
+    return kEvenRing + even_merge_bytes<HD, KVH>() + 16 * even_slots<HD>() + 16 * KVH + 40 + (2 * batch + 1) * 4 + 1024;
 }
 
 // What a sequence (chunked form: a query) reads.
@@ -126,12 +127,12 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *aligned = smem_raw + (base - raw);
     float *merge = reinterpret_cast<float *>(aligned + kEvenRing);   // [KVH][8 rows][HD + 2]
-    int *before = reinterpret_cast<int *>(aligned + kEvenRing + even_merge_bytes<HD, KVH>());   // pages before sequence b
-    int *lengths = before + kEvenMaxBatch + 1;
-    int *warp_pages = lengths + kEvenMaxBatch;
-    const uint32_t bar_full = base + kEvenRing + even_merge_bytes<HD, KVH>() + (2 * kEvenMaxBatch + 1) * 4 + 60;
+    const uint32_t bar_full = base + kEvenRing + even_merge_bytes<HD, KVH>();
     const uint32_t bar_empty = bar_full + 8 * SLOTS;
     const uint32_t bar_merge = bar_empty + 8 * SLOTS;   // [KVH][written, read]
+    int *warp_pages = reinterpret_cast<int *>(aligned + kEvenRing + even_merge_bytes<HD, KVH>() + 16 * SLOTS + 16 * KVH);   // [warps]
+    int *before = warp_pages + 10;            // [batch + 1]: pages before sequence b
+    int *lengths = before + p.batch + 1;      // [batch]
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
@@ -542,9 +543,10 @@ template <typename T, int HD, int KVH, int FORM>
 int launch_even(cudaStream_t stream, const DecodeParams &params, const StepExtras &extras, const ChunkedDecode &chunked,
                 const void *key_cache, const void *value_cache, int slots) {
     static int configured[kMaxDevices] = {0};
-    constexpr int smem = even_smem_bytes<HD, KVH>();
-    static_assert(smem <= 227 * 1024, "shared memory of one CTA");
-    SINGE_CUDA_TRY(ensure_dynamic_shared(paged_decode_even_kernel<T, HD, KVH, FORM>, smem, configured));
+    constexpr int most = even_smem_bytes<HD, KVH>(kEvenMaxBatch);
+    static_assert(most <= 227 * 1024, "shared memory of one CTA");
+    SINGE_CUDA_TRY(ensure_dynamic_shared(paged_decode_even_kernel<T, HD, KVH, FORM>, most, configured));
+    const int smem = even_smem_bytes<HD, KVH>(params.batch);
     // tokens before heads: a box lands as one 16-row tile per head
     const uint64_t dims[4] = {static_cast<uint64_t>(HD), kPageTokens, static_cast<uint64_t>(KVH),
                               static_cast<uint64_t>(params.physical_blocks)};

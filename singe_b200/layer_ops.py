@@ -26,6 +26,13 @@ class Ops:
         self.dtype = getattr(torch, dtype)
         self.is_bf16 = dtype == "bfloat16"
         self.suffix = "bf16" if self.is_bf16 else "f32"
+        self._side = None
+
+    def side_stream(self):
+        """A stream beside the current one, the same for all layers of a decoder."""
+        if self._side is None:
+            self._side = self.torch.cuda.Stream()
+        return self._side
 
     def call(self, name: str, *arguments) -> None:
         code = getattr(ks.lib(), name)(*[a.data_ptr() if hasattr(a, "data_ptr") else a for a in arguments])

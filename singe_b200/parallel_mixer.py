@@ -136,20 +136,29 @@ class ChunkedAttention:
         pages = (table.page_count(), table.page_size, c.kv_heads, self.size)
         return zeros(*pages), zeros(*pages), zeros(sequences, c.taps - 1, self.span)
 
+    def even_splits(self, rows: int, key_bound: int) -> int:
+        c = self.config
+        return int(ks.lib().singe_paged_kv_decode_even_splits(rows, c.heads, c.kv_heads, self.size, min(c.chunk + TILED_PAGE - 1, key_bound),
+                                                              TILED_PAGE)) if self.tiled else 0
+
+    def fills_machine(self, rows: int, key_bound: int) -> bool:
+        """Whether the decode attention of ``rows`` queries runs as one CTA per SM that takes its shared memory."""
+        return self.even_splits(rows, key_bound) > 0
+
     def scratch(self, rows: int, key_bound: int):
         """Partial results of the split decode attention for ``rows`` queries over at most ``key_bound`` keys."""
         if not self.tiled:
             return None
         torch, c = self.ops.torch, self.config
-        bound = min(c.chunk + TILED_PAGE - 1, key_bound)
-        splits = int(ks.lib().singe_paged_kv_decode_even_splits(rows, c.heads, c.kv_heads, self.size, bound, TILED_PAGE) or
-                     ks.lib().singe_paged_kv_decode_default_splits(rows, c.kv_heads, bound, TILED_PAGE))
+        splits = self.even_splits(rows, key_bound) or int(ks.lib().singe_paged_kv_decode_default_splits(
+            rows, c.kv_heads, min(c.chunk + TILED_PAGE - 1, key_bound), TILED_PAGE))
         attn = torch.empty((rows, c.heads, splits, self.size), dtype=torch.float32, device="cuda")
         lse = torch.empty((rows, c.heads, splits), dtype=torch.float32, device="cuda")
         return splits, attn, lse
 
-    def attend(self, stream, step: StepRows, projected, cache, out, status, scratch=None) -> None:
-        """out = W_o of the heads' outputs; ``projected`` holds this mixer's columns of the input projection."""
+    def prepare(self, stream, step: StepRows, projected, cache, out, status, scratch=None):
+        """Enqueues what stands before the attention; returns what enqueues the rest.  out = W_o of the heads' outputs;
+        ``projected`` holds this mixer's columns of the input projection."""
         ops, c, size = self.ops, self.config, self.size
         torch = ops.torch
         keys, values, state = cache
@@ -172,18 +181,22 @@ class ChunkedAttention:
         if step.longest > 1:
             ops.call(f"singe_conv_state_{ops.suffix}", stream, *conv, state, step.first, step.fresh_tokens, t, sequences, c.taps,
                      self.span)
-        if rows is not None:
-            self._prompt(stream, rows, query, keys, values, packed_keys, packed_values, attended, status)
-        if not self.tiled:
-            self._decode(stream, step, query, step.sequence_of, step.row_lens, keys, values, attended, status, None)
-        elif step.short_rows is None:
-            self._decode(stream, step, query, step.short_sequences, step.short_lens, keys, values, attended, status, scratch)
-        elif step.short_count > 0:
-            short = buffer(step.short_count, c.heads)
-            self._decode(stream, step, query.index_select(0, step.short_rows), step.short_sequences, step.short_lens, keys, values,
-                         short, status, scratch)
-            attended.index_copy_(0, step.short_rows, short)
-        ops.linear(stream, out, attended, self.out)
+
+        def finish() -> None:
+            if rows is not None:
+                self._prompt(stream, rows, query, keys, values, packed_keys, packed_values, attended, status)
+            if not self.tiled:
+                self._decode(stream, step, query, step.sequence_of, step.row_lens, keys, values, attended, status, None)
+            elif step.short_rows is None:
+                self._decode(stream, step, query, step.short_sequences, step.short_lens, keys, values, attended, status, scratch)
+            elif step.short_count > 0:
+                short = buffer(step.short_count, c.heads)
+                self._decode(stream, step, query.index_select(0, step.short_rows), step.short_sequences, step.short_lens, keys, values,
+                             short, status, scratch)
+                attended.index_copy_(0, step.short_rows, short)
+            ops.linear(stream, out, attended, self.out)
+
+        return finish
 
     def _decode(self, stream, step, query, sequence_of, lens, keys, values, attended, status, scratch) -> None:
         """Every query over the cached keys of its own chunk."""
@@ -242,8 +255,9 @@ class GatedDelta:
         return (torch.zeros((sequences, c.heads, c.dim, c.vdim), dtype=torch.float32, device="cuda"),
                 torch.zeros((sequences, c.taps - 1, self.span), dtype=self.ops.dtype, device="cuda"))
 
-    def attend(self, stream, step: StepRows, projected, cache, out, status, scratch=None) -> None:
-        """out = W_o of the heads' outputs; ``projected`` holds this mixer's columns of the input projection."""
+    def prepare(self, stream, step: StepRows, projected, cache, out, status):
+        """Enqueues what stands before the recurrence; returns what enqueues the rest.  out = W_o of the heads' outputs;
+        ``projected`` holds this mixer's columns of the input projection."""
         ops, c = self.ops, self.config
         torch = ops.torch
         state, conv_state = cache
@@ -264,16 +278,20 @@ class GatedDelta:
         operands = [attended, attended.stride(0), mixed, mixed.stride(0), inverse, strength, strength.stride(0), decay,
                     decay.stride(0), self.decay_rate, self.decay_bias, self.norm, state]
         sizes = [c.heads, c.kv_heads, c.dim, c.vdim, self.key_at, self.value_at, self.columns, self.eps]
-        rows = step.whole if self.blocked else None
-        if rows is not None:
-            scratch = torch.empty(int(ks.lib().singe_gated_delta_prompt_scratch(c.heads, c.dim, c.vdim, t, rows.blocks)),
-                                  dtype=torch.uint8, device="cuda")
-            ops.call("singe_gated_delta_prompt_bf16", stream, *operands, step.context, t, *sizes, rows.rows, rows.tokens, rows.blocks,
-                     rows.segments, rows.count, scratch)
-        if rows is None or step.short_count > 0:
-            ops.call(f"singe_gated_delta_step_{ops.suffix}", stream, *operands, step.first, step.fresh_tokens, step.context, t,
-                     sequences, *sizes, 0x7fffffff if rows is None else FEW_TOKENS)
-        ops.linear(stream, out, attended, self.out)
+
+        def finish() -> None:
+            rows = step.whole if self.blocked else None
+            if rows is not None:
+                scratch = torch.empty(int(ks.lib().singe_gated_delta_prompt_scratch(c.heads, c.dim, c.vdim, t, rows.blocks)),
+                                      dtype=torch.uint8, device="cuda")
+                ops.call("singe_gated_delta_prompt_bf16", stream, *operands, step.context, t, *sizes, rows.rows, rows.tokens, rows.blocks,
+                         rows.segments, rows.count, scratch)
+            if rows is None or step.short_count > 0:
+                ops.call(f"singe_gated_delta_step_{ops.suffix}", stream, *operands, step.first, step.fresh_tokens, step.context, t,
+                         sequences, *sizes, 0x7fffffff if rows is None else FEW_TOKENS)
+            ops.linear(stream, out, attended, self.out)
+
+        return finish
 
 
 class ParallelMixer:
@@ -300,5 +318,29 @@ class ParallelMixer:
         self.ops.linear(stream, projected, normed, self.project)
         width = normed.shape[1]
         right = delta.shape[1] - width
-        self.left.attend(stream, step, projected[:, :self.split], cache[:3], delta[:, :width], status, scratch)
-        self.right.attend(stream, step, projected[:, self.split:], cache[3:], delta[:, right:], status)
+        right_part = projected[:, self.split:], cache[3:], delta[:, right:], status
+        left_part = projected[:, :self.split], cache[:3], delta[:, :width], status, scratch
+        if step.longest > 1:
+            self.left.prepare(stream, step, *left_part)()
+            self.right.prepare(stream, step, *right_part)()
+            return
+        # One token per sequence: the sides share nothing but the projections, and the right one runs on a stream of its own beside
+        # the left one's attention.  Where that attention's CTAs take the shared memory of every SM they start behind all that stands
+        # before the recurrence, which would else wait for them (64 sequences of 2048 tokens 853 us a step, 863 without, 932 one
+        # side after the other; 16 of 3000 578, 636 and 635); where they do not, the second meeting is not worth it (4 of 500 480, 438
+        # and 510).  What the right side allocates belongs to its stream; the rest outlives the join.
+        torch = self.ops.torch
+        main, side = torch.cuda.current_stream(), self.ops.side_stream()
+        filling = self.left.fills_machine(normed.shape[0], step.table.shape[1] * cache[0].shape[1])
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            recurrence = self.right.prepare(int(side.cuda_stream), step, *right_part)
+            if not filling:
+                recurrence()
+        attention = self.left.prepare(stream, step, *left_part)
+        if filling:
+            main.wait_stream(side)
+            with torch.cuda.stream(side):
+                recurrence()
+        attention()
+        main.wait_stream(side)
