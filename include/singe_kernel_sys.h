@@ -192,7 +192,8 @@ size_t singe_paged_kv_decode_default_splits(size_t batch, size_t kv_heads, size_
 
 /* For callers of singe_decode_step_attention_bf16 and singe_chunked_attention_bf16 (whose partials are the library's own
  * matter): the max_splits whose scratch has room for the form that shares the cached pages evenly among the SMs, or 0 where
- * the split grid serves the shape.  With less room the split grid serves it too. */
+ * the split grid serves the shape.  With less room the split grid serves it too, and a decode step whose batch * kv_heads rows
+ * fit three CTAs an SM. */
 size_t singe_paged_kv_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound,
                                          size_t block_size);
 

@@ -789,6 +789,10 @@ int decode_half(cudaStream_t stream, int element, void *out, const void *query, 
                                   head_dim, block_size, physical_blocks, stride, scale);
 }
 
+// The step's fused form takes even shares only where its rows alone are more than the split grid's one wave (three CTAs an SM).
+// Until then its caller's splits make one wave of equal CTAs, which start beside the projection before them where a persistent
+// CTA waits for the whole SM (a Llama-shaped step over six layers, us, even shares and splits: 27 sequences of 652 keys 899 and
+// 842, 40 of 2048 1107 and 1084; beyond, 64 of 200 898 and 926, 64 of 2048 1306 and 1384).
 int decode_splitk_half(cudaStream_t stream, int element, void *out, float *attn_scratch, float *lse_scratch,
                        const void *query, const void *key_cache, const void *value_cache, const int32_t *lens,
                        const uint32_t *table, size_t batch, size_t heads, size_t kv_heads, size_t head_dim,
@@ -808,7 +812,7 @@ int decode_splitk_half(cudaStream_t stream, int element, void *out, float *attn_
     return paged_decode_splitk(stream, element, out, attn_scratch, lse_scratch, query, key_cache, value_cache, lens,
                                table, batch, heads, kv_heads, head_dim, physical_blocks, stride, max_splits, scale,
                                partials_only, status != nullptr ? status : device_error_word(), nullptr, hints, rotation,
-                               tickets, fused, fused != nullptr);
+                               tickets, fused, fused != nullptr && batch * kv_heads > 3 * static_cast<size_t>(device_sm_count()));
 }
 
 template <typename T>

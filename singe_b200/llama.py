@@ -220,21 +220,20 @@ class LlamaDecoder(PagedDecoder):
         self.fast_decode = fast
         # rotary embedding, cache write and attention of a decode step in one launch (singe_decode_step_attention_bf16)
         self.fuse_attention = fuse_attention and fast
-        if max_splits <= 0 and self.fuse_attention and not fold_in_kernel:
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        if max_splits <= 0 and self.fuse_attention and not fold_in_kernel and sequences * self.kv_heads > 3 * sms:
             # scratch for the form that shares the cached pages evenly among the SMs, where it serves this shape
             max_splits = int(ks.lib().singe_paged_kv_decode_even_splits(sequences, self.heads, self.kv_heads, config.head_dim,
                                                                         self.stride * config.page_size, config.page_size))
         if max_splits <= 0:
             max_splits = choose_decode_splits(sequences * self.kv_heads, self.stride * config.page_size,
-                                              2 * 2 * config.head_dim,
-                                              torch.cuda.get_device_properties(0).multi_processor_count)
+                                              2 * 2 * config.head_dim, sms)
         self.max_splits = max_splits
         self.attn_scratch = torch.empty((t, self.heads, max_splits, config.head_dim), dtype=torch.float32, device=dev)
         self.lse_scratch = torch.empty((t, self.heads, max_splits), dtype=torch.float32, device=dev)
         # Optional: with one wave of decode CTAs (three fit an SM) the last split of a row can fold the row inside the
         # decode kernel instead of a combine launch.  Measured slower on B200 (+6 us per layer at the 8-way shard's
         # shapes: the fence and the ticket sit on every CTA's exit path), so it is off unless asked for.
-        sms = torch.cuda.get_device_properties(0).multi_processor_count
         self.tickets = (torch.zeros(t * self.kv_heads, dtype=i32, device=dev)
                         if fold_in_kernel and t * self.kv_heads * max_splits <= 3 * sms else None)
 

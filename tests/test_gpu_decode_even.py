@@ -55,14 +55,16 @@ def test_even_decode_reports_page_ids_outside_the_cache():
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(32, 8, 128), (8, 4, 64)])
 @pytest.mark.parametrize("hinted", [False, True])
 def test_even_decode_step_adds_its_key(heads, kv_heads, head_dim, hinted):
-    lens = [1, 300, 16, 17, 2049, 0, 513, 33]     # keys including the new one; an idle row
+    # keys including the new one; an idle row; as many sequences as the form wants for a step (over three rows an SM)
+    lens = [1, 300, 16, 17, 2049, 0, 513, 33] * (8 if kv_heads == 8 else 14)
+    assert len(lens) * kv_heads > 3 * torch.cuda.get_device_properties(0).multi_processor_count
     case = workloads.paged_decode_case(seed=6, heads=heads, kv_heads=kv_heads, head_dim=head_dim, lens=lens, max_len=LONG)
     _, k, v = _inputs(case, seed=7)
     width = (heads + 2 * kv_heads) * head_dim
     qkv = workloads.normal_bf16(np.random.default_rng(8), (case.batch, width))
     positions = np.maximum(np.asarray(lens, dtype=np.int64) - 1, 0)
     pages = np.asarray([case.block_table[b, p // 16] for b, p in enumerate(positions)], dtype=np.int64)
-    pages[5] = case.physical_blocks - 1           # a page that no sequence holds
+    pages[5::8] = case.physical_blocks - 1        # a page that no sequence holds
     slots = positions % 16
     cos, sin = rotary_tables(head_dim, 500000.0, 4096)
     splits = even_splits(case)
