@@ -40,6 +40,11 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int PENDING>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
+// Every thread of every CTA of the cluster takes part; what they wrote to shared memory before it is visible to all behind it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 template <int D, int R, int BM, int G>
 struct Layout {
     static constexpr int kTeam = 16 * BM / R;          // threads that share a key tile
@@ -53,7 +58,9 @@ struct Layout {
     static_assert(G == 1 || kTeam * (R * D / 16 + 2 * R) <= kTeamFloats, "the fold reuses a team's buffers");
 };
 
-template <int D, int R, int BM, int G>
+// C > 1: a cluster of C CTAs shares a row tile, each with every C-th step of G key tiles; the others park their rows and the
+// first folds them out of their shared memory.
+template <int D, int R, int BM, int G, int C>
 __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(const DenseF32 p, const int row_tiles) {
     using L = Layout<D, R, BM, G>;
     constexpr int kColumns = D / 64;   // float4 groups of output columns a thread owns
@@ -76,9 +83,10 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     };
 
     // the heaviest row tiles (the last ones, under a causal mask) are dispatched first
-    const int pairs = gridDim.x / row_tiles;
-    const int first_row = (row_tiles - 1 - static_cast<int>(blockIdx.x) / pairs) * BM;
-    const int pair = static_cast<int>(blockIdx.x) % pairs;
+    const int rank = static_cast<int>(blockIdx.x) % C, block = static_cast<int>(blockIdx.x) / C;
+    const int pairs = gridDim.x / C / row_tiles;
+    const int first_row = (row_tiles - 1 - block / pairs) * BM;
+    const int pair = block % pairs;
     const int head = pair % p.heads;
     const long long batch = pair / p.heads;
     const int kv_head = head / (p.heads / p.kv_heads);
@@ -101,7 +109,7 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     };
 
     grid_dependency_wait();
-    int key0 = first_key + team * kKeys;
+    int key0 = first_key + (rank * G + team) * kKeys;
     if (key0 < end_key) {
         load_keys(k_tile, keys, L::kPitch, key0);
         load_keys(v_tile, values, D, key0);
@@ -120,7 +128,7 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     float4 out[R][kColumns];
     int begin[R], end[R];
     // a sink is one key of weight exp(sink - sink) = 1 and value zero; one thread of a row counts it
-    const float sink = p.sinks != nullptr && team == 0 ? p.sinks[head] : -INFINITY;
+    const float sink = p.sinks != nullptr && team == 0 && rank == 0 ? p.sinks[head] : -INFINITY;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const int row = first_row + ty + i * L::kRows;
@@ -135,7 +143,7 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     // A score is s * unit, rounded only together with the base it is weighed against.
     const float unit = p.softcap > 0.0f || p.scale == 0.0f ? 1.0f : p.scale;
     const float hidden = unit < 0.0f ? INFINITY : -INFINITY;
-    for (; key0 < end_key; key0 += G * kKeys) {
+    for (; key0 < end_key; key0 += C * G * kKeys) {
         copy_wait<1>();   // the keys; the values may still be on their way
         team_sync();
         // Even and odd dimensions are summed apart, as packed pairs, kBlock dimensions in a row; then the blocks of a group,
@@ -208,9 +216,9 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
             }
         }
         team_sync();   // every thread has read the keys
-        const bool more = key0 + G * kKeys < end_key;
+        const bool more = key0 + C * G * kKeys < end_key;
         if (more) {
-            load_keys(k_tile, keys, L::kPitch, key0 + G * kKeys);
+            load_keys(k_tile, keys, L::kPitch, key0 + C * G * kKeys);
         } else {
             copy_commit();
         }
@@ -289,7 +297,7 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
         }
         team_sync();   // every thread has read the values
         if (more) {
-            load_keys(v_tile, values, D, key0 + G * kKeys);
+            load_keys(v_tile, values, D, key0 + C * G * kKeys);
         } else {
             copy_commit();
         }
@@ -300,47 +308,69 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
 #pragma unroll
         for (int offset = 8; offset > 0; offset >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], offset);
     }
-    // teams fold pairwise: the upper half parks its rows in the lower half's buffers, which nobody reads any more
+    // Rows are folded pairwise: one side parks its rows where the other reads them, one float of every thread, then the next.
+    constexpr int kEach = 2 + 4 * kColumns;
+    auto park = [&](float *parked) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            float *at = parked + i * kEach * L::kTeam;
+            at[0] = top[i];
+            at[L::kTeam] = sum[i];
+#pragma unroll
+            for (int c = 0; c < kColumns; ++c) {
+                at[(2 + 4 * c) * L::kTeam] = out[i][c].x;
+                at[(3 + 4 * c) * L::kTeam] = out[i][c].y;
+                at[(4 + 4 * c) * L::kTeam] = out[i][c].z;
+                at[(5 + 4 * c) * L::kTeam] = out[i][c].w;
+            }
+        }
+    };
+    auto fold = [&](auto read) {   // read(n): the n-th float this thread's counterpart parked
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float other = read(i * kEach);
+            const float most = fmaxf(top[i], other);
+            const float base = most == -INFINITY ? 0.0f : most;
+            const float mine = expf(top[i] - base), theirs = expf(other - base);
+            top[i] = most;
+            sum[i] = sum[i] * mine + read(i * kEach + 1) * theirs;
+#pragma unroll
+            for (int c = 0; c < kColumns; ++c) {
+                out[i][c].x = out[i][c].x * mine + read(i * kEach + 2 + 4 * c) * theirs;
+                out[i][c].y = out[i][c].y * mine + read(i * kEach + 3 + 4 * c) * theirs;
+                out[i][c].z = out[i][c].z * mine + read(i * kEach + 4 + 4 * c) * theirs;
+                out[i][c].w = out[i][c].w * mine + read(i * kEach + 5 + 4 * c) * theirs;
+            }
+        }
+    };
+    // the upper half of the teams parks in the lower half's buffers, which nobody reads any more
 #pragma unroll
     for (int half = G / 2; half > 0; half /= 2) {
         __syncthreads();
-        constexpr int kEach = 2 + 4 * kColumns;
-        float *parked = shared + BM * L::kPitch + (team % half) * L::kTeamFloats + t;   // one float of every thread, then the next
-        if (team >= half && team < 2 * half) {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                float *at = parked + i * kEach * L::kTeam;
-                at[0] = top[i];
-                at[L::kTeam] = sum[i];
-#pragma unroll
-                for (int c = 0; c < kColumns; ++c) {
-                    at[(2 + 4 * c) * L::kTeam] = out[i][c].x;
-                    at[(3 + 4 * c) * L::kTeam] = out[i][c].y;
-                    at[(4 + 4 * c) * L::kTeam] = out[i][c].z;
-                    at[(5 + 4 * c) * L::kTeam] = out[i][c].w;
-                }
-            }
-        }
+        float *parked = shared + BM * L::kPitch + (team % half) * L::kTeamFloats + t;
+        if (team >= half && team < 2 * half) park(parked);
         __syncthreads();
-        if (team < half) {
+        if (team < half) fold([&](int n) { return parked[n * L::kTeam]; });
+    }
+    if constexpr (C > 1) {
+        __syncthreads();   // (with one team, all have read their tiles)
+        float *parked = shared + BM * L::kPitch + t;
+        if (team == 0 && rank > 0) park(parked);
+        cluster_sync();
+        if (team == 0 && rank == 0) {
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const float *at = parked + i * kEach * L::kTeam;
-                const float other = at[0];
-                const float most = fmaxf(top[i], other);
-                const float base = most == -INFINITY ? 0.0f : most;
-                const float mine = expf(top[i] - base), theirs = expf(other - base);
-                top[i] = most;
-                sum[i] = sum[i] * mine + at[L::kTeam] * theirs;
-#pragma unroll
-                for (int c = 0; c < kColumns; ++c) {
-                    out[i][c].x = out[i][c].x * mine + at[(2 + 4 * c) * L::kTeam] * theirs;
-                    out[i][c].y = out[i][c].y * mine + at[(3 + 4 * c) * L::kTeam] * theirs;
-                    out[i][c].z = out[i][c].z * mine + at[(4 + 4 * c) * L::kTeam] * theirs;
-                    out[i][c].w = out[i][c].w * mine + at[(5 + 4 * c) * L::kTeam] * theirs;
-                }
+            for (int r = 1; r < C; ++r) {
+                uint32_t theirs;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(smem_u32(parked)), "r"(r));
+                fold([&](int n) {
+                    float value;
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(value) : "r"(theirs + n * L::kTeam * 4));
+                    return value;
+                });
             }
         }
+        cluster_sync();    // nobody leaves before its rows have been read
+        if (rank > 0) return;
     }
     if (team > 0) return;
 #pragma unroll
@@ -364,15 +394,15 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
     }
 }
 
-template <int D, int R, int BM, int G>
+template <int D, int R, int BM, int G, int C = 1>
 int launch(cudaStream_t stream, const DenseF32 &p, size_t pairs) {
     using L = Layout<D, R, BM, G>;
     static int raised[kMaxDevices] = {0};
     constexpr int kBytes = L::kFloats * 4;
-    SINGE_CUDA_TRY(ensure_dynamic_shared(dense_attention_f32_kernel<D, R, BM, G>, kBytes, raised));
+    SINGE_CUDA_TRY(ensure_dynamic_shared(dense_attention_f32_kernel<D, R, BM, G, C>, kBytes, raised));
     const int row_tiles = (p.query_len + BM - 1) / BM;
-    SINGE_CUDA_TRY(launch_dependent(dense_attention_f32_kernel<D, R, BM, G>, dim3(static_cast<unsigned>(pairs * row_tiles)),
-                                    dim3(L::kThreads), kBytes, stream, kLaunchGlue, 1, p, row_tiles));
+    SINGE_CUDA_TRY(launch_dependent(dense_attention_f32_kernel<D, R, BM, G, C>, dim3(static_cast<unsigned>(pairs * row_tiles * C)),
+                                    dim3(L::kThreads), kBytes, stream, kLaunchGlue, C, p, row_tiles));
     return launch_status();
 }
 
@@ -390,6 +420,16 @@ int dense_attention_f32(cudaStream_t stream, const DenseF32 &p, size_t batch) {
     const size_t pairs = batch * static_cast<size_t>(p.heads);
     const size_t sms = static_cast<size_t>(device_sm_count());
     const size_t blocks = pairs * ((static_cast<size_t>(p.query_len) + 31) / 32);
+    // A grid that leaves half of the SMs idle gives each row tile a cluster of two CTAs with two teams each, once there are more
+    // keys than two teams' first tiles (us without and with: 4 causal heads of 64, 200 keys 13.9 and 10.7, 512 24.6 and 16.6; of
+    // 128, 512 44.3 and 26.5; 128 keys 9.4 and 10.6).  Under a causal mask the short walks make room: up to four fifths of the SMs
+    // where walks are long (8 heads x 400 22.0 and 20.3, 4 x 900 42.0 and 31.7, of 128 79.2 and 50.8; not 8 x 512, 128 tiles, 24.7
+    // and 25.9, nor 12 x 256 14.6 and 19.1).
+    long long longest = p.key_len;
+    if (p.window > 0 && longest > p.window) longest = p.window;
+    if (longest > 2 * kKeys && (2 * blocks <= sms || (p.causal && longest >= 6 * kKeys && 5 * blocks <= 4 * sms))) {
+        return p.head_dim <= 64 ? launch<64, 4, 32, 2, 2>(stream, p, pairs) : launch<128, 4, 32, 2, 2>(stream, p, pairs);
+    }
     if (p.head_dim <= 64) {
         // Four teams need more than two key tiles to share.  A grid that does not cover the SMs leaves each CTA alone on its SM,
         // and the longest walk decides (us with four teams and with two: 8 heads x 130 causal keys 11.3 and 12.6, x 512 24.1 and
