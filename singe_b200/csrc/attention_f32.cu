@@ -11,13 +11,15 @@
 // scale is applied by the FMA that takes a score's distance from the row's base.  Against 64 bits, 128 heads of 128 columns
 // over 16, 40 and 100 causal keys, in units of the general kernel's error: 1.00, 0.99, 0.95 (64 columns 0.99, 0.98, 0.94); four
 // chains of a quarter of the dimensions each, scaled afterwards: 1.19, 1.17, 1.11.  They took 4 % less time, but 8 % more in the
-// form of four teams, where their registers spilled.  (Packed value products as well, with every weight stored
-// twice, cost 3 - 9 % more: the wider reads.)  Thread (ty, tx) owns rows ty, ty + BM/R, ... and keys tx,
-// tx + 16, ...: a row's scores lie in 16 neighbouring lanes, and rows one apart keep the 16-byte reads of a warp on
-// different banks (rows are padded by 16 bytes).
+// form of four teams, where their registers spilled.  The value products take pairs of columns at a time (sums and order as one by
+// one; with the halving of last tiles below 2 - 18 % less time: 8 heads x 512 causal keys of 64 24.4 us -> 23.6, of 128 44.3 -> 42.0,
+// 8 x 100 of 128 14.1 -> 12.0); reading every weight twice from shared memory instead cost 3 - 9 % more.
+// Thread (ty, tx) owns rows ty, ty + BM/R, ... and keys tx, tx + 16, ...: a row's scores lie in 16 neighbouring lanes, and rows
+// one apart keep the 16-byte reads of a warp on different banks (rows are padded by 16 bytes).
 // Teams of threads walk alternate key tiles, each in buffers of its own, and are folded at the end through shared memory: the
 // chain of key tiles is what a call of few CTAs waits for.
-// 8 heads x 512 causal keys of 64: 417 us -> 24.1; x 900: 1011 -> 41.7; x 1500 of 128: 3367 -> 182.
+// A last tile is walked as far as its last visible key: scores by halves of 32 keys, value products by groups of 16.
+// 8 heads x 512 causal keys of 64: 417 us -> 23.6; x 900: 1011 -> 39.8; x 1500 of 128: 3367 -> 170.
 // Keys a row does not see take no part at all, whatever their bits are: in tiles that hold hidden keys the value
 // products are predicated, not multiplied by zero.
 #include "common.cuh"
@@ -154,66 +156,74 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
         }
+        auto score = [&](auto columns) {   // how many of a thread's keys; the others lie behind the last visible one
+            constexpr int kOf = decltype(columns)::value;
 #pragma unroll 1
-        for (int group = 0; group < D; group += kGroup) {
-            // (in narrow heads, where threads have 128 registers, a pair is folded at the end of its block)
-            std::conditional_t<D == 64, float, float2> total[R][4];
+            for (int group = 0; group < D; group += kGroup) {
+                // (in narrow heads, where threads have 128 registers, a pair is folded at the end of its block)
+                std::conditional_t<D == 64, float, float2> total[R][4];
 #pragma unroll
-            for (int first = 0; first < kGroup; first += kBlock) {
-                float2 part[R][4];
-#pragma unroll
-                for (int i = 0; i < R; ++i) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) part[i][j] = make_float2(0.0f, 0.0f);
-                }
-#pragma unroll
-                for (int d = 0; d < kBlock; d += 4) {
-                    const int at = group + first + d;
-                    float4 a[R], b[4];
-#pragma unroll
-                    for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4 *>(q_tile + (ty + i * L::kRows) * L::kPitch + at);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(k_tile + (tx + 16 * j) * L::kPitch + at);
+                for (int first = 0; first < kGroup; first += kBlock) {
+                    float2 part[R][4];
 #pragma unroll
                     for (int i = 0; i < R; ++i) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) part[i][j] = __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), part[i][j]);
+                        for (int j = 0; j < kOf; ++j) part[i][j] = make_float2(0.0f, 0.0f);
+                    }
+#pragma unroll
+                    for (int d = 0; d < kBlock; d += 4) {
+                        const int at = group + first + d;
+                        float4 a[R], b[4];
+#pragma unroll
+                        for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4 *>(q_tile + (ty + i * L::kRows) * L::kPitch + at);
+#pragma unroll
+                        for (int j = 0; j < kOf; ++j) b[j] = *reinterpret_cast<const float4 *>(k_tile + (tx + 16 * j) * L::kPitch + at);
+#pragma unroll
+                        for (int i = 0; i < R; ++i) {
+#pragma unroll
+                            for (int j = 0; j < kOf; ++j) part[i][j] = __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), part[i][j]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < R; ++i) {
+#pragma unroll
+                            for (int j = 0; j < kOf; ++j) part[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), part[i][j]);
+                        }
                     }
 #pragma unroll
                     for (int i = 0; i < R; ++i) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) part[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), part[i][j]);
+                        for (int j = 0; j < kOf; ++j) {
+                            if constexpr (D == 64) {
+                                const float sum_of_block = part[i][j].x + part[i][j].y;
+                                total[i][j] = first == 0 ? sum_of_block : total[i][j] + sum_of_block;
+                            } else {
+                                total[i][j] = first == 0 ? part[i][j] : __fadd2_rn(total[i][j], part[i][j]);
+                            }
+                        }
                     }
                 }
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < kOf; ++j) {
                         if constexpr (D == 64) {
-                            const float sum_of_block = part[i][j].x + part[i][j].y;
-                            total[i][j] = first == 0 ? sum_of_block : total[i][j] + sum_of_block;
+                            s[i][j] += total[i][j];
                         } else {
-                            total[i][j] = first == 0 ? part[i][j] : __fadd2_rn(total[i][j], part[i][j]);
+                            const float sum_of_group = total[i][j].x + total[i][j].y;
+                            if (group % (2 * kGroup) == 0) {
+                                two[i][j] = sum_of_group;
+                            } else {
+                                s[i][j] += two[i][j] + sum_of_group;
+                            }
                         }
                     }
                 }
             }
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if constexpr (D == 64) {
-                        s[i][j] += total[i][j];
-                    } else {
-                        const float sum_of_group = total[i][j].x + total[i][j].y;
-                        if (group % (2 * kGroup) == 0) {
-                            two[i][j] = sum_of_group;
-                        } else {
-                            s[i][j] += two[i][j] + sum_of_group;
-                        }
-                    }
-                }
-            }
+        };
+        if (end_key - key0 > kKeys / 2) {
+            score(std::integral_constant<int, 4>{});
+        } else {
+            score(std::integral_constant<int, 2>{});
         }
         team_sync();   // every thread has read the keys
         const bool more = key0 + C * G * kKeys < end_key;
@@ -265,8 +275,9 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
         copy_wait<1>();   // the values; the next keys may still be on their way
         team_sync();
         auto weigh = [&](auto whole_tile) {
+            const int last = decltype(whole_tile)::value || G == 4 ? kKeys : min(kKeys, end_key - key0);   // (four teams have no register for it)
 #pragma unroll 4
-            for (int k = 0; k < kKeys; k += 4) {
+            for (int k = 0; k < last; k += 4) {
                 float4 w[R];
 #pragma unroll
                 for (int i = 0; i < R; ++i) w[i] = *reinterpret_cast<const float4 *>(weights + (ty + i * L::kRows) * L::kWeightPitch + k);
@@ -281,10 +292,10 @@ __global__ void __launch_bounds__(16 * BM / R * G) dense_attention_f32_kernel(co
                         const float weight = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
 #pragma unroll
                         for (int c = 0; c < kColumns; ++c) {
-                            out[i][c].x = fmaf(weight, v[c].x, out[i][c].x);
-                            out[i][c].y = fmaf(weight, v[c].y, out[i][c].y);
-                            out[i][c].z = fmaf(weight, v[c].z, out[i][c].z);
-                            out[i][c].w = fmaf(weight, v[c].w, out[i][c].w);
+                            const float2 both = make_float2(weight, weight);
+                            const float2 low = __ffma2_rn(both, make_float2(v[c].x, v[c].y), make_float2(out[i][c].x, out[i][c].y));
+                            const float2 high = __ffma2_rn(both, make_float2(v[c].z, v[c].w), make_float2(out[i][c].z, out[i][c].w));
+                            out[i][c] = make_float4(low.x, low.y, high.x, high.y);
                         }
                     }
                 }
@@ -421,10 +432,10 @@ int dense_attention_f32(cudaStream_t stream, const DenseF32 &p, size_t batch) {
     const size_t sms = static_cast<size_t>(device_sm_count());
     const size_t blocks = pairs * ((static_cast<size_t>(p.query_len) + 31) / 32);
     // A grid that leaves half of the SMs idle gives each row tile a cluster of two CTAs with two teams each, once there are more
-    // keys than two teams' first tiles (us without and with: 4 causal heads of 64, 200 keys 13.9 and 10.7, 512 24.6 and 16.6; of
-    // 128, 512 44.3 and 26.5; 128 keys 9.4 and 10.6).  Under a causal mask the short walks make room: up to four fifths of the SMs
-    // where walks are long (8 heads x 400 22.0 and 20.3, 4 x 900 42.0 and 31.7, of 128 79.2 and 50.8; not 8 x 512, 128 tiles, 24.7
-    // and 25.9, nor 12 x 256 14.6 and 19.1).
+    // keys than two teams' first tiles (us without and with: 4 causal heads of 64, 200 keys 12.3 and 10.2, 512 23.4 and 16.0; of
+    // 128, 512 41.5 and 24.9; 128 keys 9.0 and 10.2).  Under a causal mask the short walks make room: up to four fifths of the SMs
+    // where walks are long (8 heads x 400 20.5 and 19.5, 4 x 900 39.4 and 29.6, of 128 72.0 and 46.1; not 8 x 512, 128 tiles, 23.6
+    // and 24.7, nor 12 x 256 13.9 and 17.4).
     long long longest = p.key_len;
     if (p.window > 0 && longest > p.window) longest = p.window;
     if (longest > 2 * kKeys && (2 * blocks <= sms || (p.causal && longest >= 6 * kKeys && 5 * blocks <= 4 * sms))) {
@@ -432,18 +443,25 @@ int dense_attention_f32(cudaStream_t stream, const DenseF32 &p, size_t batch) {
     }
     if (p.head_dim <= 64) {
         // Four teams need more than two key tiles to share.  A grid that does not cover the SMs leaves each CTA alone on its SM,
-        // and the longest walk decides (us with four teams and with two: 8 heads x 130 causal keys 11.3 and 12.6, x 512 24.1 and
-        // 26.4; x 128 whole 9.7 and 9.1).  Else the mean walk does: from three tiles on (200 heads x 200 whole keys
-        // 135 and 141, 64 x 400 causal 82 and 84, 24 x 1500 causal 270 and 297; 64 x 256 causal 41.6 and 41.2, 200 x 130 causal
-        // 65 and 62).  64 rows and no teams never win by more than 3 % and lose up to half.
+        // and the longest walk decides (us with four teams and with two: 8 heads x 512 causal keys 23.6 and 25.7, x 900 39.8 and
+        // 44.1; x 128 whole 9.6 and 8.9).  Else the mean walk does: from three tiles on (200 heads x 200 whole keys
+        // 124 and 128, 64 x 400 causal 77.9 and 78.5, 24 x 1500 causal 256 and 281; 64 x 256 causal 39.1 and 38.1, 200 x 130 causal
+        // 59.9 and 55.0).  64 rows and no teams never win by more than 3 % and lose up to half.
         long long walk = p.key_len;
         if (blocks > sms && p.causal) walk = (min(p.query_len, p.key_len) + 1) / 2;
         if (p.window > 0 && walk > p.window) walk = p.window;
         return walk > (blocks > sms ? 3 : 2) * kKeys ? launch<64, 4, 32, 4>(stream, p, pairs) : launch<64, 4, 32, 2>(stream, p, pairs);
     }
-    // Two teams' tiles of 128 columns fill an SM's shared memory, 64 rows without teams read each key half as often: that
-    // gains once the grid is two waves (24 heads x 1500 keys: 883 us against 978) and loses below (12 x 700: 104 against 65).
-    return blocks < 4 * sms ? launch<128, 4, 32, 2>(stream, p, pairs) : launch<128, 4, 64, 1>(stream, p, pairs);
+    // Two teams' tiles of 128 columns fill an SM's shared memory, so a CTA has an SM to itself and whole walks come in waves.  64
+    // rows without teams read each key half as often and take 16/9 of a wave's time: they win where their waves are few enough
+    // (us with two teams and with 64 rows, whole: 12 heads x 500, 2 waves and 1, 82.5 and 74.7; x 900, 3 and 2, 215 and 260; 24 x
+    // 600, 4 and 2, 193 and 176; x 900, 5 and 3, 360 and 389; x 1500, 8 and 4, 902 and 847).  Causal walks fill each other's
+    // gaps: 64 rows gain from three and a half waves on (12 x 700 59 and 100, 12 x 1200 166 and 170, 12 x 1500 234 and 227, 24 x
+    // 700 117 and 105, 48 x 700 236 and 212).
+    auto waves = [&](size_t ctas) { return (ctas + sms - 1) / sms; };
+    const size_t tall = pairs * ((static_cast<size_t>(p.query_len) + 63) / 64);
+    const bool teams = p.causal ? 2 * blocks < 7 * sms : 9 * waves(blocks) <= 16 * waves(tall);
+    return teams ? launch<128, 4, 32, 2>(stream, p, pairs) : launch<128, 4, 64, 1>(stream, p, pairs);
 }
 
 }  // namespace singe

@@ -1,4 +1,4 @@
-"""Dense f32 attention whose row tiles are shared by two CTAs, against 64-bit sums."""
+"""Dense f32 attention against 64-bit sums: row tiles that two CTAs share, and last key tiles."""
 import pytest
 import torch
 
@@ -36,4 +36,24 @@ def test_shared_row_tiles(h, g, l, s, d, causal, window, with_sinks):
         scores = torch.cat([scores, sinks.double()[None, :, None, None].expand(1, h, l, 1)], -1)
     expect = torch.nan_to_num(torch.softmax(scores, -1))[..., :s] @ wide(v)
     # f32 sums over at most s + d terms of values below 6: 2^-24 * 630 * 6 = 2.3e-4 at worst, the root of that many in practice
+    assert (out.double() - expect).abs().max() < 2e-5
+
+
+# a last key tile of 1 to 64 keys, for each form: two and four teams, 64 rows
+@pytest.mark.parametrize("last", [1, 31, 32, 33, 63, 64])
+@pytest.mark.parametrize("h,before,d", [(80, 64, 64), (80, 320, 64), (80, 128, 128), (200, 128, 128)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_last_tiles(last, h, before, d, causal):
+    l = s = before + last
+    gen = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randn(1, h, m, d, device="cuda", generator=gen) for m in (l, s, s))
+    out = torch.full_like(q, float("nan"))
+    code = ks.lib().singe_attend_f32(int(torch.cuda.current_stream().cuda_stream), out.data_ptr(), q.data_ptr(), k.data_ptr(),
+                                     v.data_ptr(), 1, h, h, l, s, d, d ** -0.5, int(causal), 0, 0.0, None)
+    assert code == ks.OK
+    scores = q.double() @ k.double().transpose(-1, -2) * d ** -0.5
+    if causal:
+        scores.masked_fill_(torch.ones(l, s, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    expect = torch.softmax(scores, -1) @ v.double()
+    # f32 sums over at most s + d terms of values below 6: 2^-24 * 512 * 6 = 1.8e-4 at worst, the root of that many in practice
     assert (out.double() - expect).abs().max() < 2e-5
