@@ -11,7 +11,7 @@
 //   * pieces of equal size leave SMs idle in the last wave (2049 keys x 64 sequences: 4.6 waves of 512 keys) and ragged
 //     lengths make it worse; here every SM gets the same number of pages to within one.
 // Measured, bf16 and f16 (us, by the split grid and here, with the fold): 32 sequences of 128 - 4096 keys, 8 heads of 128 57.1 and
-// 52.5; 64 x 1024 59.5 and 49.3; 4 x 4096 24.7 and 18.9; 32 x 4096 of 64 61.3 and 49.6.  A Llama-shaped decode step of 64 x 2048
+// 52.5; 64 x 1024 59.5 and 49.3; 4 x 4096 24.7 and 18.0; 32 x 4096 of 64 61.3 and 49.6.  A Llama-shaped decode step of 64 x 2048
 // keys over six layers 1462 and 1384.  Against 64 bits the error is 0.84 of the split grid's (2.0e-3 -> 1.7e-3, the rounding of the
 // output): the weights enter the value product as two terms, in rows of the 16-row tile that carry no query head.
 // Structure: one persistent CTA per SM.  Warp 8 (producer) brings K and V of a step -- eight (page, head) tiles, so one page of
@@ -153,6 +153,12 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
         prefetch_tensor_map(&v_map);
     }
     if (FORM != kEvenChunked && warp == 0) warm_l2(x.warm, blockIdx.x, gridDim.x, lane);
+    {
+        // The table is read behind the lengths: till then every CTA has some of its lines on their way to L2 (1 % of a call).
+        const size_t words = static_cast<size_t>(FORM == kEvenChunked ? chunked.sequences : p.batch) * p.table_stride;
+        const size_t word = (static_cast<size_t>(tid) * gridDim.x + blockIdx.x) * 32;
+        if (word < words) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.table + word));
+    }
     if (!stable) grid_dependency_wait();
 
     // ---- pages before each sequence ----
@@ -454,8 +460,11 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
 }
 
 // Folds the segments of every sequence that has more than one, with the arithmetic of decode_combine_kernel.  `TEAM` warps share a
-// row, each every TEAM-th segment: few sequences have many segments (37 each of four: 3.3 us by one warp).  A warp's
-// lanes hold the weights of all segments, and its first segments' values are on their way before the weights are known.
+// row, each every TEAM-th segment: few sequences have many segments, and a warp waits once for each batch of them.  A warp's
+// lanes hold the weights of all segments, and its first segments' values are on their way before the weights are known (us a
+// call, four of them early by eight warps and twelve: 2 x 7168 keys of 64 16.8 and 14.1, ragged 3 x 2901 of 128 11.5 and 10.3).
+// Warps for a row, eight, four, two and one: 8 x 1088 of 128 12.6, 13.2, 14.0, 14.0; 15 x 580 14.6, 14.2, 14.3, 14.6; 28 x 310
+// 17.3, 14.7, 14.7, 14.2; 48 x 298 24.3, 20.0, 18.9, 17.8.
 constexpr int kFoldWarps = 8;
 
 template <typename T, int HD, int TEAM>
@@ -465,7 +474,7 @@ __global__ void __launch_bounds__(32 * kFoldWarps)
     grid_dependency_wait();
     constexpr int kColumns = HD / 32;   // columns of a lane
     constexpr int kRounds = kEvenMaxCtas / 32;
-    constexpr int kEarly = 4;
+    constexpr int kEarly = TEAM == 8 ? 12 : 8;
     struct __align__(kColumns * 4) Columns { float v[kColumns]; };
     __shared__ Columns parts[TEAM > 1 ? kFoldWarps : 1][32];
     const int b = blockIdx.y;
@@ -506,17 +515,17 @@ __global__ void __launch_bounds__(32 * kFoldWarps)
     Columns value = {};
 #pragma unroll
     for (int i = 0; i < kEarly; ++i) {
-        const float w = __shfl_sync(0xffffffffu, weight[0], member + i * TEAM);   // (below 32)
+        const float w = __shfl_sync(0xffffffffu, weight[i * TEAM / 32], (member + i * TEAM) % 32);
 #pragma unroll
         for (int c = 0; c < kColumns; ++c) {
             if (member + i * TEAM < segments) value.v[c] = fmaf(w, early[i].v[c], value.v[c]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < kRounds; ++i) {
+    for (int i = kEarly * TEAM / 32; i < kRounds; ++i) {
         const int end = min(segments - i * 32, 32);
 #pragma unroll 4
-        for (int s = member + (i == 0 ? kEarly * TEAM : 0); s < end; s += TEAM) {
+        for (int s = member + max(kEarly * TEAM - i * 32, 0); s < end; s += TEAM) {
             const Columns part = *reinterpret_cast<const Columns *>(partial + static_cast<size_t>(i * 32 + s) * step);
             const float w = __shfl_sync(0xffffffffu, weight[i], s);
 #pragma unroll
@@ -571,7 +580,9 @@ int launch_even(cudaStream_t stream, const DecodeParams &params, const StepExtra
                                 dim3(32 * kFoldWarps), 0, stream, kLaunchCombine, 1, static_cast<T *>(params.out),
                                 params.attn_partial, params.lse_partial, rows, params.heads);
     };
-    SINGE_CUDA_TRY(params.batch < 16 ? fold(even_combine_kernel<T, HD, 8>, 8) : fold(even_combine_kernel<T, HD, 1>, 1));
+    SINGE_CUDA_TRY(params.batch < 12   ? fold(even_combine_kernel<T, HD, 8>, 8)
+                   : params.batch < 20 ? fold(even_combine_kernel<T, HD, 4>, 4)
+                                       : fold(even_combine_kernel<T, HD, 1>, 1));
     return launch_status();
 }
 
@@ -591,19 +602,23 @@ int launch_even_shape(cudaStream_t stream, const DecodeParams &params, const Ste
 // How many slots of [heads, head_dim] f32 partials and [heads] log sums the even form wants for a call of the tiled kernel
 // (paged_decode_fast_path) with at most `bound` keys a sequence; 0: the split grid serves it.
 // Lengths are device data, so the rule knows only what they may grow to.  Below 32 MB of keys and values setting up (a scan of
-// the lengths, then the block table, then the first pages) and folding cost as much as the even shares gain: 64 x 64 keys 8.8 us
-// (split grid 8.6 - 9.7), 16 x 256 9.2 (9.2 - 9.6), 4 x 1100 of 64 8.6 (7.6); at 32 MB 8 x 1024 13.8 (17.3), 2 x 4096
-// 15.6 (19.6), 64 x 256 of 64 14.1 (16.4).  Sequences of one split each need no fold there: they stay while they fill the grid
+// the lengths, then the block table, then the first pages) and folding cost as much as the even shares gain, 24 MB for heads of
+// 128 whose sequences the split grid has to split as well (us, calls one after the other, split grid and here; "to" is the shortest of a
+// ragged batch): 4 x 1536 of 128 11.0 and 10.1, 384 to 1536 10.5 and 9.7; 20 x 307 14.2 and 10.5; 4 x 2901 19.2 and 13.5; 8 x
+// 640, 20 MB, 10.0 and 10.4; 48 x 128, not split, 7.4 and 10.9; heads of 64, 14 x 877 12.6 and 10.6, but 219 to 877 8.9 and 9.6; at 32
+// MB 8 x 2176 16.4 and 13.1, 544 to 2176 10.5 and 10.3.  (Ragged batches of 13 - 20 of these may still lose: 478 to 1911 x 15 13.7
+// and 14.4, whole 21.9 and 18.0.)  Sequences of one split each need no fold there: they stay while they fill the grid
 // (three CTAs an SM) one and a half times, 96 x 256 24.1 against 25.1 here; 64 x 256, 1.15 times, 27.1 against 18.9.
 size_t paged_decode_even_slots(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t bound) {
-    constexpr size_t kLeastBytes = size_t{32} << 20;
     const size_t sms = static_cast<size_t>(device_sm_count());
     const size_t stride = (bound + kPageTokens - 1) / kPageTokens;
     if ((kv_heads != 8 && kv_heads != 4) || batch > kEvenMaxBatch || sms > kEvenMaxCtas || 2 * batch > heads * head_dim ||
         stride > (size_t{1} << 30) / batch) {
         return 0;
     }
-    if (batch * stride * kPageTokens * kv_heads * head_dim * 4 < kLeastBytes) return 0;
+    const bool split = bound > 128 && batch * kv_heads <= 3 * sms;
+    const size_t least = size_t{head_dim == 128 && split ? 24u : 32u} << 20;
+    if (batch * stride * kPageTokens * kv_heads * head_dim * 4 < least) return 0;
     if (bound <= 512 && 2 * batch * kv_heads > 9 * sms) return 0;
     return sms + batch;
 }

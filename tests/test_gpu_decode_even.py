@@ -15,9 +15,10 @@ pytestmark = pytest.mark.gpu
 
 LONG = 65536     # a bound on the lengths that has the even form serve short ones too
 
-# one sequence; runs that end inside, at and before a sequence's last page; empty sequences; more sequences than threads
+# one sequence; runs that end inside, at and before a sequence's last page; empty sequences; more sequences than threads; sequences
+# of more segments than the fold has under way at once, with eight, four and one warps for a row
 LENGTHS = [[1], [16 * 300], [16 * 148 * 2], [0, 33, 0, 512, 0], [1, 15, 16, 17, 2049, 31, 32, 33, 4097, 100],
-           [(37 * i) % 90 for i in range(300)], [5000] + [3] * 40]
+           [(37 * i) % 90 for i in range(300)], [5000] + [3] * 40, [3000] + [(211 * i) % 700 for i in range(13)]]
 
 
 def even_splits(case):
