@@ -285,6 +285,18 @@ __device__ __forceinline__ uint4 narrow(const Eight &x) {
                       pack2<__nv_bfloat16>(x.v[6], x.v[7]));
 }
 
+// Brings a thread's columns of `count` neighbouring rows on their way to shared memory, where `held` is its place for the first and
+// `step` leads to the next: one latency for a tile, and no registers for what is on its way (us, four prompts of 1500 tokens, the
+// next row in registers and a tile in shared memory: the attention's inputs 84.9 and 78.0, the recurrence's 57.9 and 52.6).
+__device__ __forceinline__ void fetch_rows(const ConvRows &p, int c, int token0, int count, uint4 *held, int step) {
+    for (int i = 0; i < count; ++i) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(held + i * step)),
+                     "l"(static_cast<const __nv_bfloat16 *>(p.projected) + (token0 + i) * p.stride + c)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void rows_arrived() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ uint4 load_eight(const void *base, long long element) {
     return *reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(base) + element);
 }
@@ -295,7 +307,6 @@ struct TapWindow {
     uint4 taps[N], bias;
     uint4 past[N > 1 ? N - 1 : 1];  // past[j]: the row j + 1 tokens back
     bool there[N > 1 ? N - 1 : 1];  // false: before the sequence's start
-    uint4 ahead;                    // the next row, on its way while this one is worked on
     bool follows;                   // the window stands just before the next token of its sequence
 
     __device__ __forceinline__ void start(const ConvRows &p, int c) {
@@ -304,8 +315,6 @@ struct TapWindow {
         bias = p.bias != nullptr ? load_eight(p.bias, c) : make_uint4(0u, 0u, 0u, 0u);
         follows = false;
     }
-
-    __device__ __forceinline__ void fetch(const ConvRows &p, int c, int token) { ahead = load_eight(p.projected, token * p.stride + c); }
 
     // The convolution at `token`, a sequence's new token number `at`, whose row is `now`; moves the window on, and with `shift` the
     // sequence's state.
@@ -389,14 +398,16 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 384 ? 2 : 1) attention_inp
     __shared__ float2 scratch[2][32];
     __shared__ TileToken tokens[kTileTokens];
     __shared__ long long cells[kTileTokens], packs[kTileTokens];  // rows of the cache and of the packed arrays, or negative
-    extern __shared__ float2 turns[];                             // [tile][pairs]: cosine, sine
+    extern __shared__ uint4 held_rows[];                          // [tile][threads]
+    float2 *turns = reinterpret_cast<float2 *>(held_rows + tile * blockDim.x);  // [tile][pairs]: cosine, sine
     const int c = threadIdx.x * 8, warps = (blockDim.x + 31) >> 5;
     const int token0 = blockIdx.x * tile;
     const bool live = c < p.rows.span;
     TapWindow<N> window;
     if (live) window.start(p.rows, c);  // weights: they do not wait for the kernel before
     grid_dependency_wait();
-    if (live) window.fetch(p.rows, c, token0);
+    uint4 *held = held_rows + threadIdx.x;
+    if (live) fetch_rows(p.rows, c, token0, min(tile, rows - token0), held, blockDim.x);
     look_up_tile(p.rows, tokens, token0, tile, rows);
     for (int i = threadIdx.x; i < tile && token0 + i < rows; i += blockDim.x) {
         long long page = p.write_pages[token0 + i], slot = p.write_slots[token0 + i];
@@ -430,13 +441,13 @@ __global__ void __launch_bounds__(THREADS, THREADS <= 384 ? 2 : 1) attention_inp
     if (is_key) gain = widen(load_eight(p.key_norm, within));
     const bool normed = is_query || is_key;
     const size_t key_width = static_cast<size_t>(p.kv_heads) * p.key_size, value_width = static_cast<size_t>(p.kv_heads) * p.value_size;
+    rows_arrived();   // (a thread reads no row but its own)
     __syncthreads();
     int parity = 0;
     for (int i = 0; i < tile && token0 + i < rows; ++i) {
         const int token = token0 + i;
         const TileToken now = tokens[i];
-        const uint4 row = window.ahead;
-        if (live && i + 1 < tile && token + 1 < rows) window.fetch(p.rows, c, token + 1);
+        const uint4 row = live ? held[i * blockDim.x] : make_uint4(0u, 0u, 0u, 0u);
         T *query = static_cast<T *>(p.query) + token * p.query_stride;
         if (now.fresh <= 0) {
             for (int at = c; at < p.heads * p.key_size; at += blockDim.x * 8) {
@@ -512,14 +523,16 @@ template <int N>
 __global__ void __launch_bounds__(kConvThreads, 4) recurrence_inputs_wide_kernel(const RecurrenceInputs p, int rows, int tile) {
     grid_launch_dependents();
     __shared__ TileToken tokens[kTileTokens];
+    __shared__ uint4 held_rows[kTileTokens][kConvThreads];
     const int c = (blockIdx.y * kConvThreads + threadIdx.x) * 8;
     const int token0 = blockIdx.x * tile;
     const bool live = c < p.rows.span;
     TapWindow<N> window;
     if (live) window.start(p.rows, c);
     grid_dependency_wait();
-    if (live) window.fetch(p.rows, c, token0);
+    if (live) fetch_rows(p.rows, c, token0, min(tile, rows - token0), &held_rows[0][threadIdx.x], kConvThreads);
     look_up_tile(p.rows, tokens, token0, tile, rows);
+    rows_arrived();   // (a thread reads no row but its own)
     __syncthreads();
     const int units = p.unit_heads * p.dim, lanes = p.dim / 8;
     const bool first = c < units, second = c >= p.second_at && c < p.second_at + units;
@@ -527,8 +540,7 @@ __global__ void __launch_bounds__(kConvThreads, 4) recurrence_inputs_wide_kernel
     for (int i = 0; i < tile && token0 + i < rows; ++i) {
         const int token = token0 + i;
         const TileToken now = tokens[i];
-        const uint4 row = window.ahead;
-        if (live && i + 1 < tile && token + 1 < rows) window.fetch(p.rows, c, token + 1);
+        const uint4 row = live ? held_rows[i][threadIdx.x] : make_uint4(0u, 0u, 0u, 0u);
         uint4 out = make_uint4(0u, 0u, 0u, 0u);
         float square = 0.0f;
         if (now.fresh <= 0) {
@@ -575,6 +587,11 @@ auto recurrence_inputs_kernel_for(unsigned) {
         if (p.rows.count == 2) kernel = CHOOSE<2>(THREADS);                                                                \
         if (p.rows.count == 3) kernel = CHOOSE<3>(THREADS);                                                                \
         if (p.rows.count == 4) kernel = CHOOSE<4>(THREADS);                                                                \
+        static int raised[kWideTaps + 1][3][kMaxDevices] = {};                                                             \
+        if ((SHARED) > 48 * 1024) {                                                                                        \
+            SINGE_CUDA_TRY(ensure_dynamic_shared(kernel, static_cast<int>(SHARED),                                         \
+                                                 raised[p.rows.count][(THREADS) <= 384 ? 0 : (THREADS) <= 768 ? 1 : 2]));  \
+        }                                                                                                                  \
         SINGE_CUDA_TRY(launch_dependent(kernel, GRID, dim3(THREADS), SHARED, static_cast<cudaStream_t>(stream), kLaunchGlue, 1, p, \
                                         static_cast<int>(rows), tile));                                                    \
         return launch_status();                                                                                            \
@@ -640,7 +657,8 @@ int attention_inputs(singe_stream_t stream, const AttentionInputs &p, size_t row
         const int tile = conv_tile(rows, 1);
         const unsigned threads = static_cast<unsigned>((p.rows.span / 8 + 31) / 32 * 32);
         const dim3 grid(static_cast<unsigned>((rows + tile - 1) / tile));
-        SINGE_WIDE_CONV(attention_inputs_kernel_for, grid, threads, static_cast<size_t>(tile) * p.pairs * sizeof(float2));
+        SINGE_WIDE_CONV(attention_inputs_kernel_for, grid, threads,
+                        static_cast<size_t>(tile) * (threads * sizeof(uint4) + p.pairs * sizeof(float2)));
     }
     const size_t bytes = 4 * sizeof(T);
     const bool out_wide = p.key_size % 4 == 0 && p.value_size % 4 == 0 && p.query_stride % 4 == 0 && aligned_to(p.query, bytes) &&
