@@ -157,9 +157,9 @@ def sum_over_ranks(value: float, group) -> float:
 # headline: config 2 paged decode
 # ----------------------------------------------------------------------------------------------------------
 
-# DRAM bytes one launch of paged_decode_kernel moves on the config-2 workload (seed 1), from an ncu capture of this
-# very command (dram__bytes_read.sum + dram__bytes_write.sum): 277.49 MB read + 7.69 MB written (split-K partials, output).
-DECODE_DRAM_TRAFFIC = 285_181_184
+# DRAM bytes one launch of paged_decode_even_kernel moves on the config-2 workload (seed 1), from an ncu capture of the same
+# call (dram__bytes_read.sum + dram__bytes_write.sum): 277.53 MB read + 5.42 MB written (partials, output).
+DECODE_DRAM_TRAFFIC = 282_945_024
 
 
 def decode_device_inputs(case, seed: int):
@@ -377,10 +377,10 @@ def run_decode(args, rank, world, group):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": DECODE_DRAM_TRAFFIC,
                      "traffic_unit": "bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                                     "paged_decode_kernel on this workload)",
+                                     "paged_decode_even_kernel on this workload)",
                      "algorithmic_bytes": int(my_bytes),
                      "peak_source": peaks["source"], "launch_us": round(launch_seconds * 1e6, 2),
-                     "kernels": "paged_decode_kernel + decode_combine_kernel"},
+                     "kernels": "paged_decode_even_kernel + even_combine_kernel"},
     }
     return line, case
 
