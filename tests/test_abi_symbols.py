@@ -51,10 +51,13 @@ def test_status_strings_and_host_only_helpers_need_no_gpu():
     assert lib.singe_paged_kv_decode_default_splits(64, 8, 4096, 16) == 4      # 1024-key pieces
     assert lib.singe_paged_kv_decode_default_splits(128, 8, 1024, 16) == 2     # 512-key pieces of a short bound
     assert lib.singe_paged_kv_decode_default_splits(1, 1, 2048, 16) == 16      # one row: the finest split
-    # scratch for one segment per SM and sequence, where pages are shared evenly: from 32 MB of keys and values on
+    # scratch for one segment per SM and sequence, where pages are shared evenly: from 32 MB of keys and values on, 24 MB for heads
+    # of 128 whose sequences would be split
     even = lib.singe_paged_kv_decode_even_splits
     assert even(32, 32, 8, 128, 4096, 16) == 6 and even(8, 32, 8, 128, 1024, 16) == 20
-    assert even(8, 32, 8, 128, 1008, 16) == 0 and even(96, 32, 8, 128, 512, 16) == 0 and even(32, 32, 2, 128, 4096, 16) == 0
+    assert even(8, 32, 8, 128, 768, 16) == 20 and even(8, 32, 8, 128, 752, 16) == 0 and even(48, 32, 8, 128, 128, 16) == 0
+    assert even(8, 32, 8, 64, 2048, 16) == 20 and even(8, 32, 8, 64, 2032, 16) == 0
+    assert even(96, 32, 8, 128, 512, 16) == 0 and even(32, 32, 2, 128, 4096, 16) == 0
     assert even(32, 32, 8, 128, 4096, 32) == 0 and even(32, 32, 8, 96, 4096, 16) == 0
 
 
