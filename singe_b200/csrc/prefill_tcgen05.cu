@@ -111,7 +111,7 @@ struct PrefillParams {
 // output is not finite (a hidden key's value may be anything, and zero times infinity is not zero).
 // Bound by the tensor core and the special-function unit alike: 8 + 16 MMAs of 128 x 128 x 16 and 16384 exponentials a
 // key tile.  One step of four 510-token chunks and 28 decoding sequences behind 0 - 3000 tokens of context, 32 query heads on 8:
-// 158 us with the rows behind; 175 before one thread issued the MMAs and the weights came in halves, 238 with items in order of their pair
+// 150 us with the rows behind; 158 before the items were decoded ahead, 175 before one thread issued the MMAs and the weights came in halves, 238 with items in order of their pair
 // index and lone tiles a key tile at a time, 40.2 ms by one warp per row and head.
 // Against 64 bits, this step and twelve of other sizes: outputs 1.6585e-3 off by either kernel, which is their rounding to bf16
 // (the squares of the two errors differ by 4e-6 squared: two terms, and long sums in the tensor core); log sums 5.6e-8, by the
@@ -347,6 +347,13 @@ __device__ __forceinline__ void scale_o_row(uint32_t tmem_o, float factor) {
     tmem_wait_st();
 }
 
+// 32 bytes by one lane.  The lanes of a warp store to rows of their own, a line each, so what counts is how many stores there are.
+__device__ __forceinline__ void store_sector(void *to, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(to), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
 // One unit of work: 256 query rows (tiles A and B) of one (sequence, head).
 struct Item {
     int head;
@@ -366,6 +373,12 @@ struct Item {
     bool alternate; // TENSOR: a single query tile, whose key tiles go to tile A's and tile B's places in turn
     bool valid;     // false: the sequence's offsets leave the packed tensors
 };
+
+// The items of a CTA's first rounds are decoded by its warps side by side before the roles part: item by item, the softmax waited
+// 2600 clk for its look-ups between two items, and another 4100 for the stores of 32 rows' lines, 16 bytes a lane (a key tile's step
+// takes 2950).  With stores of 32 bytes 8192 + 4096 + 2048 + 1024 tokens 726 -> 691 us at the power limit, eight prompts of 209 - 3355
+// 268 -> 250, the tensor surface's mixed step 157 -> 150.
+constexpr int kHeldItems = 64;
 
 __device__ __forceinline__ int pairs_of(int len_q) { return (max(len_q, 0) + kPair - 1) / kPair; }
 
@@ -578,6 +591,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     int pack = 0;
     int ordered = -1;                  // TENSOR: entries in `order`, or -1: items go by `counts`
     unsigned *order = nullptr;
+    Item *held = reinterpret_cast<Item *>(counts + kMaxRankTiles + kRedoCapacity);  // [kHeldItems]
     volatile float2 *share = nullptr;  // TENSOR: base and sum of tile B's rows of an alternating item
     if constexpr (TENSOR) {
         // (the redo list's place and what follows it)
@@ -594,6 +608,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         __syncthreads();
         ordered = order_items<WINDOW>(p, table, pack, counts, costs, entries, order, shared_ranks, warp, lane);
         if (ordered < 0) order = nullptr;
+        held = reinterpret_cast<Item *>(costs);  // (and the entries' place: both are done with)
+        static_assert(kHeldItems * sizeof(Item) <= 2 * kMaxOrdered * sizeof(int), "the ordering's scratch holds the items");
         __syncthreads();  // `counts` may be used again below
     }
     if (SAFE && !p.exact && *reinterpret_cast<volatile unsigned *>(&g_out_of_range_seen) == 0u) {
@@ -669,6 +685,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         return share_index(round);
     };
 
+    for (int round = warp; round < kHeldItems; round += kPrefillThreads / 32) {
+        const int index = item_index(round);
+        if (index < 0) break;
+        const Item item = decode(index);
+        if (lane == 0) held[round] = item;
+    }
+    auto item_at = [&](int round, int index) -> Item { return round < kHeldItems ? held[round] : decode(index); };
     if (tid == 0) {
         for (int i = 0; i < kBarriers; ++i) {
             const bool by_warps = i >= 16;  // p_full, o_empty, share
@@ -708,7 +731,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         for (int round = 0; (PAGED || warp == 9) && !failed; ++round) {
             const int index = item_index(round);
             if (index < 0) break;
-            const Item item = decode(index);
+            const Item item = item_at(round, index);
             if (item.key_tiles == 0) continue;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
@@ -851,8 +874,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                     item.key_tiles = 0;
                     return item;
                 }
+                item = item_at(round, index);
                 ++round;
-                item = decode(index);
                 if (item.key_tiles > 0) return item;
             }
         };
@@ -1013,7 +1036,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         for (int round = 0; !failed; ++round) {
             const int index = item_index(round);
             if (index < 0) break;
-            const Item item = decode(index);
+            const Item item = item_at(round, index);
             if (!item.valid) {
                 if (warp == 0 && lane == 0) report_status(p.error, kStatusIndexOutOfBounds);
                 continue;
@@ -1151,16 +1174,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             if (WINDOW && p.gate != nullptr) {
                 inverse /= 1.0f + __expf(-__bfloat162float(p.gate[token * p.gate_stride + item.head]));
             }
-            float probe = 0.0f;   // TENSOR: a NaN once an output is not finite
+            float probes[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // TENSOR: a NaN once an output is not finite
+            const bool sectors = (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0;  // whole sectors a lane
 #pragma unroll 1
             for (int c = 0; c < HD; c += 32) {
                 uint32_t r[32];
                 tmem_ld_x32(tmem_o + c, r);
-                tmem_wait_ld_into(r);
                 if constexpr (TENSOR) {
                     if (alternate) {
                         uint32_t b[32];
                         tmem_ld_x32(tmem_o + HD + c, b);
+                        tmem_wait_ld_into(r);
                         tmem_wait_ld_into(b);
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
@@ -1168,9 +1192,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                         }
                     }
                 }
+                if (!alternate) tmem_wait_ld_into(r);
                 if (TENSOR) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) probe = fmaf(__uint_as_float(r[i]) * inverse, 0.0f, probe);
+                    for (int i = 0; i < 32; ++i) probes[i % 4] = fmaf(__uint_as_float(r[i]) * inverse, 0.0f, probes[i % 4]);
                 }
                 if (c + 32 == HD) {
                     // O is out of tensor memory: the next item's first P V may overwrite it
@@ -1181,14 +1206,18 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 }
                 if (real) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 word;
-                        word.x = pack2<T>(__uint_as_float(r[i]) * inverse, __uint_as_float(r[i + 1]) * inverse);
-                        word.y = pack2<T>(__uint_as_float(r[i + 2]) * inverse, __uint_as_float(r[i + 3]) * inverse);
-                        word.z = pack2<T>(__uint_as_float(r[i + 4]) * inverse, __uint_as_float(r[i + 5]) * inverse);
-                        word.w = pack2<T>(__uint_as_float(r[i + 6]) * inverse, __uint_as_float(r[i + 7]) * inverse);
-                        if (empty) word = make_uint4(0u, 0u, 0u, 0u);
-                        *reinterpret_cast<uint4 *>(dst + c + i) = word;
+                    for (int i = 0; i < 32; i += 16) {
+                        uint32_t words[8];
+#pragma unroll
+                        for (int n = 0; n < 8; ++n) {
+                            words[n] = empty ? 0u : pack2<T>(__uint_as_float(r[i + 2 * n]) * inverse, __uint_as_float(r[i + 2 * n + 1]) * inverse);
+                        }
+                        if (sectors) {
+                            store_sector(dst + c + i, words);
+                        } else {
+                            reinterpret_cast<uint4 *>(dst + c + i)[0] = make_uint4(words[0], words[1], words[2], words[3]);
+                            reinterpret_cast<uint4 *>(dst + c + i)[1] = make_uint4(words[4], words[5], words[6], words[7]);
+                        }
                     }
                 }
             }
@@ -1196,7 +1225,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                 float value = empty ? -1.0e20f : (base_log2 + log2f(row_sum)) * 0.6931471805599453f;
                 if constexpr (TENSOR) {
                     value = base_log2 + log2f(row_sum);
-                    if (!in_range || empty || isnan(probe)) value = __int_as_float(0x7fc00000);  // has the row done again: see left_rows_kernel
+                    if (!in_range || empty || isnan((probes[0] + probes[1]) + (probes[2] + probes[3]))) value = __int_as_float(0x7fc00000);  // has the row done again: see left_rows_kernel
                 } else if (!SAFE && !in_range) {
                     value = __int_as_float(0x7fc00000);  // has the second launch redo the item
                     atomicExch(&g_out_of_range_seen, 1u);
@@ -1218,6 +1247,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
 }
 
 constexpr int kPrefillSmem = 6 * kTileBytes + 8 * 22 + 32 + kMaxRankTiles * 4 + kRedoCapacity * 4 + 1024;
+constexpr int kPrefillBytes = kPrefillSmem + kHeldItems * static_cast<int>(sizeof(Item));
+static_assert(kPrefillBytes <= 227 * 1024, "shared memory of one CTA");
 
 }  // namespace
 
@@ -1236,18 +1267,18 @@ template <typename T, int HD, bool PAGED, bool DENSE = false, bool WINDOW = fals
 int launch_prefill(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
                    const PrefillParams &params, unsigned persistent) {
     SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem));
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillBytes));
     if (std::is_same<T, __nv_bfloat16>::value) {
         SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem));
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillBytes));
         prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false>
-            <<<persistent, kPrefillThreads, kPrefillSmem, stream>>>(q_map, k_map, v_map, params, NoPaging{});
+            <<<persistent, kPrefillThreads, kPrefillBytes, stream>>>(q_map, k_map, v_map, params, NoPaging{});
         SINGE_TRY(launch_status());
     }
     // bf16: the redo pass over the same shares, a no-op while the device's out-of-range flag has never been raised.
     // f16 (params.exact): the only pass.  P must stay below 65504 there, so every tile takes its exact row maximum.
     prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false>
-        <<<persistent, kPrefillThreads, kPrefillSmem, stream>>>(q_map, k_map, v_map, params, NoPaging{});
+        <<<persistent, kPrefillThreads, kPrefillBytes, stream>>>(q_map, k_map, v_map, params, NoPaging{});
     return launch_status();
 }
 
