@@ -377,10 +377,11 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
                 if (lane == 0) mbar_arrive(bar_empty + 8 * slot_v);
             }
             if (failed) break;
+            // A leading product that is not finite stands alone: zero or less of an infinite value has been left out of it.
 #pragma unroll
             for (int nt = 0; nt < NTILES; ++nt) {
-                o[nt][0] += o[nt][2];
-                o[nt][1] += o[nt][3];
+                if (fabsf(o[nt][0]) < INFINITY) o[nt][0] += o[nt][2];
+                if (fabsf(o[nt][1]) < INFINITY) o[nt][1] += o[nt][3];
             }
             if (FORM == kEvenFused && counted_to == s.counted && turn == 0 && len > 0) {
                 add_new_key<T, HD>(p, x, qa, o, run_max, run_sum, b, head, row, quad, lane);

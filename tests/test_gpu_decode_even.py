@@ -43,6 +43,30 @@ def test_even_decode(lens, heads, kv_heads, head_dim, dtype):
     assert not host(out)[np.asarray(lens) == 0].any()
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,dtype", [(32, 8, 128, torch.bfloat16), (16, 4, 64, torch.float16)])
+def test_even_decode_values_that_are_not_finite(heads, kv_heads, head_dim, dtype):
+    # seen values of either infinity and NaN, in a sequence of one segment and in one of many; a finite column beside them
+    case = workloads.paged_decode_case(seed=9, heads=heads, kv_heads=kv_heads, head_dim=head_dim, lens=[40, 3000, 17], max_len=LONG)
+    assert even_splits(case) > 0
+    q, k, v = _inputs(case, seed=10)
+    for b in (0, 1):
+        for column, value in ((3, np.inf), (4, -np.inf), (5, np.nan)):
+            v[case.block_table[b, 1], 2, :, column] = value
+    operands = [dev(x, dtype) for x in (q, k, v)] + [dev(case.lens), dev_u32(case.block_table), _config(case)]
+    out = torch.empty((case.batch, heads, head_dim), dtype=dtype, device="cuda")
+    ops.paged_kv_decode_attention(out, *operands)
+    # what the split grid gives, whose weights are one term
+    splits = ks.lib().singe_paged_kv_decode_default_splits(case.batch, kv_heads, LONG, 16)
+    expect = torch.empty_like(out)
+    ops.paged_kv_decode_splitk_reduce(expect, torch.empty((case.batch, heads, splits, head_dim), device="cuda"),
+                                      torch.empty((case.batch, heads, splits), device="cuda"), *operands, splits)
+    got, expect = host(out), host(expect)
+    assert (expect[:2, :, 3] == np.inf).all() and (expect[:2, :, 4] == -np.inf).all() and np.isnan(expect[:2, :, 5]).all()
+    odd = ~np.isfinite(expect)
+    assert odd.sum() == 6 * heads and np.array_equal(got[odd], expect[odd], equal_nan=True)
+    assert_close_bf16(got[~odd], expect[~odd], "finite columns")
+
+
 def test_even_decode_reports_page_ids_outside_the_cache():
     case = workloads.paged_decode_case(seed=4, heads=8, kv_heads=4, head_dim=64, lens=[700, 40], max_len=LONG)
     q, k, v = _inputs(case, seed=5)
