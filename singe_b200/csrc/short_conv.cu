@@ -588,7 +588,7 @@ auto recurrence_inputs_kernel_for(unsigned) {
         if (p.rows.count == 3) kernel = CHOOSE<3>(THREADS);                                                                \
         if (p.rows.count == 4) kernel = CHOOSE<4>(THREADS);                                                                \
         static int raised[kWideTaps + 1][3][kMaxDevices] = {};                                                             \
-        if ((SHARED) > 48 * 1024) {                                                                                        \
+        if ((SHARED) > 0) {  /* (the limit until raised, 48 KB, holds the kernel's own arrays as well) */                  \
             SINGE_CUDA_TRY(ensure_dynamic_shared(kernel, static_cast<int>(SHARED),                                         \
                                                  raised[p.rows.count][(THREADS) <= 384 ? 0 : (THREADS) <= 768 ? 1 : 2]));  \
         }                                                                                                                  \

@@ -8,15 +8,13 @@ from singe_b200.layer_ops import Ops
 pytestmark = pytest.mark.gpu
 
 
-# rows of 192, 384, 640 and 1024 threads (24 to 136 KB of shared memory); a last tile of one row; a sequence that begins inside a tile
-@pytest.mark.parametrize("heads,kv_heads,taps", [(8, 2, 4), (16, 4, 4), (24, 8, 1), (48, 8, 3)])
-def test_tiles_equal_rows_one_at_a_time(heads, kv_heads, taps):
-    ops, dim, page_size, pairs = Ops("bfloat16"), 128, 16, 32
+def check_tiles(heads, kv_heads, taps, dim=128, vdim=128, pairs=32):
+    ops, page_size = Ops("bfloat16"), 16
     lengths = [4001, 1, 743]
     tokens = sum(lengths)
     assert tokens >= 4 * torch.cuda.get_device_properties(0).multi_processor_count * 8 and tokens % 8 == 1
     key_at, value_at = heads * dim, (heads + kv_heads) * dim
-    span, pages = value_at + kv_heads * dim, tokens // page_size + 1
+    span, pages = value_at + kv_heads * vdim, tokens // page_size + 1
     gen = torch.Generator(device="cuda").manual_seed(heads)
     normal = lambda *shape: torch.randn(*shape, device="cuda", generator=gen).bfloat16()
     projected, bias, weight, norms = normal(tokens, span), normal(span), normal(taps, span), (normal(heads * dim), normal(kv_heads * dim))
@@ -29,7 +27,7 @@ def test_tiles_equal_rows_one_at_a_time(heads, kv_heads, taps):
 
     def run(portions):
         query = torch.zeros((tokens, heads * dim), dtype=torch.bfloat16, device="cuda")
-        caches = [torch.zeros((pages, page_size, kv_heads * dim), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        caches = [torch.zeros((pages, page_size, kv_heads * size), dtype=torch.bfloat16, device="cuda") for size in (dim, vdim)]
         status = torch.zeros(1, dtype=torch.int32, device="cuda")
         for begin, end in portions:    # (a portion's rows are all new tokens of a call that starts with the whole prompt's first row)
             n = end - begin
@@ -39,10 +37,24 @@ def test_tiles_equal_rows_one_at_a_time(heads, kv_heads, taps):
                      *caches, None, None, projected[begin:end], projected.stride(0), bias, weight, kept.clone(), norms[0], norms[1],
                      frequencies, pairs, 1.0, i64(at), i32(sequence_of), i32(first - begin), i32(lengths), i32(context),
                      i64(place[begin:end] // page_size), i64(place[begin:end] % page_size), None, None, 0, n, len(lengths), taps, heads,
-                     kv_heads, dim, dim, dim, dim, key_at, value_at, span, pages, page_size, 1e-5, status)
+                     kv_heads, dim, vdim, dim, vdim, key_at, value_at, span, pages, page_size, 1e-5, status)
         assert int(status.item()) == 0
         return [query] + caches
 
     whole = run([(0, tokens)])
     few = run([(begin, min(begin + 1000, tokens)) for begin in range(0, tokens, 1000)])
     assert all(torch.equal(a, b) for a, b in zip(whole, few)) and whole[0].float().abs().sum() > 0
+
+
+# rows of 192, 384, 640 and 1024 threads (24 to 136 KB of shared memory); a last tile of one row; a sequence that begins inside a tile
+@pytest.mark.parametrize("heads,kv_heads,taps", [(8, 2, 4), (16, 4, 4), (24, 8, 1), (48, 8, 3)])
+def test_tiles_equal_rows_one_at_a_time(heads, kv_heads, taps):
+    check_tiles(heads, kv_heads, taps)
+
+
+# 48 KB to the byte behind the kernel's own arrays, from rows of 352, 384 and 320 threads
+@pytest.mark.parametrize("heads,kv_heads,taps,dim,vdim,pairs", [(16, 4, 4, 128, 64, 64), (16, 4, 2, 128, 128, 0), (6, 2, 4, 256, 256, 128)])
+def test_tiles_of_48_kilobytes(heads, kv_heads, taps, dim, vdim, pairs):
+    span = (heads + kv_heads) * dim + kv_heads * vdim
+    assert 8 * (span // 8 * 16 + pairs * 8) == 48 * 1024
+    check_tiles(heads, kv_heads, taps, dim, vdim, pairs)
