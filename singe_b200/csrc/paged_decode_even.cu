@@ -266,6 +266,13 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
         const int v_sel = mat >> 1;
         const uint32_t tile = base + turn * NHALF * BOX + head * kHalfBytes;
         if (stable) grid_dependency_wait();
+        // Ahead of every wait that may run out: the fold reads the entry of each sequence, whatever has become of its rows.
+        if (warp == 0) {
+            for (int b = first_sequence + (before[first_sequence] < lo ? 1 : 0) + lane; b < p.batch && before[b] < hi; b += 32) {
+                const int last = static_cast<int>((static_cast<long long>(before[b + 1]) * ctas - 1) / total);
+                rows[b] = {last - cta + 1, cta + b};
+            }
+        }
         int n = 0;        // steps taken
         int merges = 0;   // merges of the head's two warps so far
         uint32_t qa[KSTEPS][2];
@@ -291,10 +298,6 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
             const int to = min(counted_to, s.real);
             const bool whole = from == 0 && counted_to == s.counted;
             const int slot_of_row = cta + b;
-            if (from == 0 && warp == 0 && lane == 0) {
-                const int last = static_cast<int>((static_cast<long long>(before[b + 1]) * ctas - 1) / total);
-                rows[b] = {last - cta + 1, slot_of_row};
-            }
             if (FORM == kEvenFused) rotate_query_fragments<T, HD>(qa, p, x, b, row, quad);
             float o[NTILES][4];
 #pragma unroll
@@ -468,9 +471,18 @@ __global__ void __launch_bounds__(kEvenThreads, 1)
 // 17.3, 14.7, 14.7, 14.2; 48 x 298 24.3, 20.0, 18.9, 17.8.
 constexpr int kFoldWarps = 8;
 
+}  // namespace
+
+// Whether a sequence's segments lie in a scratch of `slots` slots, whose last one is the list.
+__host__ __device__ bool even_row_inside(int segments, int slot, int slots) {
+    return segments > 0 && segments <= kEvenMaxCtas && slot >= 0 && segments < slots && slot < slots - segments;
+}
+
+namespace {
+
 template <typename T, int HD, int TEAM>
 __global__ void __launch_bounds__(32 * kFoldWarps)
-    even_combine_kernel(T *out, const float *attn_partial, const float *lse_partial, const EvenRow *rows, int heads) {
+    even_combine_kernel(T *out, const float *attn_partial, const float *lse_partial, const EvenRow *rows, int heads, int slots) {
     grid_launch_dependents();
     grid_dependency_wait();
     constexpr int kColumns = HD / 32;   // columns of a lane
@@ -486,6 +498,8 @@ __global__ void __launch_bounds__(32 * kFoldWarps)
     const EvenRow row = rows[b];
     const int segments = row.segments;
     if (segments <= 1) return;   // written by the decode kernel
+    // (an entry that calls which share a caller's scratch have written over each other ends here)
+    if (!even_row_inside(segments, row.slot, slots)) return;
     const bool real = head < heads;
     const size_t first = static_cast<size_t>(row.slot) * heads + (real ? head : 0);
     const float *partial = attn_partial + first * HD + lane * kColumns;
@@ -579,7 +593,7 @@ int launch_even(cudaStream_t stream, const DecodeParams &params, const StepExtra
         return launch_dependent(kernel, dim3(static_cast<unsigned>((params.heads + rows_per_cta - 1) / rows_per_cta),
                                              static_cast<unsigned>(params.batch)),
                                 dim3(32 * kFoldWarps), 0, stream, kLaunchCombine, 1, static_cast<T *>(params.out),
-                                params.attn_partial, params.lse_partial, rows, params.heads);
+                                params.attn_partial, params.lse_partial, rows, params.heads, slots);
     };
     SINGE_CUDA_TRY(params.batch < 12   ? fold(even_combine_kernel<T, HD, 8>, 8)
                    : params.batch < 20 ? fold(even_combine_kernel<T, HD, 4>, 4)
