@@ -17,6 +17,7 @@ bool paged_decode_fast_path(size_t heads, size_t kv_heads, size_t head_dim, size
                             const void *value_cache, const void *query);
 size_t paged_decode_split_tokens(size_t key_len_bound, size_t max_splits, size_t block_size);
 size_t paged_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound);
+bool even_operands(const void *out, const float *attn_scratch);
 int paged_decode_splitk(cudaStream_t stream, int element, void *out, float *attn_scratch, float *lse_scratch,
                         const void *query, const void *key_cache, const void *value_cache,
                         const int32_t *actual_seq_lens, const uint32_t *block_table, size_t batch, size_t heads,
@@ -772,7 +773,7 @@ int decode_half(cudaStream_t stream, int element, void *out, const void *query, 
     }
     // The tiled kernel puts the batch in a grid dimension of at most 65535; larger batches keep the general kernel.
     if (batch <= 65535 && paged_decode_fast_path(heads, kv_heads, head_dim, block_size, key_cache, value_cache, query)) {
-        const size_t even = paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size);
+        const size_t even = even_operands(out, nullptr) ? paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size) : 0;
         const size_t splits = even > 0 ? even : wave_aware_splits(batch, kv_heads, stride * block_size, block_size);
         float *scratch = nullptr;
         const size_t rows = batch * heads * splits;

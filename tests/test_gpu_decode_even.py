@@ -43,6 +43,26 @@ def test_even_decode(lens, heads, kv_heads, head_dim, dtype):
     assert not host(out)[np.asarray(lens) == 0].any()
 
 
+def split_grid(case, operands):
+    """The call in the split grid with the pieces it chooses for itself."""
+    splits = ks.lib().singe_paged_kv_decode_default_splits(case.batch, case.kv_heads, case.block_table_batch_stride * 16, 16)
+    attn = torch.empty((case.batch, case.heads, splits, case.head_dim), device="cuda")
+    out = torch.empty_like(operands[0])
+    ops.paged_kv_decode_splitk_reduce(out, attn, torch.empty(attn.shape[:3], device="cuda"), *operands, splits)
+    return out
+
+
+def test_outputs_at_odd_places_take_the_split_grid_with_its_own_pieces():
+    case = workloads.paged_decode_case(seed=12, heads=8, kv_heads=8, head_dim=64, lens=[2500, 30, 700], max_len=LONG)
+    q, k, v = _inputs(case, seed=13)
+    operands = [dev(x, torch.bfloat16) for x in (q, k, v)] + [dev(case.lens), dev_u32(case.block_table), _config(case)]
+    room = torch.empty(q.size + 1, dtype=torch.bfloat16, device="cuda")
+    out = room[1:].view(q.shape)
+    ops.paged_kv_decode_attention(out, *operands)
+    assert even_splits(case) > 0 and out.data_ptr() % 4 == 2
+    assert torch.equal(out, split_grid(case, operands))
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,dtype", [(32, 8, 128, torch.bfloat16), (16, 4, 64, torch.float16)])
 def test_even_decode_values_that_are_not_finite(heads, kv_heads, head_dim, dtype):
     # seen values of either infinity and NaN, in a sequence of one segment and in one of many; a finite column beside them
@@ -55,11 +75,7 @@ def test_even_decode_values_that_are_not_finite(heads, kv_heads, head_dim, dtype
     operands = [dev(x, dtype) for x in (q, k, v)] + [dev(case.lens), dev_u32(case.block_table), _config(case)]
     out = torch.empty((case.batch, heads, head_dim), dtype=dtype, device="cuda")
     ops.paged_kv_decode_attention(out, *operands)
-    # what the split grid gives, whose weights are one term
-    splits = ks.lib().singe_paged_kv_decode_default_splits(case.batch, kv_heads, LONG, 16)
-    expect = torch.empty_like(out)
-    ops.paged_kv_decode_splitk_reduce(expect, torch.empty((case.batch, heads, splits, head_dim), device="cuda"),
-                                      torch.empty((case.batch, heads, splits), device="cuda"), *operands, splits)
+    expect = split_grid(case, operands)     # (its weights are one term)
     got, expect = host(out), host(expect)
     assert (expect[:2, :, 3] == np.inf).all() and (expect[:2, :, 4] == -np.inf).all() and np.isnan(expect[:2, :, 5]).all()
     odd = ~np.isfinite(expect)
