@@ -123,6 +123,11 @@ int singe_kv_cache_write_f32(singe_stream_t stream, void *key_cache, void *value
  * whose kernels can overlap on the GPU (different streams, no event between them) race on it -- run them on
  * one stream at a time or pass caller-owned scratch.  Growth never frees: a buffer that was handed out
  * (and may be baked into a captured CUDA graph) stays allocated until singe_release_workspaces().
+ * Sequences that fit one piece (512 keys or more, see singe_paged_kv_decode_default_splits) leave no partials there:
+ * calls of such sequences may overlap, on streams and in graphs.  The form that shares the cached pages evenly among
+ * the SMs always has partials; its scratch belongs to the stream, and in a capture to the graph and its stream, so that
+ * this holds for it too (but not for two executables instantiated from one graph).  A device has 64 such scratches,
+ * allocated when first needed, also in a capture; where none is to be had the split grid serves the call.
  * ================================================================================================= */
 int singe_paged_kv_decode_attention_bf16(singe_stream_t stream, void *out, const void *query,
                                          const void *key_cache, const void *value_cache,
@@ -893,7 +898,8 @@ int singe_warm_l2_with_next_launch(const void *pointer, size_t bytes);
 
 /* Frees the current device's decode workspaces (the live one and every one retired by growth) after a device
  * synchronisation.  Only when no captured graph that used them will be replayed again.  No reference
- * counterpart (the reference's operators take all scratch from the caller). */
+ * counterpart (the reference's operators take all scratch from the caller).  Scratches that captured graphs hold are
+ * kept; they are free again once their graph is gone. */
 int singe_release_workspaces(void);
 
 /* Reads and clears the library's sticky device error word for the current device (synchronises the device).

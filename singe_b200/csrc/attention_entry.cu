@@ -1,6 +1,7 @@
 // C-ABI entry points of the attention surfaces: host-side validation that mirrors the reference's
 // config validators, dispatch between the specialised kernels and the general one, and the policies
 // that describe each surface to the general kernel.
+#include <atomic>
 #include <cmath>
 #include <mutex>
 
@@ -677,12 +678,112 @@ int workspace_for(cudaStream_t stream, size_t floats, float **data) {
     return SINGE_OK;
 }
 
+// Scratch of the drop-in decode's even form.  That form uses its scratch on every call, also where no sequence is longer than a
+// piece, which the split grid serves without: calls of short sequences may overlap, on several streams and in several graphs.  So
+// it does not stand in the shared workspace.  Each stream has a scratch of its own, whose calls follow one another, and so has
+// each stream of a capture: the graph keeps it (a user object) until it and what was instantiated from it are gone, then it is
+// free for other captures.  Where none is to be had -- kEvenScratches are in use, memory is short -- the split grid serves the call.
+constexpr int kEvenScratches = 64;
+
+struct EvenScratch {
+    float *data = nullptr;
+    size_t floats = 0;
+    unsigned long long stream = 0, capture = 0;   // capture: 0 outside of one
+    std::atomic<bool> held{false};
+    std::mutex enqueue;   // of two threads' calls on one stream, neither's kernels come between the other's
+};
+
+struct EvenScratches {
+    EvenScratch all[kEvenScratches];
+    std::mutex mutex;
+};
+EvenScratches g_even_scratches[kMaxDevices];
+
+// What the runtime calls once no graph needs the scratch any more.
+void give_back_even_scratch(void *scratch) { static_cast<EvenScratch *>(scratch)->held = false; }
+
+// The scratch, of `floats` or more, of a call on `stream`, or nullptr.
+EvenScratch *even_scratch(cudaStream_t stream, size_t floats) {
+    const int device = device_slot();
+    if (device < 0) return nullptr;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0, capture = 0;
+    cudaGraph_t graph = nullptr;
+    cudaError_t error = cudaStreamGetCaptureInfo(stream, &status, &capture, &graph);
+    if (error == cudaSuccess && status == cudaStreamCaptureStatusNone) {
+        capture = 0;
+        error = cudaStreamGetId(stream, &id);   // (unlike the handle, never given to another stream)
+    } else {
+        id = reinterpret_cast<uintptr_t>(stream);   // the identifier may not be asked for in a capture
+    }
+    if (error != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (status == cudaStreamCaptureStatusInvalidated) return nullptr;
+    EvenScratches &scratches = g_even_scratches[device];
+    std::lock_guard<std::mutex> guard(scratches.mutex);
+    EvenScratch *best = nullptr, *empty = nullptr;
+    for (EvenScratch &each : scratches.all) {
+        if (each.held) {
+            if (each.stream == id && each.capture == capture && each.floats >= floats) return &each;
+        } else if (each.data == nullptr) {
+            if (empty == nullptr) empty = &each;
+        } else if (each.floats >= floats && (best == nullptr || each.floats < best->floats)) {
+            best = &each;
+        }
+    }
+    if (best == nullptr) {
+        if (empty == nullptr) return nullptr;
+        // No work of the capture depends on the allocation.  A stream's scratch that has become too small stays until the
+        // workspaces are released, as the workspace does: calls may still be using it.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        error = cudaMalloc(&empty->data, 2 * floats * sizeof(float));
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (error != cudaSuccess) {
+            empty->data = nullptr;
+            cudaGetLastError();
+            return nullptr;
+        }
+        empty->floats = 2 * floats;
+        best = empty;
+    }
+    best->held = true;
+    best->stream = id;
+    best->capture = capture;
+    if (capture != 0) {
+        cudaUserObject_t keeper = nullptr;
+        error = cudaUserObjectCreate(&keeper, best, give_back_even_scratch, 1, cudaUserObjectNoDestructorSync);
+        if (error != cudaSuccess) {
+            best->held = false;
+        } else {
+            error = cudaGraphRetainUserObject(graph, keeper, 1, cudaGraphUserObjectMove);
+            if (error != cudaSuccess) cudaUserObjectRelease(keeper, 1);   // (gives the scratch back)
+        }
+        if (error != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+    }
+    return best;
+}
+
 int release_workspaces() {
     const int device = device_slot();
     if (device < 0) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
     std::lock_guard<std::mutex> guard(g_workspace_mutex);
     Workspace &space = g_workspace[device];
     SINGE_CUDA_TRY(cudaDeviceSynchronize());
+    EvenScratches &scratches = g_even_scratches[device];
+    std::lock_guard<std::mutex> even_guard(scratches.mutex);
+    for (EvenScratch &each : scratches.all) {
+        if (each.held && each.capture != 0) continue;   // its graph gives it back
+        if (each.data != nullptr) cudaFree(each.data);
+        each.data = nullptr;
+        each.floats = 0;
+        each.held = false;
+    }
     for (int i = 0; i < space.retired_count; ++i) cudaFree(space.retired[i]);
     space.retired_count = 0;
     if (space.data != nullptr) cudaFree(space.data);
@@ -773,14 +874,21 @@ int decode_half(cudaStream_t stream, int element, void *out, const void *query, 
     }
     // The tiled kernel puts the batch in a grid dimension of at most 65535; larger batches keep the general kernel.
     if (batch <= 65535 && paged_decode_fast_path(heads, kv_heads, head_dim, block_size, key_cache, value_cache, query)) {
-        const size_t even = even_operands(out, nullptr) ? paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size) : 0;
-        const size_t splits = even > 0 ? even : wave_aware_splits(batch, kv_heads, stride * block_size, block_size);
+        auto split_into = [&](size_t splits, float *scratch, bool even) -> int {
+            return paged_decode_splitk(stream, element, out, scratch, scratch + batch * heads * splits * head_dim, query, key_cache,
+                                       value_cache, lens, table, batch, heads, kv_heads, head_dim, physical_blocks, stride,
+                                       splits, scale, false, device_error_word(), nullptr, 0u, nullptr, nullptr, nullptr, even);
+        };
+        const size_t splits = wave_aware_splits(batch, kv_heads, stride * block_size, block_size);
         float *scratch = nullptr;
-        const size_t rows = batch * heads * splits;
-        SINGE_TRY(workspace_for(stream, rows * (head_dim + 1), &scratch));
-        return paged_decode_splitk(stream, element, out, scratch, scratch + rows * head_dim, query, key_cache,
-                                   value_cache, lens, table, batch, heads, kv_heads, head_dim, physical_blocks, stride,
-                                   splits, scale, false, device_error_word(), nullptr, 0u, nullptr, nullptr, nullptr, true);
+        SINGE_TRY(workspace_for(stream, batch * heads * splits * (head_dim + 1), &scratch));
+        const size_t even = even_operands(out, nullptr) ? paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size) : 0;
+        EvenScratch *own = even > 0 ? even_scratch(stream, batch * heads * even * (head_dim + 1)) : nullptr;
+        if (own != nullptr) {
+            std::lock_guard<std::mutex> guard(own->enqueue);
+            return split_into(even, own->data, true);
+        }
+        return split_into(splits, scratch, false);
     }
     if (element == 0) {
         return decode_general<__nv_bfloat16>(stream, out, query, key_cache, value_cache, lens, table, batch, heads,

@@ -171,3 +171,95 @@ def test_even_chunked_decode(heads, kv_heads, head_dim, chunk):
                                                   batch=len(lens), heads=heads, kv_heads=kv_heads, head_dim=head_dim, block_size=16,
                                                   block_table_batch_stride=pages, scale=head_dim ** -0.5)
     assert_close_bf16(host(out), expect, f"chunks of {chunk}")
+
+
+def short_problem(seed, dtype=torch.bfloat16):
+    """Sequences of at most a piece, which the split grid serves without any scratch; operands and what a lone call gives."""
+    lens = np.random.default_rng(seed).integers(1, 513, size=80)
+    case = workloads.paged_decode_case(seed=seed, heads=16, kv_heads=8, head_dim=128, lens=lens, max_len=512)
+    assert even_splits(case) > 0
+    operands = [dev(x, dtype) for x in _inputs(case, seed)] + [dev(case.lens), dev_u32(case.block_table), _config(case)]
+    alone = torch.empty_like(operands[0])
+    ops.paged_kv_decode_attention(alone, *operands)
+    torch.cuda.synchronize()
+    assert not torch.equal(alone, split_grid(case, operands))     # (the two forms can be told apart)
+    return operands, alone
+
+
+def test_calls_of_short_sequences_overlap_on_streams():
+    problems = [short_problem(seed) for seed in (21, 22)]
+    streams = [torch.cuda.Stream() for _ in problems]
+    outs = [[torch.empty_like(alone) for _ in range(100)] for _, alone in problems]
+    torch.cuda.synchronize()
+    for i in range(100):
+        for stream, (operands, _), out in zip(streams, problems, outs):
+            ops.paged_kv_decode_attention(out[i], *operands, stream=stream)
+    torch.cuda.synchronize()
+    for (_, alone), out in zip(problems, outs):
+        assert all(torch.equal(alone, each) for each in out)
+
+
+def captured(operands, calls):
+    graph, outs = torch.cuda.CUDAGraph(), [torch.empty_like(operands[0]) for _ in range(calls)]
+    with torch.cuda.graph(graph):
+        for out in outs:
+            ops.paged_kv_decode_attention(out, *operands)
+    return graph, outs
+
+
+def test_calls_of_short_sequences_overlap_in_graphs():
+    problems = [short_problem(seed) for seed in (23, 24)]
+    graphs = [captured(operands, 40) for operands, _ in problems]
+    streams = [torch.cuda.Stream() for _ in problems]
+    for _ in range(3):
+        for _, outs in graphs:
+            for out in outs:
+                out.zero_()
+        torch.cuda.synchronize()
+        for stream, (graph, _) in zip(streams, graphs):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        out = torch.empty_like(problems[0][1])
+        ops.paged_kv_decode_attention(out, *problems[0][0])       # and a call beside them
+        torch.cuda.synchronize()
+        assert torch.equal(out, problems[0][1])
+        for (_, alone), (_, outs) in zip(problems, graphs):
+            assert all(torch.equal(alone, each) for each in outs)
+
+
+def test_graphs_that_are_gone_give_their_scratch_back():
+    operands, alone = short_problem(25)
+    for _ in range(150):              # more than there are scratches
+        graph, (out,) = captured(operands, 1)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, alone)
+        graph.reset()
+        torch.cuda.synchronize()
+
+
+def test_more_graphs_than_scratches():
+    operands, alone = short_problem(26)
+    kept = [captured(operands, 1) for _ in range(80)]
+    for graph, _ in kept:
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(out, alone) for _, (out,) in kept[:8])
+    for _, (out,) in kept:            # the last ones in the split grid
+        assert_close_bf16(host(out), host(alone), "either form")
+
+
+def test_a_capture_without_a_call_before_it_is_refused():
+    operands, alone = short_problem(27)
+    ks.lib().singe_release_workspaces()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(ops.SingeError) as refused:
+            ops.paged_kv_decode_attention(torch.empty_like(alone), *operands)
+        operands[0].add_(0)
+    assert refused.value.code == 12
+    ops.paged_kv_decode_attention(alone.clone(), *operands)
+    graph, (out,) = captured(operands, 1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, alone)
