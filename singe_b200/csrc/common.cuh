@@ -12,6 +12,7 @@
 #include <stdlib.h>
 
 #include "../../include/singe_kernel_sys.h"
+#include "raised_limit.cuh"
 
 namespace singe {
 
@@ -111,11 +112,12 @@ inline int device_slot() {
 // function, so a process that drives several GPUs sets it on each).  `done` is the launch site's own table.
 template <typename Kernel>
 inline cudaError_t ensure_dynamic_shared(Kernel kernel, int bytes, int (&done)[kMaxDevices]) {
+    static std::mutex mutex;
     const int slot = device_slot();
-    if (slot >= 0 && done[slot] >= bytes) return cudaSuccess;
-    const cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (error == cudaSuccess && slot >= 0) done[slot] = bytes;
-    return error;
+    int unknown = 0;
+    return static_cast<cudaError_t>(raise_limit(bytes, slot >= 0 ? done[slot] : unknown, mutex, [&](int needed) -> int {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, needed);
+    }));
 }
 
 template <typename... Parameters, typename... Arguments>

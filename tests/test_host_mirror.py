@@ -20,3 +20,11 @@ def test_cpp_host_mirror_validation(tmp_path):
     result = subprocess.run([str(binary)], capture_output=True, text=True)
     assert result.returncode == 0, result.stdout + result.stderr
     assert "host mirror ok" in result.stdout
+
+
+def test_limits_are_raised_and_never_lowered(tmp_path):
+    binary = tmp_path / "test_raised_limit"
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-Wall", "-pthread", os.path.join(ROOT, "tests", "host", "test_raised_limit.cpp"),
+                    "-o", str(binary)], check=True)
+    result = subprocess.run([str(binary)], capture_output=True, text=True, timeout=60)
+    assert result.returncode == 0 and "raised limit ok" in result.stdout, result.stdout
