@@ -18,6 +18,7 @@ bool paged_decode_fast_path(size_t heads, size_t kv_heads, size_t head_dim, size
                             const void *value_cache, const void *query);
 size_t paged_decode_split_tokens(size_t key_len_bound, size_t max_splits, size_t block_size);
 size_t paged_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound);
+bool paged_decode_even_pays(size_t batch, size_t kv_heads, size_t head_dim, size_t bound);
 bool even_operands(const void *out, const float *attn_scratch);
 int paged_decode_splitk(cudaStream_t stream, int element, void *out, float *attn_scratch, float *lse_scratch,
                         const void *query, const void *key_cache, const void *value_cache,
@@ -882,7 +883,8 @@ int decode_half(cudaStream_t stream, int element, void *out, const void *query, 
         const size_t splits = wave_aware_splits(batch, kv_heads, stride * block_size, block_size);
         float *scratch = nullptr;
         SINGE_TRY(workspace_for(stream, batch * heads * splits * (head_dim + 1), &scratch));
-        const size_t even = even_operands(out, nullptr) ? paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size) : 0;
+        const size_t even = even_operands(out, nullptr) && paged_decode_even_pays(batch, kv_heads, head_dim, stride * block_size)
+                                ? paged_decode_even_splits(batch, heads, kv_heads, head_dim, stride * block_size) : 0;
         EvenScratch *own = even > 0 ? even_scratch(stream, batch * heads * even * (head_dim + 1)) : nullptr;
         if (own != nullptr) {
             std::lock_guard<std::mutex> guard(own->enqueue);

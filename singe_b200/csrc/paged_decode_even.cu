@@ -621,14 +621,13 @@ int launch_even_shape(cudaStream_t stream, const DecodeParams &params, const Ste
 // 128 whose sequences the split grid has to split as well (us, calls one after the other, split grid and here; "to" is the shortest of a
 // ragged batch): 4 x 1536 of 128 11.0 and 10.1, 384 to 1536 10.5 and 9.7; 20 x 307 14.2 and 10.5; 4 x 2901 19.2 and 13.5; 8 x
 // 640, 20 MB, 10.0 and 10.4; 48 x 128, not split, 7.4 and 10.9; heads of 64, 14 x 877 12.6 and 10.6, but 219 to 877 8.9 and 9.6; at 32
-// MB 8 x 2176 16.4 and 13.1, 544 to 2176 10.5 and 10.3.  (Ragged batches of 13 - 20 of these may still lose: 478 to 1911 x 15 13.7
-// and 14.4, whole 21.9 and 18.0.)  Sequences of one split each need no fold there: they stay while they fill the grid
+// MB 8 x 2176 16.4 and 13.1, 544 to 2176 10.5 and 10.3.  (Ragged batches of more rows may lose, see paged_decode_even_pays.)  Sequences of one split each need no fold there: they stay while they fill the grid
 // (three CTAs an SM) one and a half times, 96 x 256 24.1 against 25.1 here; 64 x 256, 1.15 times, 27.1 against 18.9.
 size_t paged_decode_even_slots(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t bound) {
     const size_t sms = static_cast<size_t>(device_sm_count());
     const size_t stride = (bound + kPageTokens - 1) / kPageTokens;
     if ((kv_heads != 8 && kv_heads != 4) || batch > kEvenMaxBatch || sms > kEvenMaxCtas || 2 * batch > heads * head_dim ||
-        stride > (size_t{1} << 30) / batch) {
+        stride > (size_t{1} << 30) / batch || stride >= (size_t{1} << 27)) {   // (positions stay below 2^31)
         return 0;
     }
     const bool split = bound > 128 && batch * kv_heads <= 3 * sms;
@@ -641,6 +640,25 @@ size_t paged_decode_even_slots(size_t batch, size_t heads, size_t kv_heads, size
 // The same as a number of splits of a [batch, heads, splits, head_dim] scratch.
 size_t paged_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, size_t head_dim, size_t key_len_bound) {
     return (paged_decode_even_slots(batch, heads, kv_heads, head_dim, key_len_bound) + batch - 1) / batch;
+}
+
+// Whether a drop-in call takes the even form.  Its caller knows nothing of the lengths but the bound, so the line lies where ragged
+// batches (lengths spread from 1/4 or 1/32 of the bound up to it) stop losing, on some 600 shapes.  With at most 32 rows what the
+// split grid has to split decides, as above.  With more, ragged lengths leave that grid a single wave, which is hard to beat below
+// 40 MB of keys and values at the bound (8 heads of 128), 112 MB (heads of 64), 160 MB (4 of 128), or 48 MB where there are rows
+// enough to fill the wave without splits (us, split grid and here, lengths from a quarter of the bound, then all at it: heads of 64, 20 x
+// 1024 11.5 and 12.7, 17.2 and 14.6; 24 x 2128 on 4 12.8 and 14.2, 20.2 and 16.6; 20 x 3584 27.1 and 22.4, 32.7 and 30.8; 4 heads of
+// 128, 20 x 1632 14.1 and 14.9, 22.2 and 19.3).  Of the calls it takes none from half of the bound on loses, of 1422 ragged ones 13 by 2 - 8 %.
+// Lengths far below the bound may lose: all at a sixteenth of it, heads of 64, 32 x 140 7.8 and 9.5, 64 x 280 17.2 and 14.7.
+bool paged_decode_even_pays(size_t batch, size_t kv_heads, size_t head_dim, size_t bound) {
+    const size_t rows = batch * kv_heads, stride = (bound + kPageTokens - 1) / kPageTokens;
+    size_t least = 32;
+    if (kv_heads * head_dim == 1024) {
+        least = rows <= 32 ? 24 : 40;
+    } else if (rows > 32) {
+        least = head_dim == 128 ? (rows < 192 ? 160 : 48) : (rows < 384 ? 112 : 48);
+    }
+    return batch * stride * kPageTokens * kv_heads * head_dim * 4 >= least << 20;
 }
 
 // The decode kernels' call in the even form; params.out, scratch of `slots` slots, extras.qkv (fused) as there.

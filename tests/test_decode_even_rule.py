@@ -15,3 +15,20 @@ def test_fold_stays_inside_its_scratch(slots):
     for segments in edges:
         for slot in edges:
             assert inside(segments, slot, slots) == (0 < segments <= 256 and slot >= 0 and slot + segments <= slots - 1)
+
+
+@pytest.mark.parametrize("kv_heads,head_dim,batch,bound,pays", [
+    # few rows; ragged batches that lost, and the same from where they no longer do
+    (8, 128, 4, 1600, True), (8, 128, 1, 6000, False), (8, 128, 64, 128, False), (8, 128, 64, 160, True), (8, 128, 32, 4096, True),
+    (8, 64, 4, 4224, True), (8, 64, 20, 1024, False), (8, 64, 15, 1911, False), (8, 64, 20, 3584, True), (8, 64, 64, 400, True),
+    (4, 64, 24, 2128, False), (4, 64, 32, 4480, True), (4, 128, 20, 1632, False), (4, 128, 20, 4960, True), (4, 128, 64, 512, True)])
+def test_drop_in_calls_take_the_even_form_where_ragged_batches_do_not_lose(kv_heads, head_dim, batch, bound, pays):
+    rule = ks.lib()._ZN5singe22paged_decode_even_paysEmmmm
+    rule.argtypes, rule.restype = [ctypes.c_size_t] * 4, ctypes.c_bool
+    assert rule(batch, kv_heads, head_dim, bound) == pays
+    assert rule(batch, kv_heads, head_dim, bound // 16 * 16 - 15) == rule(batch, kv_heads, head_dim, bound // 16 * 16)
+
+
+def test_positions_of_the_even_form_stay_below_2_31():
+    splits = lambda bound: ks.lib().singe_paged_kv_decode_even_splits(1, 32, 8, 128, bound, 16)
+    assert splits(2 ** 31 - 32) > 0 and splits(2 ** 31 - 16) > 0 and splits(2 ** 31) == 0 and splits(2 ** 34) == 0
