@@ -333,14 +333,16 @@ class ParallelMixer:
         main, side = torch.cuda.current_stream(), self.ops.side_stream()
         filling = self.left.fills_machine(normed.shape[0], step.table.shape[1] * cache[0].shape[1])
         side.wait_stream(main)
-        with torch.cuda.stream(side):
-            recurrence = self.right.prepare(int(side.cuda_stream), step, *right_part)
-            if not filling:
-                recurrence()
-        attention = self.left.prepare(stream, step, *left_part)
-        if filling:
-            main.wait_stream(side)
+        try:
             with torch.cuda.stream(side):
-                recurrence()
-        attention()
-        main.wait_stream(side)
+                recurrence = self.right.prepare(int(side.cuda_stream), step, *right_part)
+                if not filling:
+                    recurrence()
+            attention = self.left.prepare(stream, step, *left_part)
+            if filling:
+                main.wait_stream(side)
+                with torch.cuda.stream(side):
+                    recurrence()
+            attention()
+        finally:
+            main.wait_stream(side)   # also where a call is refused: what the side reads is free for other use behind this

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from singe_b200 import models
-from singe_b200.parallel_mixer import ParallelMixer
+from singe_b200.parallel_mixer import ChunkedAttention, GatedDelta, ParallelMixer
 from tests import vatolorn_util as util
 
 pytestmark = pytest.mark.gpu
@@ -24,14 +24,14 @@ def one_after_the_other(self, stream, step, normed, cache, delta, status, scratc
     self.right.prepare(stream, step, projected[:, self.split:], cache[3:], delta[:, delta.shape[1] - width:], status)()
 
 
-# few sequences, and enough for the decode attention that takes every SM's shared memory
-@pytest.mark.parametrize("sequences,filling", [(2, False), (24, True)])
+# few sequences, and enough for the decode attention that takes every SM's shared memory (with 16-bit activations)
+@pytest.mark.parametrize("sequences,filling,dtype", [(2, False, "bfloat16"), (24, True, "bfloat16"), (24, False, "float32")])
 @pytest.mark.parametrize("captured", [False, True])
-def test_sides_beside_each_other(tmp_path, monkeypatch, sequences, filling, captured):
+def test_sides_beside_each_other(tmp_path, monkeypatch, sequences, filling, dtype, captured):
     directory = util.write_snapshot(tmp_path, CONFIG, util.make_weights(CONFIG, seed=3))
 
     def steps():
-        decoder = models.load_decoder(directory, sequences, 2048, "bfloat16")
+        decoder = models.load_decoder(directory, sequences, 2048, dtype)
         bound = decoder.stride * 16
         assert {layer.mixer.left.fills_machine(sequences, bound) for layer in decoder.layers} == {filling}
         decoder.fill_context(700, seed=5)
@@ -50,3 +50,23 @@ def test_sides_beside_each_other(tmp_path, monkeypatch, sequences, filling, capt
     monkeypatch.setattr(ParallelMixer, "run", one_after_the_other)
     for mine, other in zip(beside, steps()):
         assert all(torch.equal(a, b) for a, b in zip(mine, other))
+
+
+def test_a_side_is_waited_for_when_the_other_one_is_refused(tmp_path, monkeypatch):
+    decoder = models.load_decoder(util.write_snapshot(tmp_path, CONFIG, util.make_weights(CONFIG, seed=3)), 2, 2048, "bfloat16")
+    decoder.fill_context(100, seed=5)
+
+    def busy(self, stream, *_):
+        torch.cuda._sleep(400_000_000)     # a fifth of a second
+        return lambda: None
+
+    def refused(self, stream, *_):
+        raise RuntimeError("refused")
+
+    monkeypatch.setattr(GatedDelta, "prepare", busy)
+    monkeypatch.setattr(ChunkedAttention, "prepare", refused)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="refused"):
+        decoder.step(np.asarray([1, 2]))
+    assert not torch.cuda.current_stream().query()
+    torch.cuda.synchronize()
