@@ -63,6 +63,37 @@ def test_outputs_at_odd_places_take_the_split_grid_with_its_own_pieces():
     assert torch.equal(out, split_grid(case, operands))
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 8, 128), (8, 4, 64)])
+def test_even_decode_lengths_that_no_table_holds(heads, kv_heads, head_dim):
+    # below zero: no keys; beyond the table: all that it holds.  Pages that no sequence holds are not numbers
+    bound = 65536 // head_dim * 8
+    case = workloads.paged_decode_case(seed=14, heads=heads, kv_heads=kv_heads, head_dim=head_dim, lens=[bound, 40, bound, 300], max_len=bound)
+    assert even_splits(case) > 0
+    q, k, v = _inputs(case, seed=15)
+    held = np.unique(np.concatenate([case.block_table[b, : -(-n // 16)] for b, n in enumerate(case.lens)]))
+    spare = np.setdiff1d(np.arange(case.physical_blocks), held)
+    assert len(spare) > 0
+    k[spare], v[spare] = np.nan, np.inf
+    odd = dev(np.asarray([2 ** 31 - 1, -1, bound + 1, -2 ** 31], dtype=np.int32))
+    out = torch.full((4, heads, head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    operands = [dev(x, torch.bfloat16) for x in (q, k, v)]
+    ops.paged_kv_decode_attention(out, *operands, odd, dev_u32(case.block_table), _config(case))
+    case.lens[[1, 3]] = 0
+    assert_close_bf16(host(out), _oracle(case, np.nan_to_num(q), np.nan_to_num(k), np.nan_to_num(v)), "odd lengths")
+    assert not host(out)[[1, 3]].any() and ops.take_device_error() == 0
+
+
+@pytest.mark.parametrize("batch", [2048, 2049])
+def test_most_sequences_of_the_even_form(batch):
+    lens = np.random.default_rng(batch).integers(0, 40, size=batch)
+    case = workloads.paged_decode_case(seed=16, heads=32, kv_heads=4, head_dim=128, lens=lens, max_len=1024)
+    assert (even_splits(case) > 0) == (batch == 2048)
+    q, k, v = _inputs(case, seed=17)
+    out = torch.full((batch, 32, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_kv_decode_attention(out, *[dev(x, torch.bfloat16) for x in (q, k, v)], dev(case.lens), dev_u32(case.block_table), _config(case))
+    assert_close_bf16(host(out), _oracle(case, q, k, v), f"{batch} sequences")
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,dtype", [(32, 8, 128, torch.bfloat16), (16, 4, 64, torch.float16)])
 def test_even_decode_values_that_are_not_finite(heads, kv_heads, head_dim, dtype):
     # seen values of either infinity and NaN, in a sequence of one segment and in one of many; a finite column beside them
@@ -134,8 +165,10 @@ def test_even_decode_step_adds_its_key(heads, kv_heads, head_dim, hinted):
     assert_close_bf16(host(out), _oracle(case, queries, k, v), "decode step")
 
 
-@pytest.mark.parametrize("heads,kv_heads,head_dim,chunk", [(16, 4, 128, 512), (8, 8, 64, 520), (8, 8, 64, 100), (4, 4, 64, 4096)])
-def test_even_chunked_decode(heads, kv_heads, head_dim, chunk):
+# (the rule leaves short chunks to the split grid, and rows too narrow for the list: both forms are held to the same)
+@pytest.mark.parametrize("heads,kv_heads,head_dim,chunk,even", [(16, 4, 128, 512, True), (8, 8, 64, 520, True), (8, 4, 64, 4096, True),
+                                                                (8, 8, 64, 100, False), (4, 4, 64, 4096, False)])
+def test_even_chunked_decode(heads, kv_heads, head_dim, chunk, even):
     # queries in another order than their sequences, one sequence twice, a query without keys; chunks that begin inside a page
     rng = np.random.default_rng(chunk)
     sequence_of, lens = [2, 0, 1, 1, 3, 0] * 40, [700, 1, 512, 513, 0, 37] * 40
@@ -145,8 +178,8 @@ def test_even_chunked_decode(heads, kv_heads, head_dim, chunk):
                                                                 (pool, 16, kv_heads, head_dim)))
     bound = min(chunk + 15, stride * 16)
     splits = ks.lib().singe_paged_kv_decode_even_splits(len(lens), heads, kv_heads, head_dim, bound, 16)
-    if splits == 0:          # (the rule leaves short chunks to the split grid: both forms are held to the same)
-        splits = 2
+    assert (splits > 0) == even
+    splits = splits or 2
     attn = torch.full((len(lens), heads, splits, head_dim), float("nan"), device="cuda")
     lse = torch.full((len(lens), heads, splits), float("nan"), device="cuda")
     out = torch.full((len(lens), heads, head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
