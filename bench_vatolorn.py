@@ -68,7 +68,9 @@ def decode_attention(size: str, sequences: int, visible: int, peaks) -> dict:
     _, heads, kv, dim, *_ = SIZES[size]
     o = hybrid.Ops("bfloat16")
     stride = -(-2 * visible // TILED_PAGE)
-    splits = int(ks.lib().singe_paged_kv_decode_default_splits(sequences, kv, visible + TILED_PAGE - 1, TILED_PAGE))
+    bound = visible + TILED_PAGE - 1      # (as a decoder sizes it)
+    splits = int(ks.lib().singe_paged_kv_decode_even_splits(sequences, heads, kv, dim, bound, TILED_PAGE)
+                 or ks.lib().singe_paged_kv_decode_default_splits(sequences, kv, bound, TILED_PAGE))
     attn, lse = torch.empty((sequences, heads, splits, dim), device="cuda"), torch.empty((sequences, heads, splits), device="cuda")
     order, lens = torch.arange(sequences, dtype=torch.int32, device="cuda"), torch.full((sequences,), 2 * visible, dtype=torch.int32, device="cuda")
     status = torch.zeros(1, dtype=torch.int32, device="cuda")

@@ -12,13 +12,14 @@
 // over 16, 40 and 100 causal keys, in units of the general kernel's error: 1.00, 0.99, 0.95 (64 columns 0.99, 0.98, 0.94); four
 // chains of a quarter of the dimensions each, scaled afterwards: 1.19, 1.17, 1.11.  They took 4 % less time, but 8 % more in the
 // form of four teams, where their registers spilled.  The value products take pairs of columns at a time (sums and order as one by
-// one; with the halving of last tiles below 2 - 18 % less time: 8 heads x 512 causal keys of 64 24.4 us -> 23.6, of 128 44.3 -> 42.0,
-// 8 x 100 of 128 14.1 -> 12.0); reading every weight twice from shared memory instead cost 3 - 9 % more.
+// one; together with what last tiles leave out, see below: 8 heads x 512 causal keys of 64, four teams, 24.4 us -> 23.6; of 128, two teams,
+// 44.3 -> 42.0, 8 x 100 14.1 -> 12.0); reading every weight twice from shared memory instead cost 3 - 9 % more.
 // Thread (ty, tx) owns rows ty, ty + BM/R, ... and keys tx, tx + 16, ...: a row's scores lie in 16 neighbouring lanes, and rows
 // one apart keep the 16-byte reads of a warp on different banks (rows are padded by 16 bytes).
 // Teams of threads walk alternate key tiles, each in buffers of its own, and are folded at the end through shared memory: the
 // chain of key tiles is what a call of few CTAs waits for.
-// A last tile is walked as far as its last visible key: scores by halves of 32 keys, value products by groups of 16.
+// In a last tile the scores stop at a half (32 keys) that holds the last visible key; the value products stop at the next multiple of
+// four keys behind it with one team or two, while four teams walk the whole tile (no register is left for the end).
 // 8 heads x 512 causal keys of 64: 417 us -> 23.6; x 900: 1011 -> 39.8; x 1500 of 128: 3367 -> 170.
 // Keys a row does not see take no part at all, whatever their bits are: in tiles that hold hidden keys the value
 // products are predicated, not multiplied by zero.

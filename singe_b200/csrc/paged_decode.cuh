@@ -205,7 +205,7 @@ __device__ __forceinline__ void add_new_key(const DecodeParams &p, const StepExt
     const float weight = fast_exp2(score - next_max);
     run_max = next_max;
     run_sum = run_sum * correction + (quad == 0 ? weight : 0.0f);   // the quad's sums are added up below
-    // the weight takes the rounding the tensor-core path gives P
+    // the weight takes the rounding the split grid's tensor-core path gives P (the even form's cached keys have two terms)
     T packed_weight = from_float<T>(weight);
     const float rounded_weight = to_float<T>(packed_weight);
 #pragma unroll

@@ -13,7 +13,8 @@
 // Measured, bf16 and f16 (us, by the split grid and here, with the fold): 32 sequences of 128 - 4096 keys, 8 heads of 128 57.1 and
 // 52.5; 64 x 1024 59.5 and 49.3; 4 x 4096 24.7 and 18.0; 32 x 4096 of 64 61.3 and 49.6.  A Llama-shaped decode step of 64 x 2048
 // keys over six layers 1462 and 1384.  Against 64 bits the error is 0.84 of the split grid's (2.0e-3 -> 1.7e-3, the rounding of the
-// output): the weights enter the value product as two terms, in rows of the 16-row tile that carry no query head.
+// output): the weights of cached keys enter the value product as two terms, in rows of the 16-row tile that carry no query head.  The
+// one key that a fused step adds keeps the single rounded weight it has there.
 // Structure: one persistent CTA per SM.  Warp 8 (producer) brings K and V of a step -- eight (page, head) tiles, so one page of
 // eight heads or two of four -- into a ring of 32 KB slots (K and V have slots of their own, so that K's is free while V is
 // read); warp w < 8 owns head w % kv_heads and, with four heads, every other page; one tile a step, ldmatrix from the

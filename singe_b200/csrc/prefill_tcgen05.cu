@@ -375,9 +375,8 @@ struct Item {
 };
 
 // The items of a CTA's first rounds are decoded by its warps side by side before the roles part: item by item, the softmax waited
-// 2600 clk for its look-ups between two items, and another 4100 for the stores of 32 rows' lines, 16 bytes a lane (a key tile's step
-// takes 2950).  With stores of 32 bytes 8192 + 4096 + 2048 + 1024 tokens 726 -> 691 us at the power limit, eight prompts of 209 - 3355
-// 268 -> 250, the tensor surface's mixed step 157 -> 150.
+// for its look-ups between two items, and for the stores of 32 rows' lines, 16 bytes a lane.  With stores of 32 bytes 8192 + 4096 +
+// 2048 + 1024 tokens 726 -> 691 us at the power limit, eight prompts of 209 - 3355 268 -> 250, the tensor surface's mixed step 157 -> 150.
 constexpr int kHeldItems = 64;
 
 __device__ __forceinline__ int pairs_of(int len_q) { return (max(len_q, 0) + kPair - 1) / kPair; }
