@@ -29,9 +29,10 @@ class Ops:
         self._side = None
 
     def side_stream(self):
-        """A stream beside the current one, the same for all layers of a decoder."""
+        """A stream beside the current one and two events to meet it by, the same for all layers of a decoder."""
         if self._side is None:
-            self._side = self.torch.cuda.Stream()
+            cuda = self.torch.cuda
+            self._side = cuda.Stream(), cuda.Event(), cuda.Event()
         return self._side
 
     def call(self, name: str, *arguments) -> None:

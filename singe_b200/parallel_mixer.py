@@ -313,6 +313,12 @@ class ParallelMixer:
     def scratch(self, rows: int, key_bound: int):
         return self.left.scratch(rows, key_bound)
 
+    def beside(self, step: StepRows) -> bool:
+        """Whether the two sides run beside each other: for one token per sequence, where the step is captured.  Called one by one
+        from the host, a step waits for the host, and forking and meeting make that 0.1 - 0.3 ms longer (six layers: 4 sequences of 500
+        1.05 ms one side after the other, 1.19 beside, 64 of 2048 1.07 and 1.20)."""
+        return step.longest <= 1 and self.ops.torch.cuda.is_current_stream_capturing()
+
     def run(self, stream, step: StepRows, normed, cache, delta, status, scratch=None) -> None:
         projected = self.ops.rows(normed.shape[0], self.project.shape[0])
         self.ops.linear(stream, projected, normed, self.project)
@@ -320,29 +326,34 @@ class ParallelMixer:
         right = delta.shape[1] - width
         right_part = projected[:, self.split:], cache[3:], delta[:, right:], status
         left_part = projected[:, :self.split], cache[:3], delta[:, :width], status, scratch
-        if step.longest > 1:
+        if not self.beside(step):
             self.left.prepare(stream, step, *left_part)()
             self.right.prepare(stream, step, *right_part)()
             return
-        # One token per sequence: the sides share nothing but the projections, and the right one runs on a stream of its own beside
-        # the left one's attention.  Where that attention's CTAs take the shared memory of every SM they start behind all that stands
-        # before the recurrence, which would else wait for them (64 sequences of 2048 tokens 853 us a step, 863 without, 932 one
-        # side after the other; 16 of 3000 578, 636 and 635); where they do not, the second meeting is not worth it (4 of 500 480, 438
-        # and 510).  What the right side allocates belongs to its stream; the rest outlives the join.
-        torch = self.ops.torch
-        main, side = torch.cuda.current_stream(), self.ops.side_stream()
+        # The sides share nothing but the projections, and the right one runs on a stream of its own beside the left one's attention.
+        # Where that attention's CTAs take the shared memory of every SM they start behind all that stands before the recurrence,
+        # which would else wait for them (64 sequences of 2048 tokens 853 us a step, 863 without, 932 one side after the other; 16 of
+        # 3000 578, 636 and 635); where they do not, the second meeting is not worth it (4 of 500 480, 438 and 510).  What the right
+        # side needs is allocated on the current stream and held until the two have met again.
+        main = self.ops.torch.cuda.current_stream()
+        side, fork, join = self.ops.side_stream()
+        beside = int(side.cuda_stream)
         filling = self.left.fills_machine(normed.shape[0], step.table.shape[1] * cache[0].shape[1])
-        side.wait_stream(main)
+
+        def meet() -> None:
+            join.record(side)
+            main.wait_event(join)
+
+        fork.record(main)
+        side.wait_event(fork)
         try:
-            with torch.cuda.stream(side):
-                recurrence = self.right.prepare(int(side.cuda_stream), step, *right_part)
-                if not filling:
-                    recurrence()
+            recurrence = self.right.prepare(beside, step, *right_part)
+            if not filling:
+                recurrence()
             attention = self.left.prepare(stream, step, *left_part)
             if filling:
-                main.wait_stream(side)
-                with torch.cuda.stream(side):
-                    recurrence()
+                meet()
+                recurrence()
             attention()
         finally:
-            main.wait_stream(side)   # also where a call is refused: what the side reads is free for other use behind this
+            meet()   # also where a call is refused: what the side reads is free for other use behind this

@@ -29,6 +29,8 @@ def one_after_the_other(self, stream, step, normed, cache, delta, status, scratc
 @pytest.mark.parametrize("captured", [False, True])
 def test_sides_beside_each_other(tmp_path, monkeypatch, sequences, filling, dtype, captured):
     directory = util.write_snapshot(tmp_path, CONFIG, util.make_weights(CONFIG, seed=3))
+    if not captured:        # (left alone, only captured steps fork)
+        monkeypatch.setattr(ParallelMixer, "beside", lambda self, step: step.longest <= 1)
 
     def steps():
         decoder = models.load_decoder(directory, sequences, 2048, dtype)
@@ -57,12 +59,14 @@ def test_a_side_is_waited_for_when_the_other_one_is_refused(tmp_path, monkeypatc
     decoder.fill_context(100, seed=5)
 
     def busy(self, stream, *_):
-        torch.cuda._sleep(400_000_000)     # a fifth of a second
+        with torch.cuda.stream(torch.cuda.ExternalStream(stream)):
+            torch.cuda._sleep(400_000_000)     # a fifth of a second
         return lambda: None
 
     def refused(self, stream, *_):
         raise RuntimeError("refused")
 
+    monkeypatch.setattr(ParallelMixer, "beside", lambda self, step: True)
     monkeypatch.setattr(GatedDelta, "prepare", busy)
     monkeypatch.setattr(ChunkedAttention, "prepare", refused)
     torch.cuda.synchronize()
@@ -70,3 +74,21 @@ def test_a_side_is_waited_for_when_the_other_one_is_refused(tmp_path, monkeypatc
         decoder.step(np.asarray([1, 2]))
     assert not torch.cuda.current_stream().query()
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_only_captured_steps_fork(tmp_path, monkeypatch, captured):
+    decoder = models.load_decoder(util.write_snapshot(tmp_path, CONFIG, util.make_weights(CONFIG, seed=3)), 2, 2048, "bfloat16")
+    decoder.fill_context(100, seed=5)
+    streams = []
+    prepare = GatedDelta.prepare
+    monkeypatch.setattr(GatedDelta, "prepare", lambda self, stream, *rest: (streams.append(stream), prepare(self, stream, *rest))[1])
+    if captured:
+        decoder.capture()       # a warm-up ahead of the capture, then the capture
+    else:
+        decoder.step(np.asarray([1, 2]))
+    torch.cuda.synchronize()
+    layers = len(decoder.layers)
+    own = {int(layer.mixer.ops._side[0].cuda_stream) for layer in decoder.layers if layer.mixer.ops._side}
+    assert len(streams) == (2 * layers if captured else layers) and len(own) == (1 if captured else 0)
+    assert [stream in own for stream in streams] == [False] * layers + [True] * layers * captured
