@@ -374,7 +374,8 @@ struct Item {
     bool valid;     // false: the sequence's offsets leave the packed tensors
 };
 
-// The items of a CTA's first rounds are decoded by its warps side by side before the roles part: item by item, the softmax waited
+// The items of a CTA's first rounds are decoded by its warps side by side before the roles part (not where a CTA has one item only: held
+// ahead it cost 0.5 - 1 us, 3 prompts of 13 - 53 tokens 12.4 -> 13.3 us, 2 of 100 - 300 16.3 -> 17.1): item by item, the softmax waited
 // for its look-ups between two items, and for the stores of 32 rows' lines, 16 bytes a lane.  With stores of 32 bytes 8192 + 4096 +
 // 2048 + 1024 tokens 726 -> 691 us at the power limit, eight prompts of 209 - 3355 268 -> 250, the tensor surface's mixed step 157 -> 150.
 constexpr int kHeldItems = 64;
@@ -550,7 +551,8 @@ __device__ __forceinline__ int order_items(const PrefillParams &p, const Sequenc
 // 128-key tile and 64-wide half; the boxes land back to back, which is the layout one 128-row box would have).
 // HD = 128 or 64: with 64 a tile is a single 128-byte-wide box (the second half of every 32 KB buffer stays unused).
 // DENSE: uniform lengths, sequences back to back, LSE laid out [batch, heads, queries] (fmha_prefill_lse).
-template <typename T, int HD, bool SAFE, bool PAGED, bool DENSE, bool WINDOW, bool TENSOR>
+// LONE: no CTA has a second item, and none is held: see kHeldItems.
+template <typename T, int HD, bool SAFE, bool PAGED, bool DENSE, bool WINDOW, bool TENSOR, bool LONE = false>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
     prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                            const __grid_constant__ CUtensorMap v_map, const PrefillParams p,
@@ -684,13 +686,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         return share_index(round);
     };
 
-    for (int round = warp; round < kHeldItems; round += kPrefillThreads / 32) {
+    for (int round = warp; !LONE && round < kHeldItems; round += kPrefillThreads / 32) {
         const int index = item_index(round);
         if (index < 0) break;
         const Item item = decode(index);
         if (lane == 0) held[round] = item;
     }
-    auto item_at = [&](int round, int index) -> Item { return round < kHeldItems ? held[round] : decode(index); };
+    auto item_at = [&](int round, int index) -> Item { return !LONE && round < kHeldItems ? held[round] : decode(index); };
     if (tid == 0) {
         for (int i = 0; i < kBarriers; ++i) {
             const bool by_warps = i >= 16;  // p_full, o_empty, share
@@ -1262,23 +1264,32 @@ bool prefill_fast_path(size_t heads, size_t kv_heads, size_t head_dim, size_t to
 
 namespace {
 
-template <typename T, int HD, bool PAGED, bool DENSE = false, bool WINDOW = false>
-int launch_prefill(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
-                   const PrefillParams &params, unsigned persistent) {
-    SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillBytes));
-    if (std::is_same<T, __nv_bfloat16>::value) {
-        SINGE_CUDA_TRY(cudaFuncSetAttribute(prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillBytes));
-        prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false>
-            <<<persistent, kPrefillThreads, kPrefillBytes, stream>>>(q_map, k_map, v_map, params, NoPaging{});
+template <typename T, int HD, bool PAGED, bool DENSE, bool WINDOW, bool LONE>
+int launch_passes(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
+                  const PrefillParams &params, unsigned persistent) {
+    constexpr bool kTwo = std::is_same<T, __nv_bfloat16>::value;
+    const auto exact = prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false, LONE && !kTwo>;
+    SINGE_CUDA_TRY(cudaFuncSetAttribute(exact, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillBytes));
+    if (kTwo) {
+        const auto first = prefill_tcgen05_kernel<__nv_bfloat16, HD, false, PAGED, DENSE, WINDOW, false, LONE>;
+        SINGE_CUDA_TRY(cudaFuncSetAttribute(first, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillBytes));
+        first<<<persistent, kPrefillThreads, kPrefillBytes, stream>>>(q_map, k_map, v_map, params, NoPaging{});
         SINGE_TRY(launch_status());
     }
     // bf16: the redo pass over the same shares, a no-op while the device's out-of-range flag has never been raised.
     // f16 (params.exact): the only pass.  P must stay below 65504 there, so every tile takes its exact row maximum.
-    prefill_tcgen05_kernel<T, HD, true, PAGED, DENSE, WINDOW, false>
-        <<<persistent, kPrefillThreads, kPrefillBytes, stream>>>(q_map, k_map, v_map, params, NoPaging{});
+    exact<<<persistent, kPrefillThreads, kPrefillBytes, stream>>>(q_map, k_map, v_map, params, NoPaging{});
     return launch_status();
+}
+
+// One CTA for each of at most `items` items, or one for each of the `sms` SMs.
+template <typename T, int HD, bool PAGED, bool DENSE = false, bool WINDOW = false>
+int launch_prefill(cudaStream_t stream, const CUtensorMap &q_map, const CUtensorMap &k_map, const CUtensorMap &v_map,
+                   const PrefillParams &params, size_t items, size_t sms) {
+    if (items <= sms) {
+        return launch_passes<T, HD, PAGED, DENSE, WINDOW, true>(stream, q_map, k_map, v_map, params, static_cast<unsigned>(items));
+    }
+    return launch_passes<T, HD, PAGED, DENSE, WINDOW, false>(stream, q_map, k_map, v_map, params, static_cast<unsigned>(sms));
 }
 
 template <int HD, bool WINDOW>
@@ -1370,31 +1381,30 @@ int prefill_tcgen05(cudaStream_t stream, bool is_f16, void *out, float *lse, con
     const size_t items = (total_query_tokens / kPair + batch) * heads;
     if (items > 0x7fffffffull) return SINGE_ERR_LENGTH_EXCEEDS_I32;
     if (items == 0) return SINGE_OK;
-    const unsigned persistent = static_cast<unsigned>(items < static_cast<size_t>(sms) ? items : sms);
     if (lens_q == nullptr) {
         // the dense form: ragged keys only
         if (paged) return SINGE_ERR_UNSUPPORTED_CONFIGURATION;
         if (head_dim == 64) {
-            return is_f16 ? launch_prefill<__half, 64, false, true>(stream, q_map, k_map, v_map, params, persistent)
-                          : launch_prefill<__nv_bfloat16, 64, false, true>(stream, q_map, k_map, v_map, params, persistent);
+            return is_f16 ? launch_prefill<__half, 64, false, true>(stream, q_map, k_map, v_map, params, items, sms)
+                          : launch_prefill<__nv_bfloat16, 64, false, true>(stream, q_map, k_map, v_map, params, items, sms);
         }
-        return is_f16 ? launch_prefill<__half, 128, false, true>(stream, q_map, k_map, v_map, params, persistent)
-                      : launch_prefill<__nv_bfloat16, 128, false, true>(stream, q_map, k_map, v_map, params, persistent);
+        return is_f16 ? launch_prefill<__half, 128, false, true>(stream, q_map, k_map, v_map, params, items, sms)
+                      : launch_prefill<__nv_bfloat16, 128, false, true>(stream, q_map, k_map, v_map, params, items, sms);
     }
     if (head_dim == 64) {
         if (is_f16) {
-            return paged ? launch_prefill<__half, 64, true>(stream, q_map, k_map, v_map, params, persistent)
-                         : launch_prefill<__half, 64, false>(stream, q_map, k_map, v_map, params, persistent);
+            return paged ? launch_prefill<__half, 64, true>(stream, q_map, k_map, v_map, params, items, sms)
+                         : launch_prefill<__half, 64, false>(stream, q_map, k_map, v_map, params, items, sms);
         }
-        return paged ? launch_prefill<__nv_bfloat16, 64, true>(stream, q_map, k_map, v_map, params, persistent)
-                     : launch_prefill<__nv_bfloat16, 64, false>(stream, q_map, k_map, v_map, params, persistent);
+        return paged ? launch_prefill<__nv_bfloat16, 64, true>(stream, q_map, k_map, v_map, params, items, sms)
+                     : launch_prefill<__nv_bfloat16, 64, false>(stream, q_map, k_map, v_map, params, items, sms);
     }
     if (is_f16) {
-        return paged ? launch_prefill<__half, 128, true>(stream, q_map, k_map, v_map, params, persistent)
-                     : launch_prefill<__half, 128, false>(stream, q_map, k_map, v_map, params, persistent);
+        return paged ? launch_prefill<__half, 128, true>(stream, q_map, k_map, v_map, params, items, sms)
+                     : launch_prefill<__half, 128, false>(stream, q_map, k_map, v_map, params, items, sms);
     }
-    return paged ? launch_prefill<__nv_bfloat16, 128, true>(stream, q_map, k_map, v_map, params, persistent)
-                 : launch_prefill<__nv_bfloat16, 128, false>(stream, q_map, k_map, v_map, params, persistent);
+    return paged ? launch_prefill<__nv_bfloat16, 128, true>(stream, q_map, k_map, v_map, params, items, sms)
+                 : launch_prefill<__nv_bfloat16, 128, false>(stream, q_map, k_map, v_map, params, items, sms);
 }
 
 // The windowed form: keys and values are rows of kv_row_stride elements (heads side by side) with offsets of their own;
@@ -1439,11 +1449,10 @@ int prefill_tcgen05_windowed(cudaStream_t stream, void *out, float *lse, const v
     const size_t items = (total_query_tokens / kPair + batch) * heads;
     if (items > 0x7fffffffull) return SINGE_ERR_LENGTH_EXCEEDS_I32;
     const size_t sms = static_cast<size_t>(device_sm_count());
-    const unsigned persistent = static_cast<unsigned>(items < sms ? items : sms);
     if (head_dim == 64) {
-        return launch_prefill<__nv_bfloat16, 64, false, false, true>(stream, q_map, k_map, v_map, params, persistent);
+        return launch_prefill<__nv_bfloat16, 64, false, false, true>(stream, q_map, k_map, v_map, params, items, sms);
     }
-    return launch_prefill<__nv_bfloat16, 128, false, false, true>(stream, q_map, k_map, v_map, params, persistent);
+    return launch_prefill<__nv_bfloat16, 128, false, false, true>(stream, q_map, k_map, v_map, params, items, sms);
 }
 
 // Whether tensor_prefill serves a call of the Tensor surface's paged attention (bf16, no score cap).
