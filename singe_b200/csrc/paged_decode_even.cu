@@ -644,20 +644,24 @@ size_t paged_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, siz
 }
 
 // Whether a drop-in call takes the even form.  Its caller knows nothing of the lengths but the bound, so the line lies where ragged
-// batches (lengths spread from 1/4 or 1/32 of the bound up to it) stop losing, on some 600 shapes.  With at most 32 rows what the
-// split grid has to split decides, as above.  With more, ragged lengths leave that grid a single wave, which is hard to beat below
-// 40 MB of keys and values at the bound (8 heads of 128), 112 MB (heads of 64), 160 MB (4 of 128), or 48 MB where there are rows
-// enough to fill the wave without splits (us, split grid and here, lengths from a quarter of the bound, then all at it: heads of 64, 20 x
-// 1024 11.5 and 12.7, 17.2 and 14.6; 24 x 2128 on 4 12.8 and 14.2, 20.2 and 16.6; 20 x 3584 27.1 and 22.4, 32.7 and 30.8; 4 heads of
-// 128, 20 x 1632 14.1 and 14.9, 22.2 and 19.3).  Of the calls it takes none from half of the bound on loses, of 1422 ragged ones 13 by 2 - 8 %.
-// Lengths far below the bound may lose: all at a sixteenth of it, heads of 64, 32 x 140 7.8 and 9.5, 64 x 280 17.2 and 14.7.
+// batches (lengths spread from 1/4 or 1/32 of the bound up to it) lose as a whole, measured on some 600 shapes whose keys and values
+// come from HBM (us, split grid and here, lengths from a quarter of the bound, then all at it):
+//   * heads of 64 on 49 - 175 rows below 80 MB of keys and values at the bound, where ragged lengths leave the split grid a single
+//     wave: 20 x 1024 11.5 and 12.7, 17.2 and 14.6; 24 x 2128 on 4 12.8 and 14.2, 20.2 and 16.6;
+//   * 4 heads of 128 on more than 16 rows below 32 MB and on more than 32 below 40: 20 x 640 12.2 and 12.7, 13.9 and 13.5;
+//   * what the split grid need not split of 8 heads of 128 below 40 MB: 64 x 128 11.9 and 12.3, 14.3 and 13.8.
+// Of the calls it takes none with lengths from half of the bound on is slower, of 1101 from a quarter on 51 by 2 - 10 %, of 1004 from
+// 1/32 on 130, 16 of them by more than 10 %; on all but 3 of 373 shapes, by 2 % at most, all three together gain.  Lengths far below the
+// bound may lose: all at a sixteenth of it, heads of 64, 32 x 140 7.8 and 9.5, 64 x 280 17.2 and 14.7.
 bool paged_decode_even_pays(size_t batch, size_t kv_heads, size_t head_dim, size_t bound) {
     const size_t rows = batch * kv_heads, stride = (bound + kPageTokens - 1) / kPageTokens;
     size_t least = 32;
-    if (kv_heads * head_dim == 1024) {
-        least = rows <= 32 ? 24 : 40;
-    } else if (rows > 32) {
-        least = head_dim == 128 ? (rows < 192 ? 160 : 48) : (rows < 384 ? 112 : 48);
+    if (head_dim == 64) {
+        if (rows > 48 && rows < 176) least = 80;
+    } else if (kv_heads == 8) {
+        least = bound > 128 && rows <= 3 * static_cast<size_t>(device_sm_count()) ? 24 : 40;
+    } else {
+        least = rows <= 16 ? 24 : rows <= 32 ? 32 : 40;
     }
     return batch * stride * kPageTokens * kv_heads * head_dim * 4 >= least << 20;
 }
