@@ -644,22 +644,26 @@ size_t paged_decode_even_splits(size_t batch, size_t heads, size_t kv_heads, siz
 }
 
 // Whether a drop-in call takes the even form.  Its caller knows nothing of the lengths but the bound, so the line lies where ragged
-// batches (lengths spread from 1/4 or 1/32 of the bound up to it) lose as a whole, measured on some 600 shapes whose keys and values
+// batches (lengths spread from 1/4 or 1/32 of the bound up to it) lose as a whole, measured on 750 shapes whose keys and values
 // come from HBM (us, split grid and here, lengths from a quarter of the bound, then all at it):
-//   * heads of 64 on 49 - 175 rows below 80 MB of keys and values at the bound, where ragged lengths leave the split grid a single
+//   * heads of 64 on 49 - 175 rows below 96 MB of keys and values at the bound, where ragged lengths leave the split grid a single
 //     wave: 20 x 1024 11.5 and 12.7, 17.2 and 14.6; 24 x 2128 on 4 12.8 and 14.2, 20.2 and 16.6;
 //   * 4 heads of 128 on more than 16 rows below 32 MB and on more than 32 below 40: 20 x 640 12.2 and 12.7, 13.9 and 13.5;
-//   * what the split grid need not split of 8 heads of 128 below 40 MB: 64 x 128 11.9 and 12.3, 14.3 and 13.8.
-// Of the calls it takes none with lengths from half of the bound on is slower, of 1101 from a quarter on 51 by 2 - 10 %, of 1004 from
-// 1/32 on 130, 16 of them by more than 10 %; on all but 3 of 373 shapes, by 2 % at most, all three together gain.  Lengths far below the
+//   * what the split grid need not split of 8 heads of 128 below 40 MB: 64 x 128 11.9 and 12.3, 14.3 and 13.8;
+//   * four rows an SM or more up to 512 keys, where a row of the split grid is one piece and needs no fold (8 heads of 128 up to 256):
+//     81 x 320 of 64 1.1 - 1.2 times and 0.99, 166 x 400 of 128 on 4 1.04 - 1.07 and 1.06, 81 x 400 on 8 0.96 and 0.98.
+// Of the calls it takes none with lengths from half of the bound on is slower, of 1221 from a quarter on 37 by 2 - 9 %, of 1130 from
+// 1/32 on 114, 15 of them by more than 10 %; on all but 3 of 432 shapes, by 2 % at most, all three together gain.  Lengths far below the
 // bound may lose: all at a sixteenth of it, heads of 64, 32 x 140 7.8 and 9.5, 64 x 280 17.2 and 14.7.
 bool paged_decode_even_pays(size_t batch, size_t kv_heads, size_t head_dim, size_t bound) {
-    const size_t rows = batch * kv_heads, stride = (bound + kPageTokens - 1) / kPageTokens;
+    const size_t rows = batch * kv_heads, stride = (bound + kPageTokens - 1) / kPageTokens, sms = static_cast<size_t>(device_sm_count());
+    const bool wide = kv_heads * head_dim == 1024;   // 8 heads of 128
+    if (rows >= 4 * sms && bound <= (wide ? 256 : 512)) return false;
     size_t least = 32;
-    if (head_dim == 64) {
-        if (rows > 48 && rows < 176) least = 80;
-    } else if (kv_heads == 8) {
-        least = bound > 128 && rows <= 3 * static_cast<size_t>(device_sm_count()) ? 24 : 40;
+    if (wide) {
+        least = bound > 128 && rows <= 3 * sms ? 24 : 40;
+    } else if (head_dim == 64) {
+        if (rows > 48 && rows < 176) least = 96;
     } else {
         least = rows <= 16 ? 24 : rows <= 32 ? 32 : 40;
     }
